@@ -11,9 +11,9 @@
 // Rows that are a multiple of 16 bytes (<= 8192 channels, aligned pointers) take the vector kernels below; the rest
 // the scalar ones at the end.  The op is bound by HBM traffic (x once in, y once out; the backward x and dy in, dx
 // out), so a row is read ONCE with 16-byte loads and held in registers between the reductions and the write: by one
-// warp (rows of up to 32 x 16 B x 8) or by one 256-thread CTA (longer rows).  The variance is taken about the mean
+// warp (rows of up to 32 x 16 B x 8) or by one 256-thread CTA (longer rows); the backward see there.  The variance is taken about the mean
 // (two passes over the registers, as the reference's `var` does), not as E[x^2] - mean^2.  dw / db: every CTA walks
-// rows in a grid-stride loop, keeps its column sums in shared memory, leaves one partial row per CTA in a
+// rows in a grid-stride loop, keeps its column sums in registers, leaves one partial row per CTA in a
 // workspace, and a second kernel adds the partials in a fixed order -- deterministic, no atomics.
 #include <math.h>
 
@@ -84,13 +84,6 @@ __device__ __forceinline__ float2 row_sum2(float a, float b, float* red) {
   return make_float2(a, b);
 }
 
-template <typename T, int kVec>
-__device__ __forceinline__ void load_vec(const T* p, float (&out)[kVec]) {
-  const uint4 w = *reinterpret_cast<const uint4*>(p);
-  const T* e = reinterpret_cast<const T*>(&w);
-#pragma unroll
-  for (int i = 0; i < kVec; ++i) out[i] = to_f32<T>(e[i]);
-}
 // The same as pairs: the arithmetic below runs on the packed fp32x2 pipe (one instruction per two elements; each
 // lane rounds as the scalar instruction would, so results do not change).  At 16-bit widths the kernels are bound
 // by instruction issue as much as by memory.
@@ -137,14 +130,6 @@ __device__ __forceinline__ void store_pairs(T* p, const float2 (&v)[kVec / 2]) {
   } else {
     w = make_uint4(pack_pair<T>(v[0]), pack_pair<T>(v[1]), pack_pair<T>(v[2]), pack_pair<T>(v[3]));
   }
-  *reinterpret_cast<uint4*>(p) = w;
-}
-template <typename T, int kVec>
-__device__ __forceinline__ void store_vec(T* p, const float (&v)[kVec]) {
-  uint4 w;
-  T* e = reinterpret_cast<T*>(&w);
-#pragma unroll
-  for (int i = 0; i < kVec; ++i) e[i] = from_f32<T>(v[i]);
   *reinterpret_cast<uint4*>(p) = w;
 }
 
@@ -211,117 +196,209 @@ __global__ void __launch_bounds__(kThreads, kPer <= 4 ? 4 : 2) ln_fwd_kernel(LnA
   }
 }
 
-// Backward.  Grid-stride over rows (a warp's or a CTA's).  The column sums of dw, db live in shared memory, every
-// thread adding only to its own columns (in registers they cost 2 x kPer x kVec registers and left one CTA per SM).
-template <typename T, int kPer, bool kCta>
-__global__ void __launch_bounds__(kThreads) ln_bwd_kernel(LnArgs a) {
+// Backward.  A CTA is 512 threads = kRowThreads / tpr groups of tpr threads (tpr a power of two); a group takes one row
+// at a time, a thread up to kPer 16-byte chunks of it -- always the same columns, so its part of the column sums dw, db
+// stays in 2 kPer kVec registers from the first row to the last (16 columns a thread at most).  Every thread copies
+// its own chunks of x and dy into its own slots of a shared-memory ring with 16-byte cp.async, several rows ahead: no
+// barrier is needed for the data, and 64 to 128 KB per SM are in flight -- HBM needs about 44 KB per SM at its latency.
+// kBatch rows share one barrier (the row sums of groups wider than a warp); their x and dy are read from the ring a
+// second time behind it, which costs less than the registers that would hold them.
+// bf16 (8192, 8192): 142 -> 81 us (4.9 TB/s of x, dy, dx) against the column sums in shared memory without copies ahead;
+// 85 us with one row per barrier.
+constexpr int kRowThreads = 512;
+__device__ __forceinline__ void copy_async16(void* dst, const void* src, bool in) {
+  const uint32_t d = uint32_t(__cvta_generic_to_shared(dst));
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(in ? 16 : 0) : "memory");
+}
+template <typename T>
+__device__ __forceinline__ void word_pairs(const uint4 w, float2 (&out)[16 / int(sizeof(T)) / 2]) {
+  if constexpr (sizeof(T) == 4) {
+    out[0] = make_float2(__uint_as_float(w.x), __uint_as_float(w.y));
+    out[1] = make_float2(__uint_as_float(w.z), __uint_as_float(w.w));
+  } else {
+    out[0] = unpack_pair<T>(w.x);
+    out[1] = unpack_pair<T>(w.y);
+    out[2] = unpack_pair<T>(w.z);
+    out[3] = unpack_pair<T>(w.w);
+  }
+}
+
+template <int kPer>
+struct BwdRing {
+  static constexpr int kBatch = kPer == 4 ? 1 : 2;             // rows between two barriers
+  static constexpr int kAhead = 2;                             // batches in flight
+  static constexpr int kStages = kBatch * (kAhead + 1);
+  static constexpr size_t kBytes = size_t(kStages) * 2 * kPer * kRowThreads * 16;
+};
+
+template <typename T, int kPer>
+__global__ void __launch_bounds__(kRowThreads, kPer == 1 ? 2 : 1) ln_bwd_kernel(LnArgs a, int tpr) {
   constexpr int kVec = 16 / int(sizeof(T));
-  constexpr int kTpr = kCta ? kThreads : 32;
-  constexpr int kRowsPerCta = kCta ? 1 : kThreads / 32;
-  // [2][kRowsPerCta][kPad]: dw sums, then db sums, per row owner.  Column c of an owner sits at slot(c): the two
-  // 16-byte halves of a 16-bit thread's chunk go to separate planes, so that the threads of a quarter-warp touch
-  // consecutive 16-byte words (bank-conflict free) when they update their sums.
-  extern __shared__ __align__(16) float wsum[];
-  constexpr int kPad = kPer * kTpr * kVec;
-  auto slot4 = [](int p, int i4, int tin_) { return ((p * (kVec / 4) + i4) * kTpr + tin_) * 4; };
-  __shared__ float red[4 * (kThreads / 32)];   // two uses of 16 floats, alternating by row
-  const int tin = kCta ? threadIdx.x : (threadIdx.x & 31);
-  const int sub = kCta ? 0 : (threadIdx.x >> 5);
-  int flip = 0;
-  const T* w = reinterpret_cast<const T*>(a.w);
-  float* sw = wsum + sub * kPad;
-  float* sb = wsum + (kRowsPerCta + sub) * kPad;
-  const bool sums = a.part != nullptr;
-  if (sums) {
+  constexpr int kPairs = kVec / 2;
+  constexpr int kBatch = BwdRing<kPer>::kBatch, kAhead = BwdRing<kPer>::kAhead;
+  constexpr int kWarps = kRowThreads / 32;
+  extern __shared__ __align__(16) uint4 ring[];               // [kStages][x, dy][kPer][kRowThreads]
+  __shared__ __align__(16) float2 red[2][kBatch][kWarps];     // the warps' row sums, alternating by batch
+  const int tid = threadIdx.x, tin = tid & (tpr - 1), group = tid / tpr, groups = kRowThreads / tpr;
+  const int64_t blocks = (a.rows + groups - 1) / groups;      // of `groups` consecutive rows
+  const T* x = reinterpret_cast<const T*>(a.x);
+  const T* g = reinterpret_cast<const T*>(a.dy);
+  auto chunk = [&](int p) { return (p * tpr + tin) * kVec; };  // first column of this thread's chunk p
+  const int64_t step = gridDim.x;
+  auto slot = [&](int stage, int which, int p) -> uint4* { return ring + ((stage * 2 + which) * kPer + p) * kRowThreads + tid; };
+  // batch `it` of this CTA (blocks blockIdx.x + (it kBatch + r) step) into its part of the ring
+  auto fetch = [&](int64_t it, int part) {
 #pragma unroll
-    for (int p = 0; p < kPer; ++p) {
-      const int c0 = (p * kTpr + tin) * kVec;
-      if (c0 < a.C) {
+    for (int r = 0; r < kBatch; ++r) {
+      const int64_t blk = blockIdx.x + (it * kBatch + r) * step, row = blk * groups + group;
+      const bool in = blk < blocks && row < a.rows;
 #pragma unroll
-        for (int i = 0; i < kVec; i += 4) {
-          *reinterpret_cast<float4*>(sw + slot4(p, i / 4, tin)) = make_float4(0.f, 0.f, 0.f, 0.f);
-          *reinterpret_cast<float4*>(sb + slot4(p, i / 4, tin)) = make_float4(0.f, 0.f, 0.f, 0.f);
+      for (int p = 0; p < kPer; ++p) {
+        const bool have = in && chunk(p) < a.C;
+        const int64_t at = have ? row * a.C + chunk(p) : 0;
+        copy_async16(slot(part * kBatch + r, 0, p), x + at, have);
+        copy_async16(slot(part * kBatch + r, 1, p), g + at, have);
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  float2 w[kPer][kPairs], sw[kPer][kPairs], sb[kPer][kPairs];
+#pragma unroll
+  for (int p = 0; p < kPer; ++p) {
+#pragma unroll
+    for (int i = 0; i < kPairs; ++i) {
+      w[p][i] = make_float2(1.f, 1.f);
+      sw[p][i] = sb[p][i] = make_float2(0.f, 0.f);
+    }
+    if (a.w && chunk(p) < a.C) load_pairs<T, kVec>(reinterpret_cast<const T*>(a.w) + chunk(p), w[p]);
+  }
+#pragma unroll
+  for (int i = 0; i < kAhead; ++i) fetch(i, i);
+  float nmean[kBatch], nrstd[kBatch];                          // of the batch after this one
+  auto fetch_stats = [&](int64_t it) {
+#pragma unroll
+    for (int r = 0; r < kBatch; ++r) {
+      const int64_t blk = blockIdx.x + (it * kBatch + r) * step, row = blk * groups + group;
+      const bool in = blk < blocks && row < a.rows;
+      nmean[r] = in ? a.mean[row] : 0.f;
+      nrstd[r] = in ? a.rstd[row] : 0.f;
+    }
+  };
+  fetch_stats(0);
+  int part = 0, flip = 0;
+  const float2 os2 = make_float2(a.out_scale, a.out_scale);
+  // (every thread of the CTA runs the same number of iterations: the barriers match; rows past the last are zeros)
+  for (int64_t it = 0; blockIdx.x + it * kBatch * step < blocks; ++it) {
+    fetch(it + kAhead, part == 0 ? kAhead : part - 1);         // (the slots of the last batch: this thread has read them)
+    float2 mean2[kBatch], rstd2[kBatch];
+#pragma unroll
+    for (int r = 0; r < kBatch; ++r) {
+      mean2[r] = make_float2(-nmean[r], -nmean[r]);
+      rstd2[r] = make_float2(nrstd[r], nrstd[r]);
+    }
+    fetch_stats(it + 1);
+    asm volatile("cp.async.wait_group %0;" ::"n"(kAhead) : "memory");
+    float t1[kBatch], t2[kBatch];
+#pragma unroll
+    for (int r = 0; r < kBatch; ++r) {
+      float2 s1 = make_float2(0.f, 0.f), s2 = make_float2(0.f, 0.f);
+#pragma unroll
+      for (int p = 0; p < kPer; ++p) {
+        float2 xh[kPairs], d[kPairs];
+        word_pairs<T>(*slot(part * kBatch + r, 0, p), xh);
+        word_pairs<T>(*slot(part * kBatch + r, 1, p), d);
+        if (chunk(p) < a.C) {
+#pragma unroll
+          for (int i = 0; i < kPairs; ++i) {
+            xh[i] = __fmul2_rn(__fadd2_rn(xh[i], mean2[r]), rstd2[r]);
+            const float2 gy = __fmul2_rn(os2, d[i]);
+            sw[p][i] = __ffma2_rn(gy, xh[i], sw[p][i]);
+            sb[p][i] = __fadd2_rn(sb[p][i], gy);
+            const float2 dh = __fmul2_rn(gy, w[p][i]);
+            s1 = __fadd2_rn(s1, dh);
+            s2 = __ffma2_rn(dh, xh[i], s2);
+          }
+        }
+      }
+      t1[r] = s1.x + s1.y;
+      t2[r] = s2.x + s2.y;
+    }
+    for (int o = min(tpr, 32) >> 1; o > 0; o >>= 1) {
+#pragma unroll
+      for (int r = 0; r < kBatch; ++r) {
+        t1[r] += __shfl_xor_sync(0xffffffffu, t1[r], o);
+        t2[r] += __shfl_xor_sync(0xffffffffu, t2[r], o);
+      }
+    }
+    if (tpr > 32) {
+      // (the buffer is rewritten two batches on, after the next batch's barrier has shown that everyone has read it)
+      if ((tid & 31) == 0) {
+#pragma unroll
+        for (int r = 0; r < kBatch; ++r) red[flip][r][tid >> 5] = make_float2(t1[r], t2[r]);
+      }
+      __syncthreads();
+#pragma unroll
+      for (int r = 0; r < kBatch; ++r) {
+        t1[r] = t2[r] = 0.f;
+        const float4* q = reinterpret_cast<const float4*>(&red[flip][r][group * (tpr >> 5)]);
+        for (int k = 0; k < (tpr >> 6); ++k) {
+          const float4 v = q[k];
+          t1[r] += v.x + v.z;
+          t2[r] += v.y + v.w;
+        }
+      }
+      flip ^= 1;
+    }
+#pragma unroll
+    for (int r = 0; r < kBatch; ++r) {
+      const int64_t row = (blockIdx.x + (it * kBatch + r) * step) * groups + group;
+      if (row >= a.rows) continue;                             // (a block past the last starts past the last row)
+      const float c1 = t1[r] / float(a.C), c2 = t2[r] / float(a.C);
+      T* dx = reinterpret_cast<T*>(a.dx) + row * a.C;
+      const float2 nc1 = make_float2(-c1, -c1), nc2 = make_float2(-c2, -c2);
+#pragma unroll
+      for (int p = 0; p < kPer; ++p) {
+        if (chunk(p) < a.C) {
+          float2 xh[kPairs], d[kPairs], out[kPairs];
+          word_pairs<T>(*slot(part * kBatch + r, 0, p), xh);
+          word_pairs<T>(*slot(part * kBatch + r, 1, p), d);
+#pragma unroll
+          for (int i = 0; i < kPairs; ++i) {
+            xh[i] = __fmul2_rn(__fadd2_rn(xh[i], mean2[r]), rstd2[r]);
+            const float2 dh = __fmul2_rn(__fmul2_rn(os2, d[i]), w[p][i]);
+            out[i] = __fmul2_rn(rstd2[r], __ffma2_rn(xh[i], nc2, __fadd2_rn(dh, nc1)));
+          }
+          store_pairs<T, kVec>(dx + chunk(p), out);
         }
       }
     }
+    part = part == kAhead ? 0 : part + 1;
   }
-  // (in a CTA-per-row kernel every thread of the CTA runs the same number of iterations: the barriers in row_sum match)
-  for (int64_t row = int64_t(blockIdx.x) * kRowsPerCta + sub; row < a.rows; row += int64_t(gridDim.x) * kRowsPerCta) {
-    const T* x = reinterpret_cast<const T*>(a.x) + row * a.C;
-    const T* g = reinterpret_cast<const T*>(a.dy) + row * a.C;
-    const float mean = a.mean[row], rstd = a.rstd[row];
-    float xh[kPer][kVec], dxh[kPer][kVec];
-    float s1 = 0.f, s2 = 0.f;
+  if (!a.part) return;
+  // this CTA's partial row: the groups' sums added in group order, through the ring's memory
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  __syncthreads();
+  float* all = reinterpret_cast<float*>(ring);                 // [dw, db][groups][C]
+  float* mine_w = all + int64_t(group) * a.C;
+  float* mine_b = all + int64_t(groups + group) * a.C;
 #pragma unroll
-    for (int p = 0; p < kPer; ++p) {
-      const int c0 = (p * kTpr + tin) * kVec;
-      if (c0 < a.C) {
-        load_vec<T, kVec>(x + c0, xh[p]);
-        load_vec<T, kVec>(g + c0, dxh[p]);
-      }
-    }
+  for (int p = 0; p < kPer; ++p) {
+    if (chunk(p) < a.C) {
 #pragma unroll
-    for (int p = 0; p < kPer; ++p) {
-      const int c0 = (p * kTpr + tin) * kVec;
-      if (c0 < a.C) {
-        float wv[kVec];
-        if (w) load_vec<T, kVec>(w + c0, wv);   // (a few KB that stay in L1)
-#pragma unroll
-        for (int i = 0; i < kVec; i += 4) {
-          float4 aw, ab;
-          if (sums) {
-            aw = *reinterpret_cast<const float4*>(sw + slot4(p, i / 4, tin));
-            ab = *reinterpret_cast<const float4*>(sb + slot4(p, i / 4, tin));
-          }
-          float* pw = reinterpret_cast<float*>(&aw);
-          float* pb = reinterpret_cast<float*>(&ab);
-#pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            const float xhv = (xh[p][i + u] - mean) * rstd;
-            const float gy = a.out_scale * dxh[p][i + u];
-            pw[u] = fmaf(gy, xhv, pw[u]);
-            pb[u] += gy;
-            const float d = w ? gy * wv[i + u] : gy;
-            xh[p][i + u] = xhv;
-            dxh[p][i + u] = d;
-            s1 += d;
-            s2 = fmaf(d, xhv, s2);
-          }
-          if (sums) {
-            *reinterpret_cast<float4*>(sw + slot4(p, i / 4, tin)) = aw;
-            *reinterpret_cast<float4*>(sb + slot4(p, i / 4, tin)) = ab;
-          }
-        }
-      }
-    }
-    const float2 cs = row_sum2<kCta>(s1, s2, red + 16 * flip);
-    flip ^= 1;
-    const float c1 = cs.x / float(a.C), c2 = cs.y / float(a.C);
-    T* dx = reinterpret_cast<T*>(a.dx) + row * a.C;
-#pragma unroll
-    for (int p = 0; p < kPer; ++p) {
-      const int c0 = (p * kTpr + tin) * kVec;
-      if (c0 < a.C) {
-        float out[kVec];
-#pragma unroll
-        for (int i = 0; i < kVec; ++i) out[i] = rstd * (dxh[p][i] - c1 - xh[p][i] * c2);
-        store_vec<T, kVec>(dx + c0, out);
+      for (int i = 0; i < kPairs; i += 2) {
+        *reinterpret_cast<float4*>(mine_w + chunk(p) + 2 * i) = make_float4(sw[p][i].x, sw[p][i].y, sw[p][i + 1].x, sw[p][i + 1].y);
+        *reinterpret_cast<float4*>(mine_b + chunk(p) + 2 * i) = make_float4(sb[p][i].x, sb[p][i].y, sb[p][i + 1].x, sb[p][i + 1].y);
       }
     }
   }
-  if (!sums) return;
-  // this CTA's partial row: the row owners' sums added in owner order
+  __syncthreads();
   float* pw = a.part + int64_t(blockIdx.x) * a.C;
   float* pb = a.part + (int64_t(gridDim.x) + blockIdx.x) * a.C;
-  __syncthreads();
-  for (int c = threadIdx.x; c < a.C; c += kThreads) {
-    const int chunk = c / kVec, i = c % kVec;
-    const int at = slot4(chunk / kTpr, i / 4, chunk % kTpr) + (i & 3);
+  for (int c = tid; c < a.C; c += kRowThreads) {
     float tw = 0.f, tb = 0.f;
-#pragma unroll
-    for (int k = 0; k < kRowsPerCta; ++k) {
-      tw += wsum[k * kPad + at];
-      tb += wsum[(kRowsPerCta + k) * kPad + at];
+    for (int k = 0; k < groups; ++k) {
+      tw += all[int64_t(k) * a.C + c];
+      tb += all[int64_t(groups + k) * a.C + c];
     }
     pw[c] = tw;
     pb[c] = tb;
@@ -440,27 +517,38 @@ struct Shape {
   bool cta;
 };
 
-// the smallest per-thread chunk count that covers a row; the backward keeps twice the registers per chunk
-bool pick(int C, int dtype, bool backward, Shape* s) {
+// Forward: the smallest per-thread chunk count that covers a row.
+bool pick(int C, int dtype, Shape* s) {
   s->vec = dtype == NB200_F32 ? 4 : 8;
   if (C <= 0 || C % s->vec) return false;
-  const int max_per = backward ? (dtype == NB200_F32 ? 8 : 4) : 8;
-  const int warp_max = backward ? 4 : 8;
-  for (int per = 1; per <= warp_max; per *= 2)
+  for (int per = 1; per <= 8; per *= 2)
     if (C <= 32 * s->vec * per) { s->per = per; s->cta = false; return true; }
-  for (int per = 1; per <= max_per; per *= 2)
-    if (C <= kThreads * s->vec * per) { s->per = per; s->cta = true; return true; }
+  for (int per = 1; per <= 8; per *= 2)
+    if (C <= kThreads * s->vec * per && C <= 8192) { s->per = per; s->cta = true; return true; }
   return false;
 }
 
+// Backward: chunks per thread (as few as cover a row with 512 threads: fewer registers, more rows per CTA) and
+// threads per row.
+struct BwdShape { int per, tpr; };
+bool pick_bwd(int C, int dtype, BwdShape* s) {
+  const int vec = dtype == NB200_F32 ? 4 : 8;
+  if (C <= 0 || C % vec || C > 8192) return false;
+  s->per = 1;
+  while (C > kRowThreads * vec * s->per) s->per *= 2;
+  s->tpr = 1;
+  while (s->tpr * vec * s->per < C) s->tpr *= 2;
+  return true;
+}
+
 // The backward's grid: as many CTAs as are resident at once (`per_sm` from the occupancy calculator; more CTAs only
-// add partial rows to sum), at most one per row unit.  per_sm = 8 bounds it for sizing the workspace.
-int bwd_grid(int64_t rows, const Shape& s, int per_sm) {
+// add partial rows to sum), at most one per block of rows.  per_sm = 2 bounds it for sizing the workspace.
+int bwd_grid(int64_t rows, const BwdShape& s, int per_sm) {
   int sms = 0, dev = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (sms <= 0) sms = 148;
-  const int64_t units = s.cta ? rows : (rows + kThreads / 32 - 1) / (kThreads / 32);
+  const int64_t groups = kRowThreads / s.tpr, units = (rows + groups - 1) / groups;
   const int64_t cap = int64_t(sms) * per_sm;
   return int(units < cap ? (units > 0 ? units : 1) : cap);
 }
@@ -477,22 +565,22 @@ int check_common(const nb200_layer_norm_params* p, const char* what) {
   return NB200_OK;
 }
 
-template <typename T, bool kBwd, typename F>
+template <typename T, typename F>
 int dispatch(const Shape& s, F&& go) {
   // go(kernel) launches; one instantiation per (chunks, warp / CTA)
   if (!s.cta) {
     switch (s.per) {
-      case 1: return go(kBwd ? ln_bwd_kernel<T, 1, false> : ln_fwd_kernel<T, 1, false>);
-      case 2: return go(kBwd ? ln_bwd_kernel<T, 2, false> : ln_fwd_kernel<T, 2, false>);
-      case 4: return go(kBwd ? ln_bwd_kernel<T, 4, false> : ln_fwd_kernel<T, 4, false>);
-      default: return go(kBwd ? ln_bwd_kernel<T, 4, false> : ln_fwd_kernel<T, 8, false>);
+      case 1: return go(ln_fwd_kernel<T, 1, false>);
+      case 2: return go(ln_fwd_kernel<T, 2, false>);
+      case 4: return go(ln_fwd_kernel<T, 4, false>);
+      default: return go(ln_fwd_kernel<T, 8, false>);
     }
   }
   switch (s.per) {
-    case 1: return go(kBwd ? ln_bwd_kernel<T, 1, true> : ln_fwd_kernel<T, 1, true>);
-    case 2: return go(kBwd ? ln_bwd_kernel<T, 2, true> : ln_fwd_kernel<T, 2, true>);
-    case 4: return go(kBwd ? ln_bwd_kernel<T, 4, true> : ln_fwd_kernel<T, 4, true>);
-    default: return go(kBwd ? ln_bwd_kernel<T, sizeof(T) == 4 ? 8 : 4, true> : ln_fwd_kernel<T, 8, true>);
+    case 1: return go(ln_fwd_kernel<T, 1, true>);
+    case 2: return go(ln_fwd_kernel<T, 2, true>);
+    case 4: return go(ln_fwd_kernel<T, 4, true>);
+    default: return go(ln_fwd_kernel<T, 8, true>);
   }
 }
 
@@ -503,20 +591,39 @@ int fwd_t(const nb200_layer_norm_params* p, const Shape& s, cudaStream_t st) {
   a.rows = p->rows; a.C = p->channels; a.eps = p->eps; a.out_scale = p->out_scale;
   const int64_t blocks = s.cta ? p->rows : (p->rows + kThreads / 32 - 1) / (kThreads / 32);
   if (blocks > 0x7fffffff) { set_error("layer_norm: too many rows"); return NB200_ERR_UNSUPPORTED; }
-  return dispatch<T, false>(s, [&](auto kernel) {
+  return dispatch<T>(s, [&](auto kernel) {
     kernel<<<unsigned(blocks), kThreads, 0, st>>>(a);
     count_launch();
     return check_launch("layer_norm_fwd_kernel");
   });
 }
 
+template <typename T, int kPer>
+int bwd_launch(const LnArgs& a, const BwdShape& s, int* grid, cudaStream_t st) {
+  constexpr size_t smem = BwdRing<kPer>::kBytes;
+  auto kernel = ln_bwd_kernel<T, kPer>;
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess) {
+    set_error("layer_norm_bwd: cudaFuncSetAttribute(%zu): %s", smem, cudaGetErrorString(cudaGetLastError()));
+    return NB200_ERR_LAUNCH;
+  }
+  int per_sm = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kRowThreads, smem) != cudaSuccess || per_sm < 1) {
+    cudaGetLastError();
+    per_sm = 1;
+  }
+  *grid = bwd_grid(a.rows, s, per_sm < 2 ? per_sm : 2);
+  kernel<<<unsigned(*grid), kRowThreads, smem, st>>>(a, s.tpr);
+  count_launch();
+  return check_launch("layer_norm_bwd_kernel");
+}
+
 template <typename T>
-int bwd_t(const nb200_layer_norm_params* p, const Shape& s, cudaStream_t st) {
+int bwd_t(const nb200_layer_norm_params* p, const BwdShape& s, cudaStream_t st) {
   LnArgs a{};
   a.x = p->x; a.w = p->weight; a.dy = p->dy; a.dx = p->dx; a.mean = p->mean; a.rstd = p->rstd;
   a.rows = p->rows; a.C = p->channels; a.eps = p->eps; a.out_scale = p->out_scale;
   const bool want_params = p->dweight || p->dbias;
-  int grid = bwd_grid(p->rows, s, 8);
+  int grid = bwd_grid(p->rows, s, 2);
   if (want_params) {
     const size_t need = sizeof(float) * 2 * size_t(grid) * size_t(p->channels);
     if (!p->workspace || p->workspace_bytes < need) {
@@ -526,26 +633,14 @@ int bwd_t(const nb200_layer_norm_params* p, const Shape& s, cudaStream_t st) {
     }
     a.part = static_cast<float*>(p->workspace);
   }
-  // (rows padded to the kernel's per * threads * vec columns)
-  const size_t smem = want_params ? sizeof(float) * 2 * (s.cta ? 1 : kThreads / 32) * size_t(s.per) *
-                                        (s.cta ? kThreads : 32) * s.vec
-                                  : 0;
-  int rc = dispatch<T, true>(s, [&](auto kernel) {
-    if (smem > 48 * 1024 &&
-        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess) {
-      set_error("layer_norm_bwd: cudaFuncSetAttribute(%zu): %s", smem, cudaGetErrorString(cudaGetLastError()));
-      return int(NB200_ERR_LAUNCH);
-    }
-    int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kThreads, smem) != cudaSuccess || per_sm < 1) {
-      cudaGetLastError();
-      per_sm = 1;
-    }
-    grid = bwd_grid(p->rows, s, per_sm < 8 ? per_sm : 8);
-    kernel<<<unsigned(grid), kThreads, smem, st>>>(a);
-    count_launch();
-    return check_launch("layer_norm_bwd_kernel");
-  });
+  int rc;
+  if (s.per == 1) {
+    rc = bwd_launch<T, 1>(a, s, &grid, st);
+  } else if (s.per == 2) {
+    rc = bwd_launch<T, 2>(a, s, &grid, st);
+  } else {
+    rc = bwd_launch<T, sizeof(T) == 4 ? 4 : 2>(a, s, &grid, st);   // (four chunks: fp32 only)
+  }
   if (rc || !want_params) return rc;
   ln_bwd_finish_kernel<T><<<(p->channels + 31) / 32, kThreads, 0, st>>>(
       a.part, grid, p->channels, static_cast<T*>(p->dweight), static_cast<T*>(p->dbias));
@@ -596,13 +691,13 @@ int bwd_generic_t(const nb200_layer_norm_params* p, cudaStream_t st) {
 }
 
 // the vector kernels need 16-byte rows: channels a multiple of 16 bytes (<= 8192) and aligned pointers
-bool vector_path(const nb200_layer_norm_params* p, bool backward, Shape* s) {
-  Shape b;
-  if (!pick(p->channels, p->dtype, true, &b)) return false;       // (one limit for both directions)
-  if (!pick(p->channels, p->dtype, backward, s)) return false;
-  if (!aligned16(p->x) || (p->weight && !aligned16(p->weight))) return false;
-  if (backward) return aligned16(p->dy) && aligned16(p->dx);
-  return aligned16(p->y) && (!p->bias || aligned16(p->bias));
+bool vector_fwd(const nb200_layer_norm_params* p, Shape* s) {
+  return pick(p->channels, p->dtype, s) && aligned16(p->x) && (!p->weight || aligned16(p->weight)) && aligned16(p->y) &&
+         (!p->bias || aligned16(p->bias));
+}
+bool vector_bwd(const nb200_layer_norm_params* p, BwdShape* s) {
+  return pick_bwd(p->channels, p->dtype, s) && aligned16(p->x) && (!p->weight || aligned16(p->weight)) &&
+         aligned16(p->dy) && aligned16(p->dx);
 }
 
 }  // namespace
@@ -614,8 +709,8 @@ extern "C" NB200_API int nb200_layer_norm_workspace_bytes(const nb200_layer_norm
   if (!bytes) { set_error("bytes out-pointer is NULL"); return NB200_ERR_INVALID; }
   if (int rc = check_common(p, "layer_norm_workspace_bytes")) return rc;
   // (sized for the vector kernels' per-CTA partial rows, which is never less than the scalar kernels' [2][C])
-  Shape s;
-  const int grid = pick(p->channels, p->dtype, true, &s) ? bwd_grid(p->rows, s, 8) : 1;
+  BwdShape s;
+  const int grid = pick_bwd(p->channels, p->dtype, &s) ? bwd_grid(p->rows, s, 2) : 1;
   *bytes = sizeof(float) * 2 * size_t(grid) * size_t(p->channels);
   return NB200_OK;
 }
@@ -627,7 +722,7 @@ extern "C" NB200_API int nb200_layer_norm_fwd(const nb200_layer_norm_params* p, 
   cudaStream_t st = static_cast<cudaStream_t>(cuda_stream);
   prof_call_begin(st);
   Shape s;
-  const bool vec = vector_path(p, false, &s);
+  const bool vec = vector_fwd(p, &s);
   switch (p->dtype) {
     case NB200_F32: return vec ? fwd_t<float>(p, s, st) : fwd_generic_t<float>(p, st);
     case NB200_BF16: return vec ? fwd_t<__nv_bfloat16>(p, s, st) : fwd_generic_t<__nv_bfloat16>(p, st);
@@ -644,8 +739,8 @@ extern "C" NB200_API int nb200_layer_norm_bwd(const nb200_layer_norm_params* p, 
   }
   cudaStream_t st = static_cast<cudaStream_t>(cuda_stream);
   prof_call_begin(st);
-  Shape s;
-  const bool vec = vector_path(p, true, &s);
+  BwdShape s;
+  const bool vec = vector_bwd(p, &s);
   switch (p->dtype) {
     case NB200_F32: return vec ? bwd_t<float>(p, s, st) : bwd_generic_t<float>(p, st);
     case NB200_BF16: return vec ? bwd_t<__nv_bfloat16>(p, s, st) : bwd_generic_t<__nv_bfloat16>(p, st);

@@ -106,3 +106,11 @@ def test_empty_input():
 
     y = norm.layer_norm(torch.empty(0, 64, device="cuda"), torch.ones(64, device="cuda"))
     assert y.shape == (0, 64)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("rows,c", [(1, 8), (1, 8192), (67, 24), (130, 1032), (297, 2048), (301, 2056), (449, 4104), (595, 4096)])
+def test_backward_row_groups_at_their_edges(rows, c, dtype):
+    # one row; blocks of rows cut short; one, two and (fp32) four chunks a thread, full and just above the limit of the
+    # next smaller count; more rows than CTAs are resident, so that the ring of copies wraps around
+    _run((rows, c), dtype)
