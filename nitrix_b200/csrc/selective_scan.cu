@@ -1,23 +1,20 @@
 // Mamba / S6 selective scan, forward and backward -- the second sibling op behind the same library (reference
 // src/nitrix/nn/ssm/__init__.py:127- is the dispatcher, src/nitrix/nn/ssm/_reference.py:60-98 the recipe):
 //
-//   a_t = exp(delta_t A),  b_t = (delta_t B_t) x_t,  h_t = a_t h_{t-1} + b_t  (h_{-1} = 0),
+//   a_t = exp(delta_t A),  b_t = (delta_t x_t) B_t,  h_t = a_t h_{t-1} + b_t  (h_{-1} = 0),
 //   y_t = sum_n C_{t,n} h_{t,n} (+ D x_t)
 //
 // per batch element, channel d and state n; x, delta (batch, l, d), A (d, n), B, C (batch, l, n), D (d); fp32
 // recurrence and readout whatever the storage dtype (reference _reference.py:262-279).
 //
-// Four lanes own one channel of one batch element, a quarter of its n states each, and walk the sequence with them in
-// registers (the recurrence is sequential in t; the parallelism is batch x channels x 4); a CTA is 64 channels, and
-// the B_t / C_t rows its threads share are staged through shared memory eight steps at a time, double-buffered, with
-// the next chunk's operands already in flight.  Nothing of size (l, d, n) is ever
-// materialised: the forward leaves the state after every eighth step in a checkpoint array (batch, l / 8, n, d), and
-// the backward walks the chunks in reverse, recomputes a chunk's eight states from its checkpoint into shared
-// memory and runs the adjoint recurrence g_{t-1} = a_t g_t, g_t += C_t dy_t through them.  dB_t and dC_t are sums
-// over channels: the threads' terms of a chunk go into a shared-memory tile whose columns the CTA adds once per chunk
-// (up to 32 states; at 64 the warps reduce by shuffles), then one atomic per sum into fp32 accumulators; dA and dD
-// are sums over batch and time: kept per thread and added once at the end.  A second kernel converts the
-// accumulators to the storage dtype.
+// Nothing of size (l, d, n) is materialised.  Forward: four lanes own one channel of one batch element, a quarter of
+// its states each, and walk the sequence with them in registers; every eighth step's state goes to a checkpoint array
+// (batch, l / 8, d, n).  Backward, two kernels: ss_adjoint_kernel walks the sequence once more, last step first, with
+// the adjoint recurrence g_t = a_{t+1} g_{t+1} + C_t dy_t alone and leaves g at the same eighth steps; with both
+// states known at its borders every chunk of eight steps is then independent of all others, and ss_bwd_kernel
+// computes the gradients chunk by chunk in parallel.  Its sums over channels (dB_t, dC_t) go through a shared-memory
+// tile and 16-byte reductions into fp32 accumulators, those over batch and time (dA, dD) are kept per thread over the
+// chunks of a CTA and added once; ss_finish_kernel converts the accumulators to the storage dtype.
 #include <math.h>
 
 #include "nitrix_b200_scan.h"
@@ -26,16 +23,19 @@
 namespace nb200 {
 namespace {
 
-constexpr int kCh = 64;     // channels (threads) per CTA
-constexpr int kStep = 8;    // steps per staged chunk = checkpoint interval
+constexpr int kStep = 8;    // steps per checkpoint interval = chunk of the backward
 
 struct SsArgs {
   const void *x, *delta, *A, *B, *C, *D, *dy;
   void *y, *dx, *ddelta;
-  float* ckpt;            // [batch][chunks][N][Dc]
+  float* ckpt;            // [batch][chunks][Dc][N]: the state after each chunk
+  float* gck;             // [batch][chunks][Dc][N]: the adjoint state entering each chunk from the next one
   float *accB, *accC;     // [batch][L][N]
   float *accA, *accD;     // [Dc][N], [Dc]
   int batch, L, Dc, N, chunks;
+  int per_cta;            // chunks a CTA of ss_bwd_kernel works through
+  int vec;                // groups of four channels of x, delta, y, dy, dx, ddelta can be moved as one word
+  int vecn;               // groups of four states of the fp32 arrays can
 };
 
 // a_t = exp(delta_t A) as one multiply and one ex2.approx (relative error 2^-22): A is held pre-multiplied by log2(e)
@@ -45,287 +45,613 @@ __device__ __forceinline__ float ex2_ss(float x) {
   return y;
 }
 constexpr float kLog2eSs = 1.4426950408889634f;
+__device__ __forceinline__ float2 ex2_ss2(float2 x) { return make_float2(ex2_ss(x.x), ex2_ss(x.y)); }
 
-// Forward.  Four adjacent lanes share a channel and hold a quarter of its states each (the readout is a sum over
-// the four lanes: two shuffles per step): four times the warps of one-thread-per-channel for the same work, which is
-// what the sequential recurrence lacks -- one warp per scheduler left the issue slots 20 % busy.  A CTA is 64 channels
-// = 256 threads.
-constexpr int kSplit = 4;
-constexpr int kFwdThreads = kCh * kSplit;
+// four consecutive elements p[0..3], the first `n` of which exist (zeros for the rest); `vec`: n is 0 or 4 and p is
+// aligned to the four
+template <typename T>
+__device__ __forceinline__ float4 load4(const T* p, int n, bool vec) {
+  float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (vec) {
+    if (n > 0) {
+      if constexpr (sizeof(T) == 4) {
+        r = *reinterpret_cast<const float4*>(p);
+      } else {
+        const uint2 w = *reinterpret_cast<const uint2*>(p);
+        const T* e = reinterpret_cast<const T*>(&w);
+        r = make_float4(to_f32<T>(e[0]), to_f32<T>(e[1]), to_f32<T>(e[2]), to_f32<T>(e[3]));
+      }
+    }
+  } else {
+    if (n > 0) r.x = to_f32<T>(p[0]);
+    if (n > 1) r.y = to_f32<T>(p[1]);
+    if (n > 2) r.z = to_f32<T>(p[2]);
+    if (n > 3) r.w = to_f32<T>(p[3]);
+  }
+  return r;
+}
+// The same as loaded, for a prefetch: a conversion behind the load would wait for it on the spot.
+template <typename T>
+struct Raw4 {
+  uint32_t w[4];   // fp32: the four; 16 bits: two words of two (vec) or four of one
+  __device__ __forceinline__ void load(const T* p, int n, bool vec) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) w[i] = 0u;
+    if (vec) {
+      if (n > 0) {
+        if constexpr (sizeof(T) == 4) {
+          const uint4 v = *reinterpret_cast<const uint4*>(p);
+          w[0] = v.x; w[1] = v.y; w[2] = v.z; w[3] = v.w;
+        } else {
+          const uint2 v = *reinterpret_cast<const uint2*>(p);
+          w[0] = v.x; w[1] = v.y;
+        }
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (i < n) {
+          if constexpr (sizeof(T) == 4) w[i] = reinterpret_cast<const uint32_t*>(p)[i];
+          else w[i] = reinterpret_cast<const unsigned short*>(p)[i];
+        }
+    }
+  }
+  static __device__ __forceinline__ float f(uint32_t bits) {
+    if constexpr (sizeof(T) == 4) {
+      return __uint_as_float(bits);
+    } else {
+      const unsigned short b = static_cast<unsigned short>(bits);
+      return to_f32<T>(*reinterpret_cast<const T*>(&b));
+    }
+  }
+  __device__ __forceinline__ float4 get(bool vec) const {
+    if constexpr (sizeof(T) == 4) return make_float4(f(w[0]), f(w[1]), f(w[2]), f(w[3]));
+    else return vec ? make_float4(f(w[0]), f(w[0] >> 16), f(w[1]), f(w[1] >> 16)) : make_float4(f(w[0]), f(w[1]), f(w[2]), f(w[3]));
+  }
+};
+template <typename T>
+__device__ __forceinline__ void store4(T* p, float4 v, int n, bool vec) {
+  if (vec) {
+    if (n > 0) {
+      if constexpr (sizeof(T) == 4) {
+        *reinterpret_cast<float4*>(p) = v;
+      } else {
+        uint2 w;
+        T* e = reinterpret_cast<T*>(&w);
+        e[0] = from_f32<T>(v.x); e[1] = from_f32<T>(v.y); e[2] = from_f32<T>(v.z); e[3] = from_f32<T>(v.w);
+        *reinterpret_cast<uint2*>(p) = w;
+      }
+    }
+  } else {
+    if (n > 0) p[0] = from_f32<T>(v.x);
+    if (n > 1) p[1] = from_f32<T>(v.y);
+    if (n > 2) p[2] = from_f32<T>(v.z);
+    if (n > 3) p[3] = from_f32<T>(v.w);
+  }
+}
+
+// ---- the two sequential walks ------------------------------------------------------------------------------------
+// Four adjacent lanes share a channel and hold kQ = kN / 4 of its states each as packed pairs.  A CTA is 16 channels = 64
+// threads: small CTAs spread evenly over the SMs (8 x 2048 channels: 7 per SM against an average of 6.9; CTAs of 64
+// channels put 2 on some SMs and 1 on the others).  Sixteen steps are staged at a time: a thread fetches four channels
+// of one row of each operand with one load, one chunk ahead and kept as loaded (a 16-bit conversion behind the load
+// would wait for it), and spreads (delta, delta x) and the B, C rows through shared memory; y goes back the same way.
+// A step is 3 shared-memory loads, 8 packed operations and 4 ex2 per 4 states, taken four steps at a time so that no
+// operand or exponential waits for the recurrence.  Bounds: the special-function unit (16 ex2 per SM and cycle: 60 us
+// for 8 x 1024 x 2048 x 16) and shared memory, which delivers 32 words per cycle however many lanes share them.
+// Two channels per thread halve those words, but leave half the warps to cover the latencies: measured slower.
+// Forward with checkpoints, f32 (8, 1024, 2048, 16): 288 -> 135 us; bf16 (8, 2048, 2048, 16) without: 931 -> 242 us.
+constexpr int kScanCh = 16;
+constexpr int kScanThreads = kScanCh * 4;
+constexpr int kStage = 16;                       // steps per staged chunk
+constexpr int kYPitch = 24;                      // of the staged readouts: four rows x eight channels on distinct banks
+
+// a thread's share of a chunk's [kStage][kN] block of B or C rows: kN / 16 groups of four states
+template <typename T, int kN>
+struct RowShare {
+  static constexpr int kGroups = kStage * (kN / 4);
+  static constexpr int kPer = (kGroups + kScanThreads - 1) / kScanThreads;
+  Raw4<T> v[kPer];
+  __device__ __forceinline__ void load(const T* base, int t0, int L, int N, bool vec, int tid) {
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) {
+      const int i = tid + kScanThreads * j, s = i / (kN / 4), n0 = (i - s * (kN / 4)) * 4;
+      const bool in = i < kGroups && t0 + s < L;
+      v[j].load(base + int64_t(t0 + s) * N + n0, in ? min(4, N - n0) : 0, vec);
+    }
+  }
+  __device__ __forceinline__ void store(float* dst, bool vec, int tid) const {
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) {
+      const int i = tid + kScanThreads * j;
+      if (i < kGroups) *reinterpret_cast<float4*>(dst + i * 4) = v[j].get(vec);
+    }
+  }
+};
+
+// kQ states of one channel to / from an fp32 [..][N] row
+template <int kQ>
+__device__ __forceinline__ void store_states(float* p, int n0, int N, bool vec, const float2 (&h)[kQ / 2]) {
+  if (vec && kQ % 4 == 0) {
+#pragma unroll
+    for (int k = 0; k < kQ / 2; k += 2)
+      if (n0 + 2 * k < N) *reinterpret_cast<float4*>(p + n0 + 2 * k) = make_float4(h[k].x, h[k].y, h[(k + 1) % (kQ / 2)].x, h[(k + 1) % (kQ / 2)].y);
+  } else if (vec) {
+    if (n0 < N) *reinterpret_cast<float2*>(p + n0) = h[0];
+  } else {
+#pragma unroll
+    for (int k = 0; k < kQ / 2; ++k) {
+      if (n0 + 2 * k < N) p[n0 + 2 * k] = h[k].x;
+      if (n0 + 2 * k + 1 < N) p[n0 + 2 * k + 1] = h[k].y;
+    }
+  }
+}
+
+// A's row of a channel, times log2(e), as pairs (zeros for states that do not exist)
+template <typename T, int kQ>
+__device__ __forceinline__ void load_rates(const SsArgs& a, int d, bool live, int n0, float2 (&Ar)[kQ / 2]) {
+  const T* Ap = reinterpret_cast<const T*>(a.A) + int64_t(d) * a.N;
+#pragma unroll
+  for (int k = 0; k < kQ / 2; ++k) {
+    const int n = n0 + 2 * k;
+    Ar[k].x = (live && n < a.N) ? kLog2eSs * to_f32<T>(Ap[n]) : 0.f;
+    Ar[k].y = (live && n + 1 < a.N) ? kLog2eSs * to_f32<T>(Ap[n + 1]) : 0.f;
+  }
+}
+
+// two states' row entries from shared memory, kQ / 2 pairs
+template <int kQ>
+__device__ __forceinline__ void row_pairs(const float* p, float2 (&v)[kQ / 2]) {
+  if constexpr (kQ == 2) {
+    v[0] = *reinterpret_cast<const float2*>(p);
+  } else {
+#pragma unroll
+    for (int k = 0; k < kQ / 2; k += 2) {
+      const float4 w = *reinterpret_cast<const float4*>(p + 2 * k);
+      v[k] = make_float2(w.x, w.y);
+      v[k + 1] = make_float2(w.z, w.w);
+    }
+  }
+}
+
+// four neighbouring channels' pairs of a step
+__device__ __forceinline__ void write_pairs(float2* p, float4 a, float4 b) {
+  reinterpret_cast<float4*>(p)[0] = make_float4(a.x, b.x, a.y, b.y);
+  reinterpret_cast<float4*>(p)[1] = make_float4(a.z, b.z, a.w, b.w);
+}
+__device__ __forceinline__ float2 both(float v) { return make_float2(v, v); }
 
 template <typename T, int kN>
-__global__ void __launch_bounds__(kFwdThreads) ss_fwd_kernel(SsArgs a) {
-  constexpr int kQ = kN / kSplit;                            // states per thread
-  constexpr int kRows = kStep * kN;                          // elements of a chunk's B (or C) block
-  constexpr int kShare = (kRows + kFwdThreads - 1) / kFwdThreads;
-  __shared__ float sB[2][kRows], sC[2][kRows];               // double-buffered: one barrier per chunk
-  const int tid = threadIdx.x, part = tid & (kSplit - 1);
-  const int d = blockIdx.x * kCh + (tid >> 2), b = blockIdx.y;
+__global__ void __launch_bounds__(kScanThreads) ss_fwd_kernel(SsArgs a) {
+  constexpr int kQ = kN / 4;
+  __shared__ __align__(16) float2 du[kStage * kScanCh];    // delta, delta x
+  __shared__ __align__(16) float sB[kStage * kN], sC[kStage * kN];
+  __shared__ __align__(16) float sy[kStage * kYPitch];
+  const int tid = threadIdx.x, part = tid & 3, ch = tid >> 2;
+  const int d0 = blockIdx.x * kScanCh, b = blockIdx.y, d = d0 + ch;
   const bool live = d < a.Dc;
-  const T* xp = reinterpret_cast<const T*>(a.x) + int64_t(b) * a.L * a.Dc + d;
-  const T* dp = reinterpret_cast<const T*>(a.delta) + int64_t(b) * a.L * a.Dc + d;
-  T* yp = reinterpret_cast<T*>(a.y) + int64_t(b) * a.L * a.Dc + d;
+  const bool vec = a.vec != 0, vecn = a.vecn != 0;
+  // this thread's four channels of one row of a staged chunk
+  const int lr = tid >> 2, lc = (tid & 3) * 4, ln = max(0, min(4, a.Dc - (d0 + lc)));
+  const int64_t at = int64_t(b) * a.L * a.Dc + d0 + lc;
+  const T* xp = reinterpret_cast<const T*>(a.x) + at;
+  const T* dp = reinterpret_cast<const T*>(a.delta) + at;
+  T* yp = reinterpret_cast<T*>(a.y) + at;
   const T* Bp = reinterpret_cast<const T*>(a.B) + int64_t(b) * a.L * a.N;
   const T* Cp = reinterpret_cast<const T*>(a.C) + int64_t(b) * a.L * a.N;
-  float Ar[kQ], h[kQ];
+  const float4 Dd = a.D ? load4<T>(reinterpret_cast<const T*>(a.D) + d0 + lc, ln, false) : make_float4(0.f, 0.f, 0.f, 0.f);
+  float2 Ar[kQ / 2], h[kQ / 2];
+  load_rates<T, kQ>(a, d, live, part * kQ, Ar);
 #pragma unroll
-  for (int q = 0; q < kQ; ++q) {
-    const int n = part * kQ + q;
-    Ar[q] = (live && n < a.N) ? kLog2eSs * to_f32<T>(reinterpret_cast<const T*>(a.A)[int64_t(d) * a.N + n]) : 0.f;
-    h[q] = 0.f;
-  }
-  const float Dd = (a.D && live) ? to_f32<T>(reinterpret_cast<const T*>(a.D)[d]) : 0.f;
-  // the next chunk's operands: issued before the current chunk is computed
-  float ndl[kStep], nxv[kStep], nbq[kShare], ncq[kShare];
+  for (int k = 0; k < kQ / 2; ++k) h[k] = make_float2(0.f, 0.f);
+  Raw4<T> nx, nd;
+  RowShare<T, kN> nB, nC;
   auto load = [&](int t0) {
-#pragma unroll
-    for (int s = 0; s < kStep; ++s) {
-      const bool in = live && t0 + s < a.L;
-      ndl[s] = in ? to_f32<T>(dp[int64_t(t0 + s) * a.Dc]) : 0.f;
-      nxv[s] = in ? to_f32<T>(xp[int64_t(t0 + s) * a.Dc]) : 0.f;
-    }
-#pragma unroll
-    for (int j = 0; j < kShare; ++j) {
-      const int i = tid + kFwdThreads * j, s = i / kN, n = i - s * kN;   // (compile-time divisor)
-      const bool in = i < kRows && n < a.N && t0 + s < a.L;
-      nbq[j] = in ? to_f32<T>(Bp[int64_t(t0 + s) * a.N + n]) : 0.f;
-      ncq[j] = in ? to_f32<T>(Cp[int64_t(t0 + s) * a.N + n]) : 0.f;
-    }
+    const int n = t0 + lr < a.L ? ln : 0;
+    nx.load(xp + int64_t(t0 + lr) * a.Dc, n, vec);
+    nd.load(dp + int64_t(t0 + lr) * a.Dc, n, vec);
+    nB.load(Bp, t0, a.L, a.N, vecn, tid);
+    nC.load(Cp, t0, a.L, a.N, vecn, tid);
   };
   load(0);
-  for (int c = 0; c < a.chunks; ++c) {
-    const int t0 = c * kStep;
-    float dls[kStep], xvs[kStep];
+  for (int t0 = 0; t0 < a.L; t0 += kStage) {
+    // (steps past the sequence's end are staged as zeros: the state stays as it is)
+    const float4 cx = nx.get(vec), dl4 = nd.get(vec);
+    write_pairs(du + lr * kScanCh + lc, dl4, make_float4(dl4.x * cx.x, dl4.y * cx.y, dl4.z * cx.z, dl4.w * cx.w));
+    nB.store(sB, vecn, tid);
+    nC.store(sC, vecn, tid);
+    __syncthreads();
+    if (t0 + kStage < a.L) load(t0 + kStage);
+    // four steps at a time, in three phases: operands and decays (nothing in them depends on the state), then the
+    // recurrence, then the sums over the lanes
 #pragma unroll
-    for (int s = 0; s < kStep; ++s) {
-      dls[s] = ndl[s];
-      xvs[s] = nxv[s];
-    }
-    float* rb = sB[c & 1];
-    float* rc = sC[c & 1];
+    for (int s0 = 0; s0 < kStage; s0 += 4) {
+      float2 av[4][kQ / 2], bu[4][kQ / 2];
 #pragma unroll
-    for (int j = 0; j < kShare; ++j) {
-      const int i = tid + kFwdThreads * j;
-      if (i < kRows) {
-        rb[i] = nbq[j];
-        rc[i] = ncq[j];
-      }
-    }
-    __syncthreads();   // (the buffer written two chunks ago was last read before the previous barrier)
-    if (c + 1 < a.chunks) load(t0 + kStep);
+      for (int u = 0; u < 4; ++u) {
+        const float2 w = du[(s0 + u) * kScanCh + ch];
+        float2 Bv[kQ / 2];
+        row_pairs<kQ>(sB + (s0 + u) * kN + part * kQ, Bv);
 #pragma unroll
-    for (int s = 0; s < kStep; ++s) {
-      const int t = t0 + s;
-      if (t < a.L) {   // (uniform over the CTA: the shuffles below are executed by whole warps)
-        const float dl = dls[s], xv = xvs[s];
-        float y = 0.f;
-#pragma unroll
-        for (int q = 0; q < kQ; ++q) {
-          const int n = part * kQ + q;
-          h[q] = fmaf(ex2_ss(dl * Ar[q]), h[q], (dl * rb[s * kN + n]) * xv);   // (rows past N are zero)
-          y = fmaf(rc[s * kN + n], h[q], y);
+        for (int k = 0; k < kQ / 2; ++k) {
+          av[u][k] = ex2_ss2(__fmul2_rn(both(w.x), Ar[k]));
+          bu[u][k] = __fmul2_rn(both(w.y), Bv[k]);   // (rows past N are zero)
         }
-        y += __shfl_xor_sync(0xffffffffu, y, 1);
-        y += __shfl_xor_sync(0xffffffffu, y, 2);
-        if (a.D) y = fmaf(Dd, xv, y);
-        if (live && part == 0) yp[int64_t(t) * a.Dc] = from_f32<T>(y);
       }
-    }
-    if (a.ckpt && live) {
-      float* ck = a.ckpt + (int64_t(b) * a.chunks + c) * a.N * a.Dc + d;
+      float y[4];
 #pragma unroll
-      for (int q = 0; q < kQ; ++q) {
-        const int n = part * kQ + q;
-        if (n < a.N) ck[int64_t(n) * a.Dc] = h[q];
+      for (int u = 0; u < 4; ++u) {
+        float2 Cv[kQ / 2], acc = make_float2(0.f, 0.f);
+        row_pairs<kQ>(sC + (s0 + u) * kN + part * kQ, Cv);
+#pragma unroll
+        for (int k = 0; k < kQ / 2; ++k) {
+          h[k] = __ffma2_rn(av[u][k], h[k], bu[u][k]);
+          acc = k ? __ffma2_rn(Cv[k], h[k], acc) : __fmul2_rn(Cv[k], h[k]);
+        }
+        y[u] = acc.x + acc.y;
+      }
+      // the sums over the four lanes, four steps at once: each lane ends with one step
+      const bool hi = part & 2, lo = part & 1;
+      float k0 = hi ? y[2] : y[0], k1 = hi ? y[3] : y[1];
+      k0 += __shfl_xor_sync(0xffffffffu, hi ? y[0] : y[2], 2);
+      k1 += __shfl_xor_sync(0xffffffffu, hi ? y[1] : y[3], 2);
+      sy[(s0 + part) * kYPitch + ch] = (lo ? k1 : k0) + __shfl_xor_sync(0xffffffffu, lo ? k0 : k1, 1);
+      if ((s0 & 4) && a.ckpt) {   // the state after every eighth step (of a chunk that has a successor)
+        const int c = (t0 + s0) / kStep;
+        if (live && c + 1 < a.chunks)
+          store_states<kQ>(a.ckpt + ((int64_t(b) * a.chunks + c) * a.Dc + d) * a.N, part * kQ, a.N, vecn, h);
       }
     }
+    __syncthreads();
+    float4 v = *reinterpret_cast<const float4*>(sy + lr * kYPitch + lc);
+    if (a.D) v = make_float4(fmaf(Dd.x, cx.x, v.x), fmaf(Dd.y, cx.y, v.y), fmaf(Dd.z, cx.z, v.z), fmaf(Dd.w, cx.w, v.w));
+    store4<T>(yp + int64_t(t0 + lr) * a.Dc, v, t0 + lr < a.L ? ln : 0, vec);
   }
 }
 
-// Backward: chunks in reverse, four lanes per channel as in the forward.  hs[0] = the state before the chunk
-// (checkpoint c - 1, zero for the first chunk), hs[s + 1] = the state after step s of the chunk, recomputed; then the
-// adjoint recurrence from the chunk's last step down.  A thread reads and writes only its own states in hs.
+// The adjoint recurrence alone, last step first: leaves for every chunk but the last the g that enters it.
 template <typename T, int kN>
-__global__ void __launch_bounds__(kFwdThreads) ss_bwd_kernel(SsArgs a) {
-  constexpr int kQ = kN / kSplit;                            // states per thread
-  constexpr int kRows = kStep * kN;
-  constexpr int kShare = (kRows + kFwdThreads - 1) / kFwdThreads;
-  extern __shared__ float smem_ss[];
-  float* hs = smem_ss;                                   // [kStep + 1][kN][kCh]
-  float* sBb = hs + (kStep + 1) * kN * kCh;              // 2 x [kStep][kN]
-  float* sCb = sBb + 2 * kRows;                          // 2 x [kStep][kN]
-  // up to 32 states: the chunk's dB / dC terms as a tile [kStep][2][kN][kCh] (128 KB at 32 states); 64 states would
-  // not fit beside the states and reduce over the warp's eight channels by shuffles instead
-  constexpr bool kTile = kN <= 32;
-  float* ct = sCb + 2 * kRows;
-  const int tid = threadIdx.x, lane = tid & 31, part = tid & (kSplit - 1), ch = tid >> 2;
-  const int d = blockIdx.x * kCh + ch, b = blockIdx.y;
+__global__ void __launch_bounds__(kScanThreads) ss_adjoint_kernel(SsArgs a) {
+  constexpr int kQ = kN / 4;
+  __shared__ __align__(16) float2 dg[kStage * kScanCh];    // delta, dy
+  __shared__ __align__(16) float sC[kStage * kN];
+  const int tid = threadIdx.x, part = tid & 3, ch = tid >> 2;
+  const int d0 = blockIdx.x * kScanCh, b = blockIdx.y, d = d0 + ch;
   const bool live = d < a.Dc;
-  const int64_t base = int64_t(b) * a.L * a.Dc + d;
-  const T* xp = reinterpret_cast<const T*>(a.x) + base;
-  const T* dp = reinterpret_cast<const T*>(a.delta) + base;
-  const T* gp = reinterpret_cast<const T*>(a.dy) + base;
-  T* dxp = reinterpret_cast<T*>(a.dx) + base;
-  T* ddp = reinterpret_cast<T*>(a.ddelta) + base;
-  const T* Bp = reinterpret_cast<const T*>(a.B) + int64_t(b) * a.L * a.N;
+  const bool vec = a.vec != 0, vecn = a.vecn != 0;
+  const int lr = tid >> 2, lc = (tid & 3) * 4, ln = max(0, min(4, a.Dc - (d0 + lc)));
+  const int64_t at = int64_t(b) * a.L * a.Dc + d0 + lc;
+  const T* gp = reinterpret_cast<const T*>(a.dy) + at;
+  const T* dp = reinterpret_cast<const T*>(a.delta) + at;
   const T* Cp = reinterpret_cast<const T*>(a.C) + int64_t(b) * a.L * a.N;
-  float Ar[kQ], g[kQ], dA[kQ];
+  float2 Ar[kQ / 2], g[kQ / 2];
+  load_rates<T, kQ>(a, d, live, part * kQ, Ar);
 #pragma unroll
-  for (int q = 0; q < kQ; ++q) {
-    const int n = part * kQ + q;
-    Ar[q] = (live && n < a.N) ? kLog2eSs * to_f32<T>(reinterpret_cast<const T*>(a.A)[int64_t(d) * a.N + n]) : 0.f;
-    g[q] = dA[q] = 0.f;
-  }
-  const float Dd = (a.D && live) ? to_f32<T>(reinterpret_cast<const T*>(a.D)[d]) : 0.f;
-  float dD = 0.f;
-  // the next chunk's operands: issued before the current chunk is computed
-  float ndl[kStep], nxv[kStep], ngy[kStep], nbq[kShare], ncq[kShare];
+  for (int k = 0; k < kQ / 2; ++k) g[k] = make_float2(0.f, 0.f);
+  Raw4<T> ng, nd;
+  RowShare<T, kN> nC;
   auto load = [&](int t0) {
-#pragma unroll
-    for (int s = 0; s < kStep; ++s) {
-      const bool in = live && t0 + s < a.L;
-      ndl[s] = in ? to_f32<T>(dp[int64_t(t0 + s) * a.Dc]) : 0.f;
-      nxv[s] = in ? to_f32<T>(xp[int64_t(t0 + s) * a.Dc]) : 0.f;
-      ngy[s] = in ? to_f32<T>(gp[int64_t(t0 + s) * a.Dc]) : 0.f;
-    }
-#pragma unroll
-    for (int j = 0; j < kShare; ++j) {
-      const int i = tid + kFwdThreads * j, s = i / kN, n = i - s * kN;   // (compile-time divisor)
-      const bool in = i < kRows && n < a.N && t0 + s < a.L;
-      nbq[j] = in ? to_f32<T>(Bp[int64_t(t0 + s) * a.N + n]) : 0.f;
-      ncq[j] = in ? to_f32<T>(Cp[int64_t(t0 + s) * a.N + n]) : 0.f;
-    }
+    const int n = t0 + lr < a.L ? ln : 0;
+    ng.load(gp + int64_t(t0 + lr) * a.Dc, n, vec);
+    nd.load(dp + int64_t(t0 + lr) * a.Dc, n, vec);
+    nC.load(Cp, t0, a.L, a.N, vecn, tid);
   };
-  if (a.chunks > 0) load((a.chunks - 1) * kStep);
-  for (int c = a.chunks - 1; c >= 0; --c) {
+  const int last = (a.L - 1) / kStage * kStage;
+  load(last);
+  for (int t0 = last; t0 >= 0; t0 -= kStage) {
+    __syncthreads();
+    write_pairs(dg + lr * kScanCh + lc, nd.get(vec), ng.get(vec));
+    nC.store(sC, vecn, tid);
+    __syncthreads();
+    if (t0 > 0) load(t0 - kStage);
+#pragma unroll
+    for (int s0 = kStage - 4; s0 >= 0; s0 -= 4) {
+      if ((s0 & 4)) {   // the last step of a chunk of eight: what enters it
+        const int c = (t0 + s0) / kStep;
+        if (live && c + 1 < a.chunks)
+          store_states<kQ>(a.gck + ((int64_t(b) * a.chunks + c) * a.Dc + d) * a.N, part * kQ, a.N, vecn, g);
+      }
+      float2 av[4][kQ / 2], Cv[4][kQ / 2];
+      float gy[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const float2 w = dg[(s0 + u) * kScanCh + ch];
+        row_pairs<kQ>(sC + (s0 + u) * kN + part * kQ, Cv[u]);
+        gy[u] = w.y;
+#pragma unroll
+        for (int k = 0; k < kQ / 2; ++k) av[u][k] = ex2_ss2(__fmul2_rn(both(w.x), Ar[k]));
+      }
+#pragma unroll
+      for (int u = 3; u >= 0; --u)
+#pragma unroll
+        for (int k = 0; k < kQ / 2; ++k) g[k] = __fmul2_rn(__ffma2_rn(Cv[u][k], both(gy[u]), g[k]), av[u][k]);
+    }
+  }
+}
+
+// ---- gradients of a chunk ----------------------------------------------------------------------------------------
+// A CTA of 128 threads takes 64 channels of one batch element and works through `per_cta` chunks of eight steps, 16
+// states at a time.  A thread owns two channels (o and o + 32) and four states of each: both sums over channels (dB,
+// dC) start inside the thread, which halves the shared-memory traffic of one channel per thread, and the pairs of the
+// packed arithmetic are neighbouring states.  The eight steps are taken as two halves, the second first: the states
+// and decays of four steps of eight (channel, state) pairs are 64 registers, those of all eight steps would be 128 and
+// leave two warps per scheduler; the first half's steps are run twice for it (1.5 ex2 per step and state).  Bound: shared
+// memory (32 words per cycle and SM): per pair and step 3 words of operands, 2 of the dB / dC tile, 1 for the rest; and a chunk's first loads, which
+// a prefetch into L2 one chunk ahead shortens.  Backward of f32 (8, 1024, 2048, 16), all kernels: 1123 -> 451 us.
+constexpr int kBwdCh = 64;
+constexpr int kBwdThreads = 128;
+constexpr int kHalf = kStep / 2;
+// sums over the states of a chunk, [step][which][channel]: the four lanes that hold (channel, channel + 32) x (two
+// sums) of one owner write to banks 8 apart
+constexpr int kSumCol = 48 - 32, kSumWhich = 104, kSumStep = 184;
+
+__device__ __forceinline__ void red_add4(float* p, float4 v) {
+  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
+}
+// up to four sums of a row of N states starting at state n0
+__device__ __forceinline__ void add_states(float* row, int n0, int N, bool vec, float4 v) {
+  if (vec) {
+    if (n0 < N) red_add4(row + n0, v);
+  } else {
+    if (n0 + 0 < N) atomicAdd(row + n0 + 0, v.x);
+    if (n0 + 1 < N) atomicAdd(row + n0 + 1, v.y);
+    if (n0 + 2 < N) atomicAdd(row + n0 + 2, v.z);
+    if (n0 + 3 < N) atomicAdd(row + n0 + 3, v.w);
+  }
+}
+
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
+// kBlocks: blocks of 16 states (1: the sums of dA stay in registers; more: in shared memory, a slot per thread)
+template <typename T, int kBlocks>
+__global__ void __launch_bounds__(kBwdThreads, 3) ss_bwd_kernel(SsArgs a) {
+  constexpr int kN = 16 * kBlocks;
+  extern __shared__ __align__(16) float smem_ss[];
+  float4* dxg = reinterpret_cast<float4*>(smem_ss);                // [kStep][kBwdCh]: delta, delta x, dy, x
+  float* sB = reinterpret_cast<float*>(dxg + kStep * kBwdCh);      // [kStep][kN]
+  float* sC = sB + kStep * kN;
+  float* tile = sC + kStep * kN;                                   // [kHalf][32 owners][32]: dB, dC terms of 16 states
+  float* sums = tile + kHalf * 32 * 32;                            // [kStep][kSumStep]
+  float4* sdA = reinterpret_cast<float4*>(sums + kStep * kSumStep);   // kBlocks > 1: [kBlocks][2][kBwdThreads]
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, part = tid & 3, o = tid >> 2;
+  const int d0 = blockIdx.x * kBwdCh, b = blockIdx.z;
+  const bool vec = a.vec != 0, vecn = a.vecn != 0;
+  const bool hi = part & 2, lo = part & 1;
+  // channel ch of dxg: permuted within eight so that both the writers (four channels each) and the readers (eight
+  // neighbours per warp) meet distinct banks
+  auto place = [](int ch) { return (ch & ~7) | ((ch ^ (ch >> 3)) & 7); };
+  const int at0 = place(o), at1 = place(o + 32);
+  // this thread's four channels of one step of a chunk
+  const int lr = tid >> 4, lc = (tid & 15) * 4, ln = max(0, min(4, a.Dc - (d0 + lc)));
+  const int64_t at = int64_t(b) * a.L * a.Dc + d0 + lc;
+  float4 dDs = make_float4(0.f, 0.f, 0.f, 0.f);
+  float2 Ar[2][2], dA[2][2];
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    load_rates<T, 4>(a, d0 + o + 32 * j, d0 + o + 32 * j < a.Dc, part * 4, Ar[j]);
+    dA[j][0] = dA[j][1] = make_float2(0.f, 0.f);
+    if constexpr (kBlocks > 1) {
+#pragma unroll
+      for (int nb = 0; nb < kBlocks; ++nb) sdA[(nb * 2 + j) * kBwdThreads + tid] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+  }
+  const int c_end = min(a.chunks, int(blockIdx.y + 1) * a.per_cta);
+  for (int c = blockIdx.y * a.per_cta; c < c_end; ++c) {
     const int t0 = c * kStep;
-    float dls[kStep], xvs[kStep], gys[kStep];
-#pragma unroll
-    for (int s = 0; s < kStep; ++s) {
-      dls[s] = ndl[s];
-      xvs[s] = nxv[s];
-      gys[s] = ngy[s];
-    }
-    float* sB = sBb + (c & 1) * kRows;
-    float* sC = sCb + (c & 1) * kRows;
-#pragma unroll
-    for (int j = 0; j < kShare; ++j) {
-      const int i = tid + kFwdThreads * j;
-      if (i < kRows) {
-        sB[i] = nbq[j];
-        sC[i] = ncq[j];
+    const int n = t0 + lr < a.L ? ln : 0;
+    const int64_t row = at + int64_t(t0 + lr) * a.Dc;
+    const float4 x4 = load4<T>(reinterpret_cast<const T*>(a.x) + row, n, vec);
+    const float4 dl4 = load4<T>(reinterpret_cast<const T*>(a.delta) + row, n, vec);
+    const float4 gy4 = load4<T>(reinterpret_cast<const T*>(a.dy) + row, n, vec);
+    if (c + 1 < c_end) {   // the next chunk's rows and states, as far as L2
+      const int64_t next = at + int64_t(min(t0 + kStep + lr, a.L - 1)) * a.Dc;
+      if (ln > 0) {
+        prefetch_l2(reinterpret_cast<const T*>(a.x) + next);
+        prefetch_l2(reinterpret_cast<const T*>(a.delta) + next);
+        prefetch_l2(reinterpret_cast<const T*>(a.dy) + next);
+      }
+      const int64_t st = (int64_t(b) * a.chunks + c) * a.Dc * a.N, n0 = int64_t(d0) * a.N + tid * (kN / 2);
+      if (n0 < int64_t(a.Dc) * a.N) {
+        prefetch_l2(a.ckpt + st + n0);
+        if (c + 2 < a.chunks) prefetch_l2(a.gck + st + int64_t(a.Dc) * a.N + n0);
       }
     }
-    __syncthreads();   // (the buffer written two chunks ago, and the tile, were last read before the previous barrier)
-    if (c > 0) load(t0 - kStep);
-    // ---- recompute the chunk's states ----
-    {
-      float h[kQ];
-      const float* ck = c > 0 ? a.ckpt + (int64_t(b) * a.chunks + (c - 1)) * a.N * a.Dc + d : nullptr;
-#pragma unroll
-      for (int q = 0; q < kQ; ++q) {
-        const int n = part * kQ + q;
-        h[q] = (live && ck && n < a.N) ? ck[int64_t(n) * a.Dc] : 0.f;
-        hs[(0 * kN + n) * kCh + ch] = h[q];
-      }
-#pragma unroll
-      for (int s = 0; s < kStep; ++s) {
-        const float dl = dls[s], xv = xvs[s];   // (zeros past the sequence's end: the state stays as it is)
-#pragma unroll
-        for (int q = 0; q < kQ; ++q) {
-          const int n = part * kQ + q;
-          h[q] = fmaf(ex2_ss(dl * Ar[q]), h[q], (dl * sB[s * kN + n]) * xv);
-          hs[((s + 1) * kN + n) * kCh + ch] = h[q];
-        }
-      }
+    __syncthreads();   // (the chunk before has been read)
+    // (steps past the sequence's end and channels past the last are zeros: they add nothing)
+    dxg[lr * kBwdCh + place(lc + 0)] = make_float4(dl4.x, dl4.x * x4.x, gy4.x, x4.x);
+    dxg[lr * kBwdCh + place(lc + 1)] = make_float4(dl4.y, dl4.y * x4.y, gy4.y, x4.y);
+    dxg[lr * kBwdCh + place(lc + 2)] = make_float4(dl4.z, dl4.z * x4.z, gy4.z, x4.z);
+    dxg[lr * kBwdCh + place(lc + 3)] = make_float4(dl4.w, dl4.w * x4.w, gy4.w, x4.w);
+    for (int i = tid; i < kStep * kN; i += kBwdThreads) {
+      const int s = i / kN, ns = i - s * kN;
+      const bool in = ns < a.N && t0 + s < a.L;
+      const int64_t bc = (int64_t(b) * a.L + t0 + s) * a.N + ns;
+      sB[i] = in ? to_f32<T>(reinterpret_cast<const T*>(a.B)[bc]) : 0.f;
+      sC[i] = in ? to_f32<T>(reinterpret_cast<const T*>(a.C)[bc]) : 0.f;
     }
-    // ---- adjoint recurrence, last step of the chunk first ----
+    __syncthreads();
+#pragma unroll 1
+    for (int nb = 0; nb < kBlocks; ++nb) {
+      const int n0 = nb * 16 + part * 4;
+      float2 h0[2][2], g[2][2];
 #pragma unroll
-    for (int s = kStep - 1; s >= 0; --s) {
-      const int t = t0 + s;
-      if (t >= a.L) continue;   // (uniform over the CTA)
-      const float dl = dls[s], xv = xvs[s], gy = gys[s];
-      float ddl = 0.f, dxv = 0.f;
-      if (part == 0) dD = fmaf(gy, xv, dD);
+      for (int j = 0; j < 2; ++j) {
+        const int d = d0 + o + 32 * j;
+        const int have = d < a.Dc ? max(0, min(4, a.N - n0)) : 0;
+        const int64_t st = ((int64_t(b) * a.chunks + c) * a.Dc + d) * a.N + n0;
+        const float4 hv = load4<float>(a.ckpt + st - int64_t(a.Dc) * a.N, c > 0 ? have : 0, vecn);
+        const float4 gv = load4<float>(a.gck + st, c + 1 < a.chunks ? have : 0, vecn);
+        h0[j][0] = make_float2(hv.x, hv.y);
+        h0[j][1] = make_float2(hv.z, hv.w);
+        g[j][0] = make_float2(gv.x, gv.y);
+        g[j][1] = make_float2(gv.z, gv.w);
+        if constexpr (kBlocks > 1) load_rates<T, 4>(a, d, d < a.Dc, n0, Ar[j]);
+      }
+#pragma unroll 1
+      for (int half = 1; half >= 0; --half) {
+        float2 hs[2][2];                        // the state before the half
 #pragma unroll
-      for (int q = 0; q < kQ; ++q) {
-        const int n = part * kQ + q;
-        // a dead lane (past the last channel) and a state past N carry zeros throughout
-        const float hprev = hs[(s * kN + n) * kCh + ch], hcur = hs[((s + 1) * kN + n) * kCh + ch];
-        const float av = ex2_ss(dl * Ar[q]);
-        const float bt = sB[s * kN + n];
-        g[q] = fmaf(sC[s * kN + n], gy, g[q]);       // dL/dh_t
-        const float da = g[q] * hprev * av;          // dL/d(delta_t A_n), natural units
-        ddl = fmaf(da, Ar[q] * (1.f / kLog2eSs), ddl);
-        dA[q] = fmaf(da, dl, dA[q]);
-        ddl = fmaf(g[q] * bt, xv, ddl);
-        dxv = fmaf(g[q] * dl, bt, dxv);
-        // dB_t, dC_t: sums over the channels
-        if constexpr (kTile) {
-          // this thread's terms go into the chunk's tile; the CTA adds the columns once per chunk (below)
-          ct[((s * 2 + 0) * kN + n) * kCh + ch] = g[q] * dl * xv;
-          ct[((s * 2 + 1) * kN + n) * kCh + ch] = gy * hcur;
-        } else {
-          // the warp's eight channels by shuffles (lanes 4 apart hold the same states), then one atomic each
-          float vb = g[q] * dl * xv, vc = gy * hcur;
+        for (int j = 0; j < 2; ++j) { hs[j][0] = h0[j][0]; hs[j][1] = h0[j][1]; }
+        if (half == 1) {
 #pragma unroll
-          for (int o = 16; o >= kSplit; o >>= 1) {
-            vb += __shfl_xor_sync(0xffffffffu, vb, o);
-            vc += __shfl_xor_sync(0xffffffffu, vc, o);
-          }
-          if (lane < kSplit && n < a.N) {
-            atomicAdd(a.accB + (int64_t(b) * a.L + t) * a.N + n, vb);
-            atomicAdd(a.accC + (int64_t(b) * a.L + t) * a.N + n, vc);
+          for (int s = 0; s < kHalf; ++s) {
+            const float4 Bw = *reinterpret_cast<const float4*>(sB + s * kN + n0);
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+              const float2 w = *reinterpret_cast<const float2*>(dxg + s * kBwdCh + (j ? at1 : at0));
+              const float2 dl = both(w.x), u = both(w.y);
+              hs[j][0] = __ffma2_rn(ex2_ss2(__fmul2_rn(dl, Ar[j][0])), hs[j][0], __fmul2_rn(u, make_float2(Bw.x, Bw.y)));
+              hs[j][1] = __ffma2_rn(ex2_ss2(__fmul2_rn(dl, Ar[j][1])), hs[j][1], __fmul2_rn(u, make_float2(Bw.z, Bw.w)));
+            }
           }
         }
-        g[q] *= av;                                  // dL/dh_{t-1} so far
-      }
-      // dx_t, ddelta_t: sums over the channel's states, i.e. over the four lanes
-      ddl += __shfl_xor_sync(0xffffffffu, ddl, 1);
-      ddl += __shfl_xor_sync(0xffffffffu, ddl, 2);
-      dxv += __shfl_xor_sync(0xffffffffu, dxv, 1);
-      dxv += __shfl_xor_sync(0xffffffffu, dxv, 2);
-      if (a.D) dxv = fmaf(Dd, gy, dxv);
-      if (live && part == 0) {
-        dxp[int64_t(t) * a.Dc] = from_f32<T>(dxv);
-        ddp[int64_t(t) * a.Dc] = from_f32<T>(ddl);
-      }
-    }
-    if constexpr (kTile) {
-      // column sums of the chunk's tile: sum v = (step, B or C, n) over the 64 channels, read with a per-thread skew
-      // so that the threads of a warp hit different banks; then one atomic per sum and CTA
-      __syncthreads();
-      for (int v = tid; v < kStep * 2 * kN; v += kFwdThreads) {
-        const int sv = v / (2 * kN), rest = v - sv * 2 * kN, which = rest / kN, n = rest - which * kN;
-        const int t = t0 + sv;
-        if (n < a.N && t < a.L) {
-          const float* col = ct + v * kCh;
-          float acc = 0.f;
-#pragma unroll 8
-          for (int k = 0; k < kCh; ++k) acc += col[(k + tid) & (kCh - 1)];
-          atomicAdd((which ? a.accC : a.accB) + (int64_t(b) * a.L + t) * a.N + n, acc);
+        float2 av[kHalf][2][2], h[kHalf][2][2];
+        float4 w[kHalf][2];
+        const int sb = half * kHalf;
+#pragma unroll
+        for (int s = 0; s < kHalf; ++s) {
+          const float4 Bw = *reinterpret_cast<const float4*>(sB + (sb + s) * kN + n0);
+          const float2 Bv[2] = {make_float2(Bw.x, Bw.y), make_float2(Bw.z, Bw.w)};
+#pragma unroll
+          for (int j = 0; j < 2; ++j) {
+            w[s][j] = dxg[(sb + s) * kBwdCh + (j ? at1 : at0)];
+            const float2 dl = both(w[s][j].x), u = both(w[s][j].y);
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+              av[s][j][k] = ex2_ss2(__fmul2_rn(dl, Ar[j][k]));
+              h[s][j][k] = __ffma2_rn(av[s][j][k], s ? h[s - 1][j][k] : hs[j][k], __fmul2_rn(u, Bv[k]));
+            }
+          }
+        }
+        __syncthreads();   // (the tile's last sums have been read)
+#pragma unroll
+        for (int s = kHalf - 1; s >= 0; --s) {
+          const float4 Bw = *reinterpret_cast<const float4*>(sB + (sb + s) * kN + n0);
+          const float4 Cw = *reinterpret_cast<const float4*>(sC + (sb + s) * kN + n0);
+          const float2 Bv[2] = {make_float2(Bw.x, Bw.y), make_float2(Bw.z, Bw.w)};
+          const float2 Cv[2] = {make_float2(Cw.x, Cw.y), make_float2(Cw.z, Cw.w)};
+          float2 dB[2], dC[2];
+          float s1[2], s2[2];
+#pragma unroll
+          for (int j = 0; j < 2; ++j) {
+            const float2 dl = both(w[s][j].x), u = both(w[s][j].y), gy = both(w[s][j].z);
+            float2 e1 = make_float2(0.f, 0.f), e2 = make_float2(0.f, 0.f);
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+              const float2 gt = __ffma2_rn(Cv[k], gy, g[j][k]);                                  // dL/dh_t
+              const float2 ga = __fmul2_rn(gt, av[s][j][k]);                                     // dL/dh_{t-1} so far
+              const float2 da = __fmul2_rn(ga, s ? h[s - 1][j][k] : hs[j][k]);                   // dL/d(delta_t A_n)
+              e1 = __ffma2_rn(da, Ar[j][k], e1);
+              dA[j][k] = __ffma2_rn(da, dl, dA[j][k]);
+              e2 = __ffma2_rn(gt, Bv[k], e2);
+              dB[k] = j ? __ffma2_rn(gt, u, dB[k]) : __fmul2_rn(gt, u);
+              dC[k] = j ? __ffma2_rn(gy, h[s][j][k], dC[k]) : __fmul2_rn(gy, h[s][j][k]);
+              g[j][k] = ga;
+            }
+            s1[j] = e1.x + e1.y;
+            s2[j] = e2.x + e2.y;
+          }
+          // a row is one owner's 16 dB and 16 dC terms, the halves swapped in every other row (bank conflicts)
+          float* tr = tile + (s * 32 + o) * 32;
+          *reinterpret_cast<float4*>(tr + part * 4 + (o & 1 ? 16 : 0)) = make_float4(dB[0].x, dB[0].y, dB[1].x, dB[1].y);
+          *reinterpret_cast<float4*>(tr + part * 4 + (o & 1 ? 0 : 16)) = make_float4(dC[0].x, dC[0].y, dC[1].x, dC[1].y);
+          // sums over the states: over the four lanes, each of which ends with one channel and one of the two sums
+          float k1 = hi ? s1[1] : s1[0], k2 = hi ? s2[1] : s2[0];
+          k1 += __shfl_xor_sync(0xffffffffu, hi ? s1[0] : s1[1], 2);
+          k2 += __shfl_xor_sync(0xffffffffu, hi ? s2[0] : s2[1], 2);
+          float r = (lo ? k2 : k1) + __shfl_xor_sync(0xffffffffu, lo ? k1 : k2, 1);
+          float* out = sums + (sb + s) * kSumStep + (lo ? kSumWhich : 0) + o + (hi ? 32 + kSumCol : 0);
+          if (kBlocks > 1 && nb > 0) r += *out;
+          *out = r;
+        }
+        __syncthreads();
+        // column sums of the half's tile: a warp takes one step, a lane four of its 32 columns of eight owners
+        {
+          const int vg = lane & 7, slot = lane >> 3, t = t0 + sb + warp;
+          float2 p0 = make_float2(0.f, 0.f), p1 = make_float2(0.f, 0.f);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const float4 v = *reinterpret_cast<const float4*>(tile + (warp * 32 + slot * 8 + i) * 32 + (vg ^ (i & 1 ? 4 : 0)) * 4);
+            p0 = __fadd2_rn(p0, make_float2(v.x, v.y));
+            p1 = __fadd2_rn(p1, make_float2(v.z, v.w));
+          }
+#pragma unroll
+          for (int m = 8; m < 32; m <<= 1) {
+            p0.x += __shfl_xor_sync(0xffffffffu, p0.x, m);
+            p0.y += __shfl_xor_sync(0xffffffffu, p0.y, m);
+            p1.x += __shfl_xor_sync(0xffffffffu, p1.x, m);
+            p1.y += __shfl_xor_sync(0xffffffffu, p1.y, m);
+          }
+          if (slot == 0 && t < a.L)
+            add_states((vg < 4 ? a.accB : a.accC) + (int64_t(b) * a.L + t) * a.N, nb * 16 + (vg & 3) * 4, a.N, vecn,
+                       make_float4(p0.x, p0.y, p1.x, p1.y));
         }
       }
-      // (the tile is rewritten only after the next chunk's barrier)
+      if constexpr (kBlocks > 1) {
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          float4* slot = sdA + (nb * 2 + j) * kBwdThreads + tid;
+          const float4 was = *slot;
+          *slot = make_float4(was.x + dA[j][0].x, was.y + dA[j][0].y, was.z + dA[j][1].x, was.w + dA[j][1].y);
+          dA[j][0] = dA[j][1] = make_float2(0.f, 0.f);
+        }
+      }
+    }
+    // dx_t = delta_t sum_n g B + D dy_t,  ddelta_t = sum_n g h_{t-1} a A + x_t sum_n g B   (the last barrier above
+    // stands between these sums and their writers)
+    const float* sr = sums + lr * kSumStep + lc + (lc >= 32 ? kSumCol : 0);
+    const float4 v1 = *reinterpret_cast<const float4*>(sr), v2 = *reinterpret_cast<const float4*>(sr + kSumWhich);
+    const float4* own = dxg + lr * kBwdCh;
+    const float4 e0 = own[place(lc)], e1 = own[place(lc + 1)], e2 = own[place(lc + 2)], e3 = own[place(lc + 3)];
+    const float4 dl = make_float4(e0.x, e1.x, e2.x, e3.x), gy = make_float4(e0.z, e1.z, e2.z, e3.z), x = make_float4(e0.w, e1.w, e2.w, e3.w);
+    constexpr float kLn2 = 1.f / kLog2eSs;
+    store4<T>(reinterpret_cast<T*>(a.ddelta) + row,
+              make_float4(fmaf(x.x, v2.x, v1.x * kLn2), fmaf(x.y, v2.y, v1.y * kLn2), fmaf(x.z, v2.z, v1.z * kLn2), fmaf(x.w, v2.w, v1.w * kLn2)), n, vec);
+    float4 dx = make_float4(dl.x * v2.x, dl.y * v2.y, dl.z * v2.z, dl.w * v2.w);
+    if (a.D) {
+      const float4 Dd = load4<T>(reinterpret_cast<const T*>(a.D) + d0 + lc, ln, false);
+      dx = make_float4(fmaf(Dd.x, gy.x, dx.x), fmaf(Dd.y, gy.y, dx.y), fmaf(Dd.z, gy.z, dx.z), fmaf(Dd.w, gy.w, dx.w));
+      dDs = make_float4(fmaf(gy.x, x.x, dDs.x), fmaf(gy.y, x.y, dDs.y), fmaf(gy.z, x.z, dDs.z), fmaf(gy.w, x.w, dDs.w));
+    }
+    store4<T>(reinterpret_cast<T*>(a.dx) + row, dx, n, vec);
+  }
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    const int d = d0 + o + 32 * j;
+    if (d < a.Dc) {
+      if constexpr (kBlocks > 1) {
+        for (int nb = 0; nb < kBlocks; ++nb)
+          add_states(a.accA + int64_t(d) * a.N, nb * 16 + part * 4, a.N, vecn, sdA[(nb * 2 + j) * kBwdThreads + tid]);
+      } else {
+        add_states(a.accA + int64_t(d) * a.N, part * 4, a.N, vecn, make_float4(dA[j][0].x, dA[j][0].y, dA[j][1].x, dA[j][1].y));
+      }
     }
   }
-  if (live) {
-#pragma unroll
-    for (int q = 0; q < kQ; ++q) {
-      const int n = part * kQ + q;
-      if (n < a.N) atomicAdd(a.accA + int64_t(d) * a.N + n, dA[q]);
-    }
-    if (a.accD && part == 0) atomicAdd(a.accD + d, dD);
+  if (a.accD) {
+    // (lanes 16 apart hold two steps of the same channels)
+    dDs.x += __shfl_xor_sync(0xffffffffu, dDs.x, 16);
+    dDs.y += __shfl_xor_sync(0xffffffffu, dDs.y, 16);
+    dDs.z += __shfl_xor_sync(0xffffffffu, dDs.z, 16);
+    dDs.w += __shfl_xor_sync(0xffffffffu, dDs.w, 16);
+    if (lane < 16) add_states(a.accD + d0 + lc, 0, ln, false, dDs);
   }
 }
 
+// The fp32 accumulators in the storage dtype: four arrays in one launch.
+struct SsFinish {
+  const float* src[4];
+  void* dst[4];
+  int64_t n[4];
+};
 template <typename T>
-__global__ void __launch_bounds__(256) ss_finish_kernel(const float* acc, T* out, int64_t n) {
-  const int64_t i = int64_t(blockIdx.x) * 256 + threadIdx.x;
-  if (i < n) out[i] = from_f32<T>(acc[i]);
+__global__ void __launch_bounds__(256) ss_finish_kernel(SsFinish f) {
+  const float* src = f.src[blockIdx.y];
+  T* dst = static_cast<T*>(f.dst[blockIdx.y]);
+  for (int64_t i = int64_t(blockIdx.x) * 256 + threadIdx.x; i < f.n[blockIdx.y]; i += int64_t(gridDim.x) * 256)
+    dst[i] = from_f32<T>(src[i]);
 }
 
-int pick_n(int N) { return N <= 16 ? 16 : (N <= 32 ? 32 : (N <= 64 ? 64 : 0)); }
+int pick_n(int N) { return N <= 8 ? 8 : (N <= 16 ? 16 : (N <= 32 ? 32 : (N <= 64 ? 64 : 0))); }
 
 int check_common(const nb200_selective_scan_params* p, const char* what) {
   if (!p) { set_error("%s: NULL parameter block", what); return NB200_ERR_INVALID; }
@@ -341,78 +667,115 @@ int check_common(const nb200_selective_scan_params* p, const char* what) {
   return NB200_OK;
 }
 
+bool aligned(const void* p, size_t to) { return reinterpret_cast<uintptr_t>(p) % to == 0; }
+
+template <typename T>
 SsArgs args_of(const nb200_selective_scan_params* p) {
   SsArgs a{};
   a.x = p->x; a.delta = p->delta; a.A = p->A; a.B = p->B; a.C = p->C; a.D = p->D; a.dy = p->dy;
   a.y = p->y; a.dx = p->dx; a.ddelta = p->ddelta; a.ckpt = p->checkpoints;
   a.batch = p->batch; a.L = p->length; a.Dc = p->channels; a.N = p->states;
-  a.chunks = (p->length + kStep - 1) / kStep;
+  a.chunks = p->length / kStep + (p->length % kStep != 0);
+  // four channels (states) as one word: every row then starts on that word's boundary, and no group is cut short
+  constexpr size_t kWord = 4 * sizeof(T);
+  a.vec = p->channels % 4 == 0 && aligned(p->x, kWord) && aligned(p->delta, kWord) && aligned(p->y, kWord) &&
+          aligned(p->dy, kWord) && aligned(p->dx, kWord) && aligned(p->ddelta, kWord);
+  a.vecn = p->states % 4 == 0 && aligned(p->B, kWord) && aligned(p->C, kWord) && aligned(p->checkpoints, 16) &&
+           aligned(p->workspace, 16);
   return a;
 }
 
+dim3 scan_grid(const nb200_selective_scan_params* p) {
+  return dim3((p->channels + kScanCh - 1) / kScanCh, p->batch);
+}
 template <typename T>
 int fwd_t(const nb200_selective_scan_params* p, cudaStream_t st) {
-  SsArgs a = args_of(p);
-  dim3 grid((p->channels + kCh - 1) / kCh, p->batch);
+  SsArgs a = args_of<T>(p);
+  const dim3 grid = scan_grid(p);
   switch (pick_n(p->states)) {
-    case 16: ss_fwd_kernel<T, 16><<<grid, kFwdThreads, 0, st>>>(a); break;
-    case 32: ss_fwd_kernel<T, 32><<<grid, kFwdThreads, 0, st>>>(a); break;
-    default: ss_fwd_kernel<T, 64><<<grid, kFwdThreads, 0, st>>>(a); break;
+    case 8: ss_fwd_kernel<T, 8><<<grid, kScanThreads, 0, st>>>(a); break;
+    case 16: ss_fwd_kernel<T, 16><<<grid, kScanThreads, 0, st>>>(a); break;
+    case 32: ss_fwd_kernel<T, 32><<<grid, kScanThreads, 0, st>>>(a); break;
+    default: ss_fwd_kernel<T, 64><<<grid, kScanThreads, 0, st>>>(a); break;
   }
   count_launch();
   return check_launch("selective_scan_fwd_kernel");
 }
 
+// workspace of the backward: the fp32 accumulators, then the adjoint states between the chunks
 size_t acc_floats(const nb200_selective_scan_params* p) {
   return 2 * size_t(p->batch) * p->length * p->states + size_t(p->channels) * p->states + size_t(p->channels);
 }
+size_t ckpt_floats(const nb200_selective_scan_params* p) {
+  return size_t(p->batch) * (p->length / kStep + (p->length % kStep != 0)) * p->states * p->channels;
+}
+size_t acc_bytes(const nb200_selective_scan_params* p) { return (sizeof(float) * acc_floats(p) + 255) / 256 * 256; }
 
-template <typename T, int kN>
+template <typename T, int kBlocks>
 int bwd_launch(const SsArgs& a, dim3 grid, cudaStream_t st) {
-  const size_t smem = sizeof(float) * (size_t(kStep + 1) * kN * kCh + 4 * kStep * kN +
-                                       (kN <= 32 ? size_t(kStep) * 2 * kN * kCh : 0));
+  constexpr size_t smem = kStep * kBwdCh * sizeof(float4) +
+                          sizeof(float) * (2 * kStep * 16 * kBlocks + kHalf * 32 * 32 + kStep * kSumStep) +
+                          (kBlocks > 1 ? sizeof(float4) * kBlocks * 2 * kBwdThreads : 0);
   if (smem > 48 * 1024 &&
-      cudaFuncSetAttribute(ss_bwd_kernel<T, kN>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess) {
+      cudaFuncSetAttribute(ss_bwd_kernel<T, kBlocks>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess) {
     set_error("selective_scan_bwd: cudaFuncSetAttribute(%zu): %s", smem, cudaGetErrorString(cudaGetLastError()));
     return NB200_ERR_LAUNCH;
   }
-  ss_bwd_kernel<T, kN><<<grid, kFwdThreads, smem, st>>>(a);
+  ss_bwd_kernel<T, kBlocks><<<grid, kBwdThreads, smem, st>>>(a);
   count_launch();
   return check_launch("selective_scan_bwd_kernel");
 }
 
 template <typename T>
 int bwd_t(const nb200_selective_scan_params* p, cudaStream_t st) {
-  SsArgs a = args_of(p);
-  const size_t need = sizeof(float) * acc_floats(p);
+  SsArgs a = args_of<T>(p);
+  const size_t need = acc_bytes(p) + sizeof(float) * ckpt_floats(p);
   if (!p->workspace || p->workspace_bytes < need) {
     set_error("selective_scan_bwd: workspace of %zu bytes needed (nb200_selective_scan_workspace_bytes), %zu given",
               need, size_t(p->workspace_bytes));
     return NB200_ERR_WORKSPACE;
   }
   float* acc = static_cast<float*>(p->workspace);
-  if (cudaMemsetAsync(acc, 0, need, st) != cudaSuccess) return check_launch("selective_scan_bwd: clearing the workspace");
+  if (cudaMemsetAsync(acc, 0, sizeof(float) * acc_floats(p), st) != cudaSuccess) return check_launch("selective_scan_bwd: clearing the workspace");
   const size_t bln = size_t(p->batch) * p->length * p->states, dn = size_t(p->channels) * p->states;
   a.accB = acc; a.accC = acc + bln; a.accA = acc + 2 * bln; a.accD = p->D ? acc + 2 * bln + dn : nullptr;
+  a.gck = reinterpret_cast<float*>(static_cast<char*>(p->workspace) + acc_bytes(p));
   if (p->batch > 0 && p->length > 0) {   // (nothing to walk otherwise: dA and dD are the zeros just written)
-    dim3 grid((p->channels + kCh - 1) / kCh, p->batch);
+    if (a.chunks > 1) {
+      const dim3 grid = scan_grid(p);
+      switch (pick_n(p->states)) {
+        case 8: ss_adjoint_kernel<T, 8><<<grid, kScanThreads, 0, st>>>(a); break;
+        case 16: ss_adjoint_kernel<T, 16><<<grid, kScanThreads, 0, st>>>(a); break;
+        case 32: ss_adjoint_kernel<T, 32><<<grid, kScanThreads, 0, st>>>(a); break;
+        default: ss_adjoint_kernel<T, 64><<<grid, kScanThreads, 0, st>>>(a); break;
+      }
+      count_launch();
+      if (int rc = check_launch("selective_scan_adjoint_kernel")) return rc;
+    }
+    // chunks per CTA: as many as leave about eight CTAs for every one that the GPU holds at a time (3 x 148), so that
+    // the last wave is short; at most 16 (a CTA's own start and its sums of dA are spread well enough over those)
+    const int64_t groups = (p->channels + kBwdCh - 1) / kBwdCh;
+    int64_t per = groups * p->batch * a.chunks / (8 * 3 * 148);
+    per = per < 1 ? 1 : (per > 16 ? 16 : per);
+    const int64_t least = (int64_t(a.chunks) + 65534) / 65535;   // (grid.y)
+    a.per_cta = int(per < least ? least : per);
+    const dim3 grid(unsigned(groups), unsigned((a.chunks + a.per_cta - 1) / a.per_cta), unsigned(p->batch));
     int rc;
     switch (pick_n(p->states)) {
-      case 16: rc = bwd_launch<T, 16>(a, grid, st); break;
-      case 32: rc = bwd_launch<T, 32>(a, grid, st); break;
-      default: rc = bwd_launch<T, 64>(a, grid, st); break;
+      case 8:
+      case 16: rc = bwd_launch<T, 1>(a, grid, st); break;
+      case 32: rc = bwd_launch<T, 2>(a, grid, st); break;
+      default: rc = bwd_launch<T, 4>(a, grid, st); break;
     }
     if (rc) return rc;
   }
-  auto finish = [&](const float* src, void* dst, size_t n) {
-    if (!dst || n == 0) return;
-    ss_finish_kernel<T><<<unsigned((n + 255) / 256), 256, 0, st>>>(src, static_cast<T*>(dst), int64_t(n));
-    count_launch();
-  };
-  finish(a.accB, p->dB, bln);
-  finish(a.accC, p->dC, bln);
-  finish(a.accA, p->dA, dn);
-  if (p->D) finish(a.accD, p->dD, size_t(p->channels));
+  SsFinish f{{a.accB, a.accC, a.accA, acc + 2 * bln + dn}, {p->dB, p->dC, p->dA, p->dD},
+             {int64_t(bln), int64_t(bln), int64_t(dn), p->D ? int64_t(p->channels) : 0}};
+  int64_t most = 0;
+  for (int64_t n : f.n) most = n > most ? n : most;
+  const int64_t blocks = (most + 1023) / 1024;
+  ss_finish_kernel<T><<<dim3(unsigned(blocks < 4096 ? blocks : 4096), 4), 256, 0, st>>>(f);
+  count_launch();
   return check_launch("selective_scan_finish_kernel");
 }
 
@@ -424,14 +787,14 @@ using namespace nb200;
 extern "C" NB200_API int nb200_selective_scan_workspace_bytes(const nb200_selective_scan_params* p, size_t* bytes) {
   if (!bytes) { set_error("bytes out-pointer is NULL"); return NB200_ERR_INVALID; }
   if (int rc = check_common(p, "selective_scan_workspace_bytes")) return rc;
-  *bytes = sizeof(float) * acc_floats(p);
+  *bytes = acc_bytes(p) + sizeof(float) * ckpt_floats(p);
   return NB200_OK;
 }
 
 extern "C" NB200_API int nb200_selective_scan_checkpoint_bytes(const nb200_selective_scan_params* p, size_t* bytes) {
   if (!bytes) { set_error("bytes out-pointer is NULL"); return NB200_ERR_INVALID; }
   if (int rc = check_common(p, "selective_scan_checkpoint_bytes")) return rc;
-  *bytes = sizeof(float) * size_t(p->batch) * ((p->length + kStep - 1) / kStep) * p->states * p->channels;
+  *bytes = sizeof(float) * ckpt_floats(p);
   return NB200_OK;
 }
 

@@ -75,3 +75,12 @@ def test_without_the_skip_term_and_with_leading_axes():
 
 def test_projections_shared_over_the_batch_get_summed_gradients():
     _run((3,), 29, 72, 16, torch.float32, shared_bc=True)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("batch,length,d,n", [(8, 17, 1184, 16), (9, 40, 1061, 8), (8, 25, 1177, 5), (37, 9, 256, 12),
+                                              (8, 450, 1030, 16), (8, 450, 1030, 33)])
+def test_ragged_channels_and_states_and_several_chunks_per_cta(batch, length, d, n, dtype):
+    # channel counts that are no multiple of four (scalar loads) and states that are none, up to 8, 16 and 64; CTAs of the
+    # gradients with more than one chunk
+    _run((batch,), length, d, n, dtype)
