@@ -164,6 +164,19 @@ def lib() -> C.CDLL:
     return L
 
 
+def enqueue(fn, params, device) -> int:
+    """``fn(&params, stream)`` on the current stream of ``device`` (a ``torch.device`` with an index), which is made
+    the current device only where it is not already; returns the library's status code."""
+    import torch
+
+    index = device.index
+    stream = torch._C._cuda_getCurrentRawStream(index)   # (torch.cuda.current_stream builds a Stream object: 2 us)
+    if index == torch._C._cuda_getDevice():
+        return fn(C.byref(params), stream)
+    with torch.cuda.device(index):
+        return fn(C.byref(params), stream)
+
+
 def last_error() -> str:
     return lib().nb200_last_error().decode("utf-8", "replace")
 

@@ -103,6 +103,10 @@ def has_sm100_device() -> bool:
     try:
         import torch
 
+        if _sm100_by_device:   # a device has been seen, so the runtime is up: no need to ask for it again
+            known = _sm100_by_device.get(torch._C._cuda_getDevice())
+            if known is not None:
+                return known
         if not torch.cuda.is_available():
             return False
         dev = torch.cuda.current_device()

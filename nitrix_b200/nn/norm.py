@@ -53,9 +53,7 @@ def layer_norm_forward(x2: torch.Tensor, weight, bias, eps: float, out_scale: fl
     p.weight = None if weight is None else weight.data_ptr()
     p.bias = None if bias is None else bias.data_ptr()
     p.y, p.mean, p.rstd = y.data_ptr(), mean.data_ptr(), rstd.data_ptr()
-    with torch.cuda.device(x2.device):
-        _check(_cabi.lib().nb200_layer_norm_fwd(C.byref(p), torch.cuda.current_stream().cuda_stream),
-               "nb200_layer_norm_fwd")
+    _check(_cabi.enqueue(_cabi.lib().nb200_layer_norm_fwd, p, x2.device), "nb200_layer_norm_fwd")
     return y, mean, rstd
 
 
@@ -76,9 +74,7 @@ def layer_norm_backward(x2, weight, dy2, mean, rstd, eps: float, out_scale: floa
         p.workspace, p.workspace_bytes = ws.data_ptr(), int(need.value)
         p.dweight = None if dw is None else dw.data_ptr()
         p.dbias = None if db is None else db.data_ptr()
-    with torch.cuda.device(x2.device):
-        _check(_cabi.lib().nb200_layer_norm_bwd(C.byref(p), torch.cuda.current_stream().cuda_stream),
-               "nb200_layer_norm_bwd")
+    _check(_cabi.enqueue(_cabi.lib().nb200_layer_norm_bwd, p, x2.device), "nb200_layer_norm_bwd")
     return dx, dw, db
 
 

@@ -74,9 +74,7 @@ def selective_scan_forward(x3, delta3, A, B3, C3, D, want_checkpoints: bool):
         n = _bytes(_cabi.lib().nb200_selective_scan_checkpoint_bytes, p)
         ck = torch.empty(max(n // 4, 1), dtype=torch.float32, device=x3.device)
         p.checkpoints = ck.data_ptr()
-    with torch.cuda.device(x3.device):
-        _check(_cabi.lib().nb200_selective_scan_fwd(C.byref(p), torch.cuda.current_stream().cuda_stream),
-               "nb200_selective_scan_fwd")
+    _check(_cabi.enqueue(_cabi.lib().nb200_selective_scan_fwd, p, x3.device), "nb200_selective_scan_fwd")
     return y, ck
 
 
@@ -94,9 +92,7 @@ def selective_scan_backward(x3, delta3, A, B3, C3, D, ck, dy3):
     need = _bytes(_cabi.lib().nb200_selective_scan_workspace_bytes, p)
     ws = torch.empty(max(need, 16), dtype=torch.uint8, device=x3.device)
     p.workspace, p.workspace_bytes = ws.data_ptr(), need
-    with torch.cuda.device(x3.device):
-        _check(_cabi.lib().nb200_selective_scan_bwd(C.byref(p), torch.cuda.current_stream().cuda_stream),
-               "nb200_selective_scan_bwd")
+    _check(_cabi.enqueue(_cabi.lib().nb200_selective_scan_bwd, p, x3.device), "nb200_selective_scan_bwd")
     return dx, ddelta, dA, dB, dC, dD
 
 
