@@ -6,7 +6,7 @@
 // src/nitrix/nn/attention/_reference.py:52-77, y = x * rsqrt(mean(x^2) + 1e-6), no learnable scale, fp32
 // accumulation).  Here the pre-op keeps that place in the call sequence -- so the attention kernels and their
 // gradients are untouched -- but costs one read and one write per tensor instead of a chain of element-wise passes:
-// one warp per row, 16-byte loads, the row held in registers between the reduction and the scaling.
+// 16-byte loads, a row held in registers between the reduction and the scaling.
 //
 //   forward   y = x r,                       r = rsqrt(mean(x^2) + eps)
 //   gradient  dx = r (g - y mean(g y))       (exact, eps included: dr/dx_i = -r^3 x_i / D)
@@ -26,6 +26,7 @@ struct NormTensor {
   int64_t xs[3];      // element strides of x over (b, h, n)
   int H, N;
   int64_t rows;       // B * H * N
+  int dense;          // x is dense [rows][D] as well
 };
 
 template <typename T>
@@ -45,73 +46,88 @@ __device__ __forceinline__ __nv_bfloat16 from_f<__nv_bfloat16>(float v) { return
 template <>
 __device__ __forceinline__ __half from_f<__half>(float v) { return __float2half_rn(v); }
 
-__device__ __forceinline__ float warp_sum(float v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
+// A group of `kLanes` lanes (the power of two that covers a row with 16 bytes a lane, or two words of 16 bytes at fp32 and
+// head dims above 128) takes kRowsAhead rows, all of whose loads are issued before the first is used; the two tensors
+// have their own ranges of CTAs.  Bound by HBM.  One row per warp, whatever its length, left half of the lanes idle at
+// bf16 and head dim 128, four 64-bit divisions in front of a single load per lane, and took 40 us for the 85 MB of
+// (8, 16, 197 + 1111, 128).
+constexpr int kRowsAhead = 4;
+constexpr int kNormThreads = 256;
 
-// One warp per row; a lane holds kPer consecutive-by-32 chunks of kVec elements (16 bytes each).  D <= 32 * kVec * kPer.
-template <typename T, bool kGrad>
-__global__ void __launch_bounds__(256) qk_rms_norm_kernel(NormTensor a, NormTensor b, int D) {
+template <typename T, bool kGrad, int kLanes>
+__global__ void __launch_bounds__(kNormThreads) qk_rms_norm_kernel(NormTensor a, NormTensor b, int D, unsigned blocks_a) {
   constexpr int kVec = 16 / int(sizeof(T));
-  constexpr int kPer = sizeof(T) == 4 ? 2 : 1;     // head dims up to 256
-  const int lane = threadIdx.x & 31;
-  const int64_t row_all = int64_t(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  const bool second = row_all >= a.rows;
+  constexpr int kPer = sizeof(T) == 4 && kLanes == 32 ? 2 : 1;     // head dims up to 256
+  constexpr int kGroups = kNormThreads / kLanes;
+  const bool second = blockIdx.x >= blocks_a;
   const NormTensor& t = second ? b : a;
-  const int64_t row = second ? row_all - a.rows : row_all;
-  if (row >= t.rows) return;
-  const int64_t n = row % t.N, bh = row / t.N;
-  const int64_t h = bh % t.H, bb = bh / t.H;
-  const T* x = reinterpret_cast<const T*>(t.x) + bb * t.xs[0] + h * t.xs[1] + n * t.xs[2];
-  float xv[kPer][kVec], gv[kPer][kVec];
-  float ss = 0.f;
+  const int lane = threadIdx.x % kLanes, group = threadIdx.x / kLanes;
+  const int64_t row0 = int64_t(blockIdx.x - (second ? blocks_a : 0)) * (kGroups * kRowsAhead) + group;
+  uint4 xw[kRowsAhead][kPer], gw[kRowsAhead][kPer];
 #pragma unroll
-  for (int p = 0; p < kPer; ++p) {
-    const int c0 = (p * 32 + lane) * kVec;
-    if (c0 < D) {
-      const uint4 w = *reinterpret_cast<const uint4*>(x + c0);
-      const T* e = reinterpret_cast<const T*>(&w);
-#pragma unroll
-      for (int i = 0; i < kVec; ++i) {
-        xv[p][i] = to_f<T>(e[i]);
-        ss = fmaf(xv[p][i], xv[p][i], ss);
+  for (int r = 0; r < kRowsAhead; ++r) {
+    const int64_t row = row0 + r * kGroups;
+    const T* x = reinterpret_cast<const T*>(t.x);
+    if (row < t.rows) {
+      if (t.dense) {
+        x += row * D;
+      } else {
+        const int64_t bh = row / t.N, n = row - bh * t.N, bb = bh / t.H, h = bh - bb * t.H;
+        x += bb * t.xs[0] + h * t.xs[1] + n * t.xs[2];
       }
-      if constexpr (kGrad) {
-        const uint4 wg = *reinterpret_cast<const uint4*>(reinterpret_cast<const T*>(t.g) + row * D + c0);
-        const T* eg = reinterpret_cast<const T*>(&wg);
+    }
 #pragma unroll
-        for (int i = 0; i < kVec; ++i) gv[p][i] = to_f<T>(eg[i]);
-      }
-    } else {
-#pragma unroll
-      for (int i = 0; i < kVec; ++i) xv[p][i] = gv[p][i] = 0.f;
+    for (int p = 0; p < kPer; ++p) {
+      const int c0 = (p * kLanes + lane) * kVec;
+      const bool in = row < t.rows && c0 < D;
+      xw[r][p] = in ? *reinterpret_cast<const uint4*>(x + c0) : make_uint4(0, 0, 0, 0);
+      if constexpr (kGrad)
+        gw[r][p] = in ? *reinterpret_cast<const uint4*>(reinterpret_cast<const T*>(t.g) + row * D + c0) : make_uint4(0, 0, 0, 0);
     }
   }
-  const float r = rsqrtf(warp_sum(ss) / float(D) + kEps);
-  float m = 0.f;
-  if constexpr (kGrad) {
-    float gy = 0.f;
 #pragma unroll
-    for (int p = 0; p < kPer; ++p)
+  for (int r = 0; r < kRowsAhead; ++r) {
+    const int64_t row = row0 + r * kGroups;
+    float ss = 0.f;
 #pragma unroll
-      for (int i = 0; i < kVec; ++i) gy = fmaf(gv[p][i], xv[p][i] * r, gy);
-    m = warp_sum(gy) / float(D);
-  }
-  T* y = reinterpret_cast<T*>(t.y) + row * D;
+    for (int p = 0; p < kPer; ++p) {
+      const T* e = reinterpret_cast<const T*>(&xw[r][p]);
 #pragma unroll
-  for (int p = 0; p < kPer; ++p) {
-    const int c0 = (p * 32 + lane) * kVec;
-    if (c0 < D) {
-      uint4 w;
-      T* e = reinterpret_cast<T*>(&w);
+      for (int i = 0; i < kVec; ++i) ss = fmaf(to_f<T>(e[i]), to_f<T>(e[i]), ss);
+    }
 #pragma unroll
-      for (int i = 0; i < kVec; ++i) {
-        const float yi = xv[p][i] * r;
-        e[i] = from_f<T>(kGrad ? r * (gv[p][i] - yi * m) : yi);
+    for (int o = kLanes / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    const float rn = rsqrtf(ss / float(D) + kEps);
+    float m = 0.f;
+    if constexpr (kGrad) {
+#pragma unroll
+      for (int p = 0; p < kPer; ++p) {
+        const T* e = reinterpret_cast<const T*>(&xw[r][p]);
+        const T* eg = reinterpret_cast<const T*>(&gw[r][p]);
+#pragma unroll
+        for (int i = 0; i < kVec; ++i) m = fmaf(to_f<T>(eg[i]), to_f<T>(e[i]) * rn, m);
       }
-      *reinterpret_cast<uint4*>(y + c0) = w;
+#pragma unroll
+      for (int o = kLanes / 2; o > 0; o >>= 1) m += __shfl_xor_sync(0xffffffffu, m, o);
+      m /= float(D);
+    }
+    if (row >= t.rows) continue;
+    T* y = reinterpret_cast<T*>(t.y) + row * D;
+#pragma unroll
+    for (int p = 0; p < kPer; ++p) {
+      const int c0 = (p * kLanes + lane) * kVec;
+      if (c0 < D) {
+        const T* e = reinterpret_cast<const T*>(&xw[r][p]);
+        const T* eg = reinterpret_cast<const T*>(&gw[r][p]);
+        uint4 w;
+        T* out = reinterpret_cast<T*>(&w);
+#pragma unroll
+        for (int i = 0; i < kVec; ++i) {
+          const float yi = to_f<T>(e[i]) * rn;
+          out[i] = from_f<T>(kGrad ? rn * (to_f<T>(eg[i]) - yi * m) : yi);
+        }
+        *reinterpret_cast<uint4*>(y + c0) = w;
+      }
     }
   }
 }
@@ -132,7 +148,29 @@ int check(const nb200_qk_norm_tensor& t, int D, int dtype, bool grad, const char
   out->x = t.x; out->g = t.g; out->y = t.y;
   for (int i = 0; i < 3; ++i) out->xs[i] = t.xs[i];
   out->H = t.H; out->N = t.N;
+  // (the stride of an axis of one element says nothing)
+  out->dense = (t.N == 1 || t.xs[2] == D) && (t.H == 1 || t.xs[1] == int64_t(t.N) * D) &&
+               (t.B == 1 || t.xs[0] == int64_t(t.H) * t.N * D);
   return NB200_OK;
+}
+
+template <typename T, bool kGrad, int kLanes>
+int launch_lanes(const NormTensor& a, const NormTensor& b, int D, cudaStream_t st) {
+  constexpr int64_t kRows = kNormThreads / kLanes * kRowsAhead;     // rows of a CTA
+  const int64_t blocks_a = (a.rows + kRows - 1) / kRows, blocks = blocks_a + (b.rows + kRows - 1) / kRows;
+  if (blocks > 0x7fffffff) { set_error("qk_rms_norm: too many rows"); return NB200_ERR_UNSUPPORTED; }
+  qk_rms_norm_kernel<T, kGrad, kLanes><<<unsigned(blocks), kNormThreads, 0, st>>>(a, b, D, unsigned(blocks_a));
+  count_launch();
+  return check_launch(kGrad ? "qk_rms_norm_grad_kernel" : "qk_rms_norm_kernel");
+}
+
+template <typename T, bool kGrad>
+int launch_typed(const NormTensor& a, const NormTensor& b, int D, cudaStream_t st) {
+  const int words = D / (16 / int(sizeof(T)));
+  if (words <= 4) return launch_lanes<T, kGrad, 4>(a, b, D, st);
+  if (words <= 8) return launch_lanes<T, kGrad, 8>(a, b, D, st);
+  if (words <= 16) return launch_lanes<T, kGrad, 16>(a, b, D, st);
+  return launch_lanes<T, kGrad, 32>(a, b, D, st);
 }
 
 template <bool kGrad>
@@ -149,15 +187,11 @@ int launch(const nb200_qk_norm_tensor* q, const nb200_qk_norm_tensor* k, int D, 
   if (int rc = check(*k, D, dtype, kGrad, "k", &b)) return rc;
   const int64_t rows = a.rows + b.rows;
   if (rows == 0) return NB200_OK;
-  const int64_t blocks = (rows + 7) / 8;
-  if (blocks > 0x7fffffff) { set_error("qk_rms_norm: too many rows"); return NB200_ERR_UNSUPPORTED; }
   cudaStream_t st = static_cast<cudaStream_t>(cuda_stream);
   prof_call_begin(st);
-  if (dtype == NB200_F32) qk_rms_norm_kernel<float, kGrad><<<unsigned(blocks), 256, 0, st>>>(a, b, D);
-  else if (dtype == NB200_BF16) qk_rms_norm_kernel<__nv_bfloat16, kGrad><<<unsigned(blocks), 256, 0, st>>>(a, b, D);
-  else qk_rms_norm_kernel<__half, kGrad><<<unsigned(blocks), 256, 0, st>>>(a, b, D);
-  count_launch();
-  return check_launch(kGrad ? "qk_rms_norm_grad_kernel" : "qk_rms_norm_kernel");
+  if (dtype == NB200_F32) return launch_typed<float, kGrad>(a, b, D, st);
+  if (dtype == NB200_BF16) return launch_typed<__nv_bfloat16, kGrad>(a, b, D, st);
+  return launch_typed<__half, kGrad>(a, b, D, st);
 }
 
 }  // namespace
