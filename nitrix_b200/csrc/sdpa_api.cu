@@ -365,7 +365,11 @@ NB200_API int nb200_sdpa_workspace_bytes(const nb200_sdpa_params* p, int pass, s
   if (int rc = lower(p, pass, &lw)) return rc;
   int kernel = 0;
   if (int rc = choose(p, lw, pass, &kernel)) return rc;
-  const size_t fam = kernel == NB200_KERNEL_TCGEN05 ? tc_workspace_bytes(lw.pr, lw.dtype, lw.bias_dtype, pass) : 0;
+  size_t fam = kernel == NB200_KERNEL_TCGEN05 ? tc_workspace_bytes(lw.pr, lw.dtype, lw.bias_dtype, pass) : 0;
+  if (kernel == NB200_KERNEL_SIMT && lw.dtype == NB200_F32) {
+    if (pass == NB200_PASS_FWD && fp32_tc_fwd_applies(lw.pr)) fam = fp32_tc_fwd_bytes(lw.pr);
+    if (pass == NB200_PASS_BWD && fp32_tc_bwd_applies(lw.pr)) fam = fp32_tc_bwd_bytes(lw.pr);
+  }
   *bytes = pass == NB200_PASS_FWD ? align_up(fam) : bwd_scratch(p, lw, fam).total;
   return NB200_OK;
 }
@@ -407,6 +411,10 @@ NB200_API int nb200_sdpa_fwd(const nb200_sdpa_params* p, void* cuda_stream) {
     }
     return tc_forward(lw.pr, lw.dtype, lw.bias_dtype, p->workspace, p->workspace_bytes, st);
   }
+  // (optional: a caller without this workspace gets the kernels that need none)
+  if (lw.dtype == NB200_F32 && fp32_tc_fwd_applies(lw.pr) && p->workspace &&
+      p->workspace_bytes >= fp32_tc_fwd_bytes(lw.pr) && reinterpret_cast<uintptr_t>(p->workspace) % kAlign == 0)
+    return fp32_tc_forward(lw.pr, lw.bias_dtype, p->workspace, st);
   return simt_forward(lw.pr, lw.dtype, lw.bias_dtype, st);
 }
 
@@ -453,6 +461,9 @@ NB200_API int nb200_sdpa_bwd(const nb200_sdpa_params* p, void* cuda_stream) {
   int rc;
   if (kernel == NB200_KERNEL_TCGEN05)
     rc = tc_backward(pr, lw.dtype, lw.bias_dtype, ws + sc.family_off, fam, st);
+  else if (lw.dtype == NB200_F32 && fp32_tc_bwd_applies(pr) &&
+           p->workspace_bytes >= bwd_scratch(p, lw, fp32_tc_bwd_bytes(pr)).total)   // (optional, as in the forward)
+    rc = fp32_tc_backward(pr, lw.bias_dtype, ws + sc.family_off, st);
   else
     rc = simt_backward(pr, lw.dtype, lw.bias_dtype, st);
   if (rc) return rc;

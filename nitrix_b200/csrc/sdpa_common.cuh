@@ -98,6 +98,14 @@ int simt_backward(const Problem& pr, int dtype, int bias_dtype, cudaStream_t str
 // True when this family runs the problem's `pass` on its 3 x TF32 mma.sync kernels (fp32 operands) rather than on
 // plain FMA units.
 bool simt_family_uses_tensor_path(const Problem& pr, int dtype, int pass);
+// fp32 operands on the tcgen05 kernels (sdpa_fp32_tc.cu), as three bf16 planes in `bytes` of workspace (256-byte aligned).
+// A caller that brings no workspace runs on the kernels above, which need none.
+bool fp32_tc_fwd_applies(const Problem& pr);
+size_t fp32_tc_fwd_bytes(const Problem& pr);
+int fp32_tc_forward(const Problem& pr, int bias_dtype, void* ws, cudaStream_t stream);
+bool fp32_tc_bwd_applies(const Problem& pr);
+size_t fp32_tc_bwd_bytes(const Problem& pr);
+int fp32_tc_backward(const Problem& pr, int bias_dtype, void* ws, cudaStream_t stream);
 // delta = rowsum(out*dout) and, when dbias_accum is used, its zero-fill / final cast
 int launch_delta(const Problem& pr, int dtype, cudaStream_t stream);
 int launch_dbias_finish(const float* accum, void* dbias, int bias_dtype, const int64_t extent[4],

@@ -1,0 +1,140 @@
+"""fp32 attention on the tcgen05 kernels (three bf16 planes per operand, six products): forward and every gradient against
+a restatement in fp64 on the device, at the sizes where the kernels can go wrong.
+
+Bound: dropped products < 2^-23; the tensor core truncates each of the 24 accumulations of a 64-key step (2^-23 of the
+sum so far at most) and the accumulators are emptied every other step: 48 * 2^-23 = 5.7e-6 of the result if every
+truncation were a whole ulp, half of that on average; ex2 adds 2^-22.  So 6e-6 in the 2-norm.
+"""
+import ctypes as C
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+_BOUND = 6e-6
+
+
+def _reference(q, k, v, bias, mask, causal, scale, dout):
+    q, k, v, dout = (t.double() for t in (q, k, v, dout))
+    s = q @ k.transpose(-1, -2) * scale
+    if bias is not None:
+        s = s + bias.double()
+    if mask is not None:
+        s = s.masked_fill(~mask, -math.inf)
+    if causal:
+        s = s.masked_fill(torch.ones(s.shape[-2:], device=s.device, dtype=torch.bool).triu(1), -math.inf)
+    p = s.softmax(-1)
+    out = p @ v
+    ds = p * (dout @ v.transpose(-1, -2) - (out * dout).sum(-1, keepdim=True))
+    dbias = None
+    if bias is not None:
+        dbias = ds
+        for a, n in enumerate(bias.shape):
+            if n == 1 and ds.shape[a] != 1:
+                dbias = dbias.sum(a, keepdim=True)
+    return out, ds @ k * scale, ds.transpose(-1, -2) @ q * scale, p.transpose(-1, -2) @ dout, dbias
+
+
+def _err(a, b):
+    return float((a.double() - b).norm() / b.norm())
+
+
+def _layout(t, kind):
+    if kind == "bshd":        # a (B, S, H, D) buffer seen as (B, H, S, D)
+        return t.transpose(1, 2).contiguous().transpose(1, 2)
+    if kind == "odd":         # rows of D + 1 floats, starting one float in: no 16-byte loads
+        b = torch.zeros(t.shape[:-1] + (t.shape[-1] + 1,), device=t.device)
+        b[..., 1:] = t
+        return b[..., 1:]
+    return t
+
+
+@pytest.mark.parametrize("B,H,S,T,D,causal,bias,mask,layout", [
+    (4, 32, 64, 256, 64, False, None, None, "dense"),        # one 64-row tile per (b, h), even steps
+    (4, 48, 65, 321, 64, False, None, None, "bshd"),         # a second tile of one row; an odd last step of one key
+    (2, 64, 300, 130, 64, False, None, None, "odd"),         # second CTA of one query tile; three steps
+    (3, 40, 257, 257, 64, True, None, None, "dense"),        # causal over CTAs of two tiles
+    (2, 100, 200, 500, 32, False, None, None, "dense"),      # head dim padded to the 64 columns
+    (2, 60, 330, 200, 32, True, "full", "key", "bshd"),      # causal with more queries than keys
+    (4, 50, 130, 333, 64, False, "full", "full", "dense"),   # ragged bias and mask
+    (4, 50, 130, 333, 64, False, "shared", None, "dense"),   # fp32 sums over the batch
+    (4, 50, 130, 333, 64, True, "key", "key", "dense"),      # neither has a query axis
+    (4, 50, 190, 320, 64, False, "bf16", None, "dense"),     # a 16-bit bias of fp32 operands
+    (2, 20, 200, 200, 128, False, "full", "full", "dense"),  # head dim 128 (forward)
+    (1, 3, 100, 1111, 128, True, None, None, "odd"),
+])
+def test_against_fp64(B, H, S, T, D, causal, bias, mask, layout):
+    from nitrix_b200 import _cabi
+    from nitrix_b200.nn import attention as att
+
+    g = torch.Generator(device="cuda").manual_seed(B * 1000 + S)
+    q, k, v, dout = (torch.randn(B, H, n, D, device="cuda", generator=g) for n in (S, T, T, S))
+    q, k, v, dout = (_layout(t, layout) for t in (q, k, v, dout))
+    shape = {"full": (B, H, S, T), "shared": (1, H, S, T), "key": (1, H, 1, T), "bf16": (B, H, S, T)}
+    bias_t = None if bias is None else torch.randn(shape[bias], device="cuda", generator=g)
+    if bias == "bf16":
+        bias_t = bias_t.bfloat16()
+    mask_t = None
+    if mask is not None:
+        mask_t = torch.rand((B, 1, S if mask == "full" else 1, T), device="cuda", generator=g) > 0.2
+        mask_t[..., 0] = True
+    scale = 1.0 / math.sqrt(D)
+    L = _cabi.lib()
+    L.nb200_profile(1)
+    out, lse = att.sdpa_forward(q, k, v, bias_t, mask_t, scale=scale, causal=causal)
+    grads = att.sdpa_backward(q, k, v, bias_t, mask_t, out, lse, dout, scale=scale, causal=causal, want_dbias=bias is not None)
+    torch.cuda.synchronize()
+    ran = set(_cabi.kernel_times())
+    L.nb200_profile(0)
+    assert L.nb200_device_status(0) == 0, _cabi.last_error()
+    assert "fwd_fp32_tc_kernel" in ran, ran
+    tc_backward = D < 128 and min(S, T) > 64
+    assert ("bwd_dkv_fp32_tc_kernel" in ran) == tc_backward, ran
+    want = _reference(q, k, v, bias_t, mask_t, causal, scale, dout)
+    assert _err(out, want[0]) <= _BOUND
+    for name, a, r in zip(("dq", "dk", "dv", "dbias"), grads, want[1:]):
+        if r is not None:
+            # (a 16-bit dbias is rounded on the way out; the kernels of other paths have the fp32 budget of 1e-4)
+            assert _err(a, r) <= (5e-3 if a.dtype != torch.float32 else (_BOUND if tc_backward else 1e-4)), name
+
+
+def test_rows_without_a_kept_key_are_nan_and_leave_the_others_alone():
+    from nitrix_b200.nn import attention as att
+
+    g = torch.Generator(device="cuda").manual_seed(3)
+    q, k, v = (torch.randn(4, 50, 130, 64, device="cuda", generator=g) for _ in range(3))
+    k, v = (torch.cat([t, t, t], 2).contiguous() for t in (k, v))
+    mask = torch.ones(4, 1, 130, 390, device="cuda", dtype=torch.bool)
+    mask[:, :, 5] = False
+    out, lse = att.sdpa_forward(q, k, v, None, mask, scale=0.125)
+    assert out[:, :, 5].isnan().all() and (lse[:, :, 5] == -math.inf).all()
+    keep = [i for i in range(130) if i != 5]
+    want = (q.double() @ k.double().transpose(-1, -2) * 0.125).softmax(-1) @ v.double()
+    assert _err(out[:, :, keep], want[:, :, keep]) <= _BOUND
+
+
+def test_without_workspace_the_other_kernels_run():
+    """The workspace is optional: a C caller that brings none (the query answered 0 bytes before these kernels existed)
+    gets the mma.sync kernels, forward and backward."""
+    from nitrix_b200 import _cabi
+    from nitrix_b200.nn import attention as att
+
+    g = torch.Generator(device="cuda").manual_seed(4)
+    q, k, v, dout = (torch.randn(4, 50, 200, 64, device="cuda", generator=g) for _ in range(4))
+    want = _reference(q, k, v, None, None, False, 0.125, dout)
+    out, lse = torch.empty_like(q), torch.empty(4, 50, 200, device="cuda")
+    p = _cabi.new_params()
+    att._fill_common(p, q, k, v, out, lse, None, None, 0.125, False, _cabi.KERNEL_AUTO, None)
+    L, stream = _cabi.lib(), torch.cuda.current_stream().cuda_stream
+    assert L.nb200_sdpa_fwd(C.byref(p), stream) == _cabi.OK, _cabi.last_error()
+    dq, dk, dv = (torch.empty_like(q) for _ in range(3))
+    p.dout, p.dq, p.dk, p.dv = (t.data_ptr() for t in (dout, dq, dk, dv))
+    p.dout_stride[:] = p.dq_stride[:] = p.dk_stride[:] = p.dv_stride[:] = list(q.stride())
+    ws = torch.empty(4 * 50 * 200 * 4 + 256, dtype=torch.uint8, device="cuda")     # delta alone
+    p.workspace, p.workspace_bytes = ws.data_ptr(), ws.numel()
+    assert L.nb200_sdpa_bwd(C.byref(p), stream) == _cabi.OK, _cabi.last_error()
+    torch.cuda.synchronize()
+    for a, r in zip((out, dq, dk, dv), want):
+        assert _err(a, r) <= 1e-4
