@@ -33,6 +33,9 @@ struct Problem {
   void* dbias;
   float* delta;        // (B,H,S) fp32 scratch: rowsum(out * dout)
   float* dbias_accum;  // fp32 scratch of bias' own (un-broadcast) extent, or null
+  // its rows in blocks of 32, its keys in groups of four, [row / 32][key / 4][row % 32][key % 4] (tensor-core kernels, a
+  // bias with a query and a key axis): the number of key groups, T / 4 rounded up; 0: dense
+  int dbias_groups;
   int64_t qs[3], ks[3], vs[3], os[3], dos[3], dqs[3], dks[3], dvs[3];  // b, h, row
   int64_t bs[4], ms[4], dbs[4];                                          // b, h, row, col
   float scale;
@@ -108,7 +111,7 @@ size_t fp32_tc_bwd_bytes(const Problem& pr);
 int fp32_tc_backward(const Problem& pr, int bias_dtype, void* ws, cudaStream_t stream);
 // delta = rowsum(out*dout) and, when dbias_accum is used, its zero-fill / final cast
 int launch_delta(const Problem& pr, int dtype, cudaStream_t stream);
-int launch_dbias_finish(const float* accum, void* dbias, int bias_dtype, const int64_t extent[4],
+int launch_dbias_finish(const float* accum, int groups, void* dbias, int bias_dtype, const int64_t extent[4],
                         const int64_t stride[4], cudaStream_t stream);
 
 

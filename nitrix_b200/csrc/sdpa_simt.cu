@@ -1538,17 +1538,19 @@ __global__ void __launch_bounds__(kWarps * 32) simt_bwd_dkv_kernel(Problem pr, i
   }
 }
 
-// dbias_accum (fp32, dense over bias' own extent) -> dbias in bias dtype
-__global__ void dbias_finish_kernel(const float* accum, void* dbias, int bias_dtype, int64_t n,
+// dbias_accum (fp32, dense over bias' own extent, or its tiles blocked: Problem::dbias_groups) -> dbias in bias dtype
+__global__ void dbias_finish_kernel(const float* accum, int groups, void* dbias, int bias_dtype, int64_t n,
                                     int64_t e1, int64_t e2, int64_t e3, int64_t s0, int64_t s1,
                                     int64_t s2, int64_t s3) {
+  const int64_t tile = groups ? (e2 + 31) / 32 * groups * 128 : e2 * e3;
   for (int64_t idx = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; idx < n;
        idx += int64_t(gridDim.x) * blockDim.x) {
     int64_t r = idx;
     const int64_t i3 = r % e3; r /= e3;
     const int64_t i2 = r % e2; r /= e2;
+    const int64_t at = r * tile + (groups ? ((i2 >> 5) * groups + (i3 >> 2)) * 128 + (i2 & 31) * 4 + (i3 & 3) : i2 * e3 + i3);
     const int64_t i1 = r % e1; r /= e1;
-    store_from_f32(dbias, r * s0 + i1 * s1 + i2 * s2 + i3 * s3, bias_dtype, accum[idx]);
+    store_from_f32(dbias, r * s0 + i1 * s1 + i2 * s2 + i3 * s3, bias_dtype, accum[at]);
   }
 }
 
@@ -1969,14 +1971,14 @@ int launch_delta(const Problem& pr, int dtype, cudaStream_t st) {
   return check_launch("delta_kernel");
 }
 
-int launch_dbias_finish(const float* accum, void* dbias, int bias_dtype, const int64_t e[4],
+int launch_dbias_finish(const float* accum, int groups, void* dbias, int bias_dtype, const int64_t e[4],
                         const int64_t stride[4], cudaStream_t st) {
   const int64_t n = e[0] * e[1] * e[2] * e[3];
   if (n <= 0) return NB200_OK;
   const int threads = 256;
   const int64_t want = (n + threads - 1) / threads;
   const int blocks = int(want < 148 * 8 ? want : 148 * 8);
-  dbias_finish_kernel<<<blocks, threads, 0, st>>>(accum, dbias, bias_dtype, n, e[1], e[2], e[3], stride[0],
+  dbias_finish_kernel<<<blocks, threads, 0, st>>>(accum, groups, dbias, bias_dtype, n, e[1], e[2], e[3], stride[0],
                                                   stride[1], stride[2], stride[3]);
   count_launch();
   return check_launch("dbias_finish_kernel");

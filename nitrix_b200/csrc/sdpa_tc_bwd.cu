@@ -582,7 +582,8 @@ sdpa_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_const
     if (kKeyMajor && !kMerged && a.dbias_acc) *key_ds_sum = 0.f;
     float* acc_row = nullptr;                    // query-major, broadcast tile bias: this query's accumulator row
     if (!kKeyMajor && a.dbias_acc && orow < a.S)
-      acc_row = a.dbias_acc + b * a.acc_s[0] + h * a.acc_s[1] + int64_t(orow) * a.acc_s[2];
+      acc_row = a.dbias_acc + b * a.acc_s[0] + h * a.acc_s[1] +
+                (a.acc_groups ? int64_t(orow >> 5) * a.acc_groups * 128 + (orow & 31) * 4 : int64_t(orow) * a.acc_s[2]);
     const bool acc_vec = (a.T & 3) == 0;
     // merged: pair j of steps (2j, 2j + 1) leaves a 128-query x 64 dq tile in TMEM; this group adds its 32 columns
     // of it to the fp32 accumulator in global memory (thread = query row)
@@ -739,7 +740,10 @@ sdpa_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_const
         if constexpr (!kKeyMajor) {
           // broadcast bias: this row's ds of four consecutive keys joins the fp32 sums over the broadcast axes
           if (acc_row && r0 + 4 * c4 < a.T) {
-            if (acc_vec) {
+            if (a.acc_groups) {   // (keys past T in the last group are dropped keys: their ds is not read by anyone)
+              red_add_v4(acc_row + int64_t((r0 >> 2) + c4) * 128, __float_as_uint(ds4[0].x), __float_as_uint(ds4[0].y),
+                         __float_as_uint(ds4[1].x), __float_as_uint(ds4[1].y));
+            } else if (acc_vec) {
               red_add_v4(acc_row + r0 + 4 * c4, __float_as_uint(ds4[0].x), __float_as_uint(ds4[0].y),
                          __float_as_uint(ds4[1].x), __float_as_uint(ds4[1].y));
             } else {   // key count not a multiple of 4: rows of the accumulator are not 16-byte aligned
@@ -1139,6 +1143,7 @@ int launch_bwd(const Problem& pr, int dtype, int bias_dtype, void* ws, size_t ws
       if (a.bias_mode == kBiasTile) {
         aq.dbias_acc = pr.dbias_accum;
         for (int i = 0; i < 3; ++i) aq.acc_s[i] = pr.dbs[i];
+        aq.acc_groups = pr.dbias_groups;
       }
     } else {
       aq.dbias = pr.dbias;

@@ -41,7 +41,9 @@ struct BwdArgs {
   // stride).  A bias with a query axis is summed by the query-major kernel (ds tiles added with 16-byte
   // reductions), a per-key bias by the key-major kernel (each thread sums its key's ds over the queries it
   // streams and adds once).
-  float* dbias_acc; int64_t acc_s[3];
+  // acc_groups > 0: the accumulator's tiles are blocked (Problem::dbias_groups), so that a warp's reduction of four keys
+  // of 32 rows covers 512 contiguous bytes; acc_s[2] is not used then.
+  float* dbias_acc; int64_t acc_s[3]; int acc_groups;
   float* dq_acc;                // one-kernel backwards: fp32 sums of ds K, zero on entry (layout: see the kernels)
   int acc_rows;                 // head dim 128: rows of the dq accumulator per (batch, head) (S rounded up to 64)
   int* status;
