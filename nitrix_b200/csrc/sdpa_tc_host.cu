@@ -425,6 +425,11 @@ bool tc_supported(const Problem& original, int dtype, int bias_dtype, int pass, 
   const Problem pr = tc::staged_view(original, sg, nullptr);
   if (dtype != NB200_BF16 && dtype != NB200_F16) { *why = "dtype is not bf16/fp16"; return false; }
   if (pr.D != pr.Dv || (pr.D != 64 && pr.D != 128)) { *why = "head dims must be equal and 64 or 128"; return false; }
+  // (the kernels' sums over broadcast axes have one element per key; a bias without a key axis has one per query)
+  if (pass == NB200_PASS_BWD && original.bias && original.want_dbias && original.T > 1 && original.bs[3] == 0) {
+    *why = "gradient of a bias that is broadcast over the keys";
+    return false;
+  }
   // Lengths need not fill whole 128-row tiles, nor be multiples of anything: TMA zero-fills rows past the end, the
   // kernels mask keys past T and store only rows below S, and the operands with 16-byte row segments (bias, dbias,
   // lse, delta) are staged through padded copies when the lengths leave those segments ragged.

@@ -259,6 +259,31 @@ def test_backward_plan_takes_want_dbias_without_a_buffer():
     assert n0 >= delta + 2 * 4 * 256 * 128 * 4    # without dbias: delta rows + the one-kernel backward's fp32 dq sums
 
 
+def test_gradient_of_a_bias_without_a_key_axis_is_left_to_the_cuda_core_kernels():
+    """A (H, S, 1) bias: its forward stays on the tensor cores (a padded copy spreads it over the keys), its gradient
+    does not -- the tensor-core kernels add one sum per key, past the end of an accumulator with one per query."""
+    from nitrix_b200 import _cabi
+
+    def plan(which, want):
+        p = _cabi.new_params()
+        p.dtype = p.bias_dtype = _cabi.BF16
+        p.B, p.H, p.S, p.T, p.D, p.Dv = 2, 4, 256, 256, 64, 64
+        for f in ("q", "k", "v", "out", "lse", "dout", "dq", "dk", "dv", "bias"):
+            setattr(p, f, 0x1000)
+        for f in ("q_stride", "k_stride", "v_stride", "out_stride", "dout_stride", "dq_stride", "dk_stride", "dv_stride"):
+            getattr(p, f)[:] = [4 * 256 * 64, 256 * 64, 64, 1]
+        p.bias_stride[:] = [0, 256, 1, 0]
+        p.dbias_stride[:] = [4 * 256, 256, 1, 1]
+        p.scale, p.bh_end, p.want_dbias = 0.1, 8, want
+        kernel = C.c_int(0)
+        assert _cabi.lib().nb200_sdpa_plan(C.byref(p), which, C.byref(kernel)) == _cabi.OK, _cabi.last_error()
+        return kernel.value
+
+    assert plan(_cabi.PASS_FWD, 0) == _cabi.KERNEL_TCGEN05
+    assert plan(_cabi.PASS_BWD, 0) == _cabi.KERNEL_TCGEN05
+    assert plan(_cabi.PASS_BWD, 1) == _cabi.KERNEL_SIMT
+
+
 def test_jax_ffi_layer_is_complete_and_consistent():
     """The JAX binding cannot run here (no jax, no XLA FFI headers); it must at least compile as Python, import
     without jax, and agree with the C++ shim on the handler symbols and attribute names, and the shim must use
