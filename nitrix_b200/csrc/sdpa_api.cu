@@ -470,7 +470,9 @@ NB200_API int nb200_sdpa_bwd(const nb200_sdpa_params* p, void* cuda_stream) {
     if (e != cudaSuccess) { set_error("cudaMemsetAsync: %s", cudaGetErrorString(e)); return NB200_ERR_LAUNCH; }
   }
   if (pr.S > 0) {
-    if (int rc = launch_delta(pr, lw.dtype, st)) return rc;
+    size_t dq_off = 0, dq_bytes = 0;
+    if (kernel == NB200_KERNEL_TCGEN05) tc_bwd_dq_region(pr, lw.dtype, &dq_off, &dq_bytes);
+    if (int rc = launch_delta(pr, lw.dtype, ws + sc.family_off + dq_off, dq_bytes, &pr.dq_zeroed, st)) return rc;
   }
   int rc;
   if (kernel == NB200_KERNEL_TCGEN05)

@@ -41,6 +41,7 @@ struct Problem {
   float scale;
   int causal;
   int want_dbias;      // the backward produces a bias gradient (dbias may still be null while planning)
+  int dq_zeroed;       // the tensor-core backward's dq accumulator has been cleared (by the delta kernel)
   int mask_packed;     // 0: byte mask; 1 / 2: `mask` is a buffer made by nb200_mask_pack (2: with the transposed copy)
   int n_out_peers;     // forward: further destinations of every output row (same strides as out)
   void* out_peers[NB200_MAX_OUT_PEERS];
@@ -110,7 +111,8 @@ bool fp32_tc_bwd_applies(const Problem& pr);
 size_t fp32_tc_bwd_bytes(const Problem& pr);
 int fp32_tc_backward(const Problem& pr, int bias_dtype, void* ws, cudaStream_t stream);
 // delta = rowsum(out*dout) and, when dbias_accum is used, its zero-fill / final cast
-int launch_delta(const Problem& pr, int dtype, cudaStream_t stream);
+// `zero_bytes` (a multiple of 16) at `zero` are cleared by the same launch where the row layout allows; *zeroed tells.
+int launch_delta(const Problem& pr, int dtype, void* zero, size_t zero_bytes, int* zeroed, cudaStream_t stream);
 int launch_dbias_finish(const float* accum, int groups, void* dbias, int bias_dtype, const int64_t extent[4],
                         const int64_t stride[4], cudaStream_t stream);
 
@@ -122,6 +124,8 @@ bool tc_supported(const Problem& pr, int dtype, int bias_dtype, int pass, const 
 size_t tc_workspace_bytes(const Problem& pr, int dtype, int bias_dtype, int pass);
 int tc_forward(const Problem& pr, int dtype, int bias_dtype, void* ws, size_t ws_bytes, cudaStream_t stream);
 int tc_backward(const Problem& pr, int dtype, int bias_dtype, void* ws, size_t ws_bytes, cudaStream_t stream);
+// The part of tc_backward's workspace that holds fp32 sums of dq and is zero on entry to its kernels (no bytes: none).
+void tc_bwd_dq_region(const Problem& pr, int dtype, size_t* offset, size_t* bytes);
 // Packing of the byte mask into the tensor-core kernels' bit layout, as a call of its own (nb200_mask_pack).
 size_t tc_mask_pack_bytes(const Problem& pr, bool with_transpose);
 int tc_mask_pack(const Problem& pr, bool with_transpose, void* packed, size_t packed_bytes, cudaStream_t stream);

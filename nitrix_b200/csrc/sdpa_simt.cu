@@ -793,14 +793,18 @@ __global__ void __launch_bounds__(kWarps * 32) delta_kernel(Problem pr) {
 }
 
 // Rows with 16-byte alignment: one 16-byte load of out and of dout per thread, kLanes = Dv / (elements in 16 bytes)
-// threads per row, shuffle reduction inside the group.  Bound by HBM.
+// threads per row, shuffle reduction inside the group.  Bound by HBM.  It also clears the accumulator that the kernel
+// behind it adds dq to (twice the bytes of out): a memset of its own ran as long as this kernel and moved no operand.
 template <typename T, int kLanes>
-__global__ void __launch_bounds__(256) delta_vec_kernel(Problem pr) {
+__global__ void __launch_bounds__(256) delta_vec_kernel(Problem pr, uint4* zero, int64_t zero_words) {
   constexpr int kRows = 256 / kLanes, kVec = 16 / int(sizeof(T));
   const int sub = threadIdx.x % kLanes;
   const int i = blockIdx.x * kRows + threadIdx.x / kLanes;
   const int bh = pr.bh_begin + blockIdx.y;
   const int b = bh / pr.H, h = bh - b * pr.H;
+  for (int64_t w = (int64_t(blockIdx.y) * gridDim.x + blockIdx.x) * 256 + threadIdx.x; w < zero_words;
+       w += int64_t(gridDim.x) * gridDim.y * 256)
+    zero[w] = make_uint4(0u, 0u, 0u, 0u);
   float s = 0.f;
   if (i < pr.S) {
     const T* op = reinterpret_cast<const T*>(pr.out) + b * pr.os[0] + h * pr.os[1] + i * pr.os[2] + sub * kVec;
@@ -1938,7 +1942,8 @@ int simt_backward(const Problem& pr, int dtype, int bias_dtype, cudaStream_t st)
   }
 }
 
-int launch_delta(const Problem& pr, int dtype, cudaStream_t st) {
+int launch_delta(const Problem& pr, int dtype, void* zero, size_t zero_bytes, int* zeroed, cudaStream_t st) {
+  *zeroed = 0;
   if (pr.bh_count <= 0 || pr.S <= 0) return NB200_OK;
   const int vec = dtype == NB200_F32 ? 4 : 8;
   const bool aligned = reinterpret_cast<uintptr_t>(pr.out) % 16 == 0 && reinterpret_cast<uintptr_t>(pr.dout) % 16 == 0 &&
@@ -1947,16 +1952,19 @@ int launch_delta(const Problem& pr, int dtype, cudaStream_t st) {
   if (aligned && (pr.Dv == 64 || pr.Dv == 128 || (pr.Dv == 32 && dtype == NB200_F32))) {
     const int lanes = pr.Dv / vec, rows = 256 / lanes;
     dim3 vgrid((pr.S + rows - 1) / rows, pr.bh_count);
+    uint4* z = static_cast<uint4*>(zero);
+    const int64_t words = int64_t(zero_bytes / 16);
+    *zeroed = 1;
     if (dtype == NB200_F32) {
-      if (lanes == 8) delta_vec_kernel<float, 8><<<vgrid, 256, 0, st>>>(pr);
-      else if (lanes == 16) delta_vec_kernel<float, 16><<<vgrid, 256, 0, st>>>(pr);
-      else delta_vec_kernel<float, 32><<<vgrid, 256, 0, st>>>(pr);
+      if (lanes == 8) delta_vec_kernel<float, 8><<<vgrid, 256, 0, st>>>(pr, z, words);
+      else if (lanes == 16) delta_vec_kernel<float, 16><<<vgrid, 256, 0, st>>>(pr, z, words);
+      else delta_vec_kernel<float, 32><<<vgrid, 256, 0, st>>>(pr, z, words);
     } else if (dtype == NB200_BF16) {
-      if (lanes == 8) delta_vec_kernel<__nv_bfloat16, 8><<<vgrid, 256, 0, st>>>(pr);
-      else delta_vec_kernel<__nv_bfloat16, 16><<<vgrid, 256, 0, st>>>(pr);
+      if (lanes == 8) delta_vec_kernel<__nv_bfloat16, 8><<<vgrid, 256, 0, st>>>(pr, z, words);
+      else delta_vec_kernel<__nv_bfloat16, 16><<<vgrid, 256, 0, st>>>(pr, z, words);
     } else {
-      if (lanes == 8) delta_vec_kernel<__half, 8><<<vgrid, 256, 0, st>>>(pr);
-      else delta_vec_kernel<__half, 16><<<vgrid, 256, 0, st>>>(pr);
+      if (lanes == 8) delta_vec_kernel<__half, 8><<<vgrid, 256, 0, st>>>(pr, z, words);
+      else delta_vec_kernel<__half, 16><<<vgrid, 256, 0, st>>>(pr, z, words);
     }
     count_launch();
     return check_launch("delta_vec_kernel");

@@ -1020,13 +1020,17 @@ bool use_d128(const Problem& pr, int dtype) {
 }
 }  // namespace
 
-size_t bwd_workspace_bytes(const Problem& pr, int dtype, int) {
+void bwd_dq_region(const Problem& pr, int dtype, size_t* offset, size_t* bytes) {
   size_t mask_ws = 0;
   mask_plan_for_pass(pr, true, &mask_ws);
-  size_t bytes = round_up_256(mask_ws);
-  if (use_merged(pr)) bytes += sizeof(float) * size_t(pr.bh_count) * pr.S * pr.D;
-  else if (use_d128(pr, dtype)) bytes += d128_acc_bytes(pr);
-  return bytes;
+  *offset = round_up_256(mask_ws);
+  *bytes = use_merged(pr) ? sizeof(float) * size_t(pr.bh_count) * pr.S * pr.D : (use_d128(pr, dtype) ? d128_acc_bytes(pr) : 0);
+}
+
+size_t bwd_workspace_bytes(const Problem& pr, int dtype, int) {
+  size_t offset = 0, bytes = 0;
+  bwd_dq_region(pr, dtype, &offset, &bytes);
+  return offset + bytes;
 }
 
 int launch_bwd(const Problem& pr, int dtype, int bias_dtype, void* ws, size_t ws_bytes, int ld_rows, cudaStream_t stream) {
@@ -1081,7 +1085,7 @@ int launch_bwd(const Problem& pr, int dtype, int bias_dtype, void* ws, size_t ws
   if (merged) {
     BwdArgs ak = a;
     ak.dq_acc = reinterpret_cast<float*>(static_cast<char*>(ws) + mask_ws);
-    cudaError_t e = cudaMemsetAsync(ak.dq_acc, 0, acc_bytes, stream);
+    cudaError_t e = pr.dq_zeroed ? cudaSuccess : cudaMemsetAsync(ak.dq_acc, 0, acc_bytes, stream);
     if (e != cudaSuccess) { set_error("cudaMemsetAsync: %s", cudaGetErrorString(e)); return NB200_ERR_LAUNCH; }
     ak.out1 = pr.dv;
     ak.out2 = pr.dk;
@@ -1106,7 +1110,7 @@ int launch_bwd(const Problem& pr, int dtype, int bias_dtype, void* ws, size_t ws
     BwdArgs ak = a;
     ak.dq_acc = reinterpret_cast<float*>(static_cast<char*>(ws) + mask_ws);
     ak.acc_rows = (pr.S + kStep - 1) / kStep * kStep;
-    cudaError_t e = cudaMemsetAsync(ak.dq_acc, 0, acc_bytes, stream);
+    cudaError_t e = pr.dq_zeroed ? cudaSuccess : cudaMemsetAsync(ak.dq_acc, 0, acc_bytes, stream);
     if (e != cudaSuccess) { set_error("cudaMemsetAsync: %s", cudaGetErrorString(e)); return NB200_ERR_LAUNCH; }
     ak.out1 = pr.dv;
     ak.out2 = pr.dk;

@@ -60,6 +60,8 @@ int launch_dq_finish_d128(const Problem& pr, const float* acc, int acc_rows, boo
 
 bool bwd_supported(const Problem& pr, int dtype, int bias_dtype, const char** why);
 size_t bwd_workspace_bytes(const Problem& pr, int dtype, int bias_dtype);
+// fp32 dq sums of the one-kernel backwards: their place in that workspace
+void bwd_dq_region(const Problem& pr, int dtype, size_t* offset, size_t* bytes);
 // ld_rows: rows per (batch, head) of pr.lse / pr.delta as passed (S, or the padded count of staged copies)
 int launch_bwd(const Problem& pr, int dtype, int bias_dtype, void* ws, size_t ws_bytes, int ld_rows, cudaStream_t stream);
 

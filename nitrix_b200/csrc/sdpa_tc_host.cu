@@ -554,6 +554,10 @@ int tc_mask_pack(const Problem& pr, bool with_transpose, void* packed, size_t pa
   return tc::launch_mask_pack(pr, mp, packed, &unused, stream);
 }
 
+void tc_bwd_dq_region(const Problem& original, int dtype, size_t* offset, size_t* bytes) {
+  tc::bwd_dq_region(tc::staged_view(original, tc::plan_staging(original, NB200_PASS_BWD), nullptr), dtype, offset, bytes);
+}
+
 int tc_backward(const Problem& original, int dtype, int bias_dtype, void* ws, size_t ws_bytes, cudaStream_t stream) {
   // padded copies (bias in; lse / delta rows; dbias out) sit behind the kernels' own scratch
   const tc::Staging sg = tc::plan_staging(original, NB200_PASS_BWD);
