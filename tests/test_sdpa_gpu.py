@@ -800,3 +800,51 @@ def test_bounded_wait_times_out_and_reports():
     got, ref = run_both(q, k, v, kw, torch.bfloat16, "cuda-sm100")
     _device_ok()
     check(got, ref, torch.bfloat16)
+
+
+@pytest.mark.parametrize("dtype,d", [(torch.bfloat16, 8), (torch.bfloat16, 40), (torch.float16, 128), (torch.bfloat16, 136),
+                                     (torch.float32, 20), (torch.float32, 132), (torch.float32, 256)])
+@pytest.mark.parametrize("n", [1, 67])
+def test_qk_norm_lane_groups(dtype, d, n):
+    # head dims just in and above each group of lanes, rows that do not fill a CTA's groups, dense and strided
+    from nitrix_b200.nn import attention as att
+
+    g = torch.Generator(device="cuda").manual_seed(d)
+    q = torch.randn(2, 3, n, d, device="cuda", generator=g).to(dtype)
+    k = torch.randn(2, n + 5, 3, d, device="cuda", generator=g).to(dtype).transpose(1, 2)
+    gq, gk = torch.randn_like(q), torch.randn(k.shape, device="cuda", generator=g).to(dtype)
+    leaves = [t.detach().requires_grad_(True) for t in (q, k)]
+    assert att._qk_norm_fusable(*leaves)
+    y = att.qk_rms_norm_pair(*leaves)
+    grads = torch.autograd.grad(y, leaves, [gq, gk])
+    tol = {torch.float32: 1e-6, torch.bfloat16: 6e-3, torch.float16: 1e-3}[dtype]   # (half an ulp of the storage type)
+    for x, z, gy, dx in zip((q, k), y, (gq, gk), grads):
+        x64 = x.double().requires_grad_(True)
+        want = x64 * torch.rsqrt(x64.square().mean(-1, keepdim=True) + 1e-6)
+        assert float((z.double() - want).norm() / want.norm()) <= tol
+        r, = torch.autograd.grad(want, x64, gy.double())
+        assert float((dx.double() - r).norm() / r.norm().clamp_min(1e-3)) <= 2 * tol
+
+
+@pytest.mark.parametrize("B,H,S,T,D,causal", [(3, 2, 33, 130, 64, False), (2, 2, 129, 61, 64, True), (4, 1, 217, 217, 64, False),
+                                              (3, 2, 64, 128, 128, False), (2, 3, 100, 203, 128, True)])
+def test_shared_bias_gradient_at_the_edges_of_its_blocks(B, H, S, T, D, causal):
+    # the fp32 sums lie in blocks of 32 rows x 4 keys: rows and keys that do not fill the last block, and ones that do
+    from nitrix_b200.nn import attention as att
+
+    g = torch.Generator(device="cuda").manual_seed(S * T)
+    q, k, v, dout = (torch.randn(B, H, n, D, device="cuda", generator=g).bfloat16() for n in (S, T, T, S))
+    bias = torch.randn(1, H, S, T, device="cuda", generator=g).bfloat16()
+    scale = D ** -0.5
+    out, lse = att.sdpa_forward(q, k, v, bias, None, scale=scale, causal=causal)
+    dbias = att.sdpa_backward(q, k, v, bias, None, out, lse, dout, scale=scale, causal=causal, want_dbias=True)[3]
+    s = q.double() @ k.double().transpose(-1, -2) * scale + bias.double()
+    if causal:
+        s = s.masked_fill(torch.ones(S, T, device="cuda", dtype=torch.bool).triu(1), float('-inf'))
+    p = s.softmax(-1)
+    d = dout.double()
+    dp = d @ v.double().transpose(-1, -2)
+    want = (p * (dp - (p * dp).sum(-1, keepdim=True))).sum(0, keepdim=True)
+    assert dbias.shape == bias.shape
+    # (out is rounded to bf16 before delta is taken from it, p and ds to bf16 on the way: 2^-8 each)
+    assert float((dbias.double() - want).norm() / want.norm()) <= 1.2e-2
