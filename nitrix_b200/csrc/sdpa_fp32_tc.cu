@@ -2,11 +2,12 @@
 // into the six bf16 products that matter.
 //
 //   x = x0 + x1 + x2 exactly (8 significant bits each, by truncation: x0 the top 16 bits of x, x1 the top 16 of x - x0,
-//   x2 the rest), so a b = a0 b0 + a0 b1 + a1 b0 + a1 b1 + a0 b2 + a2 b0 up to 2^-23 |a b|; the products are exact and are
-//   accumulated in fp32 by the tensor core, the small ones first.
+//   x2 the rest), and a b = a0 b0 + a0 b1 + a1 b0 + a1 b1 + a0 b2 + a2 b0 but for a1 b2 + a2 b1 + a2 b2, which is below
+//   2^-20 |a b| and 2^-22 of it on average; the products are exact and are accumulated in fp32 by the tensor core, the
+//   small ones first.
 //
-// Six products at the bf16 rate cost what three at the tf32 rate would, keep two to three bits more than a tf32 (hi, lo)
-// pair, and need the 16-bit operand layouts only.
+// Six products at the bf16 rate cost what three at the tf32 rate would, lose less than a tf32 (hi, lo) pair (2^-20 three
+// times over), and need the 16-bit operand layouts only.
 //
 // split_planes_kernel writes the three planes of q, k, v (and dout) into the workspace as the tiles the MMA reads -- 64 rows
 // x 64 columns of bf16 in the 128-byte swizzle, 8 KB, planes of a tile side by side -- so the attention kernels fetch
@@ -117,6 +118,10 @@ __device__ __forceinline__ void prefetch_addends(const Problem& pr, int bias_siz
   }
   if (pr.mask && pr.ms[3] == 1) prefetch_l2(pr.mask + m_at + row * pr.ms[2] + key);
 }
+// neither the bias nor the mask has a query axis
+__device__ __forceinline__ bool key_only_addends(const Problem& pr) {
+  return (!pr.bias || pr.bs[2] == 0) && (!pr.mask || pr.ms[2] == 0);
+}
 constexpr int kAddPitch = 33;   // floats: a row of 32 addends plus one, so that 32 rows fall on distinct banks
 
 template <int kCols, bool kAdd>
@@ -147,7 +152,7 @@ enum FwdBar { K_FULL = 0, K_EMPTY = 2, V_FULL = 4, V_EMPTY = 6, Q_FULL = 8, S_FU
 // (round to nearest) every other step, and wherever a row's maximum has grown by more than 2^8 and it is rescaled.
 // kAdd: a bias or a mask; what it adds to the logits is staged coalesced, 32 keys at a time.
 // B8 H16 S1024 D64: 603 us on mma.sync (3 x TF32), here 182 + 26 for the planes; 204 with one query tile and single buffers
-// for K and V, two CTAs per SM.  Tensor core 65 % of the active cycles (ncu): bound by it and the waits of the two chains.
+// for K and V, two CTAs per SM; causal with a bias per (batch, head) 775 -> 390.  Tensor core 65 % of the active cycles (ncu): bound by it and the waits of the two chains.
 template <int kCols, bool kAdd>
 __global__ void __launch_bounds__(FwdLayout<kCols, kAdd>::kThreads, 1) fwd_fp32_tc_kernel(const __grid_constant__ FwdArgs a) {
   using L = FwdLayout<kCols, kAdd>;
@@ -285,7 +290,10 @@ __global__ void __launch_bounds__(FwdLayout<kCols, kAdd>::kThreads, 1) fwd_fp32_
     const float s2scale = pr.scale * kLog2e;
     float m = -INFINITY, l = 0.f;
     float* add = reinterpret_cast<float*>(smem + L::kAddend) + warp * 32 * kAddPitch;
-    // what the bias and the mask add to the warp's 32 rows x 32 keys from key k0 on: a lane reads along a key
+    // what the bias and the mask add to the warp's 32 rows x 32 keys from key k0 on: a lane reads along a key; one row
+    // stands for all where neither has a query axis
+    const bool key_only = key_only_addends(pr);
+    const int add_row = key_only ? 0 : lane * kAddPitch;
     auto stage_addends = [&](int k0) {
       const int key = k0 + lane;
       __syncwarp();
@@ -293,12 +301,17 @@ __global__ void __launch_bounds__(FwdLayout<kCols, kAdd>::kThreads, 1) fwd_fp32_
         const int64_t bo = b * pr.bs[0] + h * pr.bs[1] + key * pr.bs[3], mo = b * pr.ms[0] + h * pr.ms[1] + key * pr.ms[3];
         auto rows = [&](auto tag) {
           using BT = decltype(tag);
-#pragma unroll
-          for (int r = 0; r < 32; ++r) {
+          auto stage = [&](int r) {
             const int64_t rr = min(row0 + r, pr.S - 1);
             float v = pr.bias ? kLog2e * to_f32<BT>(reinterpret_cast<const BT*>(pr.bias)[bo + rr * pr.bs[2]]) : 0.f;
             if (pr.mask && pr.mask[mo + rr * pr.ms[2]] == 0) v = __uint_as_float(kDropped);
             add[r * kAddPitch + lane] = v;
+          };
+          if (key_only) {
+            stage(0);
+          } else {
+#pragma unroll
+            for (int r = 0; r < 32; ++r) stage(r);
           }
         };
         if (a.bias_dtype == NB200_F32) rows(float{});
@@ -314,9 +327,9 @@ __global__ void __launch_bounds__(FwdLayout<kCols, kAdd>::kThreads, 1) fwd_fp32_
     for (int j = 0; j < steps && ok; ++j) {
       const int kt = j * kRows;
       const int last = row < pr.S ? (pr.causal ? min(pr.T - 1, row) : pr.T - 1) - kt : -1;
-      if constexpr (kAdd) {
+      if constexpr (kAdd) {   // the first half's while the products run
         stage_addends(kt);
-        if (j + 1 < steps)
+        if (j + 1 < steps && !key_only)
           prefetch_addends(pr, dtype_size(a.bias_dtype), b * pr.bs[0] + h * pr.bs[1], b * pr.ms[0] + h * pr.ms[1], row, kt + kRows, kRows);
       }
       ok = __all_sync(0xffffffffu, wait_or_abort(bar(S_FULL + g), j & 1, abort_flag, a.status, 308));
@@ -333,6 +346,7 @@ __global__ void __launch_bounds__(FwdLayout<kCols, kAdd>::kThreads, 1) fwd_fp32_
 #pragma unroll
       for (int half = 0; half < 2; ++half) {
         if constexpr (kAdd) {
+          // (fetched ahead into registers instead, these cost more in spills than the wait: 390 -> 714 us on the causal case above)
           if (half == 1) stage_addends(kt + 32);
         }
 #pragma unroll
@@ -340,8 +354,7 @@ __global__ void __launch_bounds__(FwdLayout<kCols, kAdd>::kThreads, 1) fwd_fp32_
           const bool in = half * 32 + c <= last;
           float x = __uint_as_float(s[half][c]);
           if constexpr (kAdd) {
-            // (the addend of a key past the end was never written)
-            const float v = add[lane * kAddPitch + c];
+            const float v = add[add_row + c];   // (of a key past the end: never written)
             x = in && __float_as_uint(v) != kDropped ? fmaf(x, s2scale, v) : -INFINITY;
           } else {
             x = in ? x * s2scale : -INFINITY;
@@ -629,6 +642,8 @@ __global__ void __launch_bounds__(352, 1) bwd_fp32_tc_kernel(const __grid_consta
     }
     float* stage = reinterpret_cast<float*>(smem + L::kSide) + warp * 32 * kAddPitch;
     const bool want_db = !kKeyMajor && (pr.dbias != nullptr || pr.dbias_accum != nullptr);
+    const bool key_only = key_only_addends(pr);
+    const int add_row = key_only ? 0 : lane * kAddPitch;
     const int64_t b_base = b * pr.bs[0] + h * pr.bs[1], m_base = b * pr.ms[0] + h * pr.ms[1];
     const int64_t db_base = b * pr.dbs[0] + h * pr.dbs[1];
     if constexpr (!kKeyMajor) {
@@ -687,18 +702,25 @@ __global__ void __launch_bounds__(352, 1) bwd_fp32_tc_kernel(const __grid_consta
           if constexpr (kKeyMajor) {
             // lanes are neighbouring keys: read along a row of the bias / mask
             const int64_t key = min(x_row, pr.T - 1);
+            if (key_only) {
+              float v = pr.bias ? kLog2e * to_f32<BT>(reinterpret_cast<const BT*>(pr.bias)[b_base + key * pr.bs[3]]) : 0.f;
+              if (pr.mask && pr.mask[m_base + key * pr.ms[3]] == 0) v = __uint_as_float(kDropped);
 #pragma unroll
-            for (int c = 0; c < 32; ++c) {
-              const int64_t q = min(y_row0 + c, pr.S - 1);
-              add[c] = pr.bias ? kLog2e * to_f32<BT>(reinterpret_cast<const BT*>(pr.bias)[b_base + q * pr.bs[2] + key * pr.bs[3]]) : 0.f;
-              if (pr.mask && pr.mask[m_base + q * pr.ms[2] + key * pr.ms[3]] == 0) add[c] = __uint_as_float(kDropped);
+              for (int c = 0; c < 32; ++c) add[c] = v;
+            } else {
+#pragma unroll
+              for (int c = 0; c < 32; ++c) {
+                const int64_t q = min(y_row0 + c, pr.S - 1);
+                add[c] = pr.bias ? kLog2e * to_f32<BT>(reinterpret_cast<const BT*>(pr.bias)[b_base + q * pr.bs[2] + key * pr.bs[3]]) : 0.f;
+                if (pr.mask && pr.mask[m_base + q * pr.ms[2] + key * pr.ms[3]] == 0) add[c] = __uint_as_float(kDropped);
+              }
             }
           } else {
             // a lane per key here, then a lane per query row through shared memory
             const int64_t key = min(y_row0 + lane, pr.T - 1);
             __syncwarp();
 #pragma unroll 16
-            for (int r = 0; r < 32; ++r) {
+            for (int r = 0; r < (key_only ? 1 : 32); ++r) {
               const int64_t q = min(x_row0 + quad * 32 + r, pr.S - 1);
               float v = pr.bias ? kLog2e * to_f32<BT>(reinterpret_cast<const BT*>(pr.bias)[b_base + q * pr.bs[2] + key * pr.bs[3]]) : 0.f;
               if (pr.mask && pr.mask[m_base + q * pr.ms[2] + key * pr.ms[3]] == 0) v = __uint_as_float(kDropped);
@@ -710,7 +732,7 @@ __global__ void __launch_bounds__(352, 1) bwd_fp32_tc_kernel(const __grid_consta
         if (a.bias_dtype == NB200_F32) fetch(float{});
         else if (a.bias_dtype == NB200_BF16) fetch(__nv_bfloat16{});
         else fetch(__half{});
-        if (i + 1 < steps)
+        if (i + 1 < steps && !key_only)
           prefetch_addends(pr, dtype_size(a.bias_dtype), b_base, m_base, kKeyMajor ? y_row0 + kRows + lane : x_row,
                            kKeyMajor ? x_row0 + quad * 32 : y_row0 + kRows, 32);
       }
@@ -735,7 +757,7 @@ __global__ void __launch_bounds__(352, 1) bwd_fp32_tc_kernel(const __grid_consta
         float x = __uint_as_float(s[c]);
         bool keep = in;
         if constexpr (kAdd) {
-          const float v = kKeyMajor ? add[c] : stage[lane * kAddPitch + c];
+          const float v = kKeyMajor ? add[c] : stage[add_row + c];
           keep = in && __float_as_uint(v) != kDropped;
           x = fmaf(x, s2scale, v) - ref;
         } else {
@@ -754,14 +776,24 @@ __global__ void __launch_bounds__(352, 1) bwd_fp32_tc_kernel(const __grid_consta
         const int key = y_row0 + lane;
         if (key < pr.T) {
           const int n = min(32, pr.S - (x_row0 + quad * 32));
-          for (int r = 0; r < n; ++r) {
-            const int64_t at = db_base + int64_t(x_row0 + quad * 32 + r) * pr.dbs[2] + key * pr.dbs[3];
-            const float v = stage[r * kAddPitch + lane];
-            if (pr.dbias_accum) {
-              if (v != 0.f) atomicAdd(pr.dbias_accum + at, v);
+          const float* from = stage + lane;
+          const int64_t at = db_base + int64_t(x_row0 + quad * 32) * pr.dbs[2] + key * pr.dbs[3];
+          if (pr.dbias_accum) {
+            float* to = pr.dbias_accum + at;
+            if (pr.dbs[2] == 0) {                  // summed over the queries: the warp's rows first
+              float v = 0.f;
+              for (int r = 0; r < n; ++r) v += from[r * kAddPitch];
+              if (n > 0) atomicAdd(to, v);
             } else {
-              store_from_f32(pr.dbias, at, a.bias_dtype, v);
+#pragma unroll 8
+              for (int r = 0; r < n; ++r) atomicAdd(to + r * pr.dbs[2], from[r * kAddPitch]);
             }
+          } else if (a.bias_dtype == NB200_F32) {
+            float* to = reinterpret_cast<float*>(pr.dbias) + at;
+#pragma unroll 8
+            for (int r = 0; r < n; ++r) to[r * pr.dbs[2]] = from[r * kAddPitch];
+          } else {
+            for (int r = 0; r < n; ++r) store_from_f32(pr.dbias, at + r * pr.dbs[2], a.bias_dtype, from[r * kAddPitch]);
           }
         }
       }
@@ -875,6 +907,20 @@ size_t plane_bytes(const Problem& pr, int rows) {
   return size_t(pr.bh_count) * tiles_of(rows) * 3 * (padded_cols(pr.D) / 64) * kChunkBytes;
 }
 
+// The planes of a large problem are made and used for a range of (b, h) at a time, so that they take 1 GiB at most (or one
+// (b, h)): 900 pairs of S = T = 1024, D = 64.  A range is many waves of CTAs.
+constexpr size_t kPlanesLimit = size_t(1) << 30;
+Problem part_of(const Problem& pr, size_t bytes_per_bh, int done) {
+  const size_t fit = kPlanesLimit / bytes_per_bh;
+  Problem part = pr;
+  part.bh_begin = pr.bh_begin + done;
+  const int64_t left = pr.bh_count - done, most = fit > 1 ? int64_t(fit) : 1;
+  part.bh_count = int(left < most ? left : most);
+  return part;
+}
+size_t fwd_bytes_per_bh(const Problem& pr) { return (plane_bytes(pr, pr.S) + 2 * plane_bytes(pr, pr.T)) / pr.bh_count; }
+size_t bwd_bytes_per_bh(const Problem& pr) { return 2 * (plane_bytes(pr, pr.S) + plane_bytes(pr, pr.T)) / pr.bh_count; }
+
 int launch_split(const Problem& pr, const SplitArgs& sa, int operands, cudaStream_t st) {
   int tiles = 1;
   for (int i = 0; i < operands; ++i) tiles = sa.op[i].tiles > tiles ? sa.op[i].tiles : tiles;
@@ -932,27 +978,35 @@ bool takes(const Problem& pr) {
   return (pr.D == 32 || pr.D == 64 || pr.D == 128) && pr.D == pr.Dv && pr.S > 0 && pr.T > 0 && pr.bh_count > 0 &&
          pr.bh_count <= 65535;
 }
+// a bias or a mask that has to be read per query
+bool row_addends(const Problem& pr) { return (pr.bias && pr.bs[2] != 0) || (pr.mask && pr.ms[2] != 0); }
 }  // namespace
 
 // Where these kernels win over the mma.sync ones.  A CTA here is 128 rows and has an SM to itself, and a call costs a launch
 // for the planes; the others run 64-row CTAs, several to an SM, and split the keys of a small problem over warps or
-// clusters.  So: enough 64-row tiles for about half the SMs, enough work behind the start, more at head dim 32 (padded to
-// 64 here) and with a bias or a mask (read by the warps that do the soft-max).  Forward, us, here / there (D 64 unless said):
-//   B1 H1 S1536 40 / 26, B2 H4 S256 bias, mask 27 / 18, B8 H8 S128 12.6 / 9.4, B64 H8 S64 33 / 17, B2 H8 S512 D32 bias 51 / 24,
-//   B1 H8 S1024 D32 31 / 26  <  the line  <  B1 H4 S1024 31 / 31, B4 H8 S256 15.4 / 15.7, B8 H8 S192 15 / 23,
-//   B4 H6 S344 18 / 21, B8 H8 S256 D32 17 / 18, B16 H8 S200 bias 42 / 74, B8 H16 S1024 208 / 603, the same D32 S512 mask
-//   122 / 136;  D 128: B1 H1 S128 T1536 84 / 147, B32 H8 S64 26 / 19, B1 H4 S512 35 / 53, B2 H8 S1536 184 / 449.
+// clusters.  So: enough 64-row tiles for the SMs, enough work behind the start, more at head dim 32 (padded to 64 here) and
+// with a bias or a mask per query (read by the warps that do the soft-max).  Forward, us, here / there (D 64 unless said):
+//   B1 H1 S1536 40 / 26, B1 H4 S1024 31 / 31, the same causal with a key mask 50 / 37, B2 H4 S256 bias, mask 27 / 18,
+//   B8 H8 S128 12.6 / 9.4, B64 H8 S64 33 / 17, B2 H8 S512 D32 bias 51 / 24, B1 H8 S1024 D32 31 / 26  <  the line  <
+//   B4 H8 S256 15.4 / 15.7, with key bias and mask 19.9 / 20.1, B8 H8 S192 15 / 23, B4 H6 S344 18 / 21, B1 H8 S1024 31 / 45,
+//   B8 H8 S256 D32 17 / 18, B16 H8 S200 bias 42 / 74, B8 H8 S300 T700 key bias and mask 56 / 184, B8 H16 S1024 208 / 603,
+//   the same with a key mask 293 / 810, causal with bias 390 / 775; D 128: B1 H1 S128 T1536 84 / 147, B32 H8 S64 26 / 19,
+//   B1 H4 S512 35 / 53, B2 H8 S1536 184 / 449.
 bool fp32_tc_fwd_applies(const Problem& pr) {
   if (!takes(pr) || pr.T <= kRows) return false;
   if (pr.D == 128) return true;
   const int64_t ctas = tiles_of(pr.S) * pr.bh_count, work = ctas * tiles_of(pr.T);
-  if (pr.bias || pr.mask) return ctas >= 192 && work >= 1024;
-  return pr.D == 64 ? ctas >= 64 && work >= 512 : ctas >= 192 && work >= 1024;
+  if (row_addends(pr)) return ctas >= 192 && work >= 1024;
+  return pr.D == 64 ? ctas >= 128 && work >= 512 : ctas >= 192 && work >= 1024;
 }
 
-size_t fp32_tc_fwd_bytes(const Problem& pr) { return plane_bytes(pr, pr.S) + 2 * plane_bytes(pr, pr.T); }
+size_t fp32_tc_fwd_bytes(const Problem& pr) {
+  const size_t each = fwd_bytes_per_bh(pr);
+  return each * part_of(pr, each, 0).bh_count;
+}
 
-int fp32_tc_forward(const Problem& pr, int bias_dtype, void* ws, cudaStream_t st) {
+namespace {
+int forward_part(const Problem& pr, int bias_dtype, void* ws, cudaStream_t st) {
   uint8_t* base = static_cast<uint8_t*>(ws);
   FwdArgs a{};
   a.pr = pr;
@@ -977,21 +1031,35 @@ int fp32_tc_forward(const Problem& pr, int bias_dtype, void* ws, cudaStream_t st
   if (padded_cols(pr.D) == 64) return add ? launch_fwd<64, true>(a, st) : launch_fwd<64, false>(a, st);
   return add ? launch_fwd<128, true>(a, st) : launch_fwd<128, false>(a, st);
 }
+}  // namespace
+
+int fp32_tc_forward(const Problem& pr, int bias_dtype, void* ws, cudaStream_t st) {
+  for (int done = 0; done < pr.bh_count;) {
+    const Problem part = part_of(pr, fwd_bytes_per_bh(pr), done);
+    if (int rc = forward_part(part, bias_dtype, ws, st)) return rc;
+    done += part.bh_count;
+  }
+  return NB200_OK;
+}
 
 // Head dim 128 stays with the other kernels: the planes of an owner's two operands would be 192 KB of shared memory.
 // Backward, us, here / there (D 64 unless said): B1 H1 S1536 120 / 67, B2 H4 S256 bias, mask 73 / 33, B64 H8 S64 81 / 60,
 //   B4 H8 S256 D32 35 / 33, B2 H8 S512 D32 bias 118 / 89  <  the line  <  B2 H8 S256 38 / 40, B1 H4 S1024 89 / 95,
-//   B8 H8 S128 31 / 33, B32 H8 S96 60 / 93, B4 H6 S344 49 / 69, B8 H8 S256 D32 38 / 50, B16 H8 S200 bias 140 / 250,
-//   B8 H16 S1024 679 / 2019, the same causal with bias 1120 / 2366.
+//   B8 H8 S128 31 / 33, B32 H8 S96 60 / 93, B4 H6 S344 49 / 69, B8 H8 S256 D32 38 / 50, B16 H8 S200 bias 129 / 250,
+//   B8 H16 S1024 679 / 2019, the same causal with bias 917 / 2366, B8 H8 S300 T700 key bias 153 / 486.
 bool fp32_tc_bwd_applies(const Problem& pr) {
   if (!takes(pr) || pr.D == 128 || pr.T <= kRows || pr.S <= kRows) return false;
   const int64_t ctas = (tiles_of(pr.S) < tiles_of(pr.T) ? tiles_of(pr.S) : tiles_of(pr.T)) * pr.bh_count;
-  return ctas >= (pr.bias || pr.mask || pr.D == 32 ? 192 : 64);
+  return ctas >= (row_addends(pr) || pr.D == 32 ? 192 : 64);
 }
 
-size_t fp32_tc_bwd_bytes(const Problem& pr) { return 2 * plane_bytes(pr, pr.S) + 2 * plane_bytes(pr, pr.T); }
+size_t fp32_tc_bwd_bytes(const Problem& pr) {
+  const size_t each = bwd_bytes_per_bh(pr);
+  return each * part_of(pr, each, 0).bh_count;
+}
 
-int fp32_tc_backward(const Problem& pr, int bias_dtype, void* ws, cudaStream_t st) {
+namespace {
+int backward_part(const Problem& pr, int bias_dtype, void* ws, cudaStream_t st) {
   uint8_t* q = static_cast<uint8_t*>(ws);
   uint8_t* g = q + plane_bytes(pr, pr.S);
   uint8_t* k = g + plane_bytes(pr, pr.S);
@@ -1020,6 +1088,16 @@ int fp32_tc_backward(const Problem& pr, int bias_dtype, void* ws, cudaStream_t s
   a.x_tiles = int(tiles_of(pr.T));
   a.y_tiles = int(tiles_of(pr.S));
   return add ? launch_bwd<true, true>(a, st) : launch_bwd<true, false>(a, st);
+}
+}  // namespace
+
+int fp32_tc_backward(const Problem& pr, int bias_dtype, void* ws, cudaStream_t st) {
+  for (int done = 0; done < pr.bh_count;) {
+    const Problem part = part_of(pr, bwd_bytes_per_bh(pr), done);
+    if (int rc = backward_part(part, bias_dtype, ws, st)) return rc;
+    done += part.bh_count;
+  }
+  return NB200_OK;
 }
 
 }  // namespace nb200
