@@ -63,8 +63,9 @@ enum nb200_kernel {
   NB200_KERNEL_SIMT = 1,   /* fp32-arithmetic CUDA-core kernels: any shape / dtype  */
   NB200_KERNEL_TCGEN05 = 2, /* TMA + tcgen05 (TMEM accumulators): bf16 / fp16 tiles */
   /* Reported by nb200_sdpa_plan only (not a value for `kernel`): the problem runs in the NB200_KERNEL_SIMT family
-   * on its fp32-operand kernels that split every operand into two TF32 terms and use the warp-level tensor-core
-   * path (3 x TF32, fp32 accuracy) -- the counterpart of what the reference's fused path accepts, fp32 only
+   * on its fp32-operand tensor-core kernels (fp32 accuracy): every operand split into three bf16 terms on tcgen05 where
+   * the problem is large enough and `workspace` holds what nb200_sdpa_workspace_bytes reports (it may be absent or
+   * smaller), else into two TF32 terms on the warp-level path -- the counterpart of what the reference's fused path accepts, fp32 only
    * (reference attention.py:736-744). */
   NB200_KERNEL_MMA_TF32X3 = 3
 };

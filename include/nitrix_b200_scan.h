@@ -21,8 +21,8 @@
  * all work is enqueued on the caller's stream; nothing is allocated: the checkpoints
  * (nb200_selective_scan_checkpoint_bytes, fp32) belong to the caller and travel from the forward to the backward,
  * the backward's fp32 accumulators (cleared on the stream) and its adjoint states at the checkpoints' steps go through
- * `workspace` (nb200_selective_scan_workspace_bytes).  dB, dC (sums over channels) and dA, dD (sums over batch and length) are accumulated with fp32 atomics:
- * the order of those sums is not fixed.
+ * `workspace` (nb200_selective_scan_workspace_bytes).  dB, dC (sums over channels) and dA, dD (sums over batch and
+ * length) are accumulated with fp32 atomics: the order of those sums is not fixed.
  */
 #ifndef NITRIX_B200_SCAN_H_
 #define NITRIX_B200_SCAN_H_

@@ -987,14 +987,15 @@ bool row_addends(const Problem& pr) { return (pr.bias && pr.bs[2] != 0) || (pr.m
 // clusters.  So: enough 64-row tiles for the SMs, enough work behind the start, more at head dim 32 (padded to 64 here) and
 // with a bias or a mask per query (read by the warps that do the soft-max).  Forward, us, here / there (D 64 unless said):
 //   B1 H1 S1536 40 / 26, B1 H4 S1024 31 / 31, the same causal with a key mask 50 / 37, B2 H4 S256 bias, mask 27 / 18,
-//   B8 H8 S128 12.6 / 9.4, B64 H8 S64 33 / 17, B2 H8 S512 D32 bias 51 / 24, B1 H8 S1024 D32 31 / 26  <  the line  <
+//   B8 H8 S128 12.6 / 9.4, B64 H8 S64 33 / 17, B32 H16 S64 T512 121 / 93, B8 H16 S17 T1000 78 / 53, B2 H8 S512 D32 bias 51 / 24, B1 H8 S1024 D32 31 / 26  <  the line  <
 //   B4 H8 S256 15.4 / 15.7, with key bias and mask 19.9 / 20.1, B8 H8 S192 15 / 23, B4 H6 S344 18 / 21, B1 H8 S1024 31 / 45,
 //   B8 H8 S256 D32 17 / 18, B16 H8 S200 bias 42 / 74, B8 H8 S300 T700 key bias and mask 56 / 184, B8 H16 S1024 208 / 603,
 //   the same with a key mask 293 / 810, causal with bias 390 / 775; D 128: B1 H1 S128 T1536 84 / 147, B32 H8 S64 26 / 19,
-//   B1 H4 S512 35 / 53, B2 H8 S1536 184 / 449.
+//   B16 H8 S20 T300 39 / 35, B4 H8 S48 T700 49 / 71, B1 H4 S512 35 / 53, B2 H8 S1536 184 / 449.
 bool fp32_tc_fwd_applies(const Problem& pr) {
   if (!takes(pr) || pr.T <= kRows) return false;
-  if (pr.D == 128) return true;
+  if (pr.D == 128) return pr.S > kRows / 2;
+  if (pr.S <= kRows) return false;   // (half of a 128-row tile at least would be padding)
   const int64_t ctas = tiles_of(pr.S) * pr.bh_count, work = ctas * tiles_of(pr.T);
   if (row_addends(pr)) return ctas >= 192 && work >= 1024;
   return pr.D == 64 ? ctas >= 128 && work >= 512 : ctas >= 192 && work >= 1024;

@@ -53,7 +53,7 @@ def _layout(t, kind):
 
 
 @pytest.mark.parametrize("B,H,S,T,D,causal,bias,mask,layout", [
-    (4, 32, 64, 256, 64, False, None, None, "dense"),        # one 64-row tile per (b, h), even steps
+    (4, 32, 128, 256, 64, False, None, None, "dense"),       # whole tiles, an even number of steps
     (4, 48, 65, 321, 64, False, None, None, "bshd"),         # a second tile of one row; an odd last step of one key
     (2, 64, 300, 130, 64, False, None, None, "odd"),         # second CTA of one query tile; three steps
     (3, 40, 257, 257, 64, True, None, None, "dense"),        # causal over CTAs of two tiles
