@@ -151,13 +151,17 @@ NB200_API const char* nb200_last_error(void);
  * reference nn/attention/__init__.py:207-220).  Never launches. */
 NB200_API int nb200_sdpa_plan(const nb200_sdpa_params* p, int pass, int* kernel);
 
-/* Scratch bytes `pass` needs for this problem: packed mask bits (forward and backward), and for the backward
+/* Scratch bytes `pass` takes for this problem: packed mask bits (forward and backward), and for the backward
  * the delta rows (B*H*S floats), an fp32 copy of a broadcast bias' gradient, and -- bf16/fp16 at head dim 64
  * without a bias gradient, where one kernel produces dq, dk and dv -- an fp32 copy of dq (B*H*S*64 floats).
  * plus padded copies of bias / dbias / lse / delta when their rows are not 16-byte addressable (lengths that are not
- * multiples of 8, strided keys).  The tensor-core kernels take bf16/fp16 with D == Dv in {64, 128}; everything else runs
- * on the fp32 CUDA-core family (nb200_sdpa_plan tells which). */
+ * multiples of 8, strided keys), and the bf16 planes of fp32 operands.  The tensor-core kernels take bf16/fp16 with
+ * D == Dv in {64, 128}; everything else runs on the fp32 family (nb200_sdpa_plan tells which). */
 NB200_API int nb200_sdpa_workspace_bytes(const nb200_sdpa_params* p, int pass, size_t* bytes);
+
+/* The least of it with which the call still runs, on kernels that do without the rest: the planes of fp32 operands.  A
+ * workspace between the two sizes counts as the smaller one. */
+NB200_API int nb200_sdpa_workspace_least_bytes(const nb200_sdpa_params* p, int pass, size_t* bytes);
 
 /* Forward: out = softmax(scale * q k^T + bias, masked) v and lse.
  * Replaces reference attention.py:547-584 (glue) and :159-264 (kernel launch). */
@@ -182,7 +186,7 @@ NB200_API int nb200_sdpa_bwd(const nb200_sdpa_params* p, void* cuda_stream);
  * NB200_STATIC_SCRATCH_BYTES array inside the library image on every GPU that
  * loads it; p->workspace and p->workspace_bytes are ignored.
  *  - Allocates nothing: no cudaMalloc / cudaFree, no allocating library call.
- *  - A problem whose scratch (nb200_sdpa_workspace_bytes, backward pass) exceeds
+ *  - A problem whose least scratch (nb200_sdpa_workspace_least_bytes, backward pass) exceeds
  *    NB200_STATIC_SCRATCH_BYTES is rejected with NB200_ERR_WORKSPACE.
  *  - The first call on each device looks up the array's device address (with
  *    that device current); make that first call before any stream capture.

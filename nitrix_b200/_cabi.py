@@ -91,6 +91,7 @@ EXPORTS = (
     "nb200_last_error",
     "nb200_sdpa_plan",
     "nb200_sdpa_workspace_bytes",
+    "nb200_sdpa_workspace_least_bytes",
     "nb200_sdpa_fwd",
     "nb200_sdpa_bwd",
     "nb200_sdpa_bwd_static_scratch",
@@ -141,6 +142,7 @@ def lib() -> C.CDLL:
     L.nb200_profile_read.restype = C.c_size_t
     L.nb200_sdpa_plan.argtypes = [C.POINTER(SdpaParams), C.c_int, C.POINTER(C.c_int)]
     L.nb200_sdpa_workspace_bytes.argtypes = [C.POINTER(SdpaParams), C.c_int, C.POINTER(C.c_size_t)]
+    L.nb200_sdpa_workspace_least_bytes.argtypes = [C.POINTER(SdpaParams), C.c_int, C.POINTER(C.c_size_t)]
     L.nb200_sdpa_fwd.argtypes = [C.POINTER(SdpaParams), C.c_void_p]
     L.nb200_sdpa_bwd.argtypes = [C.POINTER(SdpaParams), C.c_void_p]
     L.nb200_sdpa_bwd_static_scratch.argtypes = [C.POINTER(SdpaParams), C.c_void_p]

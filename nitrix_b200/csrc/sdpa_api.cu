@@ -370,19 +370,34 @@ NB200_API int nb200_sdpa_plan(const nb200_sdpa_params* p, int pass, int* kernel)
   return NB200_OK;
 }
 
-NB200_API int nb200_sdpa_workspace_bytes(const nb200_sdpa_params* p, int pass, size_t* bytes) {
+}  // extern "C"
+
+namespace {
+// least: without what a call can do without (the fp32 planes of the tcgen05 kernels)
+int workspace_bytes(const nb200_sdpa_params* p, int pass, bool least, size_t* bytes) {
   if (!bytes) { set_error("bytes out-pointer is NULL"); return NB200_ERR_INVALID; }
   Lowered lw;
   if (int rc = lower(p, pass, &lw)) return rc;
   int kernel = 0;
   if (int rc = choose(p, lw, pass, &kernel)) return rc;
   size_t fam = kernel == NB200_KERNEL_TCGEN05 ? tc_workspace_bytes(lw.pr, lw.dtype, lw.bias_dtype, pass) : 0;
-  if (kernel == NB200_KERNEL_SIMT && lw.dtype == NB200_F32) {
+  if (!least && kernel == NB200_KERNEL_SIMT && lw.dtype == NB200_F32) {
     if (pass == NB200_PASS_FWD && fp32_tc_fwd_applies(lw.pr)) fam = fp32_tc_fwd_bytes(lw.pr);
     if (pass == NB200_PASS_BWD && fp32_tc_bwd_applies(lw.pr)) fam = fp32_tc_bwd_bytes(lw.pr);
   }
   *bytes = pass == NB200_PASS_FWD ? align_up(fam) : bwd_scratch(p, lw, kernel, fam).total;
   return NB200_OK;
+}
+}  // namespace
+
+extern "C" {
+
+NB200_API int nb200_sdpa_workspace_bytes(const nb200_sdpa_params* p, int pass, size_t* bytes) {
+  return workspace_bytes(p, pass, false, bytes);
+}
+
+NB200_API int nb200_sdpa_workspace_least_bytes(const nb200_sdpa_params* p, int pass, size_t* bytes) {
+  return workspace_bytes(p, pass, true, bytes);
 }
 
 NB200_API int nb200_mask_pack_bytes(const nb200_sdpa_params* p, int with_transpose, size_t* bytes) {

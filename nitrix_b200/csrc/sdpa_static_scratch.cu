@@ -50,8 +50,8 @@ int scratch_address(void** out) {
 
 extern "C" NB200_API int nb200_sdpa_bwd_static_scratch(const nb200_sdpa_params* p, void* cuda_stream) {
   if (!p) { nb200::set_error("params is NULL"); return NB200_ERR_INVALID; }
-  size_t need = 0;
-  if (int rc = nb200_sdpa_workspace_bytes(p, NB200_PASS_BWD, &need)) return rc;
+  size_t need = 0;   // (what the backward takes beyond this it uses only where it fits)
+  if (int rc = nb200_sdpa_workspace_least_bytes(p, NB200_PASS_BWD, &need)) return rc;
   if (need > size_t(NB200_STATIC_SCRATCH_BYTES)) {
     nb200::set_error("nb200_sdpa_bwd_static_scratch: this problem needs %zu bytes of scratch but the built-in scratch "
                      "holds %zu; use nb200_sdpa_bwd with a caller-provided workspace", need,

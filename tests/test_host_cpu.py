@@ -259,6 +259,39 @@ def test_backward_plan_takes_want_dbias_without_a_buffer():
     assert n0 >= delta + 2 * 4 * 256 * 128 * 4    # without dbias: delta rows + the one-kernel backward's fp32 dq sums
 
 
+def _backward_bytes(query="nb200_sdpa_workspace_bytes", *, B, H, S, T, D, dtype, bias=None, scale=0.125):
+    """What ``query`` answers for a backward of dense operands; ``bias``: element strides, None for no bias."""
+    from nitrix_b200 import _cabi
+
+    p = _cabi.new_params()
+    p.dtype = p.bias_dtype = dtype
+    p.B, p.H, p.S, p.T, p.D, p.Dv = B, H, S, T, D, D
+    for f in ("q", "k", "v", "out", "lse", "dout", "dq", "dk", "dv"):
+        setattr(p, f, 0x1000)
+    for f in ("q_stride", "out_stride", "dout_stride", "dq_stride"):
+        getattr(p, f)[:] = [H * S * D, S * D, D, 1]
+    for f in ("k_stride", "v_stride", "dk_stride", "dv_stride"):
+        getattr(p, f)[:] = [H * T * D, T * D, D, 1]
+    if bias is not None:
+        p.bias, p.want_dbias = 0x1000, 1
+        p.bias_stride[:] = bias
+        p.dbias_stride[:] = [H * S * T, S * T, T, 1]
+    p.scale, p.bh_end = scale, B * H
+    need = C.c_size_t(0)
+    assert getattr(_cabi.lib(), query)(C.byref(p), _cabi.PASS_BWD, C.byref(need)) == _cabi.OK, _cabi.last_error()
+    return need.value
+
+
+def test_the_planes_of_fp32_operands_are_not_part_of_the_least_workspace():
+    from nitrix_b200 import _cabi
+
+    for B, H, S, D in ((4, 8, 256, 64), (4, 6, 344, 64), (8, 16, 1024, 64)):
+        case = dict(B=B, H=H, S=S, T=S, D=D, dtype=_cabi.F32)
+        planes = 4 * B * H * ((S + 63) // 64) * 3 * 8192          # q, k, v, dout
+        assert _backward_bytes("nb200_sdpa_workspace_least_bytes", **case) == B * H * S * 4      # delta
+        assert _backward_bytes(**case) == B * H * S * 4 + planes
+
+
 def test_gradient_of_a_bias_without_a_key_axis_is_left_to_the_cuda_core_kernels():
     """A (H, S, 1) bias: its forward stays on the tensor cores (a padded copy spreads it over the keys), its gradient
     does not -- the tensor-core kernels add one sum per key, past the end of an accumulator with one per query."""

@@ -123,6 +123,14 @@ def test_static_scratch_with_tensor_core_backwards_after_a_larger_call():
     _close(got, want, torch.bfloat16)
 
 
+@pytest.mark.parametrize("shape,want_dbias", [(dict(b=4, h=8, s=256, d=64), False), (dict(b=4, h=6, s=344, d=64), False),
+                                              (dict(b=8, h=8, s=200, d=64), True)])
+def test_static_scratch_takes_fp32_problems_whose_planes_do_not_fit(shape, want_dbias):
+    # 12 MiB and more of planes, which the call can do without; delta and the bias' sums fit
+    got, want = _backward_both("bias" if want_dbias else "causal", torch.float32, want_dbias, **shape)
+    _close(got, want, torch.float32)
+
+
 def test_static_scratch_rejects_oversized_problems():
     from nitrix_b200 import _cabi
     from nitrix_b200.nn import attention as att
