@@ -159,8 +159,9 @@ NB200_API int nb200_sdpa_plan(const nb200_sdpa_params* p, int pass, int* kernel)
  * D == Dv in {64, 128}; everything else runs on the fp32 family (nb200_sdpa_plan tells which). */
 NB200_API int nb200_sdpa_workspace_bytes(const nb200_sdpa_params* p, int pass, size_t* bytes);
 
-/* The least of it with which the call still runs, on kernels that do without the rest: the planes of fp32 operands.  A
- * workspace between the two sizes counts as the smaller one. */
+/* The least of it with which the call still runs, without what it can do without: the planes of fp32 operands (other
+ * kernels run) and the padding of a broadcast bias' accumulator to blocks of 32 queries x 4 keys (it is dense then, and
+ * slower to add to).  A workspace between the two sizes counts as the smaller one. */
 NB200_API int nb200_sdpa_workspace_least_bytes(const nb200_sdpa_params* p, int pass, size_t* bytes);
 
 /* Forward: out = softmax(scale * q k^T + bias, masked) v and lse.

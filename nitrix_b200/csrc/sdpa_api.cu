@@ -263,18 +263,20 @@ int choose(const nb200_sdpa_params* p, const Lowered& lw, int pass, int* kernel)
 // accumulator for a broadcast bias gradient; family-specific scratch follows.
 struct BwdScratch { size_t delta_off, accum_off, family_off, total; int64_t accum_elems; };
 
-// Key groups of a blocked bias accumulator (Problem::dbias_groups), 0 where it is dense.
+// Key groups of a blocked bias accumulator (Problem::dbias_groups), 0 where it is dense: also below half a block of rows,
+// where clearing and reading the padding costs more than the wider reductions save (S 2, T 2048, two batches of 8 heads,
+// D 128: 75 us dense, 78 blocked).
 int dbias_groups(const Lowered& lw, int kernel) {
-  const bool tile = lw.bias_extent[2] == lw.pr.S && lw.pr.S > 1 && lw.bias_extent[3] == lw.pr.T && lw.pr.T > 1;
+  const bool tile = lw.bias_extent[2] == lw.pr.S && lw.pr.S >= 16 && lw.bias_extent[3] == lw.pr.T && lw.pr.T > 1;
   return kernel == NB200_KERNEL_TCGEN05 && tile ? (lw.pr.T + 3) / 4 : 0;
 }
 // Elements of the accumulator of one (b, h) of the bias.
-int64_t accum_tile(const Lowered& lw, int kernel) {
-  if (const int groups = dbias_groups(lw, kernel)) return int64_t((lw.pr.S + 31) / 32) * groups * 128;
+int64_t accum_tile(const Lowered& lw, int groups) {
+  if (groups) return int64_t((lw.pr.S + 31) / 32) * groups * 128;
   return lw.bias_extent[2] * lw.bias_extent[3];
 }
 
-BwdScratch bwd_scratch(const nb200_sdpa_params* p, const Lowered& lw, int kernel, size_t family_bytes) {
+BwdScratch bwd_scratch(const nb200_sdpa_params* p, const Lowered& lw, int groups, size_t family_bytes) {
   BwdScratch s{};
   size_t off = 0;
   s.delta_off = off;
@@ -282,7 +284,7 @@ BwdScratch bwd_scratch(const nb200_sdpa_params* p, const Lowered& lw, int kernel
   s.accum_off = off;
   s.accum_elems = 0;
   if ((p->dbias || p->want_dbias) && lw.bias_broadcast) {
-    s.accum_elems = lw.bias_extent[0] * lw.bias_extent[1] * accum_tile(lw, kernel);
+    s.accum_elems = lw.bias_extent[0] * lw.bias_extent[1] * accum_tile(lw, groups);
     off += align_up(sizeof(float) * size_t(s.accum_elems));
   }
   s.family_off = off;
@@ -373,7 +375,7 @@ NB200_API int nb200_sdpa_plan(const nb200_sdpa_params* p, int pass, int* kernel)
 }  // extern "C"
 
 namespace {
-// least: without what a call can do without (the fp32 planes of the tcgen05 kernels)
+// least: without what a call can do without (the fp32 planes of the tcgen05 kernels, the padding of a blocked accumulator)
 int workspace_bytes(const nb200_sdpa_params* p, int pass, bool least, size_t* bytes) {
   if (!bytes) { set_error("bytes out-pointer is NULL"); return NB200_ERR_INVALID; }
   Lowered lw;
@@ -385,7 +387,7 @@ int workspace_bytes(const nb200_sdpa_params* p, int pass, bool least, size_t* by
     if (pass == NB200_PASS_FWD && fp32_tc_fwd_applies(lw.pr)) fam = fp32_tc_fwd_bytes(lw.pr);
     if (pass == NB200_PASS_BWD && fp32_tc_bwd_applies(lw.pr)) fam = fp32_tc_bwd_bytes(lw.pr);
   }
-  *bytes = pass == NB200_PASS_FWD ? align_up(fam) : bwd_scratch(p, lw, kernel, fam).total;
+  *bytes = pass == NB200_PASS_FWD ? align_up(fam) : bwd_scratch(p, lw, least ? 0 : dbias_groups(lw, kernel), fam).total;
   return NB200_OK;
 }
 }  // namespace
@@ -458,7 +460,12 @@ NB200_API int nb200_sdpa_bwd(const nb200_sdpa_params* p, void* cuda_stream) {
   prof_mark(nullptr);   // start of this call's kernels
   if (lw.pr.bh_count == 0) return NB200_OK;
   const size_t fam = kernel == NB200_KERNEL_TCGEN05 ? tc_workspace_bytes(lw.pr, lw.dtype, lw.bias_dtype, NB200_PASS_BWD) : 0;
-  const BwdScratch sc = bwd_scratch(p, lw, kernel, fam);
+  int groups = dbias_groups(lw, kernel);
+  BwdScratch sc = bwd_scratch(p, lw, groups, fam);
+  if (groups && p->workspace_bytes < sc.total) {   // (the least workspace: a dense accumulator)
+    groups = 0;
+    sc = bwd_scratch(p, lw, 0, fam);
+  }
   if (!p->workspace || p->workspace_bytes < sc.total) {
     set_error("backward needs %zu workspace bytes, got %zu", sc.total, p->workspace ? p->workspace_bytes : size_t(0));
     return NB200_ERR_WORKSPACE;
@@ -474,10 +481,10 @@ NB200_API int nb200_sdpa_bwd(const nb200_sdpa_params* p, void* cuda_stream) {
     pr.dbias_accum = reinterpret_cast<float*>(ws + sc.accum_off);
     // dense strides over bias' own extent (of whole (b, h) tiles, where those are blocked); broadcast axes collapse to
     // stride 0
-    pr.dbias_groups = dbias_groups(lw, kernel);
+    pr.dbias_groups = groups;
     int64_t st_dense = 1;
     for (int a = 3; a >= 0; --a) {
-      if (a == 1) st_dense = accum_tile(lw, kernel);
+      if (a == 1) st_dense = accum_tile(lw, groups);
       pr.dbs[a] = lw.bias_extent[a] == 1 ? 0 : st_dense;
       st_dense *= lw.bias_extent[a];
     }
@@ -493,7 +500,7 @@ NB200_API int nb200_sdpa_bwd(const nb200_sdpa_params* p, void* cuda_stream) {
   if (kernel == NB200_KERNEL_TCGEN05)
     rc = tc_backward(pr, lw.dtype, lw.bias_dtype, ws + sc.family_off, fam, st);
   else if (lw.dtype == NB200_F32 && fp32_tc_bwd_applies(pr) &&
-           p->workspace_bytes >= bwd_scratch(p, lw, kernel, fp32_tc_bwd_bytes(pr)).total)   // (optional, as in the forward)
+           p->workspace_bytes >= bwd_scratch(p, lw, 0, fp32_tc_bwd_bytes(pr)).total)   // (optional, as in the forward)
     rc = fp32_tc_backward(pr, lw.bias_dtype, ws + sc.family_off, st);
   else
     rc = simt_backward(pr, lw.dtype, lw.bias_dtype, st);

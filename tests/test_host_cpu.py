@@ -292,6 +292,22 @@ def test_the_planes_of_fp32_operands_are_not_part_of_the_least_workspace():
         assert _backward_bytes(**case) == B * H * S * 4 + planes
 
 
+@pytest.mark.parametrize("S,T", [(2, 4096), (15, 100), (24, 8192), (217, 217), (33, 130)])
+def test_the_least_workspace_has_a_dense_bias_accumulator(S, T):
+    """The accumulator of a broadcast bias is padded to blocks of 32 queries x 4 keys where the workspace holds that, and
+    never from fewer than half a block of rows; the least workspace is that of the bias' own extent."""
+    from nitrix_b200 import _cabi
+
+    up = lambda n, to: (n + to - 1) // to * to
+    case = dict(B=2, H=8, S=S, T=T, D=64, dtype=_cabi.BF16)
+    dense, blocked = 4 * 8 * S * T, 4 * 8 * up(S, 32) * up(T, 4)
+    bias = [0, S * T, T, 1]
+    least, full = _backward_bytes("nb200_sdpa_workspace_least_bytes", bias=bias, **case), _backward_bytes(bias=bias, **case)
+    rest = least - up(dense, 256)      # delta, padded copies
+    assert full == rest + up(blocked if S >= 16 else dense, 256)
+    assert rest < up(2 * 8 * S * 4, 256) + 4 * 2 * 8 * up(S, 64) * 4 + 8 * S * up(T, 8) * 2 + 1024
+
+
 def test_gradient_of_a_bias_without_a_key_axis_is_left_to_the_cuda_core_kernels():
     """A (H, S, 1) bias: its forward stays on the tensor cores (a padded copy spreads it over the keys), its gradient
     does not -- the tensor-core kernels add one sum per key, past the end of an accumulator with one per query."""
