@@ -300,8 +300,9 @@ _call_cache: dict = {}
 
 def _call_params(key, fill):
     """A parameter block for operands of the layout that ``key`` describes, and the bytes of workspace the call needs.
-    ``fill()`` returns ``(block, bytes)``; all of the block but its pointers and the scale is remembered by the layout
-    (filling its 70 fields and asking the library took 25 us of a 60 us call), and every caller gets a copy of its own."""
+    ``fill()`` returns ``(block, bytes)``; all of the block but its pointers is remembered by the key, which holds
+    everything the library's answer depends on (the scale itself: families and scratch differ with its sign, with zero and
+    with whether 1 / scale is a number of the storage type) (filling its 70 fields and asking the library took 25 us of a 60 us call), and every caller gets a copy of its own."""
     hit = _call_cache.get(key)
     if hit is None:
         p, need = fill()
@@ -331,7 +332,7 @@ def _mask_meta(mask):
 def _planned_kernel_cached(q, k, v, bias, mask, scale, causal, which=_cabi.PASS_FWD, kernel=_cabi.KERNEL_AUTO,
                            want_dbias=False) -> int:
     """Plan for these operands, remembered by their layout (the planner is pure in it)."""
-    key = (_meta(q), _meta(k), _meta(v), _meta(bias), _meta(mask), scale > 0.0, bool(causal), q.device.index,
+    key = (_meta(q), _meta(k), _meta(v), _meta(bias), _meta(mask), float(scale), bool(causal), q.device.index,
            which, kernel, bool(want_dbias))
     chosen = _plan_cache.get(key)
     if chosen is None:
@@ -372,7 +373,7 @@ def sdpa_forward(q, k, v, bias=None, mask=None, *, scale: float, causal: bool = 
         p, need = fill()
     else:
         p, need = _call_params((_cabi.PASS_FWD, _meta(q), _meta(k), _meta(v), _meta(bias), _mask_meta(mask_b), _meta(out),
-                                scale > 0.0, bool(causal), kernel, bh_range, q.device.index), fill)
+                                float(scale), bool(causal), kernel, bh_range, q.device.index), fill)
     p.scale = float(scale)
     p.q, p.k, p.v, p.out, p.lse = q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), lse.data_ptr()
     if bias is not None:
@@ -425,7 +426,7 @@ def sdpa_backward(q, k, v, bias, mask, out, lse, dout, *, scale: float, causal: 
         return p, _workspace_need(p, _cabi.PASS_BWD)
 
     p, need = _call_params((_cabi.PASS_BWD, _meta(q), _meta(k), _meta(v), _meta(bias), _mask_meta(mask_b), _meta(out),
-                            _meta(dout), _meta(dq), _meta(dk), _meta(dv), _meta(dbias), scale > 0.0, bool(causal),
+                            _meta(dout), _meta(dq), _meta(dk), _meta(dv), _meta(dbias), float(scale), bool(causal),
                             kernel, bh_range, q.device.index), fill)
     p.scale = float(scale)
     p.q, p.k, p.v, p.out, p.lse = q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), lse.data_ptr()

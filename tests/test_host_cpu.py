@@ -308,6 +308,43 @@ def test_the_least_workspace_has_a_dense_bias_accumulator(S, T):
     assert rest < up(2 * 8 * S * 4, 256) + 4 * 2 * 8 * up(S, 64) * 4 + 8 * S * up(T, 8) * 2 + 1024
 
 
+def _workspace_of_each_call(monkeypatch, calls):
+    """Bytes of workspace that each of ``calls`` (functions of the attention module) hands to the library."""
+    from nitrix_b200.nn import attention as att
+
+    seen = []
+    monkeypatch.setattr(att, "_launch", lambda fn, p, device, what: seen.append(p.workspace_bytes))
+    for call in calls:
+        call(att)
+    return seen
+
+
+@pytest.mark.parametrize("dtype,D,with_bias,scales", [
+    (torch.bfloat16, 64, False, (0.0, -0.125, 0.125, float("inf"))),
+    (torch.float16, 128, True, (1e-5, 0.088, float("inf"), -0.088)),
+])
+def test_remembered_workspace_sizes_depend_on_the_scale(monkeypatch, dtype, D, with_bias, scales):
+    from nitrix_b200.nn import attention as att
+
+    q = torch.zeros(1, 4, 256, D, dtype=dtype)
+    lse = torch.zeros(1, 4, 256)
+    bias = torch.zeros(1, 4, 256, 256, dtype=dtype) if with_bias else None
+
+    def call(scale):
+        return lambda a: a.sdpa_backward(q, q, q, bias, None, q, lse, q, scale=scale, want_dbias=with_bias)
+
+    alone = {}
+    for scale in scales:
+        att._call_cache.clear()
+        alone[scale], = _workspace_of_each_call(monkeypatch, [call(scale)])
+    assert len(set(alone.values())) > 1
+    for order in (scales, scales[::-1]):
+        att._call_cache.clear()
+        assert _workspace_of_each_call(monkeypatch, map(call, order)) == [alone[s] for s in order]
+    att._call_cache.clear()
+    att._plan_cache.clear()
+
+
 def test_gradient_of_a_bias_without_a_key_axis_is_left_to_the_cuda_core_kernels():
     """A (H, S, 1) bias: its forward stays on the tensor cores (a padded copy spreads it over the keys), its gradient
     does not -- the tensor-core kernels add one sum per key, past the end of an accumulator with one per query."""
