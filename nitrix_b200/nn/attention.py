@@ -426,7 +426,7 @@ def sdpa_backward(q, k, v, bias, mask, out, lse, dout, *, scale: float, causal: 
         return p, _workspace_need(p, _cabi.PASS_BWD)
 
     p, need = _call_params((_cabi.PASS_BWD, _meta(q), _meta(k), _meta(v), _meta(bias), _mask_meta(mask_b), _meta(out),
-                            _meta(dout), _meta(dq), _meta(dk), _meta(dv), _meta(dbias), float(scale), bool(causal),
+                            _meta(dout), _meta(dq), _meta(dk), _meta(dv), _meta(dbias), lse.data_ptr() & 15, float(scale), bool(causal),
                             kernel, bh_range, q.device.index), fill)
     p.scale = float(scale)
     p.q, p.k, p.v, p.out, p.lse = q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), lse.data_ptr()

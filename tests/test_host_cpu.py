@@ -345,6 +345,20 @@ def test_remembered_workspace_sizes_depend_on_the_scale(monkeypatch, dtype, D, w
     att._plan_cache.clear()
 
 
+def test_remembered_workspace_sizes_depend_on_the_alignment_of_lse(monkeypatch):
+    # rows of lse that are not 16-byte aligned go through a padded copy
+    from nitrix_b200.nn import attention as att
+
+    q = torch.zeros(2, 4, 256, 64, dtype=torch.bfloat16)
+    rows = torch.zeros(2 * 4 * 256 + 1)
+    calls = [lambda a, at=at: a.sdpa_backward(q, q, q, None, None, q, rows[at:at + 2048].view(2, 4, 256), q, scale=0.1)
+             for at in (0, 1, 0)]
+    att._call_cache.clear()
+    aligned, shifted, again = _workspace_of_each_call(monkeypatch, calls)
+    att._call_cache.clear()
+    assert aligned == again < shifted
+
+
 def test_gradient_of_a_bias_without_a_key_axis_is_left_to_the_cuda_core_kernels():
     """A (H, S, 1) bias: its forward stays on the tensor cores (a padded copy spreads it over the keys), its gradient
     does not -- the tensor-core kernels add one sum per key, past the end of an accumulator with one per query."""
