@@ -360,6 +360,7 @@ def sdpa_forward(q, k, v, bias=None, mask=None, *, scale: float, causal: bool = 
     if lse is None:
         lse = torch.empty((B, H, S), dtype=torch.float32, device=q.device)
     mask_b = _mask_bytes(mask)
+    bh_range = None if bh_range is None else tuple(map(int, bh_range))
 
     def fill():
         p = _cabi.new_params()
@@ -411,6 +412,7 @@ def sdpa_backward(q, k, v, bias, mask, out, lse, dout, *, scale: float, causal: 
             raise ValueError("want_dbias without a bias")
         dbias = dbias_buf if dbias_buf is not None else torch.empty(bias.shape, dtype=bias.dtype, device=bias.device)
     mask_b = _mask_bytes(mask)
+    bh_range = None if bh_range is None else tuple(map(int, bh_range))
 
     def fill():
         p = _cabi.new_params()

@@ -359,6 +359,18 @@ def test_remembered_workspace_sizes_depend_on_the_alignment_of_lse(monkeypatch):
     assert aligned == again < shifted
 
 
+@pytest.mark.parametrize("span", [[1, 3], (1, 3), torch.tensor([1, 3]), range(1, 5, 2)])
+def test_a_range_of_pairs_may_be_any_sequence(monkeypatch, span):
+    from nitrix_b200.nn import attention as att
+
+    q, lse, seen = torch.zeros(2, 2, 64, 64), torch.zeros(2, 2, 64), []
+    monkeypatch.setattr(att, "_launch", lambda fn, p, device, what: seen.append((p.bh_begin, p.bh_end)))
+    for _ in range(2):
+        att.sdpa_forward(q, q, q, scale=0.1, bh_range=span)
+        att.sdpa_backward(q, q, q, None, None, q, lse, q, scale=0.1, bh_range=span)
+    assert seen == [(1, 3)] * 4
+
+
 def test_gradient_of_a_bias_without_a_key_axis_is_left_to_the_cuda_core_kernels():
     """A (H, S, 1) bias: its forward stays on the tensor cores (a padded copy spreads it over the keys), its gradient
     does not -- the tensor-core kernels add one sum per key, past the end of an accumulator with one per query."""
