@@ -410,6 +410,8 @@ def sdpa_backward(q, k, v, bias, mask, out, lse, dout, *, scale: float, causal: 
     if want_dbias:
         if bias is None:
             raise ValueError("want_dbias without a bias")
+        if _has_expanded_axis(bias):   # (a stride of 0 is a broadcast axis to the library, which has one gradient for it)
+            bias = bias.contiguous()
         dbias = dbias_buf if dbias_buf is not None else torch.empty(bias.shape, dtype=bias.dtype, device=bias.device)
     mask_b = _mask_bytes(mask)
     bh_range = None if bh_range is None else tuple(map(int, bh_range))
@@ -456,8 +458,10 @@ class _SDPA(torch.autograd.Function):
         # On the fused (tensor-core) path the mask is bit-packed ONCE, with the key-major copy, and the same bits
         # serve the forward and the backward; otherwise each pass reads the byte mask.
         packed = None
+        want_dbias = bias is not None and ctx.needs_input_grad[3]
+        if want_dbias and _has_expanded_axis(bias):
+            bias = bias.contiguous()   # as in sdpa_backward, here so that both passes and the plan see one layout
         if fused and mask is not None:
-            want_dbias = bias is not None and ctx.needs_input_grad[3]
             if _planned_kernel_cached(q, k, v, bias, mask, scale, causal, _cabi.PASS_BWD, kernel,
                                       want_dbias) == _cabi.KERNEL_TCGEN05:
                 packed = pack_mask(q, k, v, mask, with_transpose=True)

@@ -371,6 +371,19 @@ def test_a_range_of_pairs_may_be_any_sequence(monkeypatch, span):
     assert seen == [(1, 3)] * 4
 
 
+def test_a_bias_that_is_an_expanded_view_gets_a_gradient_at_every_position(monkeypatch):
+    """A stride of 0 is a broadcast axis to the library, which then writes one gradient for all of it."""
+    from nitrix_b200.nn import attention as att
+
+    q, lse, seen = torch.zeros(2, 4, 64, 64), torch.zeros(2, 4, 64), []
+    monkeypatch.setattr(att, "_launch", lambda fn, p, device, what: seen.append(list(p.bias_stride)))
+    bias = torch.zeros(1, 4, 64, 64).expand(2, 4, 64, 64)
+    att.sdpa_backward(q, q, q, bias, None, q, lse, q, scale=0.1, want_dbias=True)
+    att.sdpa_backward(q, q, q, bias[:1], None, q, lse, q, scale=0.1, want_dbias=True)
+    att.sdpa_backward(q, q, q, bias, None, q, lse, q, scale=0.1)
+    assert seen == [[4 * 4096, 4096, 64, 1], [0, 4096, 64, 1], [0, 4096, 64, 1]]
+
+
 def test_gradient_of_a_bias_without_a_key_axis_is_left_to_the_cuda_core_kernels():
     """A (H, S, 1) bias: its forward stays on the tensor cores (a padded copy spreads it over the keys), its gradient
     does not -- the tensor-core kernels add one sum per key, past the end of an accumulator with one per query."""

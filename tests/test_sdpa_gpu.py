@@ -848,3 +848,35 @@ def test_shared_bias_gradient_at_the_edges_of_its_blocks(B, H, S, T, D, causal):
     assert dbias.shape == bias.shape
     # (out is rounded to bf16 before delta is taken from it, p and ds to bf16 on the way: 2^-8 each)
     assert float((dbias.double() - want).norm() / want.norm()) <= 1.2e-2
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("leaf,masked", [((1, 2, 96, 130), True), ((3, 2, 96, 1), False), ((3, 1, 1, 130), True), ((1, 1, 1, 1), False)])
+def test_gradient_of_a_bias_that_is_an_expanded_view(leaf, masked, dtype):
+    # every position of the view has a gradient of its own; what the view was made from gets their sums
+    from nitrix_b200.nn import scaled_dot_product_attention
+
+    g = torch.Generator(device="cuda").manual_seed(8)
+    q, k, v, dout = (torch.randn(3, 2, n, 64, device="cuda", generator=g).to(dtype) for n in (96, 130, 130, 96))
+    w = torch.randn(leaf, device="cuda", generator=g).to(dtype).requires_grad_(True)
+    bias = w.expand(3, 2, 96, 130)
+    mask = None
+    if masked:
+        mask = torch.rand(3, 1, 96, 130, device="cuda", generator=g) > 0.2
+        mask[..., 0] = True
+    out = scaled_dot_product_attention(q, k, v, bias=bias, mask=mask)
+    dw, dview = torch.autograd.grad(out, [w, bias], dout)
+    s = q.double() @ k.double().transpose(-1, -2) * 64 ** -0.5 + bias.detach().double()
+    if masked:
+        s = s.masked_fill(~mask, float("-inf"))
+    p = s.softmax(-1)
+    dp = dout.double() @ v.double().transpose(-1, -2)
+    want = p * (dp - (p * dp).sum(-1, keepdim=True))
+    # (16 bits: out, p, ds and the result are rounded, 2^-9 each and the first three amplified by the difference taken)
+    tol = 2e-5 if dtype == torch.float32 else 1.6e-2
+    assert float((dview.double() - want).norm() / want.norm()) <= tol
+    total = want
+    for ax, n in enumerate(leaf):
+        total = total.sum(ax, keepdim=True) if n == 1 else total
+    # (sums over keys cancel: the error is measured against the terms)
+    assert float((dw.double() - total).norm()) <= tol * float(want.norm()) * max(1.0, (want.numel() / dw.numel()) ** 0.5)
