@@ -316,10 +316,28 @@ def _call_params(key, fill):
     return _cabi.SdpaParams.from_buffer_copy(hit[0]), hit[1]
 
 
-def _workspace_need(p, which: int) -> int:
+def _workspace_need(p, which: int, query: str = "nb200_sdpa_workspace_bytes") -> int:
     need = C.c_size_t(0)
-    _check(_cabi.lib().nb200_sdpa_workspace_bytes(C.byref(p), which, C.byref(need)), "nb200_sdpa_workspace_bytes")
+    _check(getattr(_cabi.lib(), query)(C.byref(p), which, C.byref(need)), query)
     return need.value
+
+
+def _workspace(p, which: int, need: int, device) -> Optional[torch.Tensor]:
+    """The call's scratch, ``need`` bytes; where the device has no room for them, the least with which the call runs (the
+    planes of fp32 operands take up to 1 GiB that the other kernels do without)."""
+    if not need:
+        return None
+    try:
+        ws = torch.empty(need, dtype=torch.uint8, device=device)
+    except torch.OutOfMemoryError:
+        least = _workspace_need(p, which, "nb200_sdpa_workspace_least_bytes")
+        if least >= need:
+            raise
+        if not least:
+            return None
+        ws = torch.empty(least, dtype=torch.uint8, device=device)
+    p.workspace, p.workspace_bytes = ws.data_ptr(), ws.numel()
+    return ws
 
 
 def _mask_meta(mask):
@@ -381,10 +399,7 @@ def sdpa_forward(q, k, v, bias=None, mask=None, *, scale: float, causal: bool = 
         p.bias = bias.data_ptr()
     if mask_b is not None:
         p.mask = (mask_b.blob if isinstance(mask_b, PackedMask) else mask_b).data_ptr()
-    ws = None
-    if need:
-        ws = torch.empty(need, dtype=torch.uint8, device=q.device)
-        p.workspace, p.workspace_bytes = ws.data_ptr(), need
+    ws = _workspace(p, _cabi.PASS_FWD, need, q.device)
     _launch(_cabi.lib().nb200_sdpa_fwd, p, q.device, "nb200_sdpa_fwd")
     del ws  # same-stream reuse is ordered by the caching allocator
     return out, lse
@@ -441,10 +456,7 @@ def sdpa_backward(q, k, v, bias, mask, out, lse, dout, *, scale: float, causal: 
         p.mask = (mask_b.blob if isinstance(mask_b, PackedMask) else mask_b).data_ptr()
     if dbias is not None:
         p.dbias = dbias.data_ptr()
-    ws = None
-    if need:
-        ws = torch.empty(need, dtype=torch.uint8, device=q.device)
-        p.workspace, p.workspace_bytes = ws.data_ptr(), need
+    ws = _workspace(p, _cabi.PASS_BWD, need, q.device)
     _launch(_cabi.lib().nb200_sdpa_bwd, p, q.device, "nb200_sdpa_bwd")
     del ws  # same-stream reuse is ordered by the caching allocator
     return dq, dk, dv, dbias

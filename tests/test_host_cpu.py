@@ -384,6 +384,28 @@ def test_a_bias_that_is_an_expanded_view_gets_a_gradient_at_every_position(monke
     assert seen == [[4 * 4096, 4096, 64, 1], [0, 4096, 64, 1], [0, 4096, 64, 1]]
 
 
+def test_a_device_without_room_for_the_planes_gets_the_least_workspace(monkeypatch):
+    from nitrix_b200.nn import attention as att
+
+    q, lse, room, empty = torch.zeros(4, 8, 256, 64), torch.zeros(4, 8, 256), [1 << 40], torch.empty
+
+    def bounded(*shape, **kw):
+        if kw.get("dtype") == torch.uint8 and shape[0] > room[0]:
+            raise torch.OutOfMemoryError("no room")
+        return empty(*shape, **kw)
+
+    monkeypatch.setattr(torch, "empty", bounded)
+    calls = [lambda a: a.sdpa_forward(q, q, q, scale=0.1),
+             lambda a: a.sdpa_backward(q, q, q, None, None, q, lse, q, scale=0.1)]
+    planes = 4 * 8 * 4 * 3 * 8192
+    assert _workspace_of_each_call(monkeypatch, calls) == [3 * planes, 4 * planes + 4 * 8 * 256 * 4]
+    room[0] = 1 << 20
+    assert _workspace_of_each_call(monkeypatch, calls) == [0, 4 * 8 * 256 * 4]
+    room[0] = 1 << 10                        # not even delta
+    with pytest.raises(torch.OutOfMemoryError):
+        _workspace_of_each_call(monkeypatch, calls)
+
+
 def test_gradient_of_a_bias_without_a_key_axis_is_left_to_the_cuda_core_kernels():
     """A (H, S, 1) bias: its forward stays on the tensor cores (a padded copy spreads it over the keys), its gradient
     does not -- the tensor-core kernels add one sum per key, past the end of an accumulator with one per query."""
