@@ -122,6 +122,9 @@ __device__ __forceinline__ void prefetch_addends(const Problem& pr, int bias_siz
 __device__ __forceinline__ bool key_only_addends(const Problem& pr) {
   return (!pr.bias || pr.bs[2] == 0) && (!pr.mask || pr.ms[2] == 0);
 }
+// The soft-max's reference lies kAbove over the last maximum taken, which a later logit may outgrow by up to 2^kAbove: no
+// p is above 1, so the un-normalised output overflows for no values of V that it would not overflow for at the maximum.
+constexpr float kAbove = 8.f;
 constexpr int kAddPitch = 33;   // floats: a row of 32 addends plus one, so that 32 rows fall on distinct banks
 
 template <int kCols, bool kAdd>
@@ -365,14 +368,14 @@ __global__ void __launch_bounds__(FwdLayout<kCols, kAdd>::kThreads, 1) fwd_fp32_
       }
       // ---- online soft-max; the reference maximum moves only when some row of the warp has outgrown it by 2^8 ----
       const float m_new = fmaxf(m, mx);
-      const bool move = __any_sync(0xffffffffu, m_new > m + 8.f);   // (true for the first kept key: m = -inf)
+      const bool move = __any_sync(0xffffffffu, m_new > m + kAbove);   // (true for the first kept key: m = -inf)
       float alpha = 1.f;
       if (move) {
         alpha = m_new == -INFINITY ? 1.f : tc::ex2(m - m_new);
         m = m_new;
         l *= alpha;
       }
-      const float m_ref = m == -INFINITY ? 0.f : m;                 // nothing kept so far: every p is 0
+      const float m_ref = m == -INFINITY ? 0.f : m + kAbove;        // nothing kept so far: every p is 0
       float sum[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
       for (int half = 0; half < 2; ++half)
@@ -447,7 +450,7 @@ __global__ void __launch_bounds__(FwdLayout<kCols, kAdd>::kThreads, 1) fwd_fp32_
           }
         }
       }
-      if (row < pr.S) pr.lse[(int64_t(b) * pr.H + h) * pr.S + row] = m + log2f(l);
+      if (row < pr.S) pr.lse[(int64_t(b) * pr.H + h) * pr.S + row] = m + kAbove + log2f(l);
     }
   }
   __syncwarp();

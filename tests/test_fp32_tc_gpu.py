@@ -115,6 +115,27 @@ def test_a_problem_whose_planes_exceed_their_limit_runs_in_ranges():
             assert _err(a[b:b + 1], r) <= _BOUND
 
 
+@pytest.mark.parametrize("with_bias", [False, True])
+def test_large_values_do_not_overflow_before_the_division(with_bias):
+    # logits that grow by 5 (2^7.2) from the second step on, less than what moves the reference maximum; the sum of 130
+    # probabilities of at most 1 times V stays below the largest fp32
+    from nitrix_b200.nn import attention as att
+
+    g = torch.Generator(device="cuda").manual_seed(12)
+    q, k = torch.ones(4, 50, 130, 64, device="cuda"), torch.zeros(4, 50, 130, 64, device="cuda")
+    v = (1.0 + torch.rand(4, 50, 130, 64, device="cuda", generator=g)) * 1e36
+    bias = None
+    if with_bias:
+        bias = torch.zeros(1, 50, 1, 130, device="cuda")
+        bias[..., 64:] = 5.0
+    else:
+        k[:, :, 64:] = 5.0 / 8.0
+    out, lse = att.sdpa_forward(q, k, v, bias, None, scale=0.125)
+    s = q.double() @ k.double().transpose(-1, -2) * 0.125 + (0.0 if bias is None else bias.double())
+    assert _err(out, s.softmax(-1) @ v.double()) <= _BOUND
+    assert float((lse.double() - s.logsumexp(-1) / math.log(2.0)).abs().max()) <= 1e-5
+
+
 def test_rows_without_a_kept_key_are_nan_and_leave_the_others_alone():
     from nitrix_b200.nn import attention as att
 
