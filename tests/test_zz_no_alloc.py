@@ -134,7 +134,7 @@ def test_static_scratch_takes_fp32_problems_whose_planes_do_not_fit(shape, want_
 @pytest.mark.parametrize("shape", [dict(b=2, h=8, s=24, t=8192, d=64), dict(b=2, h=8, s=24, t=6502, d=64)])
 def test_static_scratch_with_a_dense_bias_accumulator(shape):
     # 6.3 MB of sums, 8.4 MB in whole blocks of 32 rows; the same with keys that are no multiple of 4 (and a padded copy)
-    got, want = _backward_both("bias_mask", torch.bfloat16, True, **shape)
+    got, want = _backward_both("bias", torch.bfloat16, True, **shape)
     _close(got, want, torch.bfloat16)
 
 
