@@ -21,7 +21,8 @@
  * all work is enqueued on the caller's stream; nothing is allocated: the checkpoints
  * (nb200_selective_scan_checkpoint_bytes, fp32) belong to the caller and travel from the forward to the backward,
  * the backward's fp32 accumulators (cleared on the stream) and its adjoint states at the checkpoints' steps go through
- * `workspace` (nb200_selective_scan_workspace_bytes).  dB, dC (sums over channels) and dA, dD (sums over batch and
+ * `workspace` (nb200_selective_scan_workspace_bytes; with less, down to nb200_selective_scan_workspace_least_bytes, the
+ * backward runs for a range of batch elements or of channels at a time).  dB, dC (sums over channels) and dA, dD (sums over batch and
  * length) are accumulated with fp32 atomics: the order of those sums is not fixed.
  */
 #ifndef NITRIX_B200_SCAN_H_
@@ -60,6 +61,7 @@ typedef struct nb200_selective_scan_params {
 NB200_API int nb200_selective_scan_fwd(const nb200_selective_scan_params* p, void* cuda_stream);
 NB200_API int nb200_selective_scan_bwd(const nb200_selective_scan_params* p, void* cuda_stream);
 NB200_API int nb200_selective_scan_workspace_bytes(const nb200_selective_scan_params* p, size_t* bytes);
+NB200_API int nb200_selective_scan_workspace_least_bytes(const nb200_selective_scan_params* p, size_t* bytes);
 NB200_API int nb200_selective_scan_checkpoint_bytes(const nb200_selective_scan_params* p, size_t* bytes);
 
 #ifdef __cplusplus

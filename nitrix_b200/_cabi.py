@@ -113,6 +113,7 @@ EXPORTS = (
     "nb200_selective_scan_fwd",
     "nb200_selective_scan_bwd",
     "nb200_selective_scan_workspace_bytes",
+    "nb200_selective_scan_workspace_least_bytes",
     "nb200_selective_scan_checkpoint_bytes",
 )
 
@@ -160,6 +161,7 @@ def lib() -> C.CDLL:
     L.nb200_selective_scan_fwd.argtypes = [C.POINTER(SelectiveScanParams), C.c_void_p]
     L.nb200_selective_scan_bwd.argtypes = [C.POINTER(SelectiveScanParams), C.c_void_p]
     L.nb200_selective_scan_workspace_bytes.argtypes = [C.POINTER(SelectiveScanParams), C.POINTER(C.c_size_t)]
+    L.nb200_selective_scan_workspace_least_bytes.argtypes = [C.POINTER(SelectiveScanParams), C.POINTER(C.c_size_t)]
     L.nb200_selective_scan_checkpoint_bytes.argtypes = [C.POINTER(SelectiveScanParams), C.POINTER(C.c_size_t)]
     if L.nb200_version() != ABI_VERSION:
         raise NativeLibraryError(f"{path}: ABI {L.nb200_version()} != expected {ABI_VERSION}")

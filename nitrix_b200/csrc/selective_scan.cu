@@ -36,6 +36,9 @@ struct SsArgs {
   int per_cta;            // chunks a CTA of ss_bwd_kernel works through
   int vec;                // groups of four channels of x, delta, y, dy, dx, ddelta can be moved as one word
   int vecn;               // groups of four states of the fp32 arrays can
+  // launches of the backward for a range of channels (kRange): the first of them, and how many gck's rows hold (channel 0's
+  // states would be at gck)
+  int d_first, gD;
 };
 
 // a_t = exp(delta_t A) as one multiply and one ex2.approx (relative error 2^-22): A is held pre-multiplied by log2(e)
@@ -310,13 +313,13 @@ __global__ void __launch_bounds__(kScanThreads) ss_fwd_kernel(SsArgs a) {
 }
 
 // The adjoint recurrence alone, last step first: leaves for every chunk but the last the g that enters it.
-template <typename T, int kN>
+template <typename T, int kN, bool kRange>
 __global__ void __launch_bounds__(kScanThreads) ss_adjoint_kernel(SsArgs a) {
   constexpr int kQ = kN / 4;
   __shared__ __align__(16) float2 dg[kStage * kScanCh];    // delta, dy
   __shared__ __align__(16) float sC[kStage * kN];
   const int tid = threadIdx.x, part = tid & 3, ch = tid >> 2;
-  const int d0 = blockIdx.x * kScanCh, b = blockIdx.y, d = d0 + ch;
+  const int d0 = (kRange ? a.d_first : 0) + blockIdx.x * kScanCh, b = blockIdx.y, d = d0 + ch;
   const bool live = d < a.Dc;
   const bool vec = a.vec != 0, vecn = a.vecn != 0;
   const int lr = tid >> 2, lc = (tid & 3) * 4, ln = max(0, min(4, a.Dc - (d0 + lc)));
@@ -349,7 +352,7 @@ __global__ void __launch_bounds__(kScanThreads) ss_adjoint_kernel(SsArgs a) {
       if ((s0 & 4)) {   // the last step of a chunk of eight: what enters it
         const int c = (t0 + s0) / kStep;
         if (live && c + 1 < a.chunks)
-          store_states<kQ>(a.gck + ((int64_t(b) * a.chunks + c) * a.Dc + d) * a.N, part * kQ, a.N, vecn, g);
+          store_states<kQ>(a.gck + ((int64_t(b) * a.chunks + c) * (kRange ? a.gD : a.Dc) + d) * a.N, part * kQ, a.N, vecn, g);
       }
       float2 av[4][kQ / 2], Cv[4][kQ / 2];
       float gy[4];
@@ -403,7 +406,7 @@ __device__ __forceinline__ void add_states(float* row, int n0, int N, bool vec, 
 __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
 // kBlocks: blocks of 16 states (1: the sums of dA stay in registers; more: in shared memory, a slot per thread)
-template <typename T, int kBlocks>
+template <typename T, int kBlocks, bool kRange>
 __global__ void __launch_bounds__(kBwdThreads, 3) ss_bwd_kernel(SsArgs a) {
   constexpr int kN = 16 * kBlocks;
   extern __shared__ __align__(16) float smem_ss[];
@@ -414,7 +417,7 @@ __global__ void __launch_bounds__(kBwdThreads, 3) ss_bwd_kernel(SsArgs a) {
   float* sums = tile + kHalf * 32 * 32;                            // [kStep][kSumStep]
   float4* sdA = reinterpret_cast<float4*>(sums + kStep * kSumStep);   // kBlocks > 1: [kBlocks][2][kBwdThreads]
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, part = tid & 3, o = tid >> 2;
-  const int d0 = blockIdx.x * kBwdCh, b = blockIdx.z;
+  const int d0 = (kRange ? a.d_first : 0) + blockIdx.x * kBwdCh, b = blockIdx.z;
   const bool vec = a.vec != 0, vecn = a.vecn != 0;
   const bool hi = part & 2, lo = part & 1;
   // channel ch of dxg: permuted within eight so that both the writers (four channels each) and the readers (eight
@@ -453,7 +456,7 @@ __global__ void __launch_bounds__(kBwdThreads, 3) ss_bwd_kernel(SsArgs a) {
       const int64_t st = (int64_t(b) * a.chunks + c) * a.Dc * a.N, n0 = int64_t(d0) * a.N + tid * (kN / 2);
       if (n0 < int64_t(a.Dc) * a.N) {
         prefetch_l2(a.ckpt + st + n0);
-        if (c + 2 < a.chunks) prefetch_l2(a.gck + st + int64_t(a.Dc) * a.N + n0);
+        if (!kRange && c + 2 < a.chunks) prefetch_l2(a.gck + st + int64_t(a.Dc) * a.N + n0);
       }
     }
     __syncthreads();   // (the chunk before has been read)
@@ -479,8 +482,9 @@ __global__ void __launch_bounds__(kBwdThreads, 3) ss_bwd_kernel(SsArgs a) {
         const int d = d0 + o + 32 * j;
         const int have = d < a.Dc ? max(0, min(4, a.N - n0)) : 0;
         const int64_t st = ((int64_t(b) * a.chunks + c) * a.Dc + d) * a.N + n0;
+        const int64_t gt = kRange ? ((int64_t(b) * a.chunks + c) * a.gD + d) * a.N + n0 : st;
         const float4 hv = load4<float>(a.ckpt + st - int64_t(a.Dc) * a.N, c > 0 ? have : 0, vecn);
-        const float4 gv = load4<float>(a.gck + st, c + 1 < a.chunks ? have : 0, vecn);
+        const float4 gv = load4<float>(a.gck + gt, c + 1 < a.chunks ? have : 0, vecn);
         h0[j][0] = make_float2(hv.x, hv.y);
         h0[j][1] = make_float2(hv.z, hv.w);
         g[j][0] = make_float2(gv.x, gv.y);
@@ -706,33 +710,73 @@ int fwd_t(const nb200_selective_scan_params* p, cudaStream_t st) {
 size_t acc_floats(const nb200_selective_scan_params* p) {
   return 2 * size_t(p->batch) * p->length * p->states + size_t(p->channels) * p->states + size_t(p->channels);
 }
-size_t ckpt_floats(const nb200_selective_scan_params* p) {
-  return size_t(p->batch) * (p->length / kStep + (p->length % kStep != 0)) * p->states * p->channels;
+// The adjoint states take as much again as the checkpoints.  With less workspace the backward runs for a range of batch
+// elements, or of one element's channels in whole groups of 64, at a time, each in the same part of it.
+struct Range { int batch, channels; };
+size_t state_floats(const nb200_selective_scan_params* p, Range r) {
+  return size_t(r.batch) * (p->length / kStep + (p->length % kStep != 0)) * p->states * r.channels;
+}
+Range least_range(const nb200_selective_scan_params* p) { return {p->batch < 1 ? p->batch : 1, p->channels < kBwdCh ? p->channels : kBwdCh}; }
+Range range_of(const nb200_selective_scan_params* p, size_t floats) {
+  Range r{p->batch, p->channels};
+  if (state_floats(p, r) <= floats) return r;
+  r.batch = 1;
+  const size_t element = state_floats(p, r);
+  if (element <= floats) {
+    r.batch = int(floats / element);
+  } else {
+    r.channels = int(floats / (element / p->channels) / kBwdCh) * kBwdCh;   // (an element of one group or less fits)
+  }
+  return r;
 }
 size_t acc_bytes(const nb200_selective_scan_params* p) { return (sizeof(float) * acc_floats(p) + 255) / 256 * 256; }
 
-template <typename T, int kBlocks>
+template <typename T, int kBlocks, bool kRange>
 int bwd_launch(const SsArgs& a, dim3 grid, cudaStream_t st) {
   constexpr size_t smem = kStep * kBwdCh * sizeof(float4) +
                           sizeof(float) * (2 * kStep * 16 * kBlocks + kHalf * 32 * 32 + kStep * kSumStep) +
                           (kBlocks > 1 ? sizeof(float4) * kBlocks * 2 * kBwdThreads : 0);
   if (smem > 48 * 1024 &&
-      cudaFuncSetAttribute(ss_bwd_kernel<T, kBlocks>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess) {
+      cudaFuncSetAttribute(ss_bwd_kernel<T, kBlocks, kRange>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess) {
     set_error("selective_scan_bwd: cudaFuncSetAttribute(%zu): %s", smem, cudaGetErrorString(cudaGetLastError()));
     return NB200_ERR_LAUNCH;
   }
-  ss_bwd_kernel<T, kBlocks><<<grid, kBwdThreads, smem, st>>>(a);
+  ss_bwd_kernel<T, kBlocks, kRange><<<grid, kBwdThreads, smem, st>>>(a);
   count_launch();
   return check_launch("selective_scan_bwd_kernel");
+}
+
+// The two kernels of one range: `a` with its batch pointers at the range's first element.
+template <typename T, bool kRange>
+int bwd_range(const nb200_selective_scan_params* p, const SsArgs& a, Range r, cudaStream_t st) {
+  if (a.chunks > 1) {
+    const dim3 grid((r.channels + kScanCh - 1) / kScanCh, r.batch);
+    switch (pick_n(p->states)) {
+      case 8: ss_adjoint_kernel<T, 8, kRange><<<grid, kScanThreads, 0, st>>>(a); break;
+      case 16: ss_adjoint_kernel<T, 16, kRange><<<grid, kScanThreads, 0, st>>>(a); break;
+      case 32: ss_adjoint_kernel<T, 32, kRange><<<grid, kScanThreads, 0, st>>>(a); break;
+      default: ss_adjoint_kernel<T, 64, kRange><<<grid, kScanThreads, 0, st>>>(a); break;
+    }
+    count_launch();
+    if (int rc = check_launch("selective_scan_adjoint_kernel")) return rc;
+  }
+  const unsigned groups = (r.channels + kBwdCh - 1) / kBwdCh;
+  const dim3 grid(groups, unsigned((a.chunks + a.per_cta - 1) / a.per_cta), unsigned(r.batch));
+  switch (pick_n(p->states)) {
+    case 8:
+    case 16: return bwd_launch<T, 1, kRange>(a, grid, st);
+    case 32: return bwd_launch<T, 2, kRange>(a, grid, st);
+    default: return bwd_launch<T, 4, kRange>(a, grid, st);
+  }
 }
 
 template <typename T>
 int bwd_t(const nb200_selective_scan_params* p, cudaStream_t st) {
   SsArgs a = args_of<T>(p);
-  const size_t need = acc_bytes(p) + sizeof(float) * ckpt_floats(p);
+  const size_t need = acc_bytes(p) + sizeof(float) * state_floats(p, least_range(p));
   if (!p->workspace || p->workspace_bytes < need) {
-    set_error("selective_scan_bwd: workspace of %zu bytes needed (nb200_selective_scan_workspace_bytes), %zu given",
-              need, size_t(p->workspace_bytes));
+    set_error("selective_scan_bwd: workspace of at least %zu bytes needed (nb200_selective_scan_workspace_least_bytes), "
+              "%zu given", need, size_t(p->workspace_bytes));
     return NB200_ERR_WORKSPACE;
   }
   float* acc = static_cast<float*>(p->workspace);
@@ -741,33 +785,36 @@ int bwd_t(const nb200_selective_scan_params* p, cudaStream_t st) {
   a.accB = acc; a.accC = acc + bln; a.accA = acc + 2 * bln; a.accD = p->D ? acc + 2 * bln + dn : nullptr;
   a.gck = reinterpret_cast<float*>(static_cast<char*>(p->workspace) + acc_bytes(p));
   if (p->batch > 0 && p->length > 0) {   // (nothing to walk otherwise: dA and dD are the zeros just written)
-    if (a.chunks > 1) {
-      const dim3 grid = scan_grid(p);
-      switch (pick_n(p->states)) {
-        case 8: ss_adjoint_kernel<T, 8><<<grid, kScanThreads, 0, st>>>(a); break;
-        case 16: ss_adjoint_kernel<T, 16><<<grid, kScanThreads, 0, st>>>(a); break;
-        case 32: ss_adjoint_kernel<T, 32><<<grid, kScanThreads, 0, st>>>(a); break;
-        default: ss_adjoint_kernel<T, 64><<<grid, kScanThreads, 0, st>>>(a); break;
-      }
-      count_launch();
-      if (int rc = check_launch("selective_scan_adjoint_kernel")) return rc;
-    }
+    const Range whole = range_of(p, (p->workspace_bytes - acc_bytes(p)) / sizeof(float));
     // chunks per CTA: as many as leave about eight CTAs for every one that the GPU holds at a time (3 x 148), so that
     // the last wave is short; at most 16 (a CTA's own start and its sums of dA are spread well enough over those)
-    const int64_t groups = (p->channels + kBwdCh - 1) / kBwdCh;
-    int64_t per = groups * p->batch * a.chunks / (8 * 3 * 148);
+    const int64_t groups = (whole.channels + kBwdCh - 1) / kBwdCh;
+    int64_t per = groups * whole.batch * a.chunks / (8 * 3 * 148);
     per = per < 1 ? 1 : (per > 16 ? 16 : per);
     const int64_t least = (int64_t(a.chunks) + 65534) / 65535;   // (grid.y)
     a.per_cta = int(per < least ? least : per);
-    const dim3 grid(unsigned(groups), unsigned((a.chunks + a.per_cta - 1) / a.per_cta), unsigned(p->batch));
-    int rc;
-    switch (pick_n(p->states)) {
-      case 8:
-      case 16: rc = bwd_launch<T, 1>(a, grid, st); break;
-      case 32: rc = bwd_launch<T, 2>(a, grid, st); break;
-      default: rc = bwd_launch<T, 4>(a, grid, st); break;
+    a.gD = whole.channels;
+    for (int b = 0; b < p->batch; b += whole.batch) {
+      SsArgs part = a;
+      const size_t steps = size_t(b) * p->length, wide = steps * p->channels * sizeof(T), rows = steps * p->states;
+      part.x = static_cast<const char*>(a.x) + wide;
+      part.delta = static_cast<const char*>(a.delta) + wide;
+      part.dy = static_cast<const char*>(a.dy) + wide;
+      part.dx = static_cast<char*>(a.dx) + wide;
+      part.ddelta = static_cast<char*>(a.ddelta) + wide;
+      part.B = static_cast<const char*>(a.B) + rows * sizeof(T);
+      part.C = static_cast<const char*>(a.C) + rows * sizeof(T);
+      part.accB = a.accB + rows;
+      part.accC = a.accC + rows;
+      part.ckpt = a.ckpt + state_floats(p, {b, p->channels});
+      for (int d = 0; d < p->channels; d += whole.channels) {
+        part.d_first = d;
+        part.gck = a.gck - int64_t(d) * p->states;
+        const Range r{p->batch - b < whole.batch ? p->batch - b : whole.batch,
+                      p->channels - d < whole.channels ? p->channels - d : whole.channels};
+        if (int rc = whole.channels < p->channels ? bwd_range<T, true>(p, part, r, st) : bwd_range<T, false>(p, part, r, st)) return rc;
+      }
     }
-    if (rc) return rc;
   }
   SsFinish f{{a.accB, a.accC, a.accA, acc + 2 * bln + dn}, {p->dB, p->dC, p->dA, p->dD},
              {int64_t(bln), int64_t(bln), int64_t(dn), p->D ? int64_t(p->channels) : 0}};
@@ -787,14 +834,21 @@ using namespace nb200;
 extern "C" NB200_API int nb200_selective_scan_workspace_bytes(const nb200_selective_scan_params* p, size_t* bytes) {
   if (!bytes) { set_error("bytes out-pointer is NULL"); return NB200_ERR_INVALID; }
   if (int rc = check_common(p, "selective_scan_workspace_bytes")) return rc;
-  *bytes = acc_bytes(p) + sizeof(float) * ckpt_floats(p);
+  *bytes = acc_bytes(p) + sizeof(float) * state_floats(p, {p->batch, p->channels});
+  return NB200_OK;
+}
+
+extern "C" NB200_API int nb200_selective_scan_workspace_least_bytes(const nb200_selective_scan_params* p, size_t* bytes) {
+  if (!bytes) { set_error("bytes out-pointer is NULL"); return NB200_ERR_INVALID; }
+  if (int rc = check_common(p, "selective_scan_workspace_least_bytes")) return rc;
+  *bytes = acc_bytes(p) + sizeof(float) * state_floats(p, least_range(p));
   return NB200_OK;
 }
 
 extern "C" NB200_API int nb200_selective_scan_checkpoint_bytes(const nb200_selective_scan_params* p, size_t* bytes) {
   if (!bytes) { set_error("bytes out-pointer is NULL"); return NB200_ERR_INVALID; }
   if (int rc = check_common(p, "selective_scan_checkpoint_bytes")) return rc;
-  *bytes = sizeof(float) * ckpt_floats(p);
+  *bytes = sizeof(float) * state_floats(p, {p->batch, p->channels});
   return NB200_OK;
 }
 

@@ -78,6 +78,18 @@ def selective_scan_forward(x3, delta3, A, B3, C3, D, want_checkpoints: bool):
     return y, ck
 
 
+def _workspace(p, device) -> torch.Tensor:
+    """The backward's scratch; where the device has no room for the adjoint states of the whole batch at once (as large as
+    the checkpoints), the least with which it runs, a range after the other."""
+    try:
+        ws = torch.empty(max(_bytes(_cabi.lib().nb200_selective_scan_workspace_bytes, p), 16), dtype=torch.uint8, device=device)
+    except torch.OutOfMemoryError:
+        ws = torch.empty(max(_bytes(_cabi.lib().nb200_selective_scan_workspace_least_bytes, p), 16), dtype=torch.uint8,
+                         device=device)
+    p.workspace, p.workspace_bytes = ws.data_ptr(), ws.numel()
+    return ws
+
+
 def selective_scan_backward(x3, delta3, A, B3, C3, D, ck, dy3):
     """Enqueue the backward on the current stream: ``(dx, ddelta, dA, dB, dC, dD_or_None)``."""
     p = _params(x3, A)
@@ -89,10 +101,9 @@ def selective_scan_backward(x3, delta3, A, B3, C3, D, ck, dy3):
     p.checkpoints = None if ck is None else ck.data_ptr()
     p.dx, p.ddelta, p.dA, p.dB, p.dC = (t.data_ptr() for t in (dx, ddelta, dA, dB, dC))
     p.dD = None if dD is None else dD.data_ptr()
-    need = _bytes(_cabi.lib().nb200_selective_scan_workspace_bytes, p)
-    ws = torch.empty(max(need, 16), dtype=torch.uint8, device=x3.device)
-    p.workspace, p.workspace_bytes = ws.data_ptr(), need
+    ws = _workspace(p, x3.device)
     _check(_cabi.enqueue(_cabi.lib().nb200_selective_scan_bwd, p, x3.device), "nb200_selective_scan_bwd")
+    del ws  # same-stream reuse is ordered by the caching allocator
     return dx, ddelta, dA, dB, dC, dD
 
 

@@ -84,3 +84,40 @@ def test_ragged_channels_and_states_and_several_chunks_per_cta(batch, length, d,
     # channel counts that are no multiple of four (scalar loads) and states that are none, up to 8, 16 and 64; CTAs of the
     # gradients with more than one chunk
     _run((batch,), length, d, n, dtype)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("batch,length,d,n,pairs", [(5, 40, 200, 16, 400), (5, 40, 200, 16, 399), (5, 40, 200, 16, 199), (3, 33, 250, 5, 64),
+                                                    (3, 17, 333, 33, 130), (2, 9, 30, 8, 30)])
+def test_backward_in_ranges_of_a_smaller_workspace(monkeypatch, batch, length, d, n, pairs, dtype):
+    # room for the adjoint states of `pairs` (batch element, channel) pairs: two elements at a time and a last one, one
+    # element, groups of 64 channels with a last one cut short, the least
+    from nitrix_b200 import _cabi
+    from nitrix_b200.nn import ssm
+
+    def small(p, device):
+        full, least = (ssm._bytes(getattr(_cabi.lib(), f"nb200_selective_scan_workspace{q}_bytes"), p) for q in ("", "_least"))
+        states = 4 * ((length + 7) // 8) * n
+        size = full - (batch * d - pairs) * states
+        assert least == full - (batch * d - min(d, 64)) * states and least <= size
+        ws = torch.empty(size, dtype=torch.uint8, device=device)
+        p.workspace, p.workspace_bytes = ws.data_ptr(), size
+        return ws
+
+    monkeypatch.setattr(ssm, "_workspace", small)
+    _run((batch,), length, d, n, dtype)
+
+
+def test_a_device_without_room_for_all_adjoint_states_runs_in_ranges(monkeypatch):
+    empty, seen = torch.empty, []
+
+    def bounded(*shape, **kw):
+        if kw.get("dtype") == torch.uint8:
+            seen.append(shape[0])
+            if len(seen) == 1:
+                raise torch.OutOfMemoryError("no room")
+        return empty(*shape, **kw)
+
+    monkeypatch.setattr(torch, "empty", bounded)
+    _run((4,), 64, 128, 16, torch.float32)
+    assert len(seen) == 2 and seen[1] == seen[0] - 4 * 8 * 16 * (4 * 128 - 64)
