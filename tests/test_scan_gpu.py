@@ -121,3 +121,9 @@ def test_a_device_without_room_for_all_adjoint_states_runs_in_ranges(monkeypatch
     monkeypatch.setattr(torch, "empty", bounded)
     _run((4,), 64, 128, 16, torch.float32)
     assert len(seen) == 2 and seen[1] == seen[0] - 4 * 8 * 16 * (4 * 128 - 64)
+
+
+@pytest.mark.parametrize("length", [1, 3, 4, 5, 12, 17, 20])
+def test_sequences_that_end_inside_a_staged_chunk(length):
+    # steps are staged by sixteen and taken by four; groups past the end are left out
+    _run((3,), length, 72, 16, torch.float32)
