@@ -747,6 +747,27 @@ int bwd_launch(const SsArgs& a, dim3 grid, cudaStream_t st) {
   return check_launch("selective_scan_bwd_kernel");
 }
 
+// Chunks per CTA of the gradients: as many as leave about eight CTAs for every one that the GPU holds at a time (three per
+// SM), so that the last wave is short; more where few channels and many chunks would have more than about 192 CTAs add their
+// sums of dA and dD to the same addresses, down to about two CTAs per SM; at most 16 (a CTA's own start and its sums are
+// spread well enough over those).  us with 1 / 4 / 8 / 16: (256, 64, 64, 16) 191 / 80 / 61 / -, (8, 2048, 128, 16) 285 / 180 /
+// 183 / 174, (16, 512, 256, 16) 201 / 102 / 106 / 96, (8, 1024, 512, 16) 236 / 158 / 164 / 183, (8, 1024, 2048, 16) 502 / 451
+// / 446 / 448, (8, 128, 2048, 8) 63 / 63 / 73 / 74, (2, 333, 1030, 16) 45 / 42 / 55 / 75.
+int chunks_per_cta(int64_t groups, int64_t batch, int64_t chunks) {
+  int sms = 0, dev = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (sms <= 0) sms = 148;
+  const int64_t work = groups * batch * chunks, spread = batch * chunks / 192, filled = work / (2 * int64_t(sms));
+  int64_t per = work / (8 * 3 * int64_t(sms));
+  const int64_t shared = spread < filled ? spread : filled;
+  per = per < shared ? shared : per;
+  per = per < 1 ? 1 : (per > 16 ? 16 : per);
+  const int64_t least = (chunks + 65534) / 65535;   // (grid.y)
+  per = per < least ? least : per;
+  return int(per < chunks ? per : chunks);
+}
+
 // The two kernels of one range: `a` with its batch pointers at the range's first element.
 template <typename T, bool kRange>
 int bwd_range(const nb200_selective_scan_params* p, const SsArgs& a, Range r, cudaStream_t st) {
@@ -787,13 +808,7 @@ int bwd_t(const nb200_selective_scan_params* p, cudaStream_t st) {
   a.gck = reinterpret_cast<float*>(static_cast<char*>(p->workspace) + acc_bytes(p));
   if (p->batch > 0 && p->length > 0) {   // (nothing to walk otherwise: dA and dD are the zeros just written)
     const Range whole = range_of(p, (p->workspace_bytes - acc_bytes(p)) / sizeof(float));
-    // chunks per CTA: as many as leave about eight CTAs for every one that the GPU holds at a time (3 x 148), so that
-    // the last wave is short; at most 16 (a CTA's own start and its sums of dA are spread well enough over those)
-    const int64_t groups = (whole.channels + kBwdCh - 1) / kBwdCh;
-    int64_t per = groups * whole.batch * a.chunks / (8 * 3 * 148);
-    per = per < 1 ? 1 : (per > 16 ? 16 : per);
-    const int64_t least = (int64_t(a.chunks) + 65534) / 65535;   // (grid.y)
-    a.per_cta = int(per < least ? least : per);
+    a.per_cta = chunks_per_cta((whole.channels + kBwdCh - 1) / kBwdCh, whole.batch, a.chunks);
     a.gD = whole.channels;
     for (int b = 0; b < p->batch; b += whole.batch) {
       SsArgs part = a;

@@ -127,3 +127,9 @@ def test_a_device_without_room_for_all_adjoint_states_runs_in_ranges(monkeypatch
 def test_sequences_that_end_inside_a_staged_chunk(length):
     # steps are staged by sixteen and taken by four; groups past the end are left out
     _run((3,), length, 72, 16, torch.float32)
+
+
+@pytest.mark.parametrize("batch,length,d,n", [(256, 33, 20, 16), (300, 70, 64, 33)])
+def test_many_sequences_of_few_channels(batch, length, d, n):
+    # several chunks per CTA so that fewer CTAs add to the same sums of dA and dD, the last CTA of a sequence with fewer
+    _run((batch,), length, d, n, torch.float32)
