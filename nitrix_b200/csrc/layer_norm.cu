@@ -11,10 +11,10 @@
 // Rows that are a multiple of 16 bytes (<= 8192 channels, aligned pointers) take the vector kernels below; the rest
 // the scalar ones at the end.  The op is bound by HBM traffic (x once in, y once out; the backward x and dy in, dx
 // out), so a row is read ONCE with 16-byte loads and held in registers between the reductions and the write: by one
-// warp (rows of up to 32 x 16 B x 8) or by one 256-thread CTA (longer rows); the backward see there.  The variance is taken about the mean
-// (two passes over the registers, as the reference's `var` does), not as E[x^2] - mean^2.  dw / db: every CTA walks
-// rows in a grid-stride loop, keeps its column sums in registers, leaves one partial row per CTA in a
-// workspace, and a second kernel adds the partials in a fixed order -- deterministic, no atomics.
+// warp (rows of up to 32 x 16 B x 8) or by one 256-thread CTA (longer rows); the backward has two kernels, see there.  The
+// variance is taken about the mean (two passes over the registers, as the reference's `var` does), not as E[x^2] - mean^2.
+// dw / db: every CTA walks rows in a grid-stride loop, keeps its column sums in registers or shared memory, leaves one partial
+// row per CTA in a workspace, and a second kernel adds the partials in a fixed order -- deterministic, no atomics.
 #include <math.h>
 
 #include "nitrix_b200_norm.h"
@@ -84,6 +84,21 @@ __device__ __forceinline__ float2 row_sum2(float a, float b, float* red) {
   return make_float2(a, b);
 }
 
+template <typename T, int kVec>
+__device__ __forceinline__ void load_vec(const T* p, float (&out)[kVec]) {
+  const uint4 w = *reinterpret_cast<const uint4*>(p);
+  const T* e = reinterpret_cast<const T*>(&w);
+#pragma unroll
+  for (int i = 0; i < kVec; ++i) out[i] = to_f32<T>(e[i]);
+}
+template <typename T, int kVec>
+__device__ __forceinline__ void store_vec(T* p, const float (&v)[kVec]) {
+  uint4 w;
+  T* e = reinterpret_cast<T*>(&w);
+#pragma unroll
+  for (int i = 0; i < kVec; ++i) e[i] = from_f32<T>(v[i]);
+  *reinterpret_cast<uint4*>(p) = w;
+}
 // The same as pairs: the arithmetic below runs on the packed fp32x2 pipe (one instruction per two elements; each
 // lane rounds as the scalar instruction would, so results do not change).  At 16-bit widths the kernels are bound
 // by instruction issue as much as by memory.
@@ -232,7 +247,7 @@ struct BwdRing {
 };
 
 template <typename T, int kPer>
-__global__ void __launch_bounds__(kRowThreads, kPer == 1 ? 2 : 1) ln_bwd_kernel(LnArgs a, int tpr) {
+__global__ void __launch_bounds__(kRowThreads, kPer == 1 ? 2 : 1) ln_bwd_ring_kernel(LnArgs a, int tpr) {
   constexpr int kVec = 16 / int(sizeof(T));
   constexpr int kPairs = kVec / 2;
   constexpr int kBatch = BwdRing<kPer>::kBatch, kAhead = BwdRing<kPer>::kAhead;
@@ -375,15 +390,28 @@ __global__ void __launch_bounds__(kRowThreads, kPer == 1 ? 2 : 1) ln_bwd_kernel(
     part = part == kAhead ? 0 : part + 1;
   }
   if (!a.part) return;
-  // this CTA's partial row: the groups' sums added in group order, through the ring's memory
+  // this CTA's partial row: the groups' sums added in group order, those of a warp by shuffles, then through the ring's memory
+  for (int o = tpr; o < 32; o <<= 1) {
+#pragma unroll
+    for (int p = 0; p < kPer; ++p) {
+#pragma unroll
+      for (int i = 0; i < kPairs; ++i) {
+        sw[p][i].x += __shfl_xor_sync(0xffffffffu, sw[p][i].x, o);
+        sw[p][i].y += __shfl_xor_sync(0xffffffffu, sw[p][i].y, o);
+        sb[p][i].x += __shfl_xor_sync(0xffffffffu, sb[p][i].x, o);
+        sb[p][i].y += __shfl_xor_sync(0xffffffffu, sb[p][i].y, o);
+      }
+    }
+  }
+  const int owners = tpr < 32 ? kWarps : groups, owner = tpr < 32 ? tid >> 5 : group;
   asm volatile("cp.async.wait_all;" ::: "memory");
   __syncthreads();
-  float* all = reinterpret_cast<float*>(ring);                 // [dw, db][groups][C]
-  float* mine_w = all + int64_t(group) * a.C;
-  float* mine_b = all + int64_t(groups + group) * a.C;
+  float* all = reinterpret_cast<float*>(ring);                 // [dw, db][owners][C]
+  float* mine_w = all + int64_t(owner) * a.C;
+  float* mine_b = all + int64_t(owners + owner) * a.C;
 #pragma unroll
   for (int p = 0; p < kPer; ++p) {
-    if (chunk(p) < a.C) {
+    if (chunk(p) < a.C && (tid & 31) < tpr) {
 #pragma unroll
       for (int i = 0; i < kPairs; i += 2) {
         *reinterpret_cast<float4*>(mine_w + chunk(p) + 2 * i) = make_float4(sw[p][i].x, sw[p][i].y, sw[p][i + 1].x, sw[p][i + 1].y);
@@ -396,21 +424,141 @@ __global__ void __launch_bounds__(kRowThreads, kPer == 1 ? 2 : 1) ln_bwd_kernel(
   float* pb = a.part + (int64_t(gridDim.x) + blockIdx.x) * a.C;
   for (int c = tid; c < a.C; c += kRowThreads) {
     float tw = 0.f, tb = 0.f;
-    for (int k = 0; k < groups; ++k) {
+    for (int k = 0; k < owners; ++k) {
       tw += all[int64_t(k) * a.C + c];
-      tb += all[int64_t(groups + k) * a.C + c];
+      tb += all[int64_t(owners + k) * a.C + c];
     }
     pw[c] = tw;
     pb[c] = tb;
   }
 }
 
-// dw[c] = sum over the CTAs' partial rows.  A CTA takes 32 columns (lane = column: 128-byte reads); its eight warps
-// take the partial rows in turn, four loads in flight each, and their eight sums are added in warp order -- the
-// order of the whole sum is fixed by (grid, column) alone.
+// The other backward kernel: small CTAs with little to set up, for few rows and for rows that would leave the threads
+// above without a chunk.  Grid-stride over rows (a warp's or a CTA's).  The column sums of dw, db live in shared memory, every
+// thread adding only to its own columns (in registers they cost 2 x kPer x kVec registers and left one CTA per SM).
+template <typename T, int kPer, bool kCta>
+__global__ void __launch_bounds__(kThreads) ln_bwd_row_kernel(LnArgs a) {
+  constexpr int kVec = 16 / int(sizeof(T));
+  constexpr int kTpr = kCta ? kThreads : 32;
+  constexpr int kRowsPerCta = kCta ? 1 : kThreads / 32;
+  // [2][kRowsPerCta][kPad]: dw sums, then db sums, per row owner.  Column c of an owner sits at slot(c): the two
+  // 16-byte halves of a 16-bit thread's chunk go to separate planes, so that the threads of a quarter-warp touch
+  // consecutive 16-byte words (bank-conflict free) when they update their sums.
+  extern __shared__ __align__(16) float wsum[];
+  constexpr int kPad = kPer * kTpr * kVec;
+  auto slot4 = [](int p, int i4, int tin_) { return ((p * (kVec / 4) + i4) * kTpr + tin_) * 4; };
+  __shared__ float red[4 * (kThreads / 32)];   // two uses of 16 floats, alternating by row
+  const int tin = kCta ? threadIdx.x : (threadIdx.x & 31);
+  const int sub = kCta ? 0 : (threadIdx.x >> 5);
+  int flip = 0;
+  const T* w = reinterpret_cast<const T*>(a.w);
+  float* sw = wsum + sub * kPad;
+  float* sb = wsum + (kRowsPerCta + sub) * kPad;
+  const bool sums = a.part != nullptr;
+  if (sums) {
+#pragma unroll
+    for (int p = 0; p < kPer; ++p) {
+      const int c0 = (p * kTpr + tin) * kVec;
+      if (c0 < a.C) {
+#pragma unroll
+        for (int i = 0; i < kVec; i += 4) {
+          *reinterpret_cast<float4*>(sw + slot4(p, i / 4, tin)) = make_float4(0.f, 0.f, 0.f, 0.f);
+          *reinterpret_cast<float4*>(sb + slot4(p, i / 4, tin)) = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+      }
+    }
+  }
+  // (in a CTA-per-row kernel every thread of the CTA runs the same number of iterations: the barriers in row_sum match)
+  for (int64_t row = int64_t(blockIdx.x) * kRowsPerCta + sub; row < a.rows; row += int64_t(gridDim.x) * kRowsPerCta) {
+    const T* x = reinterpret_cast<const T*>(a.x) + row * a.C;
+    const T* g = reinterpret_cast<const T*>(a.dy) + row * a.C;
+    const float mean = a.mean[row], rstd = a.rstd[row];
+    float xh[kPer][kVec], dxh[kPer][kVec];
+    float s1 = 0.f, s2 = 0.f;
+#pragma unroll
+    for (int p = 0; p < kPer; ++p) {
+      const int c0 = (p * kTpr + tin) * kVec;
+      if (c0 < a.C) {
+        load_vec<T, kVec>(x + c0, xh[p]);
+        load_vec<T, kVec>(g + c0, dxh[p]);
+      }
+    }
+#pragma unroll
+    for (int p = 0; p < kPer; ++p) {
+      const int c0 = (p * kTpr + tin) * kVec;
+      if (c0 < a.C) {
+        float wv[kVec];
+        if (w) load_vec<T, kVec>(w + c0, wv);   // (a few KB that stay in L1)
+#pragma unroll
+        for (int i = 0; i < kVec; i += 4) {
+          float4 aw, ab;
+          if (sums) {
+            aw = *reinterpret_cast<const float4*>(sw + slot4(p, i / 4, tin));
+            ab = *reinterpret_cast<const float4*>(sb + slot4(p, i / 4, tin));
+          }
+          float* pw = reinterpret_cast<float*>(&aw);
+          float* pb = reinterpret_cast<float*>(&ab);
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const float xhv = (xh[p][i + u] - mean) * rstd;
+            const float gy = a.out_scale * dxh[p][i + u];
+            pw[u] = fmaf(gy, xhv, pw[u]);
+            pb[u] += gy;
+            const float d = w ? gy * wv[i + u] : gy;
+            xh[p][i + u] = xhv;
+            dxh[p][i + u] = d;
+            s1 += d;
+            s2 = fmaf(d, xhv, s2);
+          }
+          if (sums) {
+            *reinterpret_cast<float4*>(sw + slot4(p, i / 4, tin)) = aw;
+            *reinterpret_cast<float4*>(sb + slot4(p, i / 4, tin)) = ab;
+          }
+        }
+      }
+    }
+    const float2 cs = row_sum2<kCta>(s1, s2, red + 16 * flip);
+    flip ^= 1;
+    const float c1 = cs.x / float(a.C), c2 = cs.y / float(a.C);
+    T* dx = reinterpret_cast<T*>(a.dx) + row * a.C;
+#pragma unroll
+    for (int p = 0; p < kPer; ++p) {
+      const int c0 = (p * kTpr + tin) * kVec;
+      if (c0 < a.C) {
+        float out[kVec];
+#pragma unroll
+        for (int i = 0; i < kVec; ++i) out[i] = rstd * (dxh[p][i] - c1 - xh[p][i] * c2);
+        store_vec<T, kVec>(dx + c0, out);
+      }
+    }
+  }
+  if (!sums) return;
+  // this CTA's partial row: the row owners' sums added in owner order
+  float* pw = a.part + int64_t(blockIdx.x) * a.C;
+  float* pb = a.part + (int64_t(gridDim.x) + blockIdx.x) * a.C;
+  __syncthreads();
+  for (int c = threadIdx.x; c < a.C; c += kThreads) {
+    const int chunk = c / kVec, i = c % kVec;
+    const int at = slot4(chunk / kTpr, i / 4, chunk % kTpr) + (i & 3);
+    float tw = 0.f, tb = 0.f;
+#pragma unroll
+    for (int k = 0; k < kRowsPerCta; ++k) {
+      tw += wsum[k * kPad + at];
+      tb += wsum[(kRowsPerCta + k) * kPad + at];
+    }
+    pw[c] = tw;
+    pb[c] = tb;
+  }
+}
+
+// dw[c] = sum over the CTAs' partial rows.  A CTA takes 32 columns (lane = column: 128-byte reads); its 32 warps
+// take the partial rows in turn, four loads in flight each, and their sums are added in warp order -- the
+// order of the whole sum is fixed by (grid, column) alone.  Bound by the latency of a warp's loads: with eight warps (five
+// rounds of four at 148 partial rows, ten at 296) 4.5 to 7 us, with 32 two to three.
+constexpr int kFinishThreads = 1024;
 template <typename T>
-__global__ void __launch_bounds__(kThreads) ln_bwd_finish_kernel(const float* part, int grid, int C, T* dw, T* db) {
-  __shared__ float sw[kThreads / 32][32], sb[kThreads / 32][32];
+__global__ void __launch_bounds__(kFinishThreads) ln_bwd_finish_kernel(const float* part, int grid, int C, T* dw, T* db) {
+  __shared__ float sw[kFinishThreads / 32][32], sb[kFinishThreads / 32][32];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int c = blockIdx.x * 32 + lane;
   float tw[4] = {0.f, 0.f, 0.f, 0.f}, tb[4] = {0.f, 0.f, 0.f, 0.f};
@@ -418,14 +566,14 @@ __global__ void __launch_bounds__(kThreads) ln_bwd_finish_kernel(const float* pa
     const float* pw = part + c;
     const float* pb = part + int64_t(grid) * C + c;
     int k = warp;
-    for (; k + 3 * (kThreads / 32) < grid; k += 4 * (kThreads / 32)) {
+    for (; k + 3 * (kFinishThreads / 32) < grid; k += 4 * (kFinishThreads / 32)) {
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
-        tw[u] += pw[int64_t(k + u * (kThreads / 32)) * C];
-        tb[u] += pb[int64_t(k + u * (kThreads / 32)) * C];
+        tw[u] += pw[int64_t(k + u * (kFinishThreads / 32)) * C];
+        tb[u] += pb[int64_t(k + u * (kFinishThreads / 32)) * C];
       }
     }
-    for (; k < grid; k += kThreads / 32) {
+    for (; k < grid; k += kFinishThreads / 32) {
       tw[0] += pw[int64_t(k) * C];
       tb[0] += pb[int64_t(k) * C];
     }
@@ -436,7 +584,7 @@ __global__ void __launch_bounds__(kThreads) ln_bwd_finish_kernel(const float* pa
   if (warp == 0 && c < C) {
     float a = 0.f, b = 0.f;
 #pragma unroll
-    for (int i = 0; i < kThreads / 32; ++i) {
+    for (int i = 0; i < kFinishThreads / 32; ++i) {
       a += sw[i][lane];
       b += sb[i][lane];
     }
@@ -517,21 +665,23 @@ struct Shape {
   bool cta;
 };
 
-// Forward: the smallest per-thread chunk count that covers a row.
-bool pick(int C, int dtype, Shape* s) {
+// Forward and the row-wise backward: the smallest per-thread chunk count that covers a row (the backward keeps twice the
+// registers per chunk).
+bool pick(int C, int dtype, bool backward, Shape* s) {
   s->vec = dtype == NB200_F32 ? 4 : 8;
-  if (C <= 0 || C % s->vec) return false;
-  for (int per = 1; per <= 8; per *= 2)
+  if (C <= 0 || C % s->vec || C > 8192) return false;
+  const int warp_max = backward ? 4 : 8;
+  for (int per = 1; per <= warp_max; per *= 2)
     if (C <= 32 * s->vec * per) { s->per = per; s->cta = false; return true; }
   for (int per = 1; per <= 8; per *= 2)
-    if (C <= kThreads * s->vec * per && C <= 8192) { s->per = per; s->cta = true; return true; }
+    if (C <= kThreads * s->vec * per) { s->per = per; s->cta = true; return true; }
   return false;
 }
 
-// Backward: chunks per thread (as few as cover a row with 512 threads: fewer registers, more rows per CTA) and
+// The ring backward: chunks per thread (as few as cover a row with 512 threads: fewer registers, more rows per CTA) and
 // threads per row.
-struct BwdShape { int per, tpr; };
-bool pick_bwd(int C, int dtype, BwdShape* s) {
+struct RingShape { int per, tpr; };
+bool pick_ring(int C, int dtype, RingShape* s) {
   const int vec = dtype == NB200_F32 ? 4 : 8;
   if (C <= 0 || C % vec || C > 8192) return false;
   s->per = 1;
@@ -541,16 +691,38 @@ bool pick_bwd(int C, int dtype, BwdShape* s) {
   return true;
 }
 
+// Which backward kernel.  The ring kernel has twice the bytes in flight and its sums in registers, but 512 threads and up to
+// 196 KB to set up per CTA, and threads that a row's chunks do not fill do nothing.  us, ring / row-wise (bf16 rows x
+// channels unless f32): 4096x64 6.7 / 7.2, 32768x128 12.7 / 15.9, 2048x64 6.4 / 5.5, 32768x256 18.1 / 16.6; 16384x1024
+// 32.6 / 34.6, 8192x1024 20.8 / 17.8, 16384x768 30.7 / 22.5, 8192x2048 33.0 / 32.1, f32 8192x2048 49.5 / 41.1; 4096x4096
+// 35.2 / 37.2, 2048x4096 22.6 / 18.0, 4096x4104 40.8 / 46.3, f32 4096x4104 47.4 / 48.8; 8192x8192 87 / 145, 1024x8192
+// 21.3 / 22.5, 256x8192 13.3 / 12.8, 2048x6144 26.4 / 30.4, f32 1024x4096 15.1 / 16.1, f32 4096x2056 31.9 / 28.4.
+bool ring_backward(int64_t rows, int C, int dtype, const RingShape& s) {
+  const int vec = dtype == NB200_F32 ? 4 : 8, words = C / vec;
+  if (words <= 16) return rows >= 4096;
+  if (s.per >= 2 && 4 * words >= 3 * s.per * s.tpr) return rows >= 1024;
+  if (C >= 4096) return rows >= 4096;
+  return vec == 8 && words > 112 && words <= 128 && rows >= 16384;   // (the row-wise kernel's widest warp rows)
+}
+
 // The backward's grid: as many CTAs as are resident at once (`per_sm` from the occupancy calculator; more CTAs only
-// add partial rows to sum), at most one per block of rows.  per_sm = 2 bounds it for sizing the workspace.
-int bwd_grid(int64_t rows, const BwdShape& s, int per_sm) {
+// add partial rows to sum), at most one per unit of `unit` rows.
+int bwd_grid(int64_t rows, int unit, int per_sm) {
   int sms = 0, dev = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (sms <= 0) sms = 148;
-  const int64_t groups = kRowThreads / s.tpr, units = (rows + groups - 1) / groups;
-  const int64_t cap = int64_t(sms) * per_sm;
+  const int64_t units = (rows + unit - 1) / unit, cap = int64_t(sms) * per_sm;
   return int(units < cap ? (units > 0 ? units : 1) : cap);
+}
+// its bounds, for sizing the workspace
+constexpr int kRingPerSm = 2, kRowsPerSm = 8;
+int row_unit(const Shape& s) { return s.cta ? 1 : kThreads / 32; }
+int bwd_grid_most(int64_t rows, int C, int dtype) {
+  RingShape ring;
+  Shape s;
+  if (!pick_ring(C, dtype, &ring) || !pick(C, dtype, true, &s)) return 1;
+  return ring_backward(rows, C, dtype, ring) ? bwd_grid(rows, kRowThreads / ring.tpr, kRingPerSm) : bwd_grid(rows, row_unit(s), kRowsPerSm);
 }
 
 int check_common(const nb200_layer_norm_params* p, const char* what) {
@@ -565,22 +737,22 @@ int check_common(const nb200_layer_norm_params* p, const char* what) {
   return NB200_OK;
 }
 
-template <typename T, typename F>
+template <typename T, bool kBwd, typename F>
 int dispatch(const Shape& s, F&& go) {
   // go(kernel) launches; one instantiation per (chunks, warp / CTA)
   if (!s.cta) {
     switch (s.per) {
-      case 1: return go(ln_fwd_kernel<T, 1, false>);
-      case 2: return go(ln_fwd_kernel<T, 2, false>);
-      case 4: return go(ln_fwd_kernel<T, 4, false>);
-      default: return go(ln_fwd_kernel<T, 8, false>);
+      case 1: return go(kBwd ? ln_bwd_row_kernel<T, 1, false> : ln_fwd_kernel<T, 1, false>);
+      case 2: return go(kBwd ? ln_bwd_row_kernel<T, 2, false> : ln_fwd_kernel<T, 2, false>);
+      case 4: return go(kBwd ? ln_bwd_row_kernel<T, 4, false> : ln_fwd_kernel<T, 4, false>);
+      default: return go(kBwd ? ln_bwd_row_kernel<T, 4, false> : ln_fwd_kernel<T, 8, false>);
     }
   }
   switch (s.per) {
-    case 1: return go(ln_fwd_kernel<T, 1, true>);
-    case 2: return go(ln_fwd_kernel<T, 2, true>);
-    case 4: return go(ln_fwd_kernel<T, 4, true>);
-    default: return go(ln_fwd_kernel<T, 8, true>);
+    case 1: return go(kBwd ? ln_bwd_row_kernel<T, 1, true> : ln_fwd_kernel<T, 1, true>);
+    case 2: return go(kBwd ? ln_bwd_row_kernel<T, 2, true> : ln_fwd_kernel<T, 2, true>);
+    case 4: return go(kBwd ? ln_bwd_row_kernel<T, 4, true> : ln_fwd_kernel<T, 4, true>);
+    default: return go(kBwd ? ln_bwd_row_kernel<T, sizeof(T) == 4 ? 8 : 4, true> : ln_fwd_kernel<T, 8, true>);
   }
 }
 
@@ -591,7 +763,7 @@ int fwd_t(const nb200_layer_norm_params* p, const Shape& s, cudaStream_t st) {
   a.rows = p->rows; a.C = p->channels; a.eps = p->eps; a.out_scale = p->out_scale;
   const int64_t blocks = s.cta ? p->rows : (p->rows + kThreads / 32 - 1) / (kThreads / 32);
   if (blocks > 0x7fffffff) { set_error("layer_norm: too many rows"); return NB200_ERR_UNSUPPORTED; }
-  return dispatch<T>(s, [&](auto kernel) {
+  return dispatch<T, false>(s, [&](auto kernel) {
     kernel<<<unsigned(blocks), kThreads, 0, st>>>(a);
     count_launch();
     return check_launch("layer_norm_fwd_kernel");
@@ -599,9 +771,9 @@ int fwd_t(const nb200_layer_norm_params* p, const Shape& s, cudaStream_t st) {
 }
 
 template <typename T, int kPer>
-int bwd_launch(const LnArgs& a, const BwdShape& s, int* grid, cudaStream_t st) {
+int ring_launch(const LnArgs& a, const RingShape& s, int* grid, cudaStream_t st) {
   constexpr size_t smem = BwdRing<kPer>::kBytes;
-  auto kernel = ln_bwd_kernel<T, kPer>;
+  auto kernel = ln_bwd_ring_kernel<T, kPer>;
   if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess) {
     set_error("layer_norm_bwd: cudaFuncSetAttribute(%zu): %s", smem, cudaGetErrorString(cudaGetLastError()));
     return NB200_ERR_LAUNCH;
@@ -611,21 +783,42 @@ int bwd_launch(const LnArgs& a, const BwdShape& s, int* grid, cudaStream_t st) {
     cudaGetLastError();
     per_sm = 1;
   }
-  *grid = bwd_grid(a.rows, s, per_sm < 2 ? per_sm : 2);
+  *grid = bwd_grid(a.rows, kRowThreads / s.tpr, per_sm < kRingPerSm ? per_sm : kRingPerSm);
   kernel<<<unsigned(*grid), kRowThreads, smem, st>>>(a, s.tpr);
   count_launch();
-  return check_launch("layer_norm_bwd_kernel");
+  return check_launch("layer_norm_bwd_ring_kernel");
 }
 
 template <typename T>
-int bwd_t(const nb200_layer_norm_params* p, const BwdShape& s, cudaStream_t st) {
+int row_launch(const LnArgs& a, const Shape& s, int* grid, cudaStream_t st) {
+  // (rows padded to the kernel's per * threads * vec columns)
+  const size_t smem = a.part ? sizeof(float) * 2 * row_unit(s) * size_t(s.per) * (s.cta ? kThreads : 32) * s.vec : 0;
+  return dispatch<T, true>(s, [&](auto kernel) {
+    if (smem > 48 * 1024 &&
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess) {
+      set_error("layer_norm_bwd: cudaFuncSetAttribute(%zu): %s", smem, cudaGetErrorString(cudaGetLastError()));
+      return int(NB200_ERR_LAUNCH);
+    }
+    int per_sm = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kThreads, smem) != cudaSuccess || per_sm < 1) {
+      cudaGetLastError();
+      per_sm = 1;
+    }
+    *grid = bwd_grid(a.rows, row_unit(s), per_sm < kRowsPerSm ? per_sm : kRowsPerSm);
+    kernel<<<unsigned(*grid), kThreads, smem, st>>>(a);
+    count_launch();
+    return check_launch("layer_norm_bwd_kernel");
+  });
+}
+
+template <typename T>
+int bwd_t(const nb200_layer_norm_params* p, const RingShape& ring, const Shape& s, cudaStream_t st) {
   LnArgs a{};
   a.x = p->x; a.w = p->weight; a.dy = p->dy; a.dx = p->dx; a.mean = p->mean; a.rstd = p->rstd;
   a.rows = p->rows; a.C = p->channels; a.eps = p->eps; a.out_scale = p->out_scale;
   const bool want_params = p->dweight || p->dbias;
-  int grid = bwd_grid(p->rows, s, 2);
   if (want_params) {
-    const size_t need = sizeof(float) * 2 * size_t(grid) * size_t(p->channels);
+    const size_t need = sizeof(float) * 2 * size_t(bwd_grid_most(p->rows, p->channels, p->dtype)) * size_t(p->channels);
     if (!p->workspace || p->workspace_bytes < need) {
       set_error("layer_norm_bwd: workspace of %zu bytes needed (nb200_layer_norm_workspace_bytes), %zu given", need,
                 size_t(p->workspace_bytes));
@@ -633,16 +826,18 @@ int bwd_t(const nb200_layer_norm_params* p, const BwdShape& s, cudaStream_t st) 
     }
     a.part = static_cast<float*>(p->workspace);
   }
-  int rc;
-  if (s.per == 1) {
-    rc = bwd_launch<T, 1>(a, s, &grid, st);
-  } else if (s.per == 2) {
-    rc = bwd_launch<T, 2>(a, s, &grid, st);
+  int rc, grid = 1;
+  if (!ring_backward(p->rows, p->channels, p->dtype, ring)) {
+    rc = row_launch<T>(a, s, &grid, st);
+  } else if (ring.per == 1) {
+    rc = ring_launch<T, 1>(a, ring, &grid, st);
+  } else if (ring.per == 2) {
+    rc = ring_launch<T, 2>(a, ring, &grid, st);
   } else {
-    rc = bwd_launch<T, sizeof(T) == 4 ? 4 : 2>(a, s, &grid, st);   // (four chunks: fp32 only)
+    rc = ring_launch<T, sizeof(T) == 4 ? 4 : 2>(a, ring, &grid, st);   // (four chunks: fp32 only)
   }
   if (rc || !want_params) return rc;
-  ln_bwd_finish_kernel<T><<<(p->channels + 31) / 32, kThreads, 0, st>>>(
+  ln_bwd_finish_kernel<T><<<(p->channels + 31) / 32, kFinishThreads, 0, st>>>(
       a.part, grid, p->channels, static_cast<T*>(p->dweight), static_cast<T*>(p->dbias));
   count_launch();
   return check_launch("layer_norm_bwd_finish_kernel");
@@ -684,7 +879,7 @@ int bwd_generic_t(const nb200_layer_norm_params* p, cudaStream_t st) {
   count_launch();
   if (int rc = check_launch("layer_norm_bwd_generic_kernel")) return rc;
   if (!want_params) return NB200_OK;
-  ln_bwd_finish_kernel<T><<<(p->channels + 31) / 32, kThreads, 0, st>>>(
+  ln_bwd_finish_kernel<T><<<(p->channels + 31) / 32, kFinishThreads, 0, st>>>(
       a.part, 1, p->channels, static_cast<T*>(p->dweight), static_cast<T*>(p->dbias));
   count_launch();
   return check_launch("layer_norm_bwd_finish_kernel");
@@ -692,12 +887,12 @@ int bwd_generic_t(const nb200_layer_norm_params* p, cudaStream_t st) {
 
 // the vector kernels need 16-byte rows: channels a multiple of 16 bytes (<= 8192) and aligned pointers
 bool vector_fwd(const nb200_layer_norm_params* p, Shape* s) {
-  return pick(p->channels, p->dtype, s) && aligned16(p->x) && (!p->weight || aligned16(p->weight)) && aligned16(p->y) &&
+  return pick(p->channels, p->dtype, false, s) && aligned16(p->x) && (!p->weight || aligned16(p->weight)) && aligned16(p->y) &&
          (!p->bias || aligned16(p->bias));
 }
-bool vector_bwd(const nb200_layer_norm_params* p, BwdShape* s) {
-  return pick_bwd(p->channels, p->dtype, s) && aligned16(p->x) && (!p->weight || aligned16(p->weight)) &&
-         aligned16(p->dy) && aligned16(p->dx);
+bool vector_bwd(const nb200_layer_norm_params* p, RingShape* ring, Shape* s) {
+  return pick_ring(p->channels, p->dtype, ring) && pick(p->channels, p->dtype, true, s) && aligned16(p->x) &&
+         (!p->weight || aligned16(p->weight)) && aligned16(p->dy) && aligned16(p->dx);
 }
 
 }  // namespace
@@ -709,8 +904,7 @@ extern "C" NB200_API int nb200_layer_norm_workspace_bytes(const nb200_layer_norm
   if (!bytes) { set_error("bytes out-pointer is NULL"); return NB200_ERR_INVALID; }
   if (int rc = check_common(p, "layer_norm_workspace_bytes")) return rc;
   // (sized for the vector kernels' per-CTA partial rows, which is never less than the scalar kernels' [2][C])
-  BwdShape s;
-  const int grid = pick_bwd(p->channels, p->dtype, &s) ? bwd_grid(p->rows, s, 2) : 1;
+  const int grid = bwd_grid_most(p->rows, p->channels, p->dtype);
   *bytes = sizeof(float) * 2 * size_t(grid) * size_t(p->channels);
   return NB200_OK;
 }
@@ -739,11 +933,12 @@ extern "C" NB200_API int nb200_layer_norm_bwd(const nb200_layer_norm_params* p, 
   }
   cudaStream_t st = static_cast<cudaStream_t>(cuda_stream);
   prof_call_begin(st);
-  BwdShape s;
-  const bool vec = vector_bwd(p, &s);
+  RingShape ring;
+  Shape s;
+  const bool vec = vector_bwd(p, &ring, &s);
   switch (p->dtype) {
-    case NB200_F32: return vec ? bwd_t<float>(p, s, st) : bwd_generic_t<float>(p, st);
-    case NB200_BF16: return vec ? bwd_t<__nv_bfloat16>(p, s, st) : bwd_generic_t<__nv_bfloat16>(p, st);
-    default: return vec ? bwd_t<__half>(p, s, st) : bwd_generic_t<__half>(p, st);
+    case NB200_F32: return vec ? bwd_t<float>(p, ring, s, st) : bwd_generic_t<float>(p, st);
+    case NB200_BF16: return vec ? bwd_t<__nv_bfloat16>(p, ring, s, st) : bwd_generic_t<__nv_bfloat16>(p, st);
+    default: return vec ? bwd_t<__half>(p, ring, s, st) : bwd_generic_t<__half>(p, st);
   }
 }
