@@ -46,18 +46,16 @@ __device__ __forceinline__ __nv_bfloat16 from_f<__nv_bfloat16>(float v) { return
 template <>
 __device__ __forceinline__ __half from_f<__half>(float v) { return __float2half_rn(v); }
 
-// A group of `kLanes` lanes (the power of two that covers a row with 16 bytes a lane, or two words of 16 bytes at fp32 and
-// head dims above 128) takes kRowsAhead rows, all of whose loads are issued before the first is used; the two tensors
+// A group of `kLanes` lanes (the power of two that covers a row with kPer words of 16 bytes a lane: two at fp32 and head dims
+// above 128) takes kRowsAhead rows, all of whose loads are issued before the first is used; the two tensors
 // have their own ranges of CTAs.  Bound by HBM.  One row per warp, whatever its length, left half of the lanes idle at
 // bf16 and head dim 128, four 64-bit divisions in front of a single load per lane, and took 40 us for the 85 MB of
 // (8, 16, 197 + 1111, 128).
-constexpr int kRowsAhead = 4;
 constexpr int kNormThreads = 256;
 
-template <typename T, bool kGrad, int kLanes>
+template <typename T, bool kGrad, int kLanes, int kPer, int kRowsAhead>
 __global__ void __launch_bounds__(kNormThreads) qk_rms_norm_kernel(NormTensor a, NormTensor b, int D, unsigned blocks_a) {
   constexpr int kVec = 16 / int(sizeof(T));
-  constexpr int kPer = sizeof(T) == 4 && kLanes == 32 ? 2 : 1;     // head dims up to 256
   constexpr int kGroups = kNormThreads / kLanes;
   const bool second = blockIdx.x >= blocks_a;
   const NormTensor& t = second ? b : a;
@@ -154,14 +152,28 @@ int check(const nb200_qk_norm_tensor& t, int D, int dtype, bool grad, const char
   return NB200_OK;
 }
 
-template <typename T, bool kGrad, int kLanes>
-int launch_lanes(const NormTensor& a, const NormTensor& b, int D, cudaStream_t st) {
+template <typename T, bool kGrad, int kLanes, int kPer, int kRowsAhead>
+int launch_rows(const NormTensor& a, const NormTensor& b, int D, cudaStream_t st) {
   constexpr int64_t kRows = kNormThreads / kLanes * kRowsAhead;     // rows of a CTA
   const int64_t blocks_a = (a.rows + kRows - 1) / kRows, blocks = blocks_a + (b.rows + kRows - 1) / kRows;
   if (blocks > 0x7fffffff) { set_error("qk_rms_norm: too many rows"); return NB200_ERR_UNSUPPORTED; }
-  qk_rms_norm_kernel<T, kGrad, kLanes><<<unsigned(blocks), kNormThreads, 0, st>>>(a, b, D, unsigned(blocks_a));
+  qk_rms_norm_kernel<T, kGrad, kLanes, kPer, kRowsAhead><<<unsigned(blocks), kNormThreads, 0, st>>>(a, b, D, unsigned(blocks_a));
   count_launch();
   return check_launch(kGrad ? "qk_rms_norm_grad_kernel" : "qk_rms_norm_kernel");
+}
+
+// Rows ahead: two; one where that leaves fewer than 512 CTAs, which a call that small waits for one by one; four for a large
+// fp32 forward, whose rows are not held up by conversions.  us with 1 / 2 / 4: bf16 D 64, 512 rows 2.2 / 2.3 / 3.4, gradient
+// 2.3 / 2.7 / 3.9; bf16 D 128, 167 000 rows 19.9 / 17.7 / 21.0, gradient 25.2 / 26.8 / 34.5; f32 D 128, 167 000 rows 38.5 /
+// 35.1 / 32.0, gradient 44.9 / 42.9 / 43.4, 32 000 rows 7.2 / 6.3 / 6.7.
+template <typename T, bool kGrad, int kLanes, int kPer = 1>
+int launch_lanes(const NormTensor& a, const NormTensor& b, int D, cudaStream_t st) {
+  const int64_t ctas = (a.rows + b.rows) / (kNormThreads / kLanes);
+  if (ctas < 512) return launch_rows<T, kGrad, kLanes, kPer, 1>(a, b, D, st);
+  if constexpr (sizeof(T) == 4 && !kGrad) {
+    if (ctas >= 8192) return launch_rows<T, kGrad, kLanes, kPer, 4>(a, b, D, st);
+  }
+  return launch_rows<T, kGrad, kLanes, kPer, 2>(a, b, D, st);
 }
 
 template <typename T, bool kGrad>
@@ -170,6 +182,9 @@ int launch_typed(const NormTensor& a, const NormTensor& b, int D, cudaStream_t s
   if (words <= 4) return launch_lanes<T, kGrad, 4>(a, b, D, st);
   if (words <= 8) return launch_lanes<T, kGrad, 8>(a, b, D, st);
   if (words <= 16) return launch_lanes<T, kGrad, 16>(a, b, D, st);
+  if constexpr (sizeof(T) == 4) {
+    if (words > 32) return launch_lanes<T, kGrad, 32, 2>(a, b, D, st);
+  }
   return launch_lanes<T, kGrad, 32>(a, b, D, st);
 }
 

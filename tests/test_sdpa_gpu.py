@@ -880,3 +880,13 @@ def test_gradient_of_a_bias_that_is_an_expanded_view(leaf, masked, dtype):
         total = total.sum(ax, keepdim=True) if n == 1 else total
     # (sums over keys cancel: the error is measured against the terms)
     assert float((dw.double() - total).norm()) <= tol * float(want.norm()) * max(1.0, (want.numel() / dw.numel()) ** 0.5)
+
+
+@pytest.mark.parametrize("dtype,d", [(torch.bfloat16, 32), (torch.bfloat16, 256), (torch.float32, 64), (torch.float32, 128),
+                                     (torch.float32, 256)])
+@pytest.mark.parametrize("n", [4093, 21850, 87400])
+def test_qk_norm_rows_ahead(dtype, d, n):
+    # one, two and (fp32 forward) four rows at a time per group of lanes, the last CTA cut short
+    if n * d > 87400 * 128:
+        n = n // 3 + 1
+    test_qk_norm_lane_groups(dtype, d, n)
