@@ -2,7 +2,7 @@
 // into the six bf16 products that matter.
 //
 //   x = x0 + x1 + x2 exactly (8 significant bits each, by truncation: x0 the top 16 bits of x, x1 the top 16 of x - x0,
-//   x2 the rest), and a b = a0 b0 + a0 b1 + a1 b0 + a1 b1 + a0 b2 + a2 b0 but for a1 b2 + a2 b1 + a2 b2, which is below
+//   x2 the rest; below 2^-103 the last ones are subnormal and flushed, as a TF32 pair's are), and a b = a0 b0 + a0 b1 + a1 b0 + a1 b1 + a0 b2 + a2 b0 but for a1 b2 + a2 b1 + a2 b2, which is below
 //   2^-20 |a b| and 2^-22 of it on average; the products are exact and are accumulated in fp32 by the tensor core, the
 //   small ones first.
 //
@@ -470,7 +470,8 @@ __global__ void __launch_bounds__(FwdLayout<kCols, kAdd>::kThreads, 1) fwd_fp32_
 // warp 9 issues the products, warp 10 the accumulates (a step is 72 or 96 MMA instructions, and one thread issuing them
 // all would take longer than the tensor core).  S and dP go to registers at once, so the next step's products run under
 // this step's arithmetic.  As in the forward the accumulators are emptied every other step into fp32 sums: dq's in
-// registers, dk's in shared memory, dv's in TMEM (what each kernel has left).  Every sum is added in a fixed order.
+// registers, dk's in shared memory, dv's in TMEM (what each kernel has left).  Those and a dense dbias are summed in a
+// fixed order; a broadcast bias' gradient is added by many CTAs with fp32 atomics.
 // B8 H16 S1024 D64, both kernels and the planes: 2019 us on mma.sync, here 679 -- query-major 241 (302 with q and dout in
 // shared memory), key-major 403 (a step's 48 products at 48 cycles and 48 accumulates at 32 are 224 us).
 struct BwdArgs {
@@ -983,25 +984,44 @@ bool takes(const Problem& pr) {
 }
 // a bias or a mask that has to be read per query
 bool row_addends(const Problem& pr) { return (pr.bias && pr.bs[2] != 0) || (pr.mask && pr.ms[2] != 0); }
+int64_t owners_of(int rows) { return (int64_t(rows) + 127) / 128; }
 }  // namespace
 
 // Where these kernels win over the mma.sync ones.  A CTA here is 128 rows and has an SM to itself, and a call costs a launch
 // for the planes; the others run 64-row CTAs, several to an SM, and split the keys of a small problem over warps or
-// clusters.  So: enough 64-row tiles for the SMs, enough work behind the start, more at head dim 32 (padded to 64 here) and
-// with a bias or a mask per query (read by the warps that do the soft-max).  Forward, us, here / there (D 64 unless said):
-//   B1 H1 S1536 40 / 26, B1 H4 S1024 31 / 31, the same causal with a key mask 50 / 37, B2 H4 S256 bias, mask 27 / 18,
-//   B8 H8 S128 12.6 / 9.4, B64 H8 S64 33 / 17, B32 H16 S64 T512 121 / 93, B8 H16 S17 T1000 78 / 53, B2 H8 S512 D32 bias 51 / 24, B1 H8 S1024 D32 31 / 26  <  the line  <
-//   B4 H8 S256 15.4 / 15.7, with key bias and mask 19.9 / 20.1, B8 H8 S192 15 / 23, B4 H6 S344 18 / 21, B1 H8 S1024 31 / 45,
-//   B8 H8 S256 D32 17 / 18, B16 H8 S200 bias 42 / 74, B8 H8 S300 T700 key bias and mask 56 / 184, B8 H16 S1024 208 / 603,
-//   the same with a key mask 293 / 810, causal with bias 390 / 775; D 128: B1 H1 S128 T1536 84 / 147, B32 H8 S64 26 / 19,
-//   B16 H8 S20 T300 39 / 35, B4 H8 S48 T700 49 / 71, B1 H4 S512 35 / 53, B2 H8 S1536 184 / 449.
+// clusters.  So: enough tiles for the SMs, enough work behind the start, more with a bias or a mask per query (read by the
+// warps that do the soft-max).  Half of the tensor work at head dim 32 is padding to 64, and the others gain most of that
+// back unless the addends, which cost them more, are both there.  Forward, us, here / there:
+//  D 64: B1 H1 S1536 40 / 26, B1 H4 S1024 31 / 31, the same causal with a key mask 50 / 37, B2 H4 S256 bias, mask 27 / 18,
+//   B8 H8 S128 12.6 / 9.4, B64 H8 S64 33 / 17, B32 H16 S64 T512 121 / 93, B8 H16 S17 T1000 78 / 53, B24 H8 S128 24.4 / 22.5
+//   <  the line  <  B4 H8 S256 15.4 / 15.7, with key bias and mask 19.9 / 20.1, B8 H8 S192 15 / 23, B4 H6 S344 18 / 21, B16 H8
+//   S128 14 / 16, B1 H8 S1024 31 / 45, B16 H8 S200 bias 42 / 74, B8 H8 S300 T700 key bias and mask 56 / 184, B8 H16 S1024 208
+//   / 603, the same with a key mask 293 / 810, causal with bias 390 / 775
+//  D 32: B4 H8 S512 bias 57 / 46, B24 H8 S192 34 / 22, B16 H8 S100 T1500 75 / 70, B6 H8 S512 T100 30 / 22, B4 H8 S200 bias and
+//   mask 1.6 times, causal B32 H8 S344 1.18  <  the line  <  B4 H8 S512 22.5 / 28.9, B4 H8 S344 0.76 times (B12 H8 1.07), B4 H8 S1024 49.6 / 93.8, with bias 0.8 times, B16 H8 S512 bias 0.85
+//   times, B12 H8 S256 bias and mask 0.7 times, B16 H8 S200 key bias and mask 28.6 / 36.7
+//  D 128: B1 H1 S33 T65 5.2 / 5.6; 128 pairs of S40 T80 20.6 / 16.8, S48 T300 41.7 / 36.3, S48 T1000 124.6 / 105.8; B32 H8 S64
+//   T64 26 / 19  <  the line  <  32 pairs of S48 T300 0.77 times, 128 with bias 0.97, B1 H1 S128 T1536 84 / 147, B4 H8 S48 T700
+//   49 / 71, B1 H4 S512 35 / 53, B2 H8 S1536 184 / 449.
 bool fp32_tc_fwd_applies(const Problem& pr) {
   if (!takes(pr) || pr.T <= kRows) return false;
-  if (pr.D == 128) return pr.S > kRows / 2;
+  const bool none = !pr.bias && !pr.mask;
+  const int64_t owners = owners_of(pr.S) * pr.bh_count, area = int64_t(pr.S) * pr.T;
+  if (pr.D == 128) {
+    if (pr.S <= kRows / 2) return false;
+    return pr.S > kRows || owners <= 64 || (!none && pr.T >= 256);
+  }
   if (pr.S <= kRows) return false;   // (half of a 128-row tile at least would be padding)
+  if (pr.D == 32) {
+    const int least = pr.S < pr.T ? pr.S : pr.T;
+    if (pr.bias && pr.mask) return least > 128 && area >= 40000 && owners >= (row_addends(pr) ? 192 : 96);
+    if (row_addends(pr)) return least >= 300 && pr.S >= 512 && owners >= 192;
+    return least >= 200 && (pr.causal ? area / 2 : area) >= 100000 && owners >= 96;
+  }
   const int64_t ctas = tiles_of(pr.S) * pr.bh_count, work = ctas * tiles_of(pr.T);
   if (row_addends(pr)) return ctas >= 192 && work >= 1024;
-  return pr.D == 64 ? ctas >= 128 && work >= 512 : ctas >= 192 && work >= 1024;
+  if (none && pr.S <= 128 && pr.T <= 128 && pr.bh_count > 148) return false;   // (short CTAs in more than one wave)
+  return ctas >= 128 && work >= 512;
 }
 
 size_t fp32_tc_fwd_bytes(const Problem& pr) {
@@ -1048,13 +1068,23 @@ int fp32_tc_forward(const Problem& pr, int bias_dtype, void* ws, cudaStream_t st
 
 // Head dim 128 stays with the other kernels: the planes of an owner's two operands would be 192 KB of shared memory.
 // Backward, us, here / there (D 64 unless said): B1 H1 S1536 120 / 67, B2 H4 S256 bias, mask 73 / 33, B64 H8 S64 81 / 60,
-//   B4 H8 S256 D32 35 / 33, B2 H8 S512 D32 bias 118 / 89  <  the line  <  B2 H8 S256 38 / 40, B1 H4 S1024 89 / 95,
-//   B8 H8 S128 31 / 33, B32 H8 S96 60 / 93, B4 H6 S344 49 / 69, B8 H8 S256 D32 38 / 50, B16 H8 S200 bias 129 / 250,
-//   B8 H16 S1024 679 / 2019, the same causal with bias 917 / 2366, B8 H8 S300 T700 key bias 153 / 486.
+//   B4 H8 S65 26 / 23, B4 H8 S128 31 / 29, B4 H8 S256 D32 35 / 33, B2 H8 S512 D32 bias 118 / 89, D32: B12 H8 S192 57 / 42, B24 H8
+//   S160 87 / 73, causal B32 H8 S128 56 / 44, B12 H8 S160 mask 74 / 57
+//   <  the line  <  B2 H8 S256 38 / 40, B1 H4 S1024 89 / 95, B8 H8 S128 31 / 33, B32 H8 S96 60 / 93, B4 H6 S344 49 / 69, D32:
+//   B6 H8 S256 0.76 times, B4 H8 S344 0.68, B8 H8 S192 0.84, B12 H8 S128 bias 0.81; B16 H8 S200 bias 129 / 250, B8 H16 S1024 679 / 2019, the same
+//   causal with bias 917 / 2366, B8 H8 S300 T700 key bias 153 / 486.
 bool fp32_tc_bwd_applies(const Problem& pr) {
   if (!takes(pr) || pr.D == 128 || pr.T <= kRows || pr.S <= kRows) return false;
   const int64_t ctas = (tiles_of(pr.S) < tiles_of(pr.T) ? tiles_of(pr.S) : tiles_of(pr.T)) * pr.bh_count;
-  return ctas >= (row_addends(pr) || pr.D == 32 ? 192 : 64);
+  const bool none = !pr.bias && !pr.mask, one_tile = pr.S <= 128 && pr.T <= 128;
+  if (pr.D == 32) {
+    // (a small problem that just starts a second wave of CTAs waits for it as long as for the first)
+    const int64_t owners = owners_of(pr.S > pr.T ? pr.S : pr.T) * pr.bh_count;
+    if (ctas < 192) return false;
+    if (int64_t(pr.S) * pr.T >= 40000 || owners <= 148) return true;
+    return !none && (!row_addends(pr) || one_tile || owners >= 222);
+  }
+  return ctas >= (row_addends(pr) ? 192 : (none && one_tile ? 96 : 64));
 }
 
 size_t fp32_tc_bwd_bytes(const Problem& pr) {

@@ -101,6 +101,43 @@ def test_against_fp64(B, H, S, T, D, causal, bias, mask, layout):
             assert _err(a, r) <= (5e-3 if a.dtype != torch.float32 else (_BOUND if tc_backward else 1e-4)), name
 
 
+@pytest.mark.parametrize("B,H,S,T,D,kind,fwd,bwd", [
+    # each line of the two rules from both sides: (forward, backward) on these kernels?
+    (3, 8, 128, 128, 64, "none", False, False), (6, 8, 128, 128, 64, "none", False, True), (16, 8, 128, 128, 64, "none", True, True),
+    (24, 8, 128, 128, 64, "none", False, True), (24, 8, 128, 128, 64, "key", True, True),
+    (12, 8, 192, 192, 32, "none", False, False), (8, 8, 192, 192, 32, "none", False, True), (8, 8, 200, 200, 32, "none", False, True),
+    (4, 8, 344, 344, 32, "none", True, True), (4, 8, 512, 100, 32, "none", False, False), (12, 8, 160, 160, 32, "mask", False, False),
+    (12, 8, 128, 128, 32, "mask", False, True), (4, 8, 512, 512, 32, "mask", False, True), (6, 8, 512, 512, 32, "mask", True, True),
+    (12, 8, 200, 200, 32, "both", True, True), (3, 8, 200, 200, 32, "both", False, False),
+    (16, 8, 40, 80, 128, "none", False, False), (8, 8, 40, 80, 128, "none", True, False), (16, 8, 48, 300, 128, "mask", True, False),
+])
+def test_both_sides_of_the_lines_between_the_fp32_kernels(B, H, S, T, D, kind, fwd, bwd):
+    from nitrix_b200 import _cabi
+    from nitrix_b200.nn import attention as att
+
+    g = torch.Generator(device="cuda").manual_seed(S + T)
+    q, k, v, dout = (torch.randn(B, H, n, D, device="cuda", generator=g) for n in (S, T, T, S))
+    bias = torch.randn(B, H, S, T, device="cuda", generator=g) if kind == "both" else None
+    mask = None
+    if kind != "none":
+        mask = torch.rand((B, 1, 1 if kind == "key" else S, T), device="cuda", generator=g) > 0.2
+        mask[..., 0] = True
+    L = _cabi.lib()
+    L.nb200_profile(1)
+    out, lse = att.sdpa_forward(q, k, v, bias, mask, scale=D ** -0.5)
+    grads = att.sdpa_backward(q, k, v, bias, mask, out, lse, dout, scale=D ** -0.5, want_dbias=bias is not None)
+    torch.cuda.synchronize()
+    ran = set(_cabi.kernel_times())
+    L.nb200_profile(0)
+    assert ("fwd_fp32_tc_kernel" in ran) == fwd and ("bwd_dkv_fp32_tc_kernel" in ran) == bwd, ran
+    want = _reference(q, k, v, bias, mask, False, D ** -0.5, dout)
+    # (the mma.sync kernels have the fp32 budget of 1e-4)
+    assert _err(out, want[0]) <= (_BOUND if fwd else 1e-4)
+    for a, r in zip(grads, want[1:]):
+        if r is not None:
+            assert _err(a, r) <= (_BOUND if fwd and bwd else 1e-4)
+
+
 def test_a_problem_whose_planes_exceed_their_limit_runs_in_ranges():
     # 1100 pairs of S = T = 1024 make 1.2 GiB (forward) and 1.6 GiB (backward) of planes: two ranges each
     from nitrix_b200.nn import attention as att
