@@ -551,12 +551,11 @@ __global__ void __launch_bounds__(kThreads) ln_bwd_row_kernel(LnArgs a) {
   }
 }
 
-// dw[c] = sum over the CTAs' partial rows.  A CTA takes 32 columns (lane = column: 128-byte reads); its 32 warps
+// dw[c] = sum over the CTAs' partial rows.  A CTA takes 32 columns (lane = column: 128-byte reads); its warps
 // take the partial rows in turn, four loads in flight each, and their sums are added in warp order -- the
 // order of the whole sum is fixed by (grid, column) alone.  Bound by the latency of a warp's loads: with eight warps (five
-// rounds of four at 148 partial rows, ten at 296) 4.5 to 7 us, with 32 two to three.
-constexpr int kFinishThreads = 1024;
-template <typename T>
+// rounds of four at 148 partial rows, ten at 296) 4.5 to 7 us, with 32 two to three; up to 128 rows eight start sooner.
+template <typename T, int kFinishThreads>
 __global__ void __launch_bounds__(kFinishThreads) ln_bwd_finish_kernel(const float* part, int grid, int C, T* dw, T* db) {
   __shared__ float sw[kFinishThreads / 32][32], sb[kFinishThreads / 32][32];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -656,6 +655,15 @@ __global__ void __launch_bounds__(kThreads) ln_bwd_generic_kernel(LnArgs a) {
       }
     }
   }
+}
+
+template <typename T>
+int finish_launch(const nb200_layer_norm_params* p, const float* part, int grid, cudaStream_t st) {
+  auto kernel = grid > 128 ? ln_bwd_finish_kernel<T, 1024> : ln_bwd_finish_kernel<T, 256>;
+  kernel<<<(p->channels + 31) / 32, grid > 128 ? 1024 : 256, 0, st>>>(part, grid, p->channels, static_cast<T*>(p->dweight),
+                                                                      static_cast<T*>(p->dbias));
+  count_launch();
+  return check_launch("layer_norm_bwd_finish_kernel");
 }
 
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
@@ -837,10 +845,7 @@ int bwd_t(const nb200_layer_norm_params* p, const RingShape& ring, const Shape& 
     rc = ring_launch<T, sizeof(T) == 4 ? 4 : 2>(a, ring, &grid, st);   // (four chunks: fp32 only)
   }
   if (rc || !want_params) return rc;
-  ln_bwd_finish_kernel<T><<<(p->channels + 31) / 32, kFinishThreads, 0, st>>>(
-      a.part, grid, p->channels, static_cast<T*>(p->dweight), static_cast<T*>(p->dbias));
-  count_launch();
-  return check_launch("layer_norm_bwd_finish_kernel");
+  return finish_launch<T>(p, a.part, grid, st);
 }
 
 template <typename T>
@@ -879,10 +884,7 @@ int bwd_generic_t(const nb200_layer_norm_params* p, cudaStream_t st) {
   count_launch();
   if (int rc = check_launch("layer_norm_bwd_generic_kernel")) return rc;
   if (!want_params) return NB200_OK;
-  ln_bwd_finish_kernel<T><<<(p->channels + 31) / 32, kFinishThreads, 0, st>>>(
-      a.part, 1, p->channels, static_cast<T*>(p->dweight), static_cast<T*>(p->dbias));
-  count_launch();
-  return check_launch("layer_norm_bwd_finish_kernel");
+  return finish_launch<T>(p, a.part, 1, st);
 }
 
 // the vector kernels need 16-byte rows: channels a multiple of 16 bytes (<= 8192) and aligned pointers
