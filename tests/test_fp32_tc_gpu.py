@@ -188,6 +188,28 @@ def test_rows_without_a_kept_key_are_nan_and_leave_the_others_alone():
     assert _err(out[:, :, keep], want[:, :, keep]) <= _BOUND
 
 
+def test_bias_of_minus_infinity_drops_keys_and_infinite_operands_stay_in_their_rows():
+    from nitrix_b200.nn import attention as att
+
+    g = torch.Generator(device="cuda").manual_seed(5)
+    q, dout = (torch.randn(4, 50, 130, 64, device="cuda", generator=g) for _ in range(2))
+    k, v = (torch.randn(4, 50, 333, 64, device="cuda", generator=g) for _ in range(2))
+    bias = torch.randn(4, 50, 130, 333, device="cuda", generator=g)
+    bias[torch.rand(bias.shape, device="cuda", generator=g) < 0.2] = -math.inf
+    bias[..., 0] = 0.0
+    out, lse = att.sdpa_forward(q, k, v, bias, None, scale=0.125)
+    grads = att.sdpa_backward(q, k, v, bias, None, out, lse, dout, scale=0.125, want_dbias=True)
+    for a, r in zip((out, *grads), _reference(q, k, v, bias, None, False, 0.125, dout)):
+        assert _err(a, r) <= _BOUND
+    q[0, 0, 7, 3] = math.inf
+    v[1, 0, 5, 2] = math.inf
+    got, _ = att.sdpa_forward(q, k, v, None, None, scale=0.125)
+    bad = torch.zeros_like(got, dtype=torch.bool)
+    bad[0, 0, 7] = True
+    bad[1, 0, :, 2] = True
+    assert not got[bad].isfinite().any() and got[~bad].isfinite().all()
+
+
 def test_without_workspace_the_other_kernels_run():
     """The workspace is optional: a C caller that brings none (the query answered 0 bytes before these kernels existed)
     gets the mma.sync kernels, forward and backward."""
@@ -201,6 +223,7 @@ def test_without_workspace_the_other_kernels_run():
     p = _cabi.new_params()
     att._fill_common(p, q, k, v, out, lse, None, None, 0.125, False, _cabi.KERNEL_AUTO, None)
     L, stream = _cabi.lib(), torch.cuda.current_stream().cuda_stream
+    L.nb200_profile(1)
     assert L.nb200_sdpa_fwd(C.byref(p), stream) == _cabi.OK, _cabi.last_error()
     dq, dk, dv = (torch.empty_like(q) for _ in range(3))
     p.dout, p.dq, p.dk, p.dv = (t.data_ptr() for t in (dout, dq, dk, dv))
@@ -209,5 +232,8 @@ def test_without_workspace_the_other_kernels_run():
     p.workspace, p.workspace_bytes = ws.data_ptr(), ws.numel()
     assert L.nb200_sdpa_bwd(C.byref(p), stream) == _cabi.OK, _cabi.last_error()
     torch.cuda.synchronize()
+    ran = set(_cabi.kernel_times())
+    L.nb200_profile(0)
+    assert any("tf32x3" in name for name in ran) and not any("fp32_tc" in name or "split_planes" in name for name in ran), ran
     for a, r in zip((out, dq, dk, dv), want):
         assert _err(a, r) <= 1e-4
