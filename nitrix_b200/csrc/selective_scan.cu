@@ -224,7 +224,10 @@ __device__ __forceinline__ void write_pairs(float2* p, float4 a, float4 b) {
 }
 __device__ __forceinline__ float2 both(float v) { return make_float2(v, v); }
 
-template <typename T, int kN>
+// kShort: sequences of up to kStage - 4 steps, one loop over the groups of four that exist (one step of 128 x 2048 channels,
+// f32: 31 -> 17 us; an instantiation of its own, since the test costs the others up to a fifth by another order of the
+// instructions).
+template <typename T, int kN, bool kShort>
 __global__ void __launch_bounds__(kScanThreads) ss_fwd_kernel(SsArgs a) {
   constexpr int kQ = kN / 4;
   __shared__ __align__(16) float2 du[kStage * kScanCh];    // delta, delta x
@@ -264,12 +267,11 @@ __global__ void __launch_bounds__(kScanThreads) ss_fwd_kernel(SsArgs a) {
     nB.store(sB, vecn, tid);
     nC.store(sC, vecn, tid);
     __syncthreads();
-    if (t0 + kStage < a.L) load(t0 + kStage);
+    if (!kShort && t0 + kStage < a.L) load(t0 + kStage);
     // four steps at a time, in three phases: operands and decays (nothing in them depends on the state), then the
     // recurrence, then the sums over the lanes
 #pragma unroll
-    for (int s0 = 0; s0 < kStage; s0 += 4) {
-      if (t0 + s0 >= a.L) break;   // (the same for all threads; one step of 128 x 2048 channels: 31 -> 19 us)
+    for (int s0 = 0; s0 < (kShort ? a.L : kStage); s0 += 4) {
       float2 av[4][kQ / 2], bu[4][kQ / 2];
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
@@ -693,18 +695,23 @@ SsArgs args_of(const nb200_selective_scan_params* p) {
 dim3 scan_grid(const nb200_selective_scan_params* p) {
   return dim3((p->channels + kScanCh - 1) / kScanCh, p->batch);
 }
-template <typename T>
-int fwd_t(const nb200_selective_scan_params* p, cudaStream_t st) {
-  SsArgs a = args_of<T>(p);
+template <typename T, bool kShort>
+int fwd_launch(const nb200_selective_scan_params* p, const SsArgs& a, cudaStream_t st) {
   const dim3 grid = scan_grid(p);
   switch (pick_n(p->states)) {
-    case 8: ss_fwd_kernel<T, 8><<<grid, kScanThreads, 0, st>>>(a); break;
-    case 16: ss_fwd_kernel<T, 16><<<grid, kScanThreads, 0, st>>>(a); break;
-    case 32: ss_fwd_kernel<T, 32><<<grid, kScanThreads, 0, st>>>(a); break;
-    default: ss_fwd_kernel<T, 64><<<grid, kScanThreads, 0, st>>>(a); break;
+    case 8: ss_fwd_kernel<T, 8, kShort><<<grid, kScanThreads, 0, st>>>(a); break;
+    case 16: ss_fwd_kernel<T, 16, kShort><<<grid, kScanThreads, 0, st>>>(a); break;
+    case 32: ss_fwd_kernel<T, 32, kShort><<<grid, kScanThreads, 0, st>>>(a); break;
+    default: ss_fwd_kernel<T, 64, kShort><<<grid, kScanThreads, 0, st>>>(a); break;
   }
   count_launch();
   return check_launch("selective_scan_fwd_kernel");
+}
+
+template <typename T>
+int fwd_t(const nb200_selective_scan_params* p, cudaStream_t st) {
+  const SsArgs a = args_of<T>(p);
+  return p->length <= kStage - 4 ? fwd_launch<T, true>(p, a, st) : fwd_launch<T, false>(p, a, st);
 }
 
 // workspace of the backward: the fp32 accumulators, then the adjoint states between the chunks
