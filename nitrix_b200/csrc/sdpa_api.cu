@@ -263,7 +263,7 @@ int choose(const nb200_sdpa_params* p, const Lowered& lw, int pass, int* kernel)
 // accumulator for a broadcast bias gradient; family-specific scratch follows.
 struct BwdScratch { size_t delta_off, accum_off, family_off, total; int64_t accum_elems; };
 
-// Key groups of a blocked bias accumulator (Problem::dbias_groups), 0 where it is dense: also below half a block of rows,
+// Key groups of a blocked bias accumulator (TcBwdPrepared::dbias_groups), 0 where it is dense: also below half a block of rows,
 // where clearing and reading the padding costs more than the wider reductions save (S 2, T 2048, two batches of 8 heads,
 // D 128: 75 us dense, 78 blocked).
 int dbias_groups(const Lowered& lw, int kernel) {
@@ -460,6 +460,7 @@ NB200_API int nb200_sdpa_bwd(const nb200_sdpa_params* p, void* cuda_stream) {
   prof_mark(nullptr);   // start of this call's kernels
   if (lw.pr.bh_count == 0) return NB200_OK;
   const size_t fam = kernel == NB200_KERNEL_TCGEN05 ? tc_workspace_bytes(lw.pr, lw.dtype, lw.bias_dtype, NB200_PASS_BWD) : 0;
+  TcBwdPrepared prep{};
   int groups = dbias_groups(lw, kernel);
   BwdScratch sc = bwd_scratch(p, lw, groups, fam);
   if (groups && p->workspace_bytes < sc.total) {   // (the least workspace: a dense accumulator)
@@ -474,6 +475,7 @@ NB200_API int nb200_sdpa_bwd(const nb200_sdpa_params* p, void* cuda_stream) {
     set_error("workspace must be %zu-byte aligned", kAlign);
     return NB200_ERR_ALIGNMENT;
   }
+  prep.dbias_groups = groups;
   char* ws = static_cast<char*>(p->workspace);
   Problem& pr = lw.pr;
   pr.delta = reinterpret_cast<float*>(ws + sc.delta_off);
@@ -481,7 +483,6 @@ NB200_API int nb200_sdpa_bwd(const nb200_sdpa_params* p, void* cuda_stream) {
     pr.dbias_accum = reinterpret_cast<float*>(ws + sc.accum_off);
     // dense strides over bias' own extent (of whole (b, h) tiles, where those are blocked); broadcast axes collapse to
     // stride 0
-    pr.dbias_groups = groups;
     int64_t st_dense = 1;
     for (int a = 3; a >= 0; --a) {
       if (a == 1) st_dense = accum_tile(lw, groups);
@@ -494,11 +495,11 @@ NB200_API int nb200_sdpa_bwd(const nb200_sdpa_params* p, void* cuda_stream) {
   if (pr.S > 0) {
     size_t dq_off = 0, dq_bytes = 0;
     if (kernel == NB200_KERNEL_TCGEN05) tc_bwd_dq_region(pr, lw.dtype, &dq_off, &dq_bytes);
-    if (int rc = launch_delta(pr, lw.dtype, ws + sc.family_off + dq_off, dq_bytes, &pr.dq_zeroed, st)) return rc;
+    if (int rc = launch_delta(pr, lw.dtype, ws + sc.family_off + dq_off, dq_bytes, &prep.dq_zeroed, st)) return rc;
   }
   int rc;
   if (kernel == NB200_KERNEL_TCGEN05)
-    rc = tc_backward(pr, lw.dtype, lw.bias_dtype, ws + sc.family_off, fam, st);
+    rc = tc_backward(pr, prep, lw.dtype, lw.bias_dtype, ws + sc.family_off, fam, st);
   else if (lw.dtype == NB200_F32 && fp32_tc_bwd_applies(pr) &&
            p->workspace_bytes >= bwd_scratch(p, lw, 0, fp32_tc_bwd_bytes(pr)).total)   // (optional, as in the forward)
     rc = fp32_tc_backward(pr, lw.bias_dtype, ws + sc.family_off, st);
@@ -506,7 +507,7 @@ NB200_API int nb200_sdpa_bwd(const nb200_sdpa_params* p, void* cuda_stream) {
     rc = simt_backward(pr, lw.dtype, lw.bias_dtype, st);
   if (rc) return rc;
   if (sc.accum_elems)
-    return launch_dbias_finish(pr.dbias_accum, pr.dbias_groups, pr.dbias, lw.bias_dtype, lw.bias_extent, lw.dbias_stride, st);
+    return launch_dbias_finish(pr.dbias_accum, groups, pr.dbias, lw.bias_dtype, lw.bias_extent, lw.dbias_stride, st);
   return NB200_OK;
 }
 

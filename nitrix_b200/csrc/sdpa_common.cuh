@@ -33,15 +33,11 @@ struct Problem {
   void* dbias;
   float* delta;        // (B,H,S) fp32 scratch: rowsum(out * dout)
   float* dbias_accum;  // fp32 scratch of bias' own (un-broadcast) extent, or null
-  // its rows in blocks of 32, its keys in groups of four, [row / 32][key / 4][row % 32][key % 4] (tensor-core kernels, a
-  // bias with a query and a key axis): the number of key groups, T / 4 rounded up; 0: dense
-  int dbias_groups;
   int64_t qs[3], ks[3], vs[3], os[3], dos[3], dqs[3], dks[3], dvs[3];  // b, h, row
   int64_t bs[4], ms[4], dbs[4];                                          // b, h, row, col
   float scale;
   int causal;
   int want_dbias;      // the backward produces a bias gradient (dbias may still be null while planning)
-  int dq_zeroed;       // the tensor-core backward's dq accumulator has been cleared (by the delta kernel)
   int mask_packed;     // 0: byte mask; 1 / 2: `mask` is a buffer made by nb200_mask_pack (2: with the transposed copy)
   int n_out_peers;     // forward: further destinations of every output row (same strides as out)
   void* out_peers[NB200_MAX_OUT_PEERS];
@@ -123,7 +119,16 @@ int launch_dbias_finish(const float* accum, int groups, void* dbias, int bias_dt
 bool tc_supported(const Problem& pr, int dtype, int bias_dtype, int pass, const char** why);
 size_t tc_workspace_bytes(const Problem& pr, int dtype, int bias_dtype, int pass);
 int tc_forward(const Problem& pr, int dtype, int bias_dtype, void* ws, size_t ws_bytes, cudaStream_t stream);
-int tc_backward(const Problem& pr, int dtype, int bias_dtype, void* ws, size_t ws_bytes, cudaStream_t stream);
+// What the caller has prepared for a tensor-core backward.  (Not members of Problem, which every kernel of the CUDA-core
+// family takes by value: eight bytes more in front of its strides cost the mma.sync backwards up to 9 %.)
+struct TcBwdPrepared {
+  // dbias_accum's rows in blocks of 32, its keys in groups of four, [row / 32][key / 4][row % 32][key % 4] (a bias with a
+  // query and a key axis): the number of key groups, T / 4 rounded up; 0: dense
+  int dbias_groups;
+  int dq_zeroed;     // the dq accumulator has been cleared (by the delta kernel)
+};
+int tc_backward(const Problem& pr, const TcBwdPrepared& prep, int dtype, int bias_dtype, void* ws, size_t ws_bytes,
+                cudaStream_t stream);
 // The part of tc_backward's workspace that holds fp32 sums of dq and is zero on entry to its kernels (no bytes: none).
 void tc_bwd_dq_region(const Problem& pr, int dtype, size_t* offset, size_t* bytes);
 // Packing of the byte mask into the tensor-core kernels' bit layout, as a call of its own (nb200_mask_pack).

@@ -1542,7 +1542,7 @@ __global__ void __launch_bounds__(kWarps * 32) simt_bwd_dkv_kernel(Problem pr, i
   }
 }
 
-// dbias_accum (fp32, dense over bias' own extent, or its tiles blocked: Problem::dbias_groups) -> dbias in bias dtype
+// dbias_accum (fp32, dense over bias' own extent, or its tiles blocked: TcBwdPrepared::dbias_groups) -> dbias in bias dtype
 __global__ void dbias_finish_kernel(const float* accum, int groups, void* dbias, int bias_dtype, int64_t n,
                                     int64_t e1, int64_t e2, int64_t e3, int64_t s0, int64_t s1,
                                     int64_t s2, int64_t s3) {

@@ -1033,7 +1033,8 @@ size_t bwd_workspace_bytes(const Problem& pr, int dtype, int) {
   return offset + bytes;
 }
 
-int launch_bwd(const Problem& pr, int dtype, int bias_dtype, void* ws, size_t ws_bytes, int ld_rows, cudaStream_t stream) {
+int launch_bwd(const Problem& pr, const TcBwdPrepared& prep, int dtype, int bias_dtype, void* ws, size_t ws_bytes, int ld_rows,
+               cudaStream_t stream) {
   (void)bias_dtype;
   const char* why = "";
   const bool key_only = mask_key_only(pr);
@@ -1085,7 +1086,7 @@ int launch_bwd(const Problem& pr, int dtype, int bias_dtype, void* ws, size_t ws
   if (merged) {
     BwdArgs ak = a;
     ak.dq_acc = reinterpret_cast<float*>(static_cast<char*>(ws) + mask_ws);
-    cudaError_t e = pr.dq_zeroed ? cudaSuccess : cudaMemsetAsync(ak.dq_acc, 0, acc_bytes, stream);
+    cudaError_t e = prep.dq_zeroed ? cudaSuccess : cudaMemsetAsync(ak.dq_acc, 0, acc_bytes, stream);
     if (e != cudaSuccess) { set_error("cudaMemsetAsync: %s", cudaGetErrorString(e)); return NB200_ERR_LAUNCH; }
     ak.out1 = pr.dv;
     ak.out2 = pr.dk;
@@ -1110,7 +1111,7 @@ int launch_bwd(const Problem& pr, int dtype, int bias_dtype, void* ws, size_t ws
     BwdArgs ak = a;
     ak.dq_acc = reinterpret_cast<float*>(static_cast<char*>(ws) + mask_ws);
     ak.acc_rows = (pr.S + kStep - 1) / kStep * kStep;
-    cudaError_t e = pr.dq_zeroed ? cudaSuccess : cudaMemsetAsync(ak.dq_acc, 0, acc_bytes, stream);
+    cudaError_t e = prep.dq_zeroed ? cudaSuccess : cudaMemsetAsync(ak.dq_acc, 0, acc_bytes, stream);
     if (e != cudaSuccess) { set_error("cudaMemsetAsync: %s", cudaGetErrorString(e)); return NB200_ERR_LAUNCH; }
     ak.out1 = pr.dv;
     ak.out2 = pr.dk;
@@ -1147,7 +1148,7 @@ int launch_bwd(const Problem& pr, int dtype, int bias_dtype, void* ws, size_t ws
       if (a.bias_mode == kBiasTile) {
         aq.dbias_acc = pr.dbias_accum;
         for (int i = 0; i < 3; ++i) aq.acc_s[i] = pr.dbs[i];
-        aq.acc_groups = pr.dbias_groups;
+        aq.acc_groups = prep.dbias_groups;
       }
     } else {
       aq.dbias = pr.dbias;

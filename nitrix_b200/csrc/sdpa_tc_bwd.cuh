@@ -41,12 +41,13 @@ struct BwdArgs {
   // stride).  A bias with a query axis is summed by the query-major kernel (ds tiles added with 16-byte
   // reductions), a per-key bias by the key-major kernel (each thread sums its key's ds over the queries it
   // streams and adds once).
-  // acc_groups > 0: the accumulator's tiles are blocked (Problem::dbias_groups), so that a warp's reduction of four keys
-  // of 32 rows covers 512 contiguous bytes; acc_s[2] is not used then.
-  float* dbias_acc; int64_t acc_s[3]; int acc_groups;
+  float* dbias_acc; int64_t acc_s[3];
   float* dq_acc;                // one-kernel backwards: fp32 sums of ds K, zero on entry (layout: see the kernels)
   int acc_rows;                 // head dim 128: rows of the dq accumulator per (batch, head) (S rounded up to 64)
   int* status;
+  // acc_groups > 0: the bias accumulator's tiles are blocked (TcBwdPrepared::dbias_groups), so that a warp's reduction of four
+  // keys of 32 rows covers 512 contiguous bytes; acc_s[2] is not used then.
+  int acc_groups;
 };
 
 // One-kernel backward at head dim 128 (sdpa_tc_bwd_d128.cu): dq, dk, dv and the dbias tiles of a full-extent bias.
@@ -63,7 +64,8 @@ size_t bwd_workspace_bytes(const Problem& pr, int dtype, int bias_dtype);
 // fp32 dq sums of the one-kernel backwards: their place in that workspace
 void bwd_dq_region(const Problem& pr, int dtype, size_t* offset, size_t* bytes);
 // ld_rows: rows per (batch, head) of pr.lse / pr.delta as passed (S, or the padded count of staged copies)
-int launch_bwd(const Problem& pr, int dtype, int bias_dtype, void* ws, size_t ws_bytes, int ld_rows, cudaStream_t stream);
+int launch_bwd(const Problem& pr, const TcBwdPrepared& prep, int dtype, int bias_dtype, void* ws, size_t ws_bytes, int ld_rows,
+               cudaStream_t stream);
 
 }  // namespace tc
 }  // namespace nb200

@@ -558,7 +558,8 @@ void tc_bwd_dq_region(const Problem& original, int dtype, size_t* offset, size_t
   tc::bwd_dq_region(tc::staged_view(original, tc::plan_staging(original, NB200_PASS_BWD), nullptr), dtype, offset, bytes);
 }
 
-int tc_backward(const Problem& original, int dtype, int bias_dtype, void* ws, size_t ws_bytes, cudaStream_t stream) {
+int tc_backward(const Problem& original, const TcBwdPrepared& prep, int dtype, int bias_dtype, void* ws, size_t ws_bytes,
+                cudaStream_t stream) {
   // padded copies (bias in; lse / delta rows; dbias out) sit behind the kernels' own scratch
   const tc::Staging sg = tc::plan_staging(original, NB200_PASS_BWD);
   const size_t inner = (tc::bwd_workspace_bytes(tc::staged_view(original, sg, nullptr), dtype, bias_dtype) + 255) / 256 * 256;
@@ -568,7 +569,7 @@ int tc_backward(const Problem& original, int dtype, int bias_dtype, void* ws, si
   }
   const Problem pr = tc::staged_view(original, sg, static_cast<char*>(ws) + inner);
   if (int rc = tc::stage_in(original, pr, sg, NB200_PASS_BWD, stream)) return rc;
-  if (int rc = tc::launch_bwd(pr, dtype, bias_dtype, ws, inner, sg.rows ? sg.Sp : original.S, stream)) return rc;
+  if (int rc = tc::launch_bwd(pr, prep, dtype, bias_dtype, ws, inner, sg.rows ? sg.Sp : original.S, stream)) return rc;
   return tc::stage_out(original, pr, sg, stream);
 }
 
