@@ -218,7 +218,8 @@ __global__ void __launch_bounds__(kThreads, kPer <= 4 ? 4 : 2) ln_fwd_kernel(LnA
 // barrier is needed for the data, and 64 to 128 KB per SM are in flight -- HBM needs about 44 KB per SM at its latency.
 // kBatch rows share one barrier (the row sums of groups wider than a warp); their x and dy are read from the ring a
 // second time behind it, which costs less than the registers that would hold them.
-// bf16 (8192, 8192): 142 -> 81 us (4.9 TB/s of x, dy, dx) against the column sums in shared memory without copies ahead;
+// bf16 (8192, 8192), one operand set repeated, this kernel alone: 142 -> 81 us (4.9 TB/s of x, dy, dx; over operand sets
+// larger than L2, with the partial rows, 88) against the column sums in shared memory without copies ahead;
 // 85 us with one row per barrier.
 constexpr int kRowThreads = 512;
 __device__ __forceinline__ void copy_async16(void* dst, const void* src, bool in) {
@@ -554,7 +555,8 @@ __global__ void __launch_bounds__(kThreads) ln_bwd_row_kernel(LnArgs a) {
 // dw[c] = sum over the CTAs' partial rows.  A CTA takes 32 columns (lane = column: 128-byte reads); its warps
 // take the partial rows in turn, four loads in flight each, and their sums are added in warp order -- the
 // order of the whole sum is fixed by (grid, column) alone.  Bound by the latency of a warp's loads: with eight warps (five
-// rounds of four at 148 partial rows, ten at 296) 4.5 to 7 us, with 32 two to three; up to 128 rows eight start sooner.
+// rounds of four at 148 partial rows, ten at 296) 4.5 to 7 us, with 32 two to three; up to 128 partial
+// rows eight start sooner, and above 4096 channels they fill the GPU (8192 x 8192, all kernels: 86 us against 88).
 template <typename T, int kFinishThreads>
 __global__ void __launch_bounds__(kFinishThreads) ln_bwd_finish_kernel(const float* part, int grid, int C, T* dw, T* db) {
   __shared__ float sw[kFinishThreads / 32][32], sb[kFinishThreads / 32][32];
@@ -659,8 +661,9 @@ __global__ void __launch_bounds__(kThreads) ln_bwd_generic_kernel(LnArgs a) {
 
 template <typename T>
 int finish_launch(const nb200_layer_norm_params* p, const float* part, int grid, cudaStream_t st) {
-  auto kernel = grid > 128 ? ln_bwd_finish_kernel<T, 1024> : ln_bwd_finish_kernel<T, 256>;
-  kernel<<<(p->channels + 31) / 32, grid > 128 ? 1024 : 256, 0, st>>>(part, grid, p->channels, static_cast<T*>(p->dweight),
+  const bool wide = grid > 128 && p->channels <= 4096;
+  auto kernel = wide ? ln_bwd_finish_kernel<T, 1024> : ln_bwd_finish_kernel<T, 256>;
+  kernel<<<(p->channels + 31) / 32, wide ? 1024 : 256, 0, st>>>(part, grid, p->channels, static_cast<T*>(p->dweight),
                                                                       static_cast<T*>(p->dbias));
   count_launch();
   return check_launch("layer_norm_bwd_finish_kernel");
