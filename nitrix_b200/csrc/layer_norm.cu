@@ -707,9 +707,15 @@ bool pick_ring(int C, int dtype, RingShape* s) {
 // channels unless f32): 4096x64 6.7 / 7.2, 32768x128 12.7 / 15.9, 2048x64 6.4 / 5.5, 32768x256 18.1 / 16.6; 16384x1024
 // 32.6 / 34.6, 8192x1024 20.8 / 17.8, 16384x768 30.7 / 22.5, 8192x2048 33.0 / 32.1, f32 8192x2048 49.5 / 41.1; 4096x4096
 // 35.2 / 37.2, 2048x4096 22.6 / 18.0, 4096x4104 40.8 / 46.3, f32 4096x4104 47.4 / 48.8; 8192x8192 87 / 145, 1024x8192
-// 21.3 / 22.5, 256x8192 13.3 / 12.8, 2048x6144 26.4 / 30.4, f32 1024x4096 15.1 / 16.1, f32 4096x2056 31.9 / 28.4.
-bool ring_backward(int64_t rows, int C, int dtype, const RingShape& s) {
+// 21.3 / 22.5, 256x8192 13.3 / 12.8, 2048x6144 26.4 / 30.4, f32 1024x4096 15.1 / 16.1, f32 4096x2056 31.9 / 28.4.  For dx
+// alone: 8192x64 4.0 / 4.2, f32 32768x64 7.3 / 6.4, 4096x4096 28.7 / 25.4, f32 2048x4096 18.0 / 15.3, 2048x6144 20.1 / 17.4,
+// 2048x8192 23.5 / 29.8, 4096x6144 38.6 / 51.0, f32 8192x4096 62.8 / 64.9.
+bool ring_backward(int64_t rows, int C, int dtype, bool want_params, const RingShape& s) {
   const int vec = dtype == NB200_F32 ? 4 : 8, words = C / vec;
+  if (!want_params) {
+    if (words <= 16) return vec == 8 && rows >= 8192;
+    return (C > 4096 && rows * C >= int64_t(2048) * 8192) || (C >= 4096 && rows >= 8192);
+  }
   if (words <= 16) return rows >= 4096;
   if (s.per >= 2 && 4 * words >= 3 * s.per * s.tpr) return rows >= 1024;
   if (C >= 4096) return rows >= 4096;
@@ -733,7 +739,7 @@ int bwd_grid_most(int64_t rows, int C, int dtype) {
   RingShape ring;
   Shape s;
   if (!pick_ring(C, dtype, &ring) || !pick(C, dtype, true, &s)) return 1;
-  return ring_backward(rows, C, dtype, ring) ? bwd_grid(rows, kRowThreads / ring.tpr, kRingPerSm) : bwd_grid(rows, row_unit(s), kRowsPerSm);
+  return ring_backward(rows, C, dtype, true, ring) ? bwd_grid(rows, kRowThreads / ring.tpr, kRingPerSm) : bwd_grid(rows, row_unit(s), kRowsPerSm);
 }
 
 int check_common(const nb200_layer_norm_params* p, const char* what) {
@@ -838,7 +844,7 @@ int bwd_t(const nb200_layer_norm_params* p, const RingShape& ring, const Shape& 
     a.part = static_cast<float*>(p->workspace);
   }
   int rc, grid = 1;
-  if (!ring_backward(p->rows, p->channels, p->dtype, ring)) {
+  if (!ring_backward(p->rows, p->channels, p->dtype, want_params, ring)) {
     rc = row_launch<T>(a, s, &grid, st);
   } else if (ring.per == 1) {
     rc = ring_launch<T, 1>(a, ring, &grid, st);

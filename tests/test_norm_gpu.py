@@ -121,12 +121,15 @@ def test_backward_row_groups_at_their_edges(rows, c, dtype):
     (1023, 8192, "bfloat16", False), (1025, 8192, "bfloat16", True), (1030, 6144, "float16", True), (1030, 4104, "bfloat16", False),
     (4099, 4104, "bfloat16", True), (4095, 4096, "bfloat16", False), (16390, 1024, "bfloat16", True), (16390, 1032, "bfloat16", False),
     (300, 2056, "float32", False), (1025, 4096, "float32", True), (1025, 2048, "float32", False), (4097, 24, "float32", True),
-    (2050, 8192, "float32", True), (1, 8192, "float32", False), (4096, 1032, "float32", False)])
+    (2050, 8192, "float32", True), (1, 8192, "float32", False), (4096, 1032, "float32", False),
+    # (negative: the gradient of x alone)
+    (5000, -64, "bfloat16", False), (8200, -64, "bfloat16", True), (8200, -64, "float32", False),
+    (2040, -8192, "bfloat16", False), (2050, -8192, "bfloat16", True), (2050, -4096, "float32", False)])
 def test_backward_on_both_sides_of_the_line_between_its_kernels(rows, c, dtype, ring):
     from nitrix_b200 import _cabi
 
     _cabi.lib().nb200_profile(1)
-    _run((rows, c), getattr(torch, dtype))
+    _run((rows, abs(c)), getattr(torch, dtype), weight=c > 0, bias=c > 0)
     ran = set(_cabi.kernel_times())
     _cabi.lib().nb200_profile(0)
     assert ("layer_norm_bwd_ring_kernel" in ran) == ring and ("layer_norm_bwd_kernel" in ran) != ring, ran
