@@ -755,21 +755,22 @@ int bwd_launch(const SsArgs& a, dim3 grid, cudaStream_t st) {
 }
 
 // Chunks per CTA of the gradients: as many as leave about eight CTAs for every one that the GPU holds at a time (three per
-// SM), so that the last wave is short; more where few channels and many chunks would have more than about 192 CTAs add their
-// sums of dA and dD to the same addresses, down to about two CTAs per SM; at most 16 (a CTA's own start and its sums are
-// spread well enough over those).  us with 1 / 4 / 8 / 16: (256, 64, 64, 16) 191 / 80 / 61 / -, (8, 2048, 128, 16) 285 / 180 /
-// 183 / 174, (16, 512, 256, 16) 201 / 102 / 106 / 96, (8, 1024, 512, 16) 236 / 158 / 164 / 183, (8, 1024, 2048, 16) 502 / 451
-// / 446 / 448, (8, 128, 2048, 8) 63 / 63 / 73 / 74, (2, 333, 1030, 16) 45 / 42 / 55 / 75.
+// SM), so that the last wave is short, at most 16 (a CTA's own start and its sums are spread well enough over those); up to
+// four such waves are made one; up to six where few channels and many chunks would have more than about 192 CTAs add their
+// sums of dA and dD to the same addresses, down to about two CTAs per SM.  us with 1 / 4 / 6 / 16: (256, 64, 64, 16) 191 / 80 / 70 / -, (8, 2048, 128, 16) 285 / 180 /
+// 174 / 174, (16, 512, 256, 16) 201 / 102 / 97 / 96, (256, 128, 64, 32) 401 / 194 / 173 / 186, (64, 512, 64, 64) 482 / 354 / 341 / 371, (8, 1024, 512, 16) 236 / 158 / 162 / 183, (8, 1024, 2048, 16) 502 / 451
+// / 447 / 448, (8, 128, 2048, 8) 63 / 63 / 64 / 74, (2, 333, 1030, 16) 45 / 42 / 47 / 75.
 int chunks_per_cta(int64_t groups, int64_t batch, int64_t chunks) {
   int sms = 0, dev = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (sms <= 0) sms = 148;
   const int64_t work = groups * batch * chunks, spread = batch * chunks / 192, filled = work / (2 * int64_t(sms));
-  int64_t per = work / (8 * 3 * int64_t(sms));
-  const int64_t shared = spread < filled ? spread : filled;
-  per = per < shared ? shared : per;
+  const int64_t resident = 3 * int64_t(sms), shared = spread < filled ? spread : filled;
+  int64_t per = work / (8 * resident);
   per = per < 1 ? 1 : (per > 16 ? 16 : per);
+  const int64_t more = work <= 4 * resident ? (work + resident - 1) / resident : (shared < 6 ? shared : 6);
+  per = per < more ? more : per;
   const int64_t least = (chunks + 65534) / 65535;   // (grid.y)
   per = per < least ? least : per;
   return int(per < chunks ? per : chunks);
