@@ -998,7 +998,7 @@ int64_t owners_of(int rows) { return (int64_t(rows) + 127) / 128; }
 //   S128 14 / 16, B1 H8 S1024 31 / 45, B16 H8 S200 bias 42 / 74, B8 H8 S300 T700 key bias and mask 56 / 184, B8 H16 S1024 208
 //   / 603, the same with a key mask 293 / 810, causal with bias 390 / 775
 //  D 32: B4 H8 S512 bias 57 / 46, B24 H8 S192 34 / 22, B16 H8 S100 T1500 75 / 70, B6 H8 S512 T100 30 / 22, B4 H8 S200 bias and
-//   mask 1.6 times, causal B32 H8 S344 1.18  <  the line  <  B4 H8 S512 22.5 / 28.9, B4 H8 S344 0.76 times (B12 H8 1.07), B4 H8 S1024 49.6 / 93.8, with bias 0.8 times, B16 H8 S512 bias 0.85
+//   mask 1.6 times, causal B32 H8 S344 1.18, B5 H8 S773 T148 bias per query and key mask 45 / 33, B37 H8 S560 mask 430 / 389  <  the line  <  B4 H8 S512 22.5 / 28.9, B4 H8 S344 0.76 times (B12 H8 1.07), B4 H8 S1024 49.6 / 93.8, with bias 0.8 times, B16 H8 S512 bias 0.85
 //   times, B12 H8 S256 bias and mask 0.7 times, B4 H8 S1000 T100 bias and mask 0.77, B16 H8 S200 key bias and mask 28.6 / 36.7
 //  D 128: B1 H1 S33 T65 5.2 / 5.6; 128 pairs of S40 T80 20.6 / 16.8, S48 T300 41.7 / 36.3, S48 T1000 124.6 / 105.8; B32 H8 S64
 //   T64 26 / 19  <  the line  <  32 pairs of S48 T300 0.77 times, 128 with bias 0.97, B1 H1 S128 T1536 84 / 147, B4 H8 S48 T700
@@ -1014,8 +1014,12 @@ bool fp32_tc_fwd_applies(const Problem& pr) {
   if (pr.S <= kRows) return false;   // (half of a 128-row tile at least would be padding)
   if (pr.D == 32) {
     const int least = pr.S < pr.T ? pr.S : pr.T;
-    if (pr.bias && pr.mask) return (least > 128 || pr.S >= 512) && area >= 40000 && owners >= (row_addends(pr) ? 192 : 96);
-    if (row_addends(pr)) return least >= 300 && pr.S >= 512 && owners >= 192;
+    const bool row = row_addends(pr);
+    if (pr.bias && pr.mask) {
+      const bool alike = (pr.bs[2] != 0) == (pr.ms[2] != 0);   // (else one of the two costs the others little)
+      return (least >= 200 || (alike && (least > 128 || pr.S >= 512))) && area >= 40000 && owners >= (row ? 192 : 96);
+    }
+    if (row) return least >= 300 && pr.S >= 512 && owners >= 192 && (pr.bias || area >= 500000);
     return least >= 200 && (pr.causal ? area / 2 : area) >= 100000 && owners >= 96;
   }
   const int64_t ctas = tiles_of(pr.S) * pr.bh_count, work = ctas * tiles_of(pr.T);

@@ -107,7 +107,7 @@ def test_against_fp64(B, H, S, T, D, causal, bias, mask, layout):
     (24, 8, 128, 128, 64, "none", False, True), (24, 8, 128, 128, 64, "key", True, True),
     (12, 8, 192, 192, 32, "none", False, False), (8, 8, 192, 192, 32, "none", False, True), (8, 8, 200, 200, 32, "none", False, True),
     (4, 8, 344, 344, 32, "none", True, True), (4, 8, 512, 100, 32, "none", False, False), (12, 8, 160, 160, 32, "mask", False, False),
-    (12, 8, 128, 128, 32, "mask", False, True), (4, 8, 512, 512, 32, "mask", False, True), (6, 8, 512, 512, 32, "mask", True, True),
+    (12, 8, 128, 128, 32, "mask", False, True), (6, 8, 512, 512, 32, "mask", False, True), (4, 8, 768, 768, 32, "mask", True, True),
     (12, 8, 200, 200, 32, "both", True, True), (3, 8, 200, 200, 32, "both", False, False),
     (16, 8, 40, 80, 128, "none", False, False), (8, 8, 40, 80, 128, "none", True, False), (16, 8, 48, 300, 128, "mask", True, False),
 ])
