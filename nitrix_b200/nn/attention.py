@@ -322,22 +322,13 @@ def _workspace_need(p, which: int, query: str = "nb200_sdpa_workspace_bytes") ->
     return need.value
 
 
-def _workspace(p, which: int, need: int, device) -> Optional[torch.Tensor]:
-    """The call's scratch, ``need`` bytes; where the device has no room for them, the least with which the call runs (the
+def _least_workspace(p, which: int, need: int, device) -> Optional[torch.Tensor]:
+    """For a device without room for all of a call's ``need`` bytes of scratch: the least with which the call runs (the
     planes of fp32 operands take up to 1 GiB that the other kernels do without)."""
-    if not need:
-        return None
-    try:
-        ws = torch.empty(need, dtype=torch.uint8, device=device)
-    except torch.OutOfMemoryError:
-        least = _workspace_need(p, which, "nb200_sdpa_workspace_least_bytes")
-        if least >= need:
-            raise
-        if not least:
-            return None
-        ws = torch.empty(least, dtype=torch.uint8, device=device)
-    p.workspace, p.workspace_bytes = ws.data_ptr(), ws.numel()
-    return ws
+    least = _workspace_need(p, which, "nb200_sdpa_workspace_least_bytes")
+    if least >= need:
+        raise torch.OutOfMemoryError(f"no room for {need} bytes of workspace")
+    return torch.empty(least, dtype=torch.uint8, device=device) if least else None
 
 
 def _mask_meta(mask):
@@ -399,7 +390,14 @@ def sdpa_forward(q, k, v, bias=None, mask=None, *, scale: float, causal: bool = 
         p.bias = bias.data_ptr()
     if mask_b is not None:
         p.mask = (mask_b.blob if isinstance(mask_b, PackedMask) else mask_b).data_ptr()
-    ws = _workspace(p, _cabi.PASS_FWD, need, q.device)
+    ws = None
+    if need:
+        try:
+            ws = torch.empty(need, dtype=torch.uint8, device=q.device)
+        except torch.OutOfMemoryError:
+            ws = _least_workspace(p, _cabi.PASS_FWD, need, q.device)
+        if ws is not None:
+            p.workspace, p.workspace_bytes = ws.data_ptr(), ws.numel()
     _launch(_cabi.lib().nb200_sdpa_fwd, p, q.device, "nb200_sdpa_fwd")
     del ws  # same-stream reuse is ordered by the caching allocator
     return out, lse
@@ -456,7 +454,14 @@ def sdpa_backward(q, k, v, bias, mask, out, lse, dout, *, scale: float, causal: 
         p.mask = (mask_b.blob if isinstance(mask_b, PackedMask) else mask_b).data_ptr()
     if dbias is not None:
         p.dbias = dbias.data_ptr()
-    ws = _workspace(p, _cabi.PASS_BWD, need, q.device)
+    ws = None
+    if need:
+        try:
+            ws = torch.empty(need, dtype=torch.uint8, device=q.device)
+        except torch.OutOfMemoryError:
+            ws = _least_workspace(p, _cabi.PASS_BWD, need, q.device)
+        if ws is not None:
+            p.workspace, p.workspace_bytes = ws.data_ptr(), ws.numel()
     _launch(_cabi.lib().nb200_sdpa_bwd, p, q.device, "nb200_sdpa_bwd")
     del ws  # same-stream reuse is ordered by the caching allocator
     return dq, dk, dv, dbias
@@ -558,7 +563,7 @@ def scaled_dot_product_attention(
     if resolved == "cuda-sm100":
         chosen = _planned_kernel_cached(q4, k4, v4, bias4, mask4, resolved_scale, causal)
         fused = chosen == _cabi.KERNEL_TCGEN05
-        # fp32 operands on the 3 x TF32 tensor kernels are a fused path too (fp32 is the one dtype the reference's
+        # fp32 operands on the tensor-core kernels are a fused path too (fp32 is the one dtype the reference's
         # fused kernels accept, attention.py:736-744): only a problem that leaves the tensor paths altogether warns
         if chosen not in (_cabi.KERNEL_TCGEN05, _cabi.KERNEL_MMA_TF32X3):
             fallback(
@@ -567,7 +572,7 @@ def scaled_dot_product_attention(
                 resolved="cuda-simt",
                 reason=(
                     "the fused tcgen05 kernels take bf16/fp16 with d == d_v in {64, 128} (any query/key lengths); "
-                    "the fused 3xTF32 kernels take fp32 with d, d_v in {32, 64, 128}"
+                    "the fp32 tensor-core kernels take d, d_v in {32, 64, 128}"
                 ),
                 shapes=(tuple(q.shape), tuple(k.shape), tuple(v.shape)),
                 dtype=out_dtype,
