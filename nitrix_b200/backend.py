@@ -15,11 +15,15 @@ shared library.
     the fused TMA + tcgen05 kernels (the counterpart of the reference's
     ``'pallas-cuda'``, which is accepted as an alias);
 ``'cuda-simt'``
-    CUDA-core kernels in true fp32 arithmetic.  They take every shape and dtype
-    and are what a problem the fused kernels decline falls back to, with one
-    ``NitrixBackendFallback`` warning per (function, shapes, dtype, backend).
-    Reproducibility mode resolves ``'auto'`` to this family, as the reference
-    resolves it to its non-tensor-core engine (``backend.py:192-195``).
+    the family that takes every shape and dtype at fp32 accuracy: CUDA-core
+    kernels for 16-bit operands, for fp32 operands also tensor-core kernels on
+    which every operand is split into several terms (three of bf16 on tcgen05,
+    two of TF32 on ``mma.sync``).  A problem the fused kernels decline falls
+    back to it, with one ``NitrixBackendFallback`` warning per (function,
+    shapes, dtype, backend).  Reproducibility mode resolves ``'auto'`` to this
+    family (the reference resolves it to its non-tensor-core engine,
+    ``backend.py:192-195``): it sums everything but the gradient of a broadcast
+    bias in a fixed order.
 
 ``'jax'`` (the reference's host path) is not shipped; asking for it raises
 ``NitrixBackendError``.
