@@ -80,88 +80,115 @@ bool make_tile_map(CUtensorMap* map, const void* base, int rows, int cols, int H
 // ---- mask packing -------------------------------------------------------------
 namespace {
 
-// One CTA packs a 32-row x 32-key tile: row-major words by warp ballot over the
-// keys of a row, transposed words by ballot over the rows of a key.
-__global__ void __launch_bounds__(256) mask_pack_kernel(const uint8_t* mask, int64_t sb, int64_t sh, int64_t ss,
-                                                        int64_t st, int Hm, int Sm, int S, int T,
-                                                        uint32_t* rows_out, int words_per_row,
-                                                        uint32_t* cols_out, int words_per_col, int* kv_len) {
-  __shared__ uint8_t tile[32][33];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int bm = blockIdx.z / Hm, hm = blockIdx.z - bm * Hm;
-  const int key0 = blockIdx.x * 32, row0 = blockIdx.y * 32;
-  const uint8_t* base = mask + bm * sb + hm * sh;
-  const int n_rows = cols_out ? S : Sm;  // the transposed copy always spans every query row
-  for (int rl = warp; rl < 32; rl += 8) {
-    const int row = row0 + rl, key = key0 + lane;
-    const bool in = row < n_rows && key < T;
-    const uint8_t v = in ? (base[int64_t(Sm == 1 ? 0 : row) * ss + int64_t(key) * st] != 0) : 0;
-    tile[rl][lane] = v;
-    const uint32_t word = __ballot_sync(0xffffffffu, v != 0);
-    if (lane == 0 && row < Sm) {
-      rows_out[(int64_t(blockIdx.z) * Sm + row) * words_per_row + blockIdx.x] = word;
-      // key-only mask: remember the last kept key (1 + index) so that fully dropped tail tiles are skipped
-      if (kv_len && word != 0u) atomicMax(kv_len + blockIdx.z, key0 + 32 - __clz(word));
-    }
+// 128 at bit 7 of every non-zero byte, then one dot product gathers four bytes' bits (times 128)
+__device__ __forceinline__ uint32_t nonzero_bytes(uint32_t v) { return (((v & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) | v) & 0x80808080u; }
+__device__ __forceinline__ uint32_t keep_bits8(uint32_t lo, uint32_t hi) {
+  return __dp4a(nonzero_bytes(hi), 0x80402010u, __dp4a(nonzero_bytes(lo), 0x08040201u, 0u)) >> 7;
+}
+// keep-bits of kKeys consecutive keys, bit i = key i; keys at or past the `n`th (may be negative) are dropped.
+// 16 and 8 keys: one aligned vector load, n either >= kKeys or <= 0; 1: eight single bytes of any stride.  Lanes with
+// nothing to read load from `first` (the mask's first element) all the same, so that a row's loads need no branch.
+template <int kKeys>
+__device__ __forceinline__ uint32_t keep_bits(const uint8_t* p, const uint8_t* first, int64_t st, int n) {
+  if (n <= 0) p = first;
+  uint32_t bits;
+  if constexpr (kKeys == 16) {
+    const uint4 v = __ldg(reinterpret_cast<const uint4*>(p));
+    bits = keep_bits8(v.x, v.y) | (keep_bits8(v.z, v.w) << 8);
+  } else if constexpr (kKeys == 8) {
+    const uint2 v = __ldg(reinterpret_cast<const uint2*>(p));
+    bits = keep_bits8(v.x, v.y);
+  } else {
+    bits = 0u;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) bits |= (__ldg(p + (i < n ? i * st : 0)) != 0 && i < n) ? 1u << i : 0u;
   }
-  if (!cols_out) return;
-  __syncthreads();
-  for (int kl = warp; kl < 32; kl += 8) {
-    const int key = key0 + kl;
-    const uint32_t word = __ballot_sync(0xffffffffu, tile[lane][kl] != 0);
-    if (lane == 0 && key < T) cols_out[(int64_t(blockIdx.z) * T + key) * words_per_col + blockIdx.y] = word;
-  }
+  return n > 0 ? bits : 0u;
+}
+// a 32-key word from the bits of neighbouring lanes (each of them gets it)
+template <int kKeys>
+__device__ __forceinline__ uint32_t join_bits(uint32_t bits, int lane) {
+  constexpr int kLanes = kKeys == 16 ? 2 : 4;   // lanes per word
+  uint32_t w = bits << ((32 / kLanes) * (lane & (kLanes - 1)));
+  w |= __shfl_xor_sync(0xffffffffu, w, 1);
+  if constexpr (kLanes == 4) w |= __shfl_xor_sync(0xffffffffu, w, 2);
+  return w;
 }
 
-// Fast path for a mask with a query axis, unit key stride and 16-byte aligned rows: one CTA packs a 256-row x
-// 256-key tile.  Rows are read as 16-byte vectors (16 keys per lane, a warp covers two 256-byte row segments per
-// load); the row-major words go out as they are formed and are kept in shared memory, from which each warp then
-// builds the transposed words of 32 keys by ballot over 32 rows, 8 row-words (32 bytes) per key.
-__global__ void __launch_bounds__(256) mask_pack_tile_kernel(const uint8_t* mask, int64_t sb, int64_t sh, int64_t ss, int Hm,
-                                                             int S, int T, uint32_t* rows_out, int words_per_row,
-                                                             uint32_t* cols_out, int words_per_col) {
-  __shared__ uint32_t sw[256][9];   // [row][key word], padded against bank conflicts
+// Mask with a query axis: one CTA packs 64 rows x 256 keys, a warp eight rows, all its loads in flight; a lane takes 16
+// keys (rows that are 16-byte aligned and a multiple of 16 long), 8 (the same with 8), or eight single bytes.  The row
+// words are kept in shared memory, from which each warp then forms the transposed words of 32 keys: 32 x 32 bits turned
+// over in five exchanges between lanes.  Every word of both layouts is written, padding included, so nothing is cleared
+// before.  Bound: HBM, the mask once.  32 x 32 tiles of single bytes, or 256 x 256 tiles with a ballot per bit for lengths
+// that are multiples of 256, and a memset took (12, 1, 1216, 1216) with the transposed words 58 us, now 7.4; (4, 1, 7424,
+// 7424) 108 -> 68, without them 46 -> 47; (3, 1, 1217, 1331) without 15 -> 7; (2, 2, 256, 256) with 7.6 -> 3.1.
+template <int kKeys>
+__global__ void __launch_bounds__(256) mask_pack_kernel(const uint8_t* mask, int64_t sb, int64_t sh, int64_t ss, int64_t st,
+                                                        int Hm, int S, int T, uint32_t* rows_out, int words_per_row,
+                                                        uint32_t* cols_out, int words_per_col) {
+  constexpr int kLaneKeys = kKeys == 16 ? 16 : 8, kRowLanes = 256 / kLaneKeys, kLoads = 8 * kRowLanes / 32;
+  __shared__ uint32_t sw[64][9];   // [row][key word], padded against bank conflicts
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int bm = blockIdx.z / Hm, hm = blockIdx.z - bm * Hm;
-  const int key0 = blockIdx.x * 256, row0 = blockIdx.y * 256;
-  const uint8_t* base = mask + bm * sb + hm * sh + int64_t(row0) * ss + key0;
-#pragma unroll 4
-  for (int i = 0; i < 16; ++i) {
-    const int rl = warp * 32 + 2 * i + (lane >> 4);     // row within the tile
-    const int chunk = lane & 15;                        // 16 keys
-    const uint4 v = __ldg(reinterpret_cast<const uint4*>(base + int64_t(rl) * ss + chunk * 16));
-    const uint32_t in[4] = {v.x, v.y, v.z, v.w};
-    uint32_t bits = 0;
+  const int key0 = blockIdx.x * 256, row0 = blockIdx.y * 64;
+  const int kl = (lane % kRowLanes) * kLaneKeys, key = key0 + kl;
+  const int rl0 = warp * 8 + lane / kRowLanes;   // first row of this lane; the next ones 32 / kRowLanes further
+  const uint8_t* base = mask + bm * sb + hm * sh + key * st;
+  uint32_t bits[kLoads];
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const uint32_t nz = __vcmpne4(in[e], 0u) & 0x01010101u;          // one bit per non-zero byte
-      bits |= ((nz * 0x01020408u) >> 24 & 0xFu) << (4 * e);            // byte k of the word -> bit k
-    }
-    const uint32_t hi = __shfl_down_sync(0xffffffffu, bits, 1);
-    if (!(lane & 1)) {
-      const uint32_t word = bits | (hi << 16);
-      sw[rl][chunk >> 1] = word;
-      rows_out[(int64_t(blockIdx.z) * S + row0 + rl) * words_per_row + (key0 >> 5) + (chunk >> 1)] = word;
+  for (int i = 0; i < kLoads; ++i) {
+    const int row = row0 + rl0 + i * (32 / kRowLanes);
+    bits[i] = keep_bits<kKeys>(base + int64_t(row) * ss, mask, st, row < S ? T - key : 0);
+  }
+#pragma unroll
+  for (int i = 0; i < kLoads; ++i) {
+    const int rl = rl0 + i * (32 / kRowLanes);
+    const uint32_t w = join_bits<kKeys>(bits[i], lane);
+    if ((kl & 31) == 0) {
+      sw[rl][kl >> 5] = w;
+      if (row0 + rl < S && (key >> 5) < words_per_row) rows_out[(int64_t(blockIdx.z) * S + row0 + rl) * words_per_row + (key >> 5)] = w;
     }
   }
   if (!cols_out) return;
   __syncthreads();
-  // warp w transposes key word w: lane = key, 8 row-words each
-  uint32_t out[8];
+  uint32_t x[2] = {sw[lane][warp], sw[32 + lane][warp]};   // lane = row
 #pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    const uint32_t w = sw[32 * j + lane][warp];          // lane = row within the group of 32
-    uint32_t mine = 0;
+  for (int m = 16; m; m >>= 1) {
+    const uint32_t low = m == 16 ? 0x0000FFFFu : m == 8 ? 0x00FF00FFu : m == 4 ? 0x0F0F0F0Fu : m == 2 ? 0x33333333u : 0x55555555u;
 #pragma unroll
-    for (int b = 0; b < 32; ++b) {
-      const uint32_t t = __ballot_sync(0xffffffffu, (w >> b) & 1u);
-      if (lane == b) mine = t;
+    for (int j = 0; j < 2; ++j) {
+      const uint32_t y = __shfl_xor_sync(0xffffffffu, x[j], m);
+      x[j] = (lane & m) ? (x[j] & ~low) | ((y & ~low) >> m) : (x[j] & low) | ((y & low) << m);
     }
-    out[j] = mine;
   }
-  uint32_t* dst = cols_out + (int64_t(blockIdx.z) * T + key0 + warp * 32 + lane) * words_per_col + (row0 >> 5);
-  *reinterpret_cast<uint4*>(dst) = make_uint4(out[0], out[1], out[2], out[3]);
-  *reinterpret_cast<uint4*>(dst + 4) = make_uint4(out[4], out[5], out[6], out[7]);
+  const int mine = key0 + warp * 32 + lane;   // lane = key now; words_per_col is a multiple of 4
+  if (mine < T && (row0 >> 5) < words_per_col)
+    *reinterpret_cast<uint2*>(cols_out + (int64_t(blockIdx.z) * T + mine) * words_per_col + (row0 >> 5)) = make_uint2(x[0], x[1]);
+}
+
+// Mask without a query axis: one CTA per (batch, head) row packs it and finds 1 + its last kept key.
+template <int kKeys>
+__global__ void __launch_bounds__(1024) mask_pack_row_kernel(const uint8_t* mask, int64_t sb, int64_t sh, int64_t st, int Hm,
+                                                             int T, uint32_t* rows_out, int words_per_row, int* kv_len) {
+  static_assert(kKeys != 16, "a warp takes 256 keys");
+  __shared__ int last[32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+  const int bm = blockIdx.x / Hm, hm = blockIdx.x - bm * Hm;
+  const uint8_t* base = mask + bm * sb + hm * sh;
+  int len = 0;
+  for (int word0 = warp * 8; word0 < words_per_row; word0 += warps * 8) {
+    const int key = 32 * word0 + 8 * lane, word = key >> 5;
+    const uint32_t w = join_bits<kKeys>(keep_bits<kKeys>(base + key * st, mask, st, T - key), lane);
+    if (!(lane & 3) && word < words_per_row) rows_out[int64_t(blockIdx.x) * words_per_row + word] = w;
+    if (w) len = 32 * word + 32 - __clz(w);   // (words ascend)
+  }
+  len = __reduce_max_sync(0xffffffffu, len);
+  if (lane == 0) last[warp] = len;
+  __syncthreads();
+  if (warp == 0) {
+    len = __reduce_max_sync(0xffffffffu, lane < warps ? last[lane] : 0);
+    if (lane == 0) kv_len[blockIdx.x] = len;
+  }
 }
 
 inline int round_up(int x, int m) { return (x + m - 1) / m * m; }
@@ -404,25 +431,27 @@ int launch_mask_pack(const Problem& pr, const MaskPackPlan& plan, void* ws, Mask
   uint32_t* rows = static_cast<uint32_t*>(ws);
   uint32_t* cols = plan.cols_bytes ? reinterpret_cast<uint32_t*>(static_cast<char*>(ws) + plan.rows_bytes) : nullptr;
   const int Bm = int(plan.extent[0]), Hm = int(plan.extent[1]), Sm = int(plan.extent[2]);
-  const int n_rows = cols ? pr.S : Sm;
-  // padding words beyond ceil(T/32) (and ceil(S/32)) must read as "dropped"
   int* kv_len = plan.len_bytes ? reinterpret_cast<int*>(static_cast<char*>(ws) + plan.rows_bytes + plan.cols_bytes) : nullptr;
-  cudaError_t e = cudaMemsetAsync(ws, 0, plan.total(), stream);
-  if (e != cudaSuccess) { set_error("cudaMemsetAsync(mask bits): %s", cudaGetErrorString(e)); return NB200_ERR_LAUNCH; }
-  const bool tiled = Sm == pr.S && pr.S % 256 == 0 && pr.T % 256 == 0 && pr.ms[3] == 1 && pr.ms[2] % 16 == 0 &&
-                     (Bm == 1 || pr.ms[0] % 16 == 0) && (Hm == 1 || pr.ms[1] % 16 == 0) &&
-                     reinterpret_cast<uintptr_t>(pr.mask) % 16 == 0;
-  if (tiled) {
-    dim3 grid(pr.T / 256, pr.S / 256, Bm * Hm);
-    mask_pack_tile_kernel<<<grid, 256, 0, stream>>>(static_cast<const uint8_t*>(pr.mask), pr.ms[0], pr.ms[1], pr.ms[2], Hm,
-                                                    pr.S, pr.T, rows, plan.words_per_row, cols, plan.words_per_col);
+  // keys per load: rows that start on 16 (8) bytes and hold whole groups of as many
+  auto whole = [&](int n) {
+    return pr.T % n == 0 && pr.ms[3] == 1 && (Sm == 1 || pr.ms[2] % n == 0) && (Bm == 1 || pr.ms[0] % n == 0) &&
+           (Hm == 1 || pr.ms[1] % n == 0) && reinterpret_cast<uintptr_t>(pr.mask) % n == 0;
+  };
+  const uint8_t* mask = static_cast<const uint8_t*>(pr.mask);
+  if (kv_len) {
+    auto kernel = whole(8) ? mask_pack_row_kernel<8> : mask_pack_row_kernel<1>;
+    const int warps = (plan.words_per_row + 7) / 8;
+    kernel<<<Bm * Hm, 32 * (warps < 32 ? warps : 32), 0, stream>>>(mask, pr.ms[0], pr.ms[1], pr.ms[3], Hm, pr.T, rows,
+                                                                   plan.words_per_row, kv_len);
   } else {
-    dim3 grid((pr.T + 31) / 32, (n_rows + 31) / 32, Bm * Hm);
-    mask_pack_kernel<<<grid, 256, 0, stream>>>(pr.mask, pr.ms[0], pr.ms[1], pr.ms[2], pr.ms[3], Hm, Sm, pr.S, pr.T, rows,
-                                               plan.words_per_row, cols, plan.words_per_col, kv_len);
+    auto kernel = whole(16) ? mask_pack_kernel<16> : (whole(8) ? mask_pack_kernel<8> : mask_pack_kernel<1>);
+    // (with the transposed copy: all of its words, a multiple of 4 per key)
+    const dim3 grid((pr.T + 255) / 256, cols ? plan.words_per_col / 2 : (pr.S + 63) / 64, Bm * Hm);
+    kernel<<<grid, 256, 0, stream>>>(mask, pr.ms[0], pr.ms[1], pr.ms[2], pr.ms[3], Hm, pr.S, pr.T, rows, plan.words_per_row,
+                                     cols, plan.words_per_col);
   }
   count_launch();
-  if (int rc = check_launch(tiled ? "mask_pack_tile_kernel" : "mask_pack_kernel")) return rc;
+  if (int rc = check_launch("mask_pack_kernel")) return rc;
   mask_views(pr, plan, ws, out);
   return NB200_OK;
 }

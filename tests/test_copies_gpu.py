@@ -1,4 +1,5 @@
-"""The kernels that bring operands into the layout the attention kernels read: padded copies of a bias and its gradient."""
+"""The kernels that bring operands into the layout the attention kernels read and results out of it: padded copies of a bias
+and its gradient, packed masks, the last pass over a shared bias' gradient."""
 import pytest
 import torch
 
@@ -43,3 +44,59 @@ def test_padded_copies_of_a_bias_keep_every_element(S, T, layout):
     ref = p * (dp - (p * dp).sum(-1, keepdim=True))
     # p and ds are rounded to bf16 (2^-9), out (in delta) too
     assert float((grads[0][3].double() - ref).abs().max()) <= 2e-2 * max(1.0, float(ref.abs().max()))
+
+
+def _words(bits):
+    """(..., n) booleans -> (..., ceil(n / 32) rounded up to 4) 32-bit words, bit i of word w = element 32 w + i."""
+    n = bits.shape[-1]
+    words = (-(-n // 32) + 3) // 4 * 4
+    full = torch.zeros(*bits.shape[:-1], words * 32, dtype=torch.int64)
+    full[..., :n] = bits
+    weights = 2 ** torch.arange(32, dtype=torch.int64)
+    w = (full.reshape(*bits.shape[:-1], words, 32) * weights).sum(-1)
+    return torch.where(w >= 2 ** 31, w - 2 ** 32, w).to(torch.int32)
+
+
+@pytest.mark.parametrize("layout", ["dense", "rows_of_8", "odd_start", "key_strided"])
+@pytest.mark.parametrize("S,T", [(2, 1), (63, 16), (64, 256), (65, 264), (130, 272), (257, 511), (100, 31)])
+def test_packed_mask_bits(S, T, layout):
+    """Row-major and transposed words against a packing on the CPU, for every way the kernel reads the mask."""
+    from nitrix_b200.nn.attention import pack_mask
+
+    B, H, D = 2, 3, 64
+    g = torch.Generator().manual_seed(S * 1000 + T)
+    values = torch.randint(0, 4, (B, H, S, T), generator=g, dtype=torch.uint8) * 85      # 0, 85, 170, 255
+    if layout == "dense":
+        mask = values.cuda()
+    elif layout == "rows_of_8":
+        mask = torch.empty(B, H, S, (T + 7) // 8 * 8, dtype=torch.uint8, device="cuda")[..., :T].copy_(values)
+    elif layout == "odd_start":
+        mask = torch.empty(B, H, S, T + 1, dtype=torch.uint8, device="cuda")[..., 1:].copy_(values)
+    else:
+        mask = values.transpose(-1, -2).contiguous().cuda().transpose(-1, -2)
+    q = torch.empty(B, H, S, D, device="cuda", dtype=torch.bfloat16)
+    k = torch.empty(B, H, T, D, device="cuda", dtype=torch.bfloat16)
+    blob = pack_mask(q, k, k, mask).blob.cpu()
+    rows, cols = _words(values != 0), _words((values != 0).transpose(-1, -2))
+    at = (rows.numel() * 4 + 255) // 256 * 256
+    assert torch.equal(blob[:rows.numel() * 4].view(torch.int32).reshape(rows.shape), rows)
+    assert torch.equal(blob[at:at + cols.numel() * 4].view(torch.int32).reshape(cols.shape), cols)
+
+
+@pytest.mark.parametrize("T", [1, 31, 256, 257, 1000, 8200])
+def test_packed_key_mask_bits_and_kept_lengths(T):
+    from nitrix_b200.nn.attention import pack_mask
+
+    B, H, S, D = 5, 2, 3, 64
+    keep = torch.rand(B, 1, 1, T, generator=torch.Generator().manual_seed(T)) < 0.5
+    keep[0] = False                                   # no kept key: length 0
+    keep[1] = True
+    keep[2, ..., T // 2:] = False
+    q = torch.empty(B, H, S, D, device="cuda", dtype=torch.bfloat16)
+    k = torch.empty(B, H, T, D, device="cuda", dtype=torch.bfloat16)
+    blob = pack_mask(q, k, k, keep.cuda()).blob.cpu()
+    rows = _words(keep)
+    at = (rows.numel() * 4 + 255) // 256 * 256
+    assert torch.equal(blob[:rows.numel() * 4].view(torch.int32).reshape(rows.shape), rows)
+    lengths = torch.where(keep, torch.arange(1, T + 1), 0).amax(-1).flatten().to(torch.int32)
+    assert torch.equal(blob[at:at + 4 * B].view(torch.int32), lengths)
