@@ -100,3 +100,27 @@ def test_packed_key_mask_bits_and_kept_lengths(T):
     assert torch.equal(blob[:rows.numel() * 4].view(torch.int32).reshape(rows.shape), rows)
     lengths = torch.where(keep, torch.arange(1, T + 1), 0).amax(-1).flatten().to(torch.int32)
     assert torch.equal(blob[at:at + 4 * B].view(torch.int32), lengths)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("S,T", [(16, 16), (31, 127), (33, 129), (64, 128), (40, 257), (300, 19), (20, 15)])
+def test_gradient_of_a_shared_bias_leaves_in_any_layout(S, T, dtype):
+    """Two heads add to the same sums, in either order the same bits: the tiled last pass against the strided one."""
+    from nitrix_b200.nn.attention import sdpa_backward, sdpa_forward
+
+    g = torch.Generator(device="cuda").manual_seed(S * 1000 + T)
+    q, dout = (torch.randn(1, 2, S, 64, generator=g, device="cuda").to(dtype) for _ in range(2))
+    k, v = (torch.randn(1, 2, T, 64, generator=g, device="cuda").to(dtype) for _ in range(2))
+    bias = torch.randn(1, 1, S, T, generator=g, device="cuda").to(dtype)
+    out, lse = sdpa_forward(q, k, v, bias, scale=0.125)
+    got = []
+    for buf in (torch.empty_like(bias), torch.empty(1, 1, S, T + 3, device="cuda", dtype=dtype)[..., 1:T + 1],
+                torch.empty(1, 1, T, S, device="cuda", dtype=dtype).transpose(-1, -2)):
+        bufs = (torch.empty_like(q), torch.empty_like(k), torch.empty_like(v), buf)
+        got.append(sdpa_backward(q, k, v, bias, None, out, lse, dout, scale=0.125, want_dbias=True, grads=bufs)[3])
+    assert torch.equal(got[0], got[1]) and torch.equal(got[0], got[2])
+    p = (q.double() @ k.double().transpose(-1, -2) * 0.125 + bias.double()).softmax(-1)
+    dp = dout.double() @ v.double().transpose(-1, -2)
+    ref = (p * (dp - (p * dp).sum(-1, keepdim=True))).sum(1, keepdim=True)
+    tol = 1e-4 if dtype == torch.float32 else 2e-2
+    assert float((got[0].double() - ref).abs().max()) <= tol * max(1.0, float(ref.abs().max()))
