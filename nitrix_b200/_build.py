@@ -6,7 +6,9 @@ cross-compiles without a GPU, so this runs on a CPU-only host as well.
 
 Every ``csrc/*.cu`` is compiled to its own object file (in parallel, and only
 when the file, a header or the flags changed since its object was made); the
-objects are then linked into one shared library.
+objects are then linked into one shared library.  ``csrc/host/torch_ops.cpp``
+(the operations as C++ autograd functions) is compiled by the host compiler
+against the installed torch into a Python extension module beside it.
 """
 from __future__ import annotations
 
@@ -16,6 +18,7 @@ import os
 import pathlib
 import shutil
 import subprocess
+import sysconfig
 
 PKG = pathlib.Path(__file__).resolve().parent
 CSRC = PKG / "csrc"
@@ -31,6 +34,11 @@ COMPILE_FLAGS = [
     "-Xcompiler", "-fvisibility=hidden",
 ]
 LINK_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-shared", "-Xcompiler", "-fPIC"]
+
+
+HOST_SOURCE = CSRC / "host" / "torch_ops.cpp"
+HOST_MODULE = "_torch_ops"
+HOST_FLAGS = ["-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden"]
 
 
 def sources() -> list[pathlib.Path]:
@@ -66,9 +74,44 @@ def lib_path() -> pathlib.Path:
     return LIBDIR / LIBNAME
 
 
+def host_module_path() -> pathlib.Path:
+    return LIBDIR / (HOST_MODULE + ".so")
+
+
+def _host_digest() -> str:
+    import torch
+
+    h = hashlib.sha256(" ".join([*HOST_FLAGS, torch.__version__, sysconfig.get_python_version()]).encode())
+    for f in [HOST_SOURCE, *sorted(INCLUDE.glob("*.h"))]:
+        h.update(f.read_bytes())
+    return h.hexdigest()
+
+
+def _stamped(path: pathlib.Path, stamp: pathlib.Path, digest: str) -> bool:
+    return path.exists() and stamp.exists() and stamp.read_text().strip() == digest
+
+
 def is_current() -> bool:
-    stamp = LIBDIR / "build.sha256"
-    return lib_path().exists() and stamp.exists() and stamp.read_text().strip() == _digest()
+    return (_stamped(lib_path(), LIBDIR / "build.sha256", _digest())
+            and _stamped(host_module_path(), LIBDIR / "build_host.sha256", _host_digest()))
+
+
+def _compile_host() -> None:
+    import torch
+
+    root = pathlib.Path(torch.__file__).parent
+    cuda = pathlib.Path(_nvcc()).resolve().parent.parent
+    includes = [root / "include", root / "include" / "torch" / "csrc" / "api" / "include", sysconfig.get_paths()["include"],
+                cuda / "include", INCLUDE]
+    tmp = LIBDIR / (HOST_MODULE + ".so.tmp")
+    cmd = [os.environ.get("CXX", "g++"), *HOST_FLAGS, f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           *(f"-I{d}" for d in includes), str(HOST_SOURCE), "-o", str(tmp), f"-L{root / 'lib'}", "-lc10", "-lc10_cuda",
+           "-ltorch_cpu", "-ltorch_python"]
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        raise RuntimeError("host compiler failed:\n" + " ".join(cmd) + "\n" + res.stdout + res.stderr)
+    os.replace(tmp, host_module_path())
+    (LIBDIR / "build_host.sha256").write_text(_host_digest() + "\n")
 
 
 def _nvcc() -> str:
@@ -89,7 +132,7 @@ def _compile_one(nvcc: str, src: pathlib.Path, obj: pathlib.Path, verbose: bool)
 
 
 def build(force: bool = False, verbose: bool = False) -> pathlib.Path:
-    """Compile every ``csrc/*.cu`` and link one shared library (no-op when current)."""
+    """Compile every ``csrc/*.cu``, link one shared library and compile the host module (no-op when current)."""
     if not force and not verbose and is_current():
         return lib_path()
     nvcc = _nvcc()
@@ -104,7 +147,10 @@ def build(force: bool = False, verbose: bool = False) -> pathlib.Path:
         objs.append(obj)
         if force or verbose or not obj.exists() or not stamp.exists() or stamp.read_text().strip() != want:
             jobs.append((src, obj, stamp, want))
-    with concurrent.futures.ThreadPoolExecutor(max_workers=max(1, min(len(jobs), os.cpu_count() or 1))) as pool:
+    with concurrent.futures.ThreadPoolExecutor(max_workers=max(1, min(len(jobs) + 1, os.cpu_count() or 1))) as pool:
+        host = None
+        if force or not _stamped(host_module_path(), LIBDIR / "build_host.sha256", _host_digest()):
+            host = pool.submit(_compile_host)
         futures = {pool.submit(_compile_one, nvcc, src, obj, verbose): (src, stamp, want) for src, obj, stamp, want in jobs}
         for fut in concurrent.futures.as_completed(futures):
             src, stamp, want = futures[fut]
@@ -112,6 +158,8 @@ def build(force: bool = False, verbose: bool = False) -> pathlib.Path:
             stamp.write_text(want + "\n")
             if verbose:
                 print(f"==== {src.name}\n{log}")
+        if host is not None:
+            host.result()
     tmp = LIBDIR / (LIBNAME + ".tmp")
     cmd = [nvcc, *LINK_FLAGS, "-o", str(tmp), *map(str, objs)]
     res = subprocess.run(cmd, capture_output=True, text=True)

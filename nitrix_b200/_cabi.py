@@ -168,6 +168,27 @@ def lib() -> C.CDLL:
     return L
 
 
+@functools.lru_cache(maxsize=1)
+def torch_ops():
+    """The extension module with the differentiable operations (csrc/host/torch_ops.cpp), bound to :func:`lib`."""
+    import importlib.machinery
+    import importlib.util
+
+    import torch
+
+    path = _build.host_module_path()
+    if not path.exists():
+        raise NativeLibraryError(f"{path} is missing: build it with `python -m nitrix_b200._build`.")
+    loader = importlib.machinery.ExtensionFileLoader(_build.HOST_MODULE, str(path))
+    module = importlib.util.module_from_spec(importlib.util.spec_from_loader(_build.HOST_MODULE, loader))
+    loader.exec_module(module)
+    if module.torch_version != torch.__version__.split("+")[0]:
+        raise NativeLibraryError(f"{path} was built for torch {module.torch_version}, this is {torch.__version__}: build it anew")
+    L = lib()
+    module.bind({name: C.cast(getattr(L, name), C.c_void_p).value for name in module.entry_points()})
+    return module
+
+
 def enqueue(fn, params, device) -> int:
     """``fn(&params, stream)`` on the current stream of ``device`` (a ``torch.device`` with an index), which is made
     the current device only where it is not already; returns the library's status code."""

@@ -12,7 +12,9 @@ residuals ``(q, k, v, bias, mask, out, lse)``, cotangents
 Differences, all on purpose:
 
 * tensors are ``torch`` CUDA tensors (device memory, streams); the arithmetic
-  is done by the CUDA library behind ``include/nitrix_b200_attention.h``;
+  is done by the CUDA library behind ``include/nitrix_b200_attention.h``, the
+  differentiation rule is a C++ autograd function over it
+  (``csrc/host/torch_ops.cpp``);
 * bias and mask are passed by stride, never broadcast-materialised, and q/k/v
   stay in ``(..., h, s, d)`` layout (the reference transposes and materialises,
   ``attention.py:507-514,560-569``);
@@ -57,69 +59,17 @@ def qk_rms_norm(z: torch.Tensor) -> torch.Tensor:
     return (zf * torch.rsqrt(zf.square().mean(-1, keepdim=True) + _QK_RMS_EPS)).to(z.dtype)
 
 
-def _norm_desc(x: torch.Tensor, y: torch.Tensor, g: Optional[torch.Tensor] = None) -> "_cabi.QkNormTensor":
-    """Describes ``x`` viewed as (B, H, N, D) -- leading dims flattened -- for the fused pre-op."""
-    t = _cabi.QkNormTensor()
-    h, n = x.shape[-3], x.shape[-2]
-    x4 = x.reshape((-1, h, n, x.shape[-1])) if x.dim() != 4 else x
-    t.x, t.y, t.g = x4.data_ptr(), y.data_ptr(), (g.data_ptr() if g is not None else None)
-    t.xs[0], t.xs[1], t.xs[2] = x4.stride(0), x4.stride(1), x4.stride(2)
-    t.B, t.H, t.N = x4.shape[0], h, n
-    return t
-
-
 def _qk_norm_fusable(q: torch.Tensor, k: torch.Tensor) -> bool:
     """Both on one CUDA device, same supported dtype and head dim, rows the kernel can read with 16-byte loads."""
-    if not (q.is_cuda and k.is_cuda and q.device == k.device and q.dtype == k.dtype and q.dtype in _DTYPES):
-        return False
-    d = q.shape[-1]
-    vec = 16 // q.element_size()
-    if q.dim() < 3 or k.dim() < 3 or k.shape[-1] != d or d % vec or d > 256:
-        return False
-    for z in (q, k):
-        if z.stride(-1) != 1 or z.data_ptr() % 16:
-            return False
-        z4 = z if z.dim() == 4 else (z.reshape((-1,) + tuple(z.shape[-3:])) if z.is_contiguous() else None)
-        if z4 is None or any(st % vec for st in z4.stride()[:3]):
-            return False
-    return True
-
-
-class _QkRmsNorm(torch.autograd.Function):
-    """``(q, k) -> (qk_rms_norm(q), qk_rms_norm(k))`` as one kernel launch each way (``nb200_qk_rms_norm`` /
-    ``nb200_qk_rms_norm_grad``) instead of a chain of element-wise passes.  Same place in the call sequence as the
-    reference's pre-op (``nn/attention/__init__.py:193-197``): outside the attention kernels' own differentiation
-    rule, so autograd chains the two."""
-
-    @staticmethod
-    def forward(ctx, q, k):
-        qn, kn = torch.empty(q.shape, dtype=q.dtype, device=q.device), torch.empty(k.shape, dtype=k.dtype, device=k.device)
-        dk_ = _norm_desc(k, kn)
-        rc = _cabi.enqueue(lambda a, stream: _cabi.lib().nb200_qk_rms_norm(a, C.byref(dk_), q.shape[-1], _DTYPES[q.dtype],
-                                                                          stream), _norm_desc(q, qn), q.device)
-        if rc != 0:
-            raise RuntimeError("nb200_qk_rms_norm: " + _cabi.last_error())
-        ctx.save_for_backward(q, k)
-        return qn, kn
-
-    @staticmethod
-    def backward(ctx, gq, gk):
-        q, k = ctx.saved_tensors
-        gq, gk = gq.contiguous().to(q.dtype), gk.contiguous().to(k.dtype)
-        dq, dk = torch.empty(q.shape, dtype=q.dtype, device=q.device), torch.empty(k.shape, dtype=k.dtype, device=k.device)
-        dk_ = _norm_desc(k, dk, gk)
-        rc = _cabi.enqueue(lambda a, stream: _cabi.lib().nb200_qk_rms_norm_grad(a, C.byref(dk_), q.shape[-1],
-                                                                               _DTYPES[q.dtype], stream),
-                           _norm_desc(q, dq, gq), q.device)
-        if rc != 0:
-            raise RuntimeError("nb200_qk_rms_norm_grad: " + _cabi.last_error())
-        return dq, dk
+    return _cabi.torch_ops().qk_norm_fits(q, k)
 
 
 def qk_rms_norm_pair(q: torch.Tensor, k: torch.Tensor):
-    """``qk_rms_norm`` of q and k: the fused CUDA pre-op where its layout rules hold, else the element-wise form."""
+    """``qk_rms_norm`` of q and k: one kernel launch each way (``nb200_qk_rms_norm`` / ``nb200_qk_rms_norm_grad``) where
+    that pre-op's layout rules hold, else the element-wise form.  Same place in the call sequence as the reference's
+    (``nn/attention/__init__.py:193-197``): outside the attention kernels' own differentiation rule."""
     if _qk_norm_fusable(q, k):
-        return _QkRmsNorm.apply(q, k)
+        return _cabi.torch_ops().qk_norm(q, k)
     return qk_rms_norm(q), qk_rms_norm(k)
 
 
@@ -253,9 +203,16 @@ def _mask_bytes(mask):
     return (mask != 0).view(torch.uint8)
 
 
+_plan_cache: dict = {}
+
+
 def planned_kernel(q, k, v, bias=None, mask=None, *, scale=1.0, causal=False, which=_cabi.PASS_FWD,
                    kernel=_cabi.KERNEL_AUTO, want_dbias=False) -> int:
-    """Kernel family the library would run for these 4-D operands (no launch)."""
+    """Kernel family the library would run for these 4-D operands (no launch; remembered by their layout)."""
+    key = (_meta(q), _meta(k), _meta(v), _meta(bias), _mask_meta(mask), float(scale), bool(causal), q.device.index, which,
+           kernel, bool(want_dbias))
+    if key in _plan_cache:
+        return _plan_cache[key]
     p = _cabi.new_params()
     B, H, S, _ = q.shape
     out = q  # pointers are not dereferenced by the planner
@@ -269,6 +226,9 @@ def planned_kernel(q, k, v, bias=None, mask=None, *, scale=1.0, causal=False, wh
         p.dbias_stride[:] = [bias.shape[1] * bias.shape[2] * bias.shape[3], bias.shape[2] * bias.shape[3], bias.shape[3], 1]
     chosen = C.c_int(0)
     _check(_cabi.lib().nb200_sdpa_plan(C.byref(p), which, C.byref(chosen)), "nb200_sdpa_plan")
+    if len(_plan_cache) >= 512:
+        _plan_cache.clear()
+    _plan_cache[key] = chosen.value
     return chosen.value
 
 
@@ -284,9 +244,6 @@ def pack_mask(q, k, v, mask, *, with_transpose: bool = True) -> PackedMask:
                                                                       blob.numel(), stream), p, q.device),
            "nb200_mask_pack")
     return PackedMask(blob, 2 if with_transpose else 1, mask_b)
-
-
-_plan_cache: dict = {}
 
 
 def _meta(x: Optional[torch.Tensor]):
@@ -336,21 +293,6 @@ def _mask_meta(mask):
     if isinstance(mask, PackedMask):
         return (_meta(mask.like), mask.level, mask.blob.data_ptr() & 15)
     return _meta(mask)
-
-
-def _planned_kernel_cached(q, k, v, bias, mask, scale, causal, which=_cabi.PASS_FWD, kernel=_cabi.KERNEL_AUTO,
-                           want_dbias=False) -> int:
-    """Plan for these operands, remembered by their layout (the planner is pure in it)."""
-    key = (_meta(q), _meta(k), _meta(v), _meta(bias), _meta(mask), float(scale), bool(causal), q.device.index,
-           which, kernel, bool(want_dbias))
-    chosen = _plan_cache.get(key)
-    if chosen is None:
-        chosen = planned_kernel(q, k, v, bias, mask, scale=scale, causal=causal, which=which, kernel=kernel,
-                                want_dbias=want_dbias)
-        if len(_plan_cache) >= 512:
-            _plan_cache.clear()
-        _plan_cache[key] = chosen
-    return chosen
 
 
 def sdpa_forward(q, k, v, bias=None, mask=None, *, scale: float, causal: bool = False,
@@ -467,41 +409,6 @@ def sdpa_backward(q, k, v, bias, mask, out, lse, dout, *, scale: float, causal: 
     return dq, dk, dv, dbias
 
 
-class _SDPA(torch.autograd.Function):
-    """Differentiation rule of the fused path (reference ``attention.py:661-700``)."""
-
-    @staticmethod
-    def forward(ctx, q, k, v, bias, mask, scale, causal, kernel, fused):
-        # On the fused (tensor-core) path the mask is bit-packed ONCE, with the key-major copy, and the same bits
-        # serve the forward and the backward; otherwise each pass reads the byte mask.
-        packed = None
-        want_dbias = bias is not None and ctx.needs_input_grad[3]
-        if want_dbias and _has_expanded_axis(bias):
-            bias = bias.contiguous()   # as in sdpa_backward, here so that both passes and the plan see one layout
-        if fused and mask is not None:
-            if _planned_kernel_cached(q, k, v, bias, mask, scale, causal, _cabi.PASS_BWD, kernel,
-                                      want_dbias) == _cabi.KERNEL_TCGEN05:
-                packed = pack_mask(q, k, v, mask, with_transpose=True)
-        out, lse = sdpa_forward(q, k, v, bias, mask if packed is None else packed, scale=scale, causal=causal,
-                                kernel=kernel)
-        ctx.save_for_backward(q, k, v, bias, mask, out, lse)
-        ctx.packed = packed
-        ctx.scale, ctx.causal, ctx.kernel = scale, causal, kernel
-        ctx.mark_non_differentiable(lse)
-        ctx.set_materialize_grads(False)   # (no zeros for lse's cotangent: an allocation and a launch per backward)
-        return out, lse
-
-    @staticmethod
-    def backward(ctx, dout, _dlse):
-        if dout is None:
-            return (None,) * 9
-        q, k, v, bias, mask, out, lse = ctx.saved_tensors
-        want_dbias = bias is not None and ctx.needs_input_grad[3]
-        dq, dk, dv, dbias = sdpa_backward(q, k, v, bias, mask if ctx.packed is None else ctx.packed, out, lse, dout,
-                                          scale=ctx.scale, causal=ctx.causal, want_dbias=want_dbias, kernel=ctx.kernel)
-        return dq, dk, dv, dbias, None, None, None, None, None
-
-
 def scaled_dot_product_attention(
     q: torch.Tensor,
     k: torch.Tensor,
@@ -544,45 +451,40 @@ def scaled_dot_product_attention(
     if qk_norm:
         q, k = qk_rms_norm_pair(q, k)
 
-    h, s, d = q.shape[-3:]
-    t, dv = k.shape[-2], v.shape[-1]
-    lq, lk, lv = tuple(q.shape[:-3]), tuple(k.shape[:-3]), tuple(v.shape[:-3])
-    lead = lq if (lq == lk and lq == lv) else tuple(torch.broadcast_shapes(lq, lk, lv))
-    if k.shape[-3] != h or v.shape[-3] != h:
-        raise ValueError(f"scaled_dot_product_attention: head-count mismatch (q {h}, k {k.shape[-3]}, v {v.shape[-3]})")
-    q4, k4, v4 = _to_bhxd(q, lead, h), _to_bhxd(k, lead, h), _to_bhxd(v, lead, h)
-    bias4 = None
-    if bias is not None:
-        if bias.dtype not in _DTYPES:
-            bias = bias.to(torch.float32)
-        bias4 = _to_own_extent(bias, lead, h, s, t)
-    mask4 = None if mask is None else _to_own_extent(mask, lead, h, s, t)
-
     kernel = _KERNELS[resolved]
-    fused = False
-    if resolved == "cuda-sm100":
-        chosen = _planned_kernel_cached(q4, k4, v4, bias4, mask4, resolved_scale, causal)
-        fused = chosen == _cabi.KERNEL_TCGEN05
-        # fp32 operands on the tensor-core kernels are a fused path too (fp32 is the one dtype the reference's
-        # fused kernels accept, attention.py:736-744): only a problem that leaves the tensor paths altogether warns
-        if chosen not in (_cabi.KERNEL_TCGEN05, _cabi.KERNEL_MMA_TF32X3):
-            fallback(
-                function="scaled_dot_product_attention",
-                requested="cuda-sm100",
-                resolved="cuda-simt",
-                reason=(
-                    "the fused tcgen05 kernels take bf16/fp16 with d == d_v in {64, 128} (any query/key lengths); "
-                    "the fp32 tensor-core kernels take d, d_v in {32, 64, 128}"
-                ),
-                shapes=(tuple(q.shape), tuple(k.shape), tuple(v.shape)),
-                dtype=out_dtype,
-            )
-    needs_grad = torch.is_grad_enabled() and (
-        q4.requires_grad or k4.requires_grad or v4.requires_grad or (bias4 is not None and bias4.requires_grad))
-    if needs_grad:
-        out4, lse4 = _SDPA.apply(q4, k4, v4, bias4, mask4, resolved_scale, bool(causal), kernel, fused)
-    else:   # nothing to differentiate: skip the autograd bookkeeping
-        out4, lse4 = sdpa_forward(q4, k4, v4, bias4, mask4, scale=resolved_scale, causal=bool(causal), kernel=kernel)
+    attention = _cabi.torch_ops().attention
+    operands = (q, k, v, bias, mask)
+    lead, (h, s) = tuple(q.shape[:-3]), q.shape[-3:-1]
+    dv = v.shape[-1]
+    out4, lse4, fit = attention(*operands, resolved_scale, bool(causal), kernel, False)
+    if not fit:
+        t, lk, lv = k.shape[-2], tuple(k.shape[:-3]), tuple(v.shape[:-3])
+        lead = lead if (lead == lk and lead == lv) else tuple(torch.broadcast_shapes(lead, lk, lv))
+        if k.shape[-3] != h or v.shape[-3] != h:
+            raise ValueError(f"scaled_dot_product_attention: head-count mismatch (q {h}, k {k.shape[-3]}, v {v.shape[-3]})")
+        if bias is not None:
+            bias = _to_own_extent(bias if bias.dtype in _DTYPES else bias.to(torch.float32), lead, h, s, t)
+        if mask is not None:
+            mask = _mask_bytes(_to_own_extent(mask, lead, h, s, t))
+        operands = (_to_bhxd(q, lead, h), _to_bhxd(k, lead, h), _to_bhxd(v, lead, h), bias, mask)
+        out4, lse4, fit = attention(*operands, resolved_scale, bool(causal), kernel, False)
+        if not fit:
+            raise ValueError("scaled_dot_product_attention: q, k, v, bias and mask must be on one CUDA device")
+    if out4 is None:
+        # fp32 operands on the tensor-core kernels are a fused path too (fp32 is the one dtype the reference's fused
+        # kernels accept, attention.py:736-744): only a problem that leaves the tensor paths altogether warns
+        fallback(
+            function="scaled_dot_product_attention",
+            requested="cuda-sm100",
+            resolved="cuda-simt",
+            reason=(
+                "the fused tcgen05 kernels take bf16/fp16 with d == d_v in {64, 128} (any query/key lengths); "
+                "the fp32 tensor-core kernels take d, d_v in {32, 64, 128}"
+            ),
+            shapes=(tuple(q.shape), tuple(k.shape), tuple(v.shape)),
+            dtype=out_dtype,
+        )
+        out4, lse4, _ = attention(*operands, resolved_scale, bool(causal), kernel, True)
     out = out4 if len(lead) == 1 else out4.reshape(*lead, h, s, dv)
     if return_lse:
         return out, lse4 if len(lead) == 1 else lse4.reshape(*lead, h, s)

@@ -78,36 +78,6 @@ def layer_norm_backward(x2, weight, dy2, mean, rstd, eps: float, out_scale: floa
     return dx, dw, db
 
 
-class _LayerNorm(torch.autograd.Function):
-    """The differentiation rule of the fused op: saves (x, weight, mean, rstd), returns (dx, dweight, dbias)."""
-
-    @staticmethod
-    def forward(ctx, x, weight, bias, eps, out_scale):
-        x2 = x.reshape(-1, x.shape[-1]).contiguous()
-        w = None if weight is None else weight.to(x.dtype).contiguous()
-        b = None if bias is None else bias.to(x.dtype).contiguous()
-        y, mean, rstd = layer_norm_forward(x2, w, b, eps, out_scale)
-        ctx.save_for_backward(x2, w if w is not None else x2.new_empty(0), mean, rstd)
-        ctx.has_weight, ctx.has_bias = weight is not None, bias is not None
-        ctx.eps, ctx.out_scale, ctx.shape = eps, out_scale, x.shape
-        ctx.param_dtypes = (None if weight is None else weight.dtype, None if bias is None else bias.dtype)
-        return y.reshape(x.shape)
-
-    @staticmethod
-    def backward(ctx, dy):
-        x2, w, mean, rstd = ctx.saved_tensors
-        dy2 = dy.reshape(-1, dy.shape[-1]).to(x2.dtype).contiguous()
-        need_w = ctx.has_weight and ctx.needs_input_grad[1]
-        need_b = ctx.has_bias and ctx.needs_input_grad[2]
-        dx, dw, db = layer_norm_backward(x2, w if ctx.has_weight else None, dy2, mean, rstd, ctx.eps, ctx.out_scale,
-                                         need_w, need_b)
-        if dw is not None:
-            dw = dw.to(ctx.param_dtypes[0])
-        if db is not None:
-            db = db.to(ctx.param_dtypes[1])
-        return dx.reshape(ctx.shape), dw, db, None, None
-
-
 def layer_norm(x: torch.Tensor, weight: Optional[torch.Tensor] = None, bias: Optional[torch.Tensor] = None, *,
                eps: float = 1e-5, out_scale: float = 1.0, backend: str = "auto") -> torch.Tensor:
     """LayerNorm over the trailing axis: ``out_scale * (xhat * weight + bias)`` (reference
@@ -119,4 +89,4 @@ def layer_norm(x: torch.Tensor, weight: Optional[torch.Tensor] = None, bias: Opt
         raise TypeError(f"layer_norm: x must be a CUDA tensor of float32, bfloat16 or float16; got {x.dtype} on {x.device}")
     if x.numel() == 0:
         return torch.empty_like(x)
-    return _LayerNorm.apply(x, weight, bias, float(eps), float(out_scale))
+    return _cabi.torch_ops().layer_norm(x, weight, bias, float(eps), float(out_scale))

@@ -11,6 +11,7 @@ argument chooses among XLA formulations of the same recurrence and has no counte
 from __future__ import annotations
 
 import ctypes as C
+import functools
 from typing import Optional
 
 import torch
@@ -78,16 +79,20 @@ def selective_scan_forward(x3, delta3, A, B3, C3, D, want_checkpoints: bool):
     return y, ck
 
 
-def _workspace(p, device) -> torch.Tensor:
+def _workspace(need: int, least: int, like: torch.Tensor) -> torch.Tensor:
     """The backward's scratch; where the device has no room for the adjoint states of the whole batch at once (as large as
     the checkpoints), the least with which it runs, a range after the other."""
     try:
-        ws = torch.empty(max(_bytes(_cabi.lib().nb200_selective_scan_workspace_bytes, p), 16), dtype=torch.uint8, device=device)
+        return torch.empty(max(need, 16), dtype=torch.uint8, device=like.device)
     except torch.OutOfMemoryError:
-        ws = torch.empty(max(_bytes(_cabi.lib().nb200_selective_scan_workspace_least_bytes, p), 16), dtype=torch.uint8,
-                         device=device)
-    p.workspace, p.workspace_bytes = ws.data_ptr(), ws.numel()
-    return ws
+        return torch.empty(max(least, 16), dtype=torch.uint8, device=like.device)
+
+
+@functools.lru_cache(maxsize=1)
+def _ops():
+    ops = _cabi.torch_ops()
+    ops.set_scan_allocator(_workspace)
+    return ops
 
 
 def selective_scan_backward(x3, delta3, A, B3, C3, D, ck, dy3):
@@ -101,55 +106,12 @@ def selective_scan_backward(x3, delta3, A, B3, C3, D, ck, dy3):
     p.checkpoints = None if ck is None else ck.data_ptr()
     p.dx, p.ddelta, p.dA, p.dB, p.dC = (t.data_ptr() for t in (dx, ddelta, dA, dB, dC))
     p.dD = None if dD is None else dD.data_ptr()
-    ws = _workspace(p, x3.device)
+    ws = _workspace(_bytes(_cabi.lib().nb200_selective_scan_workspace_bytes, p),
+                    _bytes(_cabi.lib().nb200_selective_scan_workspace_least_bytes, p), x3)
+    p.workspace, p.workspace_bytes = ws.data_ptr(), ws.numel()
     _check(_cabi.enqueue(_cabi.lib().nb200_selective_scan_bwd, p, x3.device), "nb200_selective_scan_bwd")
     del ws  # same-stream reuse is ordered by the caching allocator
     return dx, ddelta, dA, dB, dC, dD
-
-
-class _SelectiveScan(torch.autograd.Function):
-    """The differentiation rule of the fused op: saves the operands and the forward's checkpoints."""
-
-    @staticmethod
-    def forward(ctx, x, delta, A, B, C_, D):
-        dt = x.dtype
-        lead = x.shape[:-2]
-        x3 = x.reshape((-1,) + tuple(x.shape[-2:])).contiguous()
-        delta3 = delta.to(dt).reshape(x3.shape).contiguous()
-        B3 = B.to(dt).expand(lead + tuple(B.shape[-2:])).reshape((-1,) + tuple(B.shape[-2:])).contiguous()
-        C3 = C_.to(dt).expand(lead + tuple(C_.shape[-2:])).reshape((-1,) + tuple(C_.shape[-2:])).contiguous()
-        A2 = A.to(dt).contiguous()
-        D1 = None if D is None else D.to(dt).contiguous()
-        need_grad = any(ctx.needs_input_grad)
-        y, ck = selective_scan_forward(x3, delta3, A2, B3, C3, D1, need_grad)
-        ctx.save_for_backward(x3, delta3, A2, B3, C3, D1 if D1 is not None else x3.new_empty(0),
-                              ck if ck is not None else x3.new_empty(0, dtype=torch.float32))
-        ctx.has_D = D is not None
-        ctx.shapes = (x.shape, delta.shape, B.shape, C_.shape)
-        ctx.dtypes = (delta.dtype, A.dtype, B.dtype, C_.dtype, None if D is None else D.dtype)
-        return y.reshape(x.shape)
-
-    @staticmethod
-    def backward(ctx, dy):
-        x3, delta3, A2, B3, C3, D1, ck = ctx.saved_tensors
-        dy3 = dy.to(x3.dtype).reshape(x3.shape).contiguous()
-        dx, ddelta, dA, dB, dC, dD = selective_scan_backward(x3, delta3, A2, B3, C3, D1 if ctx.has_D else None,
-                                                              ck if ck.numel() else None, dy3)
-        xs, ds, bs, cs = ctx.shapes
-        lead = xs[:-2]
-
-        def back_to(g3, shape):   # gradient of an operand that was broadcast over the leading axes
-            g = g3.reshape(lead + tuple(g3.shape[-2:]))
-            while g.dim() > len(shape):
-                g = g.sum(0)
-            for ax, extent in enumerate(shape):
-                if extent == 1 and g.shape[ax] != 1:
-                    g = g.sum(ax, keepdim=True)
-            return g
-
-        dl_t, a_t, b_t, c_t, d_t = ctx.dtypes
-        return (dx.reshape(xs), ddelta.reshape(ds).to(dl_t), dA.to(a_t), back_to(dB, bs).to(b_t),
-                back_to(dC, cs).to(c_t), None if dD is None else dD.to(d_t))
 
 
 def selective_scan(x: torch.Tensor, delta: torch.Tensor, A: torch.Tensor, B: torch.Tensor, C: torch.Tensor,  # noqa: N803
@@ -165,4 +127,4 @@ def selective_scan(x: torch.Tensor, delta: torch.Tensor, A: torch.Tensor, B: tor
         raise ValueError(f"selective_scan: at most 64 states per channel are supported; got n={A.shape[1]}.")
     if x.numel() == 0:
         return torch.empty_like(x)
-    return _SelectiveScan.apply(x, delta, A, B, C, D)
+    return _ops().selective_scan(x, delta, A, B, C, D)
