@@ -8,13 +8,14 @@
 // recurrence and readout whatever the storage dtype (reference _reference.py:262-279).
 //
 // Nothing of size (l, d, n) is materialised.  Forward: four lanes own one channel of one batch element, a quarter of
-// its states each, and walk the sequence with them in registers; every eighth step's state goes to a checkpoint array
-// (batch, l / 8, d, n).  Backward, two kernels: ss_adjoint_kernel walks the sequence once more, last step first, with
+// its states each, and walk the sequence with them in registers (in segments side by side where there are few channels);
+// every eighth step's state goes to a checkpoint array (batch, l / 8, d, n).  Backward, two kernels: ss_adjoint_kernel walks the sequence once more, last step first, with
 // the adjoint recurrence g_t = a_{t+1} g_{t+1} + C_t dy_t alone and leaves g at the same eighth steps; with both
 // states known at its borders every chunk of eight steps is then independent of all others, and ss_bwd_kernel
 // computes the gradients chunk by chunk in parallel.  Its sums over channels (dB_t, dC_t) go through a shared-memory
 // tile and 16-byte reductions into fp32 accumulators, those over batch and time (dA, dD) are kept per thread over the
 // chunks of a CTA and added once; ss_finish_kernel converts the accumulators to the storage dtype.
+#include <cooperative_groups.h>
 #include <math.h>
 
 #include "nitrix_b200_scan.h"
@@ -22,6 +23,8 @@
 
 namespace nb200 {
 namespace {
+
+namespace cg = cooperative_groups;
 
 constexpr int kStep = 8;    // steps per checkpoint interval = chunk of the backward
 
@@ -39,6 +42,7 @@ struct SsArgs {
   // launches of the backward for a range of channels (kRange): the first of them, and how many gck's rows hold (channel 0's
   // states would be at gck)
   int d_first, gD;
+  int seg;                // steps of a segment where the walks are split in time (kSplit), a multiple of kStage
 };
 
 // a_t = exp(delta_t A) as one multiply and one ex2.approx (relative error 2^-22): A is held pre-multiplied by log2(e)
@@ -224,12 +228,49 @@ __device__ __forceinline__ void write_pairs(float2* p, float4 a, float4 b) {
 }
 __device__ __forceinline__ float2 both(float v) { return make_float2(v, v); }
 
+// The walks split in time.  Few channels leave most of the GPU idle while a few CTAs walk a long sequence step by step, a
+// step costing its latencies alone (72 ns with one CTA per SM, where seven share one they take 132 ns together).  So a
+// cluster of up to eight CTAs takes the sequence in segments: each walks its own from an empty state, keeping its end and
+// the sum of its deltas (whose exponential is the segment's whole decay), reads those of the segments before it over
+// distributed shared memory, and walks again from the state they give.  About 1.6 times the work, four or eight times the
+// SMs (walk_splits has the figures).
+template <int kN, bool kUsed>
+struct Segment {
+  float h[kScanCh][kN];
+  float span[kScanCh];   // sum of delta
+  // Publishes this segment's end; returns in `state` what enters it, from segments first, first + step .. own - step.
+  template <int kPairs>
+  __device__ __forceinline__ void join(int first, int own, int step, int ch, int part, float my_span, const float2 (&rate)[kPairs],
+                                       float2 (&state)[kPairs]) {
+#pragma unroll
+    for (int k = 0; k < kPairs; ++k) {
+      h[ch][part * 2 * kPairs + 2 * k] = state[k].x;
+      h[ch][part * 2 * kPairs + 2 * k + 1] = state[k].y;
+      state[k] = make_float2(0.f, 0.f);
+    }
+    if (part == 0) span[ch] = my_span;
+    cg::cluster_group cluster = cg::this_cluster();
+    cluster.sync();
+    for (int s = first; s != own; s += step) {
+      const float* rh = cluster.map_shared_rank(&h[ch][part * 2 * kPairs], s);
+      const float d = *cluster.map_shared_rank(&span[ch], s);
+#pragma unroll
+      for (int k = 0; k < kPairs; ++k)
+        state[k] = __ffma2_rn(ex2_ss2(__fmul2_rn(both(d), rate[k])), state[k], make_float2(rh[2 * k], rh[2 * k + 1]));
+    }
+  }
+};
+template <int kN>
+struct Segment<kN, false> {};
+
 // kShort: sequences of up to kStage - 4 steps, one loop over the groups of four that exist (one step of 128 x 2048 channels,
 // f32: 31 -> 17 us; an instantiation of its own, since the test costs the others up to a fifth by another order of the
 // instructions).
-template <typename T, int kN, bool kShort>
+// kSplit: the sequence in segments of a.seg steps, one CTA of a cluster each.
+template <typename T, int kN, bool kShort, bool kSplit>
 __global__ void __launch_bounds__(kScanThreads) ss_fwd_kernel(SsArgs a) {
   constexpr int kQ = kN / 4;
+  __shared__ Segment<kN, kSplit> segment;
   __shared__ __align__(16) float2 du[kStage * kScanCh];    // delta, delta x
   __shared__ __align__(16) float sB[kStage * kN], sC[kStage * kN];
   __shared__ __align__(16) float sy[kStage * kYPitch];
@@ -259,15 +300,42 @@ __global__ void __launch_bounds__(kScanThreads) ss_fwd_kernel(SsArgs a) {
     nB.load(Bp, t0, a.L, a.N, vecn, tid);
     nC.load(Cp, t0, a.L, a.N, vecn, tid);
   };
-  load(0);
-  for (int t0 = 0; t0 < a.L; t0 += kStage) {
+  const int t_begin = kSplit ? int(blockIdx.z) * a.seg : 0, t_end = kSplit ? min(a.L, t_begin + a.seg) : a.L;
+  if constexpr (kSplit) {
+    // the segment from an empty state: nothing but the recurrence (the last segment's end is nobody's start)
+    float span = 0.f;
+    if (blockIdx.z + 1 < gridDim.z) {
+      load(t_begin);
+      for (int t0 = t_begin; t0 < t_end; t0 += kStage) {
+        const float4 cx = nx.get(vec), dl4 = nd.get(vec);
+        __syncthreads();   // (the steps before have been read)
+        write_pairs(du + lr * kScanCh + lc, dl4, make_float4(dl4.x * cx.x, dl4.y * cx.y, dl4.z * cx.z, dl4.w * cx.w));
+        nB.store(sB, vecn, tid);
+        __syncthreads();
+        if (t0 + kStage < t_end) load(t0 + kStage);
+#pragma unroll
+        for (int u = 0; u < kStage; ++u) {
+          const float2 w = du[u * kScanCh + ch];
+          float2 Bv[kQ / 2];
+          row_pairs<kQ>(sB + u * kN + part * kQ, Bv);
+          span += w.x;
+#pragma unroll
+          for (int k = 0; k < kQ / 2; ++k)
+            h[k] = __ffma2_rn(ex2_ss2(__fmul2_rn(both(w.x), Ar[k])), h[k], __fmul2_rn(both(w.y), Bv[k]));
+        }
+      }
+    }
+    segment.join(0, int(blockIdx.z), 1, ch, part, span, Ar, h);
+  }
+  load(kSplit ? t_begin : 0);
+  for (int t0 = kSplit ? t_begin : 0; t0 < (kSplit ? t_end : a.L); t0 += kStage) {
     // (steps past the sequence's end are staged as zeros: the state stays as it is)
     const float4 cx = nx.get(vec), dl4 = nd.get(vec);
     write_pairs(du + lr * kScanCh + lc, dl4, make_float4(dl4.x * cx.x, dl4.y * cx.y, dl4.z * cx.z, dl4.w * cx.w));
     nB.store(sB, vecn, tid);
     nC.store(sC, vecn, tid);
     __syncthreads();
-    if (!kShort && t0 + kStage < a.L) load(t0 + kStage);
+    if (!kShort && t0 + kStage < (kSplit ? t_end : a.L)) load(t0 + kStage);
     // four steps at a time, in three phases: operands and decays (nothing in them depends on the state), then the
     // recurrence, then the sums over the lanes
 #pragma unroll
@@ -313,12 +381,14 @@ __global__ void __launch_bounds__(kScanThreads) ss_fwd_kernel(SsArgs a) {
     if (a.D) v = make_float4(fmaf(Dd.x, cx.x, v.x), fmaf(Dd.y, cx.y, v.y), fmaf(Dd.z, cx.z, v.z), fmaf(Dd.w, cx.w, v.w));
     store4<T>(yp + int64_t(t0 + lr) * a.Dc, v, t0 + lr < a.L ? ln : 0, vec);
   }
+  if constexpr (kSplit) cg::this_cluster().sync();   // (nobody reads this CTA's shared memory any more)
 }
 
 // The adjoint recurrence alone, last step first: leaves for every chunk but the last the g that enters it.
-template <typename T, int kN, bool kRange>
+template <typename T, int kN, bool kRange, bool kSplit>
 __global__ void __launch_bounds__(kScanThreads) ss_adjoint_kernel(SsArgs a) {
   constexpr int kQ = kN / 4;
+  __shared__ Segment<kN, kSplit> segment;
   __shared__ __align__(16) float2 dg[kStage * kScanCh];    // delta, dy
   __shared__ __align__(16) float sC[kStage * kN];
   const int tid = threadIdx.x, part = tid & 3, ch = tid >> 2;
@@ -342,14 +412,40 @@ __global__ void __launch_bounds__(kScanThreads) ss_adjoint_kernel(SsArgs a) {
     nd.load(dp + int64_t(t0 + lr) * a.Dc, n, vec);
     nC.load(Cp, t0, a.L, a.N, vecn, tid);
   };
-  const int last = (a.L - 1) / kStage * kStage;
-  load(last);
-  for (int t0 = last; t0 >= 0; t0 -= kStage) {
+  const int first = kSplit ? int(blockIdx.z) * a.seg : 0;
+  // (below `first`: an empty segment)
+  const int last = kSplit ? min((a.L - 1) / kStage * kStage, first + a.seg - kStage) : (a.L - 1) / kStage * kStage;
+  if constexpr (kSplit) {
+    float span = 0.f;
+    if (blockIdx.z > 0) {   // as in the forward, last segment first
+      load(max(last, 0));
+      for (int t0 = last; t0 >= first; t0 -= kStage) {
+        __syncthreads();
+        write_pairs(dg + lr * kScanCh + lc, nd.get(vec), ng.get(vec));
+        nC.store(sC, vecn, tid);
+        __syncthreads();
+        if (t0 > first) load(t0 - kStage);
+#pragma unroll
+        for (int u = kStage - 1; u >= 0; --u) {
+          const float2 w = dg[u * kScanCh + ch];
+          float2 Cv[kQ / 2];
+          row_pairs<kQ>(sC + u * kN + part * kQ, Cv);
+          span += w.x;
+#pragma unroll
+          for (int k = 0; k < kQ / 2; ++k)
+            g[k] = __fmul2_rn(__ffma2_rn(Cv[k], both(w.y), g[k]), ex2_ss2(__fmul2_rn(both(w.x), Ar[k])));
+        }
+      }
+    }
+    segment.join(int(gridDim.z) - 1, int(blockIdx.z), -1, ch, part, span, Ar, g);
+  }
+  load(kSplit ? max(last, 0) : last);
+  for (int t0 = last; t0 >= first; t0 -= kStage) {
     __syncthreads();
     write_pairs(dg + lr * kScanCh + lc, nd.get(vec), ng.get(vec));
     nC.store(sC, vecn, tid);
     __syncthreads();
-    if (t0 > 0) load(t0 - kStage);
+    if (t0 > first) load(t0 - kStage);
 #pragma unroll
     for (int s0 = kStage - 4; s0 >= 0; s0 -= 4) {
       if ((s0 & 4)) {   // the last step of a chunk of eight: what enters it
@@ -373,6 +469,7 @@ __global__ void __launch_bounds__(kScanThreads) ss_adjoint_kernel(SsArgs a) {
         for (int k = 0; k < kQ / 2; ++k) g[k] = __fmul2_rn(__ffma2_rn(Cv[u][k], both(gy[u]), g[k]), av[u][k]);
     }
   }
+  if constexpr (kSplit) cg::this_cluster().sync();
 }
 
 // ---- gradients of a chunk ----------------------------------------------------------------------------------------
@@ -692,26 +789,68 @@ SsArgs args_of(const nb200_selective_scan_params* p) {
   return a;
 }
 
-dim3 scan_grid(const nb200_selective_scan_params* p) {
-  return dim3((p->channels + kScanCh - 1) / kScanCh, p->batch);
+int segment_steps(int length, int splits) {
+  const int stages = (length + kStage - 1) / kStage;
+  return (stages + splits - 1) / splits * kStage;
 }
-template <typename T, bool kShort>
-int fwd_launch(const nb200_selective_scan_params* p, const SsArgs& a, cudaStream_t st) {
-  const dim3 grid = scan_grid(p);
-  switch (pick_n(p->states)) {
-    case 8: ss_fwd_kernel<T, 8, kShort><<<grid, kScanThreads, 0, st>>>(a); break;
-    case 16: ss_fwd_kernel<T, 16, kShort><<<grid, kScanThreads, 0, st>>>(a); break;
-    case 32: ss_fwd_kernel<T, 32, kShort><<<grid, kScanThreads, 0, st>>>(a); break;
-    default: ss_fwd_kernel<T, 64, kShort><<<grid, kScanThreads, 0, st>>>(a); break;
+// Segments of the walks, 1: not split.  Two give nothing (1.6 times the work: (1, 2048, 2048, 16) 352 -> 341 us, (4, 2048,
+// 1024, 16) 446 -> 465), so four or eight, as many as leave up to eight CTAs per SM -- four from 32 states on, whose CTAs
+// hold more registers and shared memory: (4, 600, 300, 64) 248, as four segments 227, as eight 302 -- and 24 steps each.
+// All kernels of forward and backward, us before / now: bf16 (5, 1847, 136, 8) 280 / 124, (2, 1274, 277, 32) 276 / 142, f32
+// (1, 2048, 128, 16) 264 / 85, (1, 2048, 2048, 16) 352 / 219, (4, 2048, 1024, 16) 446 / 406, (3, 166, 297, 8) 37 / 32.
+int walk_splits(int64_t ctas, int64_t length, int states) {
+  int sms = 0, dev = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (sms <= 0) sms = 148;
+  const int64_t room = (states > 16 ? 4 : 8) * int64_t(sms);
+  for (int splits = 8; splits >= 4; splits /= 2)
+    if (splits * ctas <= room && length >= 24 * splits) return splits;
+  return 1;
+}
+
+// One of the walks over `grid`, as clusters of `splits` CTAs along z.
+template <typename Kernel>
+int walk_launch(Kernel kernel, dim3 grid, int splits, const SsArgs& a, cudaStream_t st, const char* what) {
+  if (splits == 1) {
+    kernel<<<grid, kScanThreads, 0, st>>>(a);
+  } else {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid.x, grid.y, unsigned(splits));
+    cfg.blockDim = dim3(kScanThreads);
+    cfg.stream = st;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = 1;
+    attr.val.clusterDim.y = 1;
+    attr.val.clusterDim.z = unsigned(splits);
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, a);
   }
   count_launch();
-  return check_launch("selective_scan_fwd_kernel");
+  return check_launch(what);
+}
+template <typename T, bool kShort, bool kSplit>
+int fwd_launch(const nb200_selective_scan_params* p, const SsArgs& a, int splits, cudaStream_t st) {
+  const dim3 grid((p->channels + kScanCh - 1) / kScanCh, p->batch);
+  auto kernel = ss_fwd_kernel<T, 64, kShort, kSplit>;
+  switch (pick_n(p->states)) {
+    case 8: kernel = ss_fwd_kernel<T, 8, kShort, kSplit>; break;
+    case 16: kernel = ss_fwd_kernel<T, 16, kShort, kSplit>; break;
+    case 32: kernel = ss_fwd_kernel<T, 32, kShort, kSplit>; break;
+  }
+  return walk_launch(kernel, grid, splits, a, st, "selective_scan_fwd_kernel");
 }
 
 template <typename T>
 int fwd_t(const nb200_selective_scan_params* p, cudaStream_t st) {
-  const SsArgs a = args_of<T>(p);
-  return p->length <= kStage - 4 ? fwd_launch<T, true>(p, a, st) : fwd_launch<T, false>(p, a, st);
+  SsArgs a = args_of<T>(p);
+  if (p->length <= kStage - 4) return fwd_launch<T, true, false>(p, a, 1, st);
+  const int splits = walk_splits(int64_t(p->channels + kScanCh - 1) / kScanCh * p->batch, p->length, p->states);
+  if (splits == 1) return fwd_launch<T, false, false>(p, a, 1, st);
+  a.seg = segment_steps(p->length, splits);
+  return fwd_launch<T, false, true>(p, a, splits, st);
 }
 
 // workspace of the backward: the fp32 accumulators, then the adjoint states between the chunks
@@ -776,19 +915,26 @@ int chunks_per_cta(int64_t groups, int64_t batch, int64_t chunks) {
   return int(per < chunks ? per : chunks);
 }
 
+template <typename T, bool kRange, bool kSplit>
+int adjoint_launch(const nb200_selective_scan_params* p, const SsArgs& a, dim3 grid, int splits, cudaStream_t st) {
+  auto kernel = ss_adjoint_kernel<T, 64, kRange, kSplit>;
+  switch (pick_n(p->states)) {
+    case 8: kernel = ss_adjoint_kernel<T, 8, kRange, kSplit>; break;
+    case 16: kernel = ss_adjoint_kernel<T, 16, kRange, kSplit>; break;
+    case 32: kernel = ss_adjoint_kernel<T, 32, kRange, kSplit>; break;
+  }
+  return walk_launch(kernel, grid, splits, a, st, "selective_scan_adjoint_kernel");
+}
+
 // The two kernels of one range: `a` with its batch pointers at the range's first element.
 template <typename T, bool kRange>
 int bwd_range(const nb200_selective_scan_params* p, const SsArgs& a, Range r, cudaStream_t st) {
   if (a.chunks > 1) {
     const dim3 grid((r.channels + kScanCh - 1) / kScanCh, r.batch);
-    switch (pick_n(p->states)) {
-      case 8: ss_adjoint_kernel<T, 8, kRange><<<grid, kScanThreads, 0, st>>>(a); break;
-      case 16: ss_adjoint_kernel<T, 16, kRange><<<grid, kScanThreads, 0, st>>>(a); break;
-      case 32: ss_adjoint_kernel<T, 32, kRange><<<grid, kScanThreads, 0, st>>>(a); break;
-      default: ss_adjoint_kernel<T, 64, kRange><<<grid, kScanThreads, 0, st>>>(a); break;
-    }
-    count_launch();
-    if (int rc = check_launch("selective_scan_adjoint_kernel")) return rc;
+    const int splits = kRange ? 1 : walk_splits(int64_t(grid.x) * grid.y, p->length, p->states);
+    SsArgs w = a;
+    w.seg = segment_steps(p->length, splits);
+    if (int rc = splits == 1 ? adjoint_launch<T, kRange, false>(p, w, grid, 1, st) : adjoint_launch<T, false, true>(p, w, grid, splits, st)) return rc;
   }
   const unsigned groups = (r.channels + kBwdCh - 1) / kBwdCh;
   const dim3 grid(groups, unsigned((a.chunks + a.per_cta - 1) / a.per_cta), unsigned(r.batch));

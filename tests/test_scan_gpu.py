@@ -133,3 +133,16 @@ def test_sequences_that_end_inside_a_staged_chunk(length):
 def test_many_sequences_of_few_channels(batch, length, d, n):
     # several chunks per CTA so that fewer CTAs add to the same sums of dA and dD, the last CTA of a sequence with fewer
     _run((batch,), length, d, n, torch.float32)
+
+
+@pytest.mark.parametrize("lead,length,d,n,dtype", [
+    ((1,), 96, 16, 8, torch.float32),        # four segments of 32 steps, the last empty
+    ((2,), 97, 5, 16, torch.float32),        # a segment of one step
+    ((1,), 192, 33, 3, torch.bfloat16),      # eight segments, two of them empty
+    ((3,), 400, 20, 32, torch.float32),      # eight of 64, the last ragged
+    ((1,), 131, 130, 64, torch.float16),
+    ((2,), 95, 40, 16, torch.float32),       # just below the line: not split
+])
+def test_walks_split_in_time(lead, length, d, n, dtype):
+    """Few channels: segments of the sequence walked side by side, joined by their decays."""
+    _run(lead, length, d, n, dtype, seed=length)
