@@ -12,13 +12,19 @@
 // CTA, and the next item's loads and first MMAs run under the current item's
 // epilogue.  Items are ordered heaviest first (causal) and, when the bias is
 // shared over the batch, batch-fastest so concurrent CTAs hit the same bias
-// tiles in L2.  Twelve warps:
+// tiles in L2.  Twelve warps at D = 128, twenty at D = 64:
 //   warp 0      TMA producer for Q (per item) and the K / V rings
 //   warp 1      TMA producer for the bias ring (128 x 64 slots)
 //   warp 2      issues tcgen05.mma for query tile 0 (one elected lane)
 //   warp 3      issues tcgen05.mma for query tile 1; owns the TMEM allocation
-//   warps 4-7   softmax of query tile 0 (one row per thread)
-//   warps 8-11  softmax of query tile 1
+//   warps 4-7   softmax of query tile 0, warps 8-11 that of query tile 1: one row per thread at D = 128, at D = 64 the
+//               first half of a row's keys, and warps 12-15, 16-19 the second
+// Two warps per scheduler cannot keep the special-function unit busy (a pair of exponentials with its arithmetic takes 17.8
+// cycles of it with two warps, 16.7 with four, 16 being its rate, and nothing covers the rest of a pass); four do, where
+// their registers suffice: D = 64 forward, fp16 B1 H16 L8192 512 -> 427 us, causal with a shared bias B8 H16 L2048 192 ->
+// 157, key padding B32 H8 L1024 114 -> 104.  At D = 128 the same split spills (1559 -> 2149 us on B4 H32 L4096 with bias and
+// mask); there the passes without tests for what a problem does not have took 1068 -> 951 (B1 H16 L16384 causal, per-key
+// bias) and 1617 -> 1551.
 // TMEM (512 columns).  D = 128: [0,128) S0, [128,256) S1, then O0, O1.  There is no
 // room for separate P tiles, so a key tile is taken as two halves of 64 keys: each
 // half has its own 64-column S buffer and its P (16-bit, 32 columns) overwrites
@@ -30,7 +36,10 @@
 // soon as softmax(j) has read S out and runs underneath it.
 // P feeds the PV MMA as the TMEM A operand; V is consumed from shared memory as
 // an MN-major B operand, so nothing is transposed or staged through shared memory.
-// All waits are bounded (sdpa_tc_common.cuh).
+// All waits on mbarriers are bounded (sdpa_tc_common.cuh); the barriers of two warps that share rows, which cannot be, are met
+// by both whatever happens.
+#include <type_traits>
+
 #include "sdpa_tc_common.cuh"
 #include "sdpa_tc_fwd.cuh"
 
@@ -41,22 +50,31 @@ using namespace sm100;
 
 namespace {
 
-constexpr int kThreads = 384;
-// register split after start-up (setmaxnreg): the softmax warps hold a whole score row
-constexpr int kProducerRegs = 56;
-constexpr int kSoftmaxRegs = 216;
+constexpr int kMaxOrder = 288;   // batch elements that a CTA ranks by kept length (item order 3)
+// Softmax warps per query tile: four (a thread owns a row) or eight (two threads share a row, each half of a pass's keys).
+template <int D>
+struct Split {
+  static constexpr int kHalves = D == 64 ? 2 : 1;
+  static constexpr int kThreads = 128 + 256 * kHalves;
+  // register split after start-up (setmaxnreg).  setmaxnreg.inc blocks (without bound) until the CTA's OWN pool -- the
+  // registers it was launched with, kLaunchRegs per thread -- holds enough released registers, so the hand-over must
+  // balance at compile time.
+  static constexpr int kLaunchRegs = kHalves == 1 ? 168 : 96;   // 65536 / kThreads rounded down to a multiple of 8
+  static constexpr int kProducerRegs = kHalves == 1 ? 56 : 64;
+  static constexpr int kSoftmaxRegs = kHalves == 1 ? 216 : 104;
+  static_assert((kLaunchRegs - kProducerRegs) * 128 >= (kSoftmaxRegs - kLaunchRegs) * 256 * kHalves,
+                "softmax warps would wait forever for registers the producer warps never release");
+};
+#ifndef NB200_POLY64
+#define NB200_POLY64 0
+#endif
 #ifndef NB200_POLY_PERIOD
 #define NB200_POLY_PERIOD 4
 #endif
-// D = 128: one pair in this many computes 2^x without the special-function unit (0: none).  There the two query
-// tiles' soft-maxes run at the same time and share the unit; at D = 64 the extra arithmetic costs more than it saves.
-constexpr int kPolyPeriod = NB200_POLY_PERIOD;
-// setmaxnreg.inc blocks (without bound) until the CTA's OWN pool -- the registers it was launched with, here
-// kLaunchRegs per thread -- holds enough released registers, so the hand-over must balance at compile time.
-constexpr int kLaunchRegs = 168;  // what __launch_bounds__(384, 1) gives: 65536 / 384 rounded down to a multiple of 8
-static_assert((kLaunchRegs - kProducerRegs) * 128 >= (kSoftmaxRegs - kLaunchRegs) * 256,
-              "softmax warps would wait forever for registers the producer warps never release");
-
+// One pair in this many computes 2^x without the special-function unit, which all softmax warps share; at D = 64 only bf16
+// with bias tiles, where the tensor core's bias add leaves issue slots (163 -> 156 us causal, 1227 -> 1151 B4 H32 L4096 with
+// bias and mask; without tiles 427 -> 447).
+constexpr int kPolyPeriod = NB200_POLY_PERIOD, kPolyPeriod64 = 16;
 #ifdef NB200_PROBE
 // Development aid (not compiled into the library): cycles one softmax warp spends in each phase of its tiles.
 __device__ unsigned long long g_fprobe[16];
@@ -96,13 +114,16 @@ struct FwdSmem {
   static constexpr int kNumBars = 4 + 4 * kStages + 16 + 3 * kBiasSlots + 2 * kAugSlots;
   static constexpr int kMisc = kBars + 8 * kNumBars;      // tmem base (4 B) + abort flag (4 B)
   static constexpr int kOrder = kMisc + 16;               // batch indices by kept length (item order 3), 16-bit each
-  static constexpr int kTotal = kOrder + 2 * kThreads;
+  static constexpr int kExchange = kOrder + 2 * kMaxOrder;   // one fp32 per query row of both tiles
+  static constexpr int kTotal = kExchange + 2 * kTile * 4;
 };
 
 // One work item: two query tiles of one (batch, head).
 struct Item {
   int b, h, q0;
-  int nt[2], nt_max;
+  int nt0, nt1, nt_max;
+  // (selected, not indexed: an array with a run-time index lives in local memory)
+  __device__ __forceinline__ int nt(int g) const { return g ? nt1 : nt0; }
 };
 
 __device__ __forceinline__ Item decode_item(const FwdArgs& a, int item, const uint16_t* order) {
@@ -157,22 +178,26 @@ __device__ __forceinline__ Item decode_item(const FwdArgs& a, int item, const ui
   // so that a batch with no kept key still produces its (NaN) rows
   const int kept = kept_key_length(a.mask, it.b, it.h, a.T);
   const int n_kt = max(1, (kept + kTile - 1) / kTile);
-#pragma unroll
-  for (int g = 0; g < 2; ++g) {
-    const int q0g = it.q0 + g * kTile;
-    it.nt[g] = q0g >= a.S ? 0 : (a.causal ? min(n_kt, q0g / kTile + 1) : n_kt);
-  }
-  it.nt_max = max(it.nt[0], it.nt[1]);
+  auto tiles = [&](int q0g) { return q0g >= a.S ? 0 : (a.causal ? min(n_kt, q0g / kTile + 1) : n_kt); };
+  it.nt0 = tiles(it.q0);
+  it.nt1 = tiles(it.q0 + kTile);
+  it.nt_max = max(it.nt0, it.nt1);
   return it;
 }
 
-template <int D, bool kBf16, bool kTileBias>
-__global__ void __launch_bounds__(kThreads, 1)
+// What the softmax warps add to the scores themselves: nothing (no bias, or the tensor core has added it; the scale is then
+// folded into the exponent), a tile of the bias, or a per-key bias and / or the scale.  Compiled apart, so that the common
+// loop neither tests for the others at every pass nor holds registers for them.
+enum SoftmaxAdd : int { kAddNone = 0, kAddTile = 1, kAddAny = 2 };
+
+template <int D, bool kBf16, bool kTileBias, int kAdd>
+__global__ void __launch_bounds__(Split<D>::kThreads, 1)
 sdpa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                    const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_bias,
                    const FwdArgs a) {
   using L = FwdSmem<D, kTileBias>;
   constexpr int kStages = L::kStages;
+  constexpr int kThreads = Split<D>::kThreads, kHalves = Split<D>::kHalves;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   // the swizzled tiles need a 1024-byte aligned base; the launch reserves the slack for rounding up
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -195,6 +220,7 @@ sdpa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   //   are computed while the softmax warps work on the current one.
   // D = 64 leaves room for separate P tiles, so the next score MMA can run under the current softmax.
   constexpr bool kAlias = D == 128;
+  constexpr int kPoly = kAlias ? kPolyPeriod : NB200_POLY64;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n_items = a.n_qblocks * a.bh_count;
@@ -202,12 +228,12 @@ sdpa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   if (threadIdx.x == 0) {
     for (int i = 0; i < L::kNumBars; ++i) {
       uint32_t count = 1;
-      if (i >= P_READY && i < P_READY + 4) count = 4;                       // one lane per softmax warp of the tile
+      if (i >= P_READY && i < P_READY + 4) count = 4 * kHalves;                       // one lane per softmax warp of the tile
       if (i >= K_EMPTY && i < K_EMPTY + kStages) count = 2;    // one arrival per MMA issuer
       if (i >= V_EMPTY && i < V_EMPTY + kStages) count = 2;
-      if (i >= O_FREE && i < O_FREE + 2) count = 4;                         // one lane per softmax warp of the tile
-      if (i >= S_FREE && i < S_FREE + 2) count = 4;
-      if (i >= B_EMPTY && i < B_EMPTY + L::kBiasSlots) count = a.bias_mma ? 1 : 4;   // MMA issuer or the tile's warps
+      if (i >= O_FREE && i < O_FREE + 2) count = 4 * kHalves;                         // one lane per softmax warp of the tile
+      if (i >= S_FREE && i < S_FREE + 2) count = 4 * kHalves;
+      if (i >= B_EMPTY && i < B_EMPTY + L::kBiasSlots) count = a.bias_mma ? 1 : (kAlias ? 4 * kHalves : 4);   // MMA issuer or the warps that read it
       if (i >= AUG_FREE && i < AUG_FREE + L::kAugSlots) count = 2;        // one arrival per MMA issuer
       mbar_init(bar(i), count);
     }
@@ -263,16 +289,17 @@ sdpa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem = *tmem_slot;
-  const uint32_t tm_S[2] = {tmem, tmem + 128};
-  const uint32_t tm_P[2] = {kAlias ? tmem : tmem + 256, kAlias ? tmem + 128 : tmem + 320};
-  const uint32_t tm_O[2] = {kAlias ? tmem + 256 : tmem + 384, kAlias ? tmem + 256 + D : tmem + 384 + D};
+  // first columns of query tile g's scores, probabilities and output
+  auto tm_S = [&](int g) { return tmem + g * 128; };
+  auto tm_P = [&](int g) { return kAlias ? tmem + g * 128 : tmem + 256 + g * 64; };
+  auto tm_O = [&](int g) { return kAlias ? tmem + 256 + g * D : tmem + 384 + g * D; };
 
   // Phase bookkeeping across items (every role derives the same numbers from the same item list):
   //   kv   key tiles streamed so far            -> ring stage kv % kStages, phase (kv / kStages) & 1
   //   tc_g tiles query tile g has processed     -> phase of s_full / p_ready / s_free / pv_done
   //   oc_g items in which query tile g was live -> phase of q_full / q_empty / o_done / o_free
   if (warp < 4) {
-  reg_dealloc<kProducerRegs>();
+  reg_dealloc<Split<D>::kProducerRegs>();
   if (warp == 0) {
     // ---------------- Q / K / V producer ----------------
     if (elect_one()) {
@@ -285,7 +312,7 @@ sdpa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         const Item it = decode_item(a, item, order);
 #pragma unroll
         for (int g = 0; g < 2; ++g) {
-          if (it.nt[g] == 0) continue;
+          if (it.nt(g) == 0) continue;
           // the previous item's last score MMA must have finished reading Q_g
           if (oc[g] > 0) ok = ok && wait_or_abort(bar(Q_EMPTY + g), (oc[g] - 1) & 1, abort_flag, a.status, 100);
           if (!ok) break;
@@ -382,7 +409,7 @@ sdpa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         // slots are filled in the order: for each key tile, for each live query tile, column half 0 then 1
         for (int j = 0; j < it.nt_max && ok; ++j) {
           for (int g = 0; g < 2 && ok; ++g) {
-            if (j >= it.nt[g]) continue;
+            if (j >= it.nt(g)) continue;
             for (int half = 0; half < 2; ++half, ++seq) {
               const int slot = seq % L::kBiasSlots;
               const uint32_t ph = (seq / L::kBiasSlots) & 1;
@@ -406,25 +433,22 @@ sdpa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     // An issuer observes every key tile of the rings, also those its query tile skips, and commits once per
     // tile to the "empty" barriers (with nothing outstanding the arrival is immediate): one arrival per
     // issuer per phase.
-    const int g_begin = warp - 2, g_end = warp - 1;
+    const int g = warp - 2;
     if (elect_one()) {
       constexpr uint32_t idesc_qk = make_idesc(kBf16, kTile, kTile, false, false);
       constexpr uint32_t idesc_pv = make_idesc(kBf16, kTile, D, false, true);
-      // descriptors are built once; a tile offset only moves the 16-byte start-address field
-      uint64_t qdesc[2], kdesc[kStages], vdesc[kStages];
-#pragma unroll
-      for (int g = 0; g < 2; ++g) qdesc[g] = make_smem_desc(sbase + L::kQ + g * L::kTileBytes, 16, 1024);
-#pragma unroll
-      for (int s = 0; s < kStages; ++s) {
-        kdesc[s] = make_smem_desc(sbase + L::kK + s * L::kTileBytes, 16, 1024);
-        vdesc[s] = make_smem_desc(sbase + L::kV + s * L::kTileBytes, kBoxBytes, 1024);
-      }
+      // descriptors are built once; a tile or stage offset only moves the 16-byte start-address field
+      const uint64_t qdesc = make_smem_desc(sbase + L::kQ + g * L::kTileBytes, 16, 1024);
+      const uint64_t kdesc0 = make_smem_desc(sbase + L::kK, 16, 1024);
+      const uint64_t vdesc0 = make_smem_desc(sbase + L::kV, kBoxBytes, 1024);
+      const uint32_t tSg = tm_S(g), tPg = tm_P(g), tOg = tm_O(g);
       bool ok = true;
-      int kv = 0, tc[2] = {0, 0}, oc[2] = {0, 0};
+      int kv = 0, tc = 0, oc = 0;
       int seq_base = 0;            // bias slots filled before this item
       uint32_t bias_phase = 0;     // bit s = parity of this issuer's next wait on its tile's "full" barrier of slot s
       for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
         const Item it = decode_item(a, item, order);
+        const int nt = it.nt(g);
         if constexpr (kAlias) {
           // D = 128: key tiles are taken in two halves of 64 keys.  A query tile's S region holds two 64-column
           // buffers, one per half, and P (16-bit, 32 columns) is written over its own buffer, so the scores of the
@@ -447,18 +471,18 @@ sdpa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
               tc_fence_after_sync();
             }
             if (u < n_sub) {
-              for (int g = g_begin; g < g_end && ok; ++g) {
-                if (j >= it.nt[g]) continue;
+              if (j < nt) {
                 if (u == 0) {
-                  ok = wait_or_abort(bar(Q_FULL + g), oc[g] & 1, abort_flag, a.status, 104);
+                  ok = wait_or_abort(bar(Q_FULL + g), oc & 1, abort_flag, a.status, 104);
                   if (!ok) break;
                   tc_fence_after_sync();
                 }
-                const uint32_t tS = tm_S[g] + hf * 64;
+                const uint32_t tS = tSg + hf * 64;
+                const uint64_t kdesc = kdesc0 + uint64_t(st * (L::kTileBytes >> 4) + ((hf * 64 * 128) >> 4));
 #pragma unroll
                 for (int kk = 0; kk < D / 16; ++kk) {
                   const uint64_t off = uint64_t(((kk / 4) * kBoxBytes + (kk % 4) * 32) >> 4);
-                  mma_ss(tS, qdesc[g] + off, kdesc[st] + off + uint64_t((hf * 64 * 128) >> 4), idesc_qk64, kk > 0 ? 1u : 0u);
+                  mma_ss(tS, qdesc + off, kdesc + off, idesc_qk64, kk > 0 ? 1u : 0u);
                 }
                 if constexpr (!kTileBias) {
                   if (a.key_mma) {
@@ -469,9 +493,8 @@ sdpa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                   }
                 }
                 mma_commit(bar(S_FULL + 2 * g + hf));
-                if (u == 2 * it.nt[g] - 1) mma_commit(bar(Q_EMPTY + g));   // Q_g may be reloaded once these are done
+                if (u == 2 * nt - 1) mma_commit(bar(Q_EMPTY + g));   // Q_g may be reloaded once these are done
               }
-              if (!ok) break;
               if (hf == 1) {
                 mma_commit(bar(K_EMPTY + st));
                 if (!kTileBias && a.key_mma) mma_commit(bar(AUG_FREE + aslot));
@@ -482,23 +505,21 @@ sdpa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                 ok = wait_or_abort(bar(V_FULL + stp), ((kv + jp) / kStages) & 1, abort_flag, a.status, 106);
                 if (!ok) break;
               }
-              for (int g = g_begin; g < g_end && ok; ++g) {
-                if (jp >= it.nt[g]) continue;
-                ok = wait_or_abort(bar(P_READY + 2 * g + hp), (tc[g] + jp) & 1, abort_flag, a.status, 107);
+              if (jp < nt) {
+                ok = wait_or_abort(bar(P_READY + 2 * g + hp), (tc + jp) & 1, abort_flag, a.status, 107);
                 // the previous item's epilogue must have read O_g out before the first half overwrites it
-                if (ok && u == 1 && oc[g] > 0)
-                  ok = wait_or_abort(bar(O_FREE + g), (oc[g] - 1) & 1, abort_flag, a.status, 115);
+                if (ok && u == 1 && oc > 0)
+                  ok = wait_or_abort(bar(O_FREE + g), (oc - 1) & 1, abort_flag, a.status, 115);
                 if (!ok) break;
                 tc_fence_after_sync();
-                const uint32_t tP = tm_S[g] + hp * 64;
+                const uint32_t tP = tSg + hp * 64;
+                const uint64_t vdesc = vdesc0 + uint64_t(stp * (L::kTileBytes >> 4) + ((hp * 4 * 2048) >> 4));
 #pragma unroll
                 for (int kk = 0; kk < kTile / 32; ++kk)
-                  mma_ts(tm_O[g], tP + kk * 8, vdesc[stp] + uint64_t(((hp * 4 + kk) * 2048) >> 4), idesc_pv,
-                         (u > 1 || kk > 0) ? 1u : 0u);
+                  mma_ts(tOg, tP + kk * 8, vdesc + uint64_t((kk * 2048) >> 4), idesc_pv, (u > 1 || kk > 0) ? 1u : 0u);
                 mma_commit(bar(PV_DONE + g));
-                if (u == 2 * it.nt[g]) mma_commit(bar(O_DONE + g));
+                if (u == 2 * nt) mma_commit(bar(O_DONE + g));
               }
-              if (!ok) break;
               if (hp == 1) mma_commit(bar(V_EMPTY + stp));
             }
           }
@@ -513,162 +534,165 @@ sdpa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
             ok = wait_or_abort(bar(AUG_FULL + aslot), ((kv + j) / L::kAugSlots) & 1, abort_flag, a.status, 118);
           if (!ok) break;
           tc_fence_after_sync();
-          for (int g = g_begin; g < g_end && ok; ++g) {
-            const int nt = it.nt[g];
-            auto round_pv = [&]() {
-              const int jj = j - 1;
-              if (j == 0 || jj >= nt) return;
-              ok = wait_or_abort(bar(P_READY + g), (tc[g] + jj) & 1, abort_flag, a.status, 107);
-              // the previous item's epilogue must have read O_g out before the first tile overwrites it
-              if (ok && jj == 0 && oc[g] > 0)
-                ok = wait_or_abort(bar(O_FREE + g), (oc[g] - 1) & 1, abort_flag, a.status, 115);
-              if (!ok) return;
-              tc_fence_after_sync();
+          // S_g was read out early in softmax(j-1): the next scores run underneath it
+          if (j < nt) {
+            const int gt = tc + j;
+            if (j == 0) ok = wait_or_abort(bar(Q_FULL + g), oc & 1, abort_flag, a.status, 104);
+            if (ok && gt > 0) ok = wait_or_abort(bar(S_FREE + g), (gt - 1) & 1, abort_flag, a.status, 111);
+            if (!ok) break;
+            tc_fence_after_sync();
+            const uint64_t kdesc = kdesc0 + uint64_t(st * (L::kTileBytes >> 4));
 #pragma unroll
-              for (int kk = 0; kk < kTile / 16; ++kk)
-                mma_ts(tm_O[g], tm_P[g] + kk * 8, vdesc[stp] + uint64_t((kk * 2048) >> 4), idesc_pv,
-                       (jj > 0 || kk > 0) ? 1u : 0u);
-              mma_commit(bar(PV_DONE + g));
-              if (jj == nt - 1) mma_commit(bar(O_DONE + g));
-            };
-            auto round_qk = [&]() {
-              if (j >= nt) return;
-              const int gt = tc[g] + j;
-              if (j == 0) ok = wait_or_abort(bar(Q_FULL + g), oc[g] & 1, abort_flag, a.status, 104);
-              if (ok && gt > 0) ok = wait_or_abort(bar(S_FREE + g), (gt - 1) & 1, abort_flag, a.status, 111);
-              if (!ok) return;
-              tc_fence_after_sync();
-#pragma unroll
-              for (int kk = 0; kk < D / 16; ++kk) {
-                const uint64_t off = uint64_t(((kk / 4) * kBoxBytes + (kk % 4) * 32) >> 4);
-                mma_ss(tm_S[g], qdesc[g] + off, kdesc[st] + off, idesc_qk, kk > 0 ? 1u : 0u);
+            for (int kk = 0; kk < D / 16; ++kk) {
+              const uint64_t off = uint64_t(((kk / 4) * kBoxBytes + (kk % 4) * 32) >> 4);
+              mma_ss(tSg, qdesc + off, kdesc + off, idesc_qk, kk > 0 ? 1u : 0u);
+            }
+            if constexpr (!kTileBias) {
+              if (a.key_mma) {
+                // S_g += W C^T: the per-key addends land on every query row
+                const uint64_t wdesc = make_smem_desc_noswizzle(sbase + L::kBias, 128, 256);
+                const uint64_t cdesc = make_smem_desc_noswizzle(sbase + L::kBias + L::kAugTileBytes * (1 + aslot), 128, 256);
+                mma_ss(tSg, wdesc, cdesc, idesc_qk, 1u);
               }
-              if constexpr (!kTileBias) {
-                if (a.key_mma) {
-                  // S_g += W C^T: the per-key addends land on every query row
-                  const uint64_t wdesc = make_smem_desc_noswizzle(sbase + L::kBias, 128, 256);
-                  const uint64_t cdesc = make_smem_desc_noswizzle(sbase + L::kBias + L::kAugTileBytes * (1 + aslot), 128, 256);
-                  mma_ss(tm_S[g], wdesc, cdesc, idesc_qk, 1u);
-                }
-              }
-              if constexpr (D == 64 && kTileBias) {
-                if (a.bias_mma) {
-                  // S_g += bias tile (hi I + lo I): each 64-key half of the tile is one slot, read K-major as it
-                  // was written by TMA.  Slot order as the bias producer fills them.
-                  constexpr uint32_t idesc_bias = make_idesc(kBf16, kTile, 64, false, false);
-                  const int seq0 = seq_base + 2 * (min(j, it.nt[0]) + min(j, it.nt[1]) + ((g == 1 && j < it.nt[0]) ? 1 : 0));
-                  const int n_ident = a.inv_scale_lo != 0.f ? 2 : 1;
-                  for (int half = 0; half < 2 && ok; ++half) {
-                    const int slot = (seq0 + half) % L::kBiasSlots;
-                    ok = wait_or_abort(bar(B_FULL + g * L::kBiasSlots + slot), (bias_phase >> slot) & 1u, abort_flag,
-                                       a.status, 116);
-                    if (!ok) return;
-                    bias_phase ^= 1u << slot;
-                    tc_fence_after_sync();
-                    const uint64_t adesc = make_smem_desc(sbase + L::kBias + slot * kBoxBytes, 16, 1024);
-                    for (int tile = 0; tile < n_ident; ++tile) {
-                      const uint64_t bdesc = make_smem_desc(sbase + L::kIdent + tile * 8192, 16, 1024);
+            }
+            if constexpr (D == 64 && kTileBias) {
+              if (a.bias_mma) {
+                // S_g += bias tile (hi I + lo I): each 64-key half of the tile is one slot, read K-major as it
+                // was written by TMA.  Slot order as the bias producer fills them.
+                constexpr uint32_t idesc_bias = make_idesc(kBf16, kTile, 64, false, false);
+                const int seq0 = seq_base + 2 * (min(j, it.nt0) + min(j, it.nt1) + ((g == 1 && j < it.nt0) ? 1 : 0));
+                const int n_ident = a.inv_scale_lo != 0.f ? 2 : 1;
+                for (int half = 0; half < 2 && ok; ++half) {
+                  const int slot = (seq0 + half) % L::kBiasSlots;
+                  ok = wait_or_abort(bar(B_FULL + g * L::kBiasSlots + slot), (bias_phase >> slot) & 1u, abort_flag,
+                                     a.status, 116);
+                  if (!ok) break;
+                  bias_phase ^= 1u << slot;
+                  tc_fence_after_sync();
+                  const uint64_t adesc = make_smem_desc(sbase + L::kBias + slot * kBoxBytes, 16, 1024);
+                  for (int tile = 0; tile < n_ident; ++tile) {
+                    const uint64_t bdesc = make_smem_desc(sbase + L::kIdent + tile * 8192, 16, 1024);
 #pragma unroll
-                      for (int kk = 0; kk < 4; ++kk)
-                        mma_ss(tm_S[g] + half * 64, adesc + uint64_t((kk * 32) >> 4), bdesc + uint64_t((kk * 32) >> 4),
-                               idesc_bias, 1u);
-                    }
-                    mma_commit(bar(B_EMPTY + slot));   // the slot may be refilled once these MMAs are done
+                    for (int kk = 0; kk < 4; ++kk)
+                      mma_ss(tSg + half * 64, adesc + uint64_t((kk * 32) >> 4), bdesc + uint64_t((kk * 32) >> 4),
+                             idesc_bias, 1u);
                   }
+                  mma_commit(bar(B_EMPTY + slot));   // the slot may be refilled once these MMAs are done
                 }
+                if (!ok) break;
               }
-              mma_commit(bar(S_FULL + g));
-              if (j == nt - 1) mma_commit(bar(Q_EMPTY + g));   // Q_g may be reloaded once these are done
-            };
-            round_qk();   // S_g was read out early in softmax(j-1): the next scores run underneath it
-            if (ok) round_pv();
+            }
+            mma_commit(bar(S_FULL + g));
+            if (j == nt - 1) mma_commit(bar(Q_EMPTY + g));   // Q_g may be reloaded once these are done
           }
-          if (!ok) break;
+          const int jj = j - 1;
+          if (j > 0 && jj < nt) {
+            ok = wait_or_abort(bar(P_READY + g), (tc + jj) & 1, abort_flag, a.status, 107);
+            // the previous item's epilogue must have read O_g out before the first tile overwrites it
+            if (ok && jj == 0 && oc > 0)
+              ok = wait_or_abort(bar(O_FREE + g), (oc - 1) & 1, abort_flag, a.status, 115);
+            if (!ok) break;
+            tc_fence_after_sync();
+            const uint64_t vdesc = vdesc0 + uint64_t(stp * (L::kTileBytes >> 4));
+#pragma unroll
+            for (int kk = 0; kk < kTile / 16; ++kk)
+              mma_ts(tOg, tPg + kk * 8, vdesc + uint64_t((kk * 2048) >> 4), idesc_pv, (jj > 0 || kk > 0) ? 1u : 0u);
+            mma_commit(bar(PV_DONE + g));
+            if (jj == nt - 1) mma_commit(bar(O_DONE + g));
+          }
           if (j < it.nt_max) mma_commit(bar(K_EMPTY + st));
           if (!kTileBias && a.key_mma && j < it.nt_max) mma_commit(bar(AUG_FREE + aslot));
           if (j > 0) mma_commit(bar(V_EMPTY + stp));
         }
         }
         kv += it.nt_max;
-        seq_base += 2 * (it.nt[0] + it.nt[1]);
-#pragma unroll
-        for (int g = 0; g < 2; ++g) {
-          tc[g] += it.nt[g];
-          oc[g] += it.nt[g] > 0 ? 1 : 0;
-        }
+        seq_base += 2 * (it.nt0 + it.nt1);
+        tc += nt;
+        oc += nt > 0 ? 1 : 0;
       }
     }
   }
   } else {
-    reg_alloc<kSoftmaxRegs>();
-    // ---------------- softmax (one query row per thread) ----------------
-    const int g = (warp - 4) >> 2;
+    reg_alloc<Split<D>::kSoftmaxRegs>();
+    // ---------------- softmax (a query row, or half of a pass's keys of one, per thread) ----------------
+    const int g = ((warp - 4) >> 2) & 1;        // query tile
+    const int half = kHalves == 1 ? 0 : (warp - 4) >> 3;   // which half of the keys
     const int wq = warp & 3;                    // TMEM lane quarter this warp may access
     const int r = wq * 32 + lane;               // row within the tile
     const uint32_t lane_addr = uint32_t(wq * 32) << 16;
-    const uint32_t tS = tm_S[g] + lane_addr, tP = tm_P[g] + lane_addr, tO = tm_O[g] + lane_addr;
+    // D = 128 takes a key tile as two halves of 64 keys (one S buffer each, P written over its own buffer);
+    // D = 64 takes it whole
+    constexpr int kSub = kAlias ? kTile / 2 : kTile;   // keys per pass
+    constexpr int kSubs = kTile / kSub;
+    constexpr int kCols = kSub / kHalves;              // keys per pass and thread
+    constexpr int kOutCols = D / kHalves;              // output columns per thread
+    const uint32_t tS = tm_S(g) + half * kCols + lane_addr, tO = tm_O(g) + half * kOutCols + lane_addr;
+    const uint32_t tP = tm_P(g) + half * (kCols / 2) + lane_addr;
+    float* const xrow = reinterpret_cast<float*>(smem + L::kExchange) + g * kTile + r;   // this row's word for exchanges
+    const uint32_t pair_bar = 1 + g * 4 + wq;   // named barrier of the two warps that share these rows
     bool ok = true;
-    // no bias and a non-negative scale: the scale is folded into the exponent's multiplier and the max runs on raw scores
-    // (the same holds when the tensor core has already added bias / scale to the scores)
+    // where nothing is added here and the scale is not negative, it is folded into the exponent's multiplier and the max
+    // runs on raw scores
     const bool key_mma = !kTileBias && a.key_mma;
-    const bool fold_scale = (a.bias_mode == kBiasNone || a.bias_mma || key_mma) && a.scale >= 0.f;
-    const float mul = fold_scale ? a.scale * kLog2e : kLog2e;   // exponent = (t - m) * mul, base 2
+    const float mul = kAdd == kAddNone ? a.scale * kLog2e : kLog2e;   // exponent = (t - m) * mul, base 2
     const float thr = mul > 0.f ? 8.f / mul : INFINITY;         // reference max lags the true max by at most 2^8
     const float2 scale2 = make_float2(a.scale, a.scale), mul2 = make_float2(mul, mul);
     uint32_t bias_phase = 0;  // bit s = parity of this tile's next wait on its "full" barrier of slot s
     int tc = 0, oc = 0, seq_base = 0;
     FPROBE_DECL;
 
-    for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
+    // A warp that gives up (`ok` false) waits no more and stores nothing, but walks on through its passes -- nothing in a
+    // pass can leave its TMEM or shared memory -- because its partner waits for it at the pair's barrier, which has no time
+    // limit of its own; and because tests of `ok` around the passes cost registers (up to 1.2 KB of spills, a factor of 2).
+    for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
       const Item it = decode_item(a, item, order);
-      const int my_nt = it.nt[g];
+      const int my_nt = it.nt(g);
       const int row = it.q0 + g * kTile + r;
       const int b = it.b, h = it.h;
-      float m = -INFINITY, l = 0.f;  // m: reference max in logit units (see the lazy rescale below)
+      float m = -INFINITY, l = 0.f;  // m: reference max in logit units (see the lazy rescale below); l: this thread's keys
 
       const uint32_t* mrow = nullptr;
       if (a.mask.rows && !(key_mma && a.mask.kv_len)) {   // a key-only mask was added to the scores as -inf
-        mrow = a.mask.rows + b * a.mask.b_stride + h * a.mask.h_stride + int64_t(min(row, a.S - 1)) * a.mask.row_stride;
+        mrow = a.mask.rows + b * a.mask.b_stride + h * a.mask.h_stride + int64_t(min(row, a.S - 1)) * a.mask.row_stride +
+               half * (kCols / 32);
       }
       const uint8_t* bias_key = nullptr;
-      if (a.bias_mode == kBiasKey && !key_mma)
+      if (kAdd == kAddAny && a.bias_mode == kBiasKey && !key_mma)
         bias_key = reinterpret_cast<const uint8_t*>(a.bias) + 2 * (b * a.bias_bs + h * a.bias_hs);
 
-      // D = 128 takes a key tile as two halves of 64 keys (one S buffer each, P written over its own buffer);
-      // D = 64 takes it whole
-      constexpr int kSub = kAlias ? kTile / 2 : kTile;   // keys per pass
-      constexpr int kSubs = kTile / kSub;
-      uint32_t mnext[kSub / 32];   // keep-bits of this row for the coming pass
-      auto load_mask_words = [](const uint32_t* src, uint32_t (&dst)[kSub / 32]) {
-        if constexpr (kSub == 64) {
-          const uint2 w = __ldg(reinterpret_cast<const uint2*>(src));
-          dst[0] = w.x; dst[1] = w.y;
-        } else {
+      uint32_t mnext[kCols / 32];   // keep-bits of this row for the coming pass
+      auto load_mask_words = [](const uint32_t* src, uint32_t (&dst)[kCols / 32]) {
+        if constexpr (kCols == 32) {
+          dst[0] = __ldg(src);
+        } else if constexpr (kCols == 128) {
           const uint4 w = __ldg(reinterpret_cast<const uint4*>(src));
           dst[0] = w.x; dst[1] = w.y; dst[2] = w.z; dst[3] = w.w;
+        } else {
+          const uint2 w = __ldg(reinterpret_cast<const uint2*>(src));
+          dst[0] = w.x; dst[1] = w.y;
         }
       };
 #pragma unroll
-      for (int i = 0; i < kSub / 32; ++i) mnext[i] = 0xffffffffu;
+      for (int i = 0; i < kCols / 32; ++i) mnext[i] = 0xffffffffu;
       if (mrow && my_nt > 0) load_mask_words(mrow, mnext);
-      for (int j = 0; j < my_nt && ok; ++j) {
+      for (int j = 0; j < my_nt; ++j) {
         const int gt = tc + j;   // this tile's running index for this query tile
 #pragma unroll 1
-        for (int hf = 0; hf < kSubs && ok; ++hf) {
-        const int key0 = j * kTile + hf * kSub;
+        for (int hf = 0; hf < kSubs; ++hf) {
+        const int key0 = j * kTile + hf * kSub + half * kCols;   // this thread's first key
         const bool first = j == 0 && hf == 0;
         const int sbar = kAlias ? 2 * g + hf : g;
         const uint32_t tSh = tS + hf * kSub;
         // keep-bits of this row for these keys
-        uint32_t keep[kSub / 32];
+        uint32_t keep[kCols / 32];
 #pragma unroll
-        for (int i = 0; i < kSub / 32; ++i) keep[i] = 0xffffffffu;
+        for (int i = 0; i < kCols / 32; ++i) keep[i] = 0xffffffffu;
         bool need_mask = false;
         if (mrow) {
           // this pass's words were fetched a pass ago; the next pass's fetch runs under this pass's arithmetic
           uint32_t all = 0xffffffffu;
 #pragma unroll
-          for (int i = 0; i < kSub / 32; ++i) {
+          for (int i = 0; i < kCols / 32; ++i) {
             keep[i] = mnext[i];
             all &= mnext[i];
           }
@@ -678,9 +702,9 @@ sdpa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         }
         int n_keep = a.T - key0;
         if (a.causal) n_keep = min(n_keep, row - key0 + 1);
-        if (n_keep < kSub) {
+        if (n_keep < kCols) {
 #pragma unroll
-          for (int i = 0; i < kSub / 32; ++i) {
+          for (int i = 0; i < kCols / 32; ++i) {
             const int n = n_keep - 32 * i;
             keep[i] &= n >= 32 ? 0xffffffffu : (n <= 0 ? 0u : ((1u << n) - 1u));
           }
@@ -689,17 +713,16 @@ sdpa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         need_mask = __any_sync(0xffffffffu, need_mask);
 
         FPROBE(0);
-        ok = wait_or_abort(bar(S_FULL + sbar), gt & 1, abort_flag, a.status, 108);
+        ok = ok && wait_or_abort(bar(S_FULL + sbar), gt & 1, abort_flag, a.status, 108);
         FPROBE(1);
-        if (!ok) break;
         tc_fence_after_sync();
 
-        // the whole score row of this pass: all TMEM loads in flight, one wait; handled as fp32 pairs
-        float2 t[kSub / 2];
+        // this thread's scores of the pass: all TMEM loads in flight, one wait; handled as fp32 pairs
+        float2 t[kCols / 2];
         {
-          uint32_t raw[kSub];
+          uint32_t raw[kCols];
 #pragma unroll
-          for (int c = 0; c < kSub / 32; ++c) tmem_ld32(tSh + c * 32, *reinterpret_cast<uint32_t(*)[32]>(&raw[c * 32]));
+          for (int c = 0; c < kCols / 32; ++c) tmem_ld32(tSh + c * 32, *reinterpret_cast<uint32_t(*)[32]>(&raw[c * 32]));
           tmem_wait_ld();
           if constexpr (!kAlias) {
             // the scores are in registers: S_g may be overwritten by the next tile's MMA right away
@@ -708,103 +731,118 @@ sdpa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
             if (lane == 0) mbar_arrive(bar(S_FREE + g));
           }
 #pragma unroll
-          for (int i = 0; i < kSub / 2; ++i)
+          for (int i = 0; i < kCols / 2; ++i)
             t[i] = make_float2(__uint_as_float(raw[2 * i]), __uint_as_float(raw[2 * i + 1]));
         }
-        // logits: t = s * scale + bias (natural units); without a bias the scale is folded into the exponent
+        // logits: t = s * scale + bias (natural units); with nothing to add the scale is folded into the exponent
         FPROBE(2);
-        if (a.bias_mode == kBiasTile && !a.bias_mma) {
+        if constexpr (kAdd == kAddTile) {
           // slots filled before this (tile, query tile): every live query tile of the earlier key tiles, and
-          // query tile 0 of this one when this is query tile 1.  One slot per 64 keys.
-          const int seq0 = seq_base + 2 * (min(j, it.nt[0]) + min(j, it.nt[1]) + ((g == 1 && j < it.nt[0]) ? 1 : 0));
+          // query tile 0 of this one when this is query tile 1.  One slot per 64 keys: of two warps that share rows both
+          // read the pass's slot at D = 128; at D = 64 each has its own and only follows the other's phase.
+          const int seq0 = seq_base + 2 * (min(j, it.nt0) + min(j, it.nt1) + ((g == 1 && j < it.nt0) ? 1 : 0));
 #pragma unroll
           for (int hh = 0; hh < kSub / 64; ++hh) {
             const int slot = (seq0 + (kAlias ? hf : hh)) % L::kBiasSlots;
-            ok = wait_or_abort(bar(B_FULL + g * L::kBiasSlots + slot), (bias_phase >> slot) & 1u, abort_flag, a.status,
-                               109);
-            if (!ok) break;
-            bias_phase ^= 1u << slot;
-            const uint8_t* srow = smem + L::kBias + slot * kBoxBytes + r * 128;
+            if (kAlias || kHalves == 1 || hh == half) {
+              ok = ok && wait_or_abort(bar(B_FULL + g * L::kBiasSlots + slot), (bias_phase >> slot) & 1u, abort_flag, a.status,
+                                       109);
+              const uint8_t* srow = smem + L::kBias + slot * kBoxBytes + r * 128;
+              const int c0 = kAlias ? half * (kCols / 8) : 0;   // first 16-byte chunk
+              constexpr int kChunks = kCols < 64 ? kCols / 8 : 8;
+              const int t0 = kCols > 64 ? hh * 32 : 0;          // (a compile-time constant: hh is unrolled)
 #pragma unroll
-            for (int c = 0; c < 8; ++c) {
-              const uint4 w = *reinterpret_cast<const uint4*>(srow + ((c ^ (r & 7)) << 4));
+              for (int c = 0; c < kChunks; ++c) {
+                const uint4 w = *reinterpret_cast<const uint4*>(srow + (((c0 + c) ^ (r & 7)) << 4));
+                const uint32_t ww[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                  t[t0 + c * 4 + e] = __ffma2_rn(t[t0 + c * 4 + e], scale2, unpack2<kBf16>(ww[e]));
+              }
+              __syncwarp();
+              if (lane == 0) mbar_arrive(bar(B_EMPTY + slot));
+            }
+            bias_phase ^= 1u << slot;
+          }
+        } else if constexpr (kAdd == kAddAny) {
+          if (bias_key) {
+            const uint4* bk = reinterpret_cast<const uint4*>(bias_key + 2 * key0);
+#pragma unroll
+            for (int c = 0; c < kCols / 8; ++c) {
+              const uint4 w = key0 + 8 * c < a.T ? __ldg(bk + c) : make_uint4(0, 0, 0, 0);   // T is a multiple of 8
               const uint32_t ww[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
-              for (int e = 0; e < 4; ++e)
-                t[hh * 32 + c * 4 + e] = __ffma2_rn(t[hh * 32 + c * 4 + e], scale2, unpack2<kBf16>(ww[e]));
+              for (int e = 0; e < 4; ++e) t[c * 4 + e] = __ffma2_rn(t[c * 4 + e], scale2, unpack2<kBf16>(ww[e]));
             }
-            __syncwarp();
-            if (lane == 0) mbar_arrive(bar(B_EMPTY + slot));
+          } else {
+#pragma unroll
+            for (int i = 0; i < kCols / 2; ++i) t[i] = __fmul2_rn(t[i], scale2);
           }
-          if (!ok) break;
-        } else if (a.bias_mode == kBiasKey && !key_mma) {
-          const uint4* bk = reinterpret_cast<const uint4*>(bias_key + 2 * key0);
-#pragma unroll
-          for (int c = 0; c < kSub / 8; ++c) {
-            const uint4 w = key0 + 8 * c < a.T ? __ldg(bk + c) : make_uint4(0, 0, 0, 0);   // T is a multiple of 8
-            const uint32_t ww[4] = {w.x, w.y, w.z, w.w};
-#pragma unroll
-            for (int e = 0; e < 4; ++e) t[c * 4 + e] = __ffma2_rn(t[c * 4 + e], scale2, unpack2<kBf16>(ww[e]));
-          }
-        } else if (!fold_scale) {
-#pragma unroll
-          for (int i = 0; i < kSub / 2; ++i) t[i] = __fmul2_rn(t[i], scale2);
         }
         FPROBE(3);
         if (need_mask) {
 #pragma unroll
-          for (int i = 0; i < kSub / 2; ++i) {
+          for (int i = 0; i < kCols / 2; ++i) {
             if (!((keep[i >> 4] >> ((2 * i) & 31)) & 1u)) t[i].x = -INFINITY;
             if (!((keep[i >> 4] >> ((2 * i + 1) & 31)) & 1u)) t[i].y = -INFINITY;
           }
         }
         FPROBE(4);
-        // row max: four independent chains of three-input max
+        // max of these keys: four independent chains of three-input max
         float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
-        for (int i = 0; i < kSub / 2; ++i) mx4[i & 3] = max3(mx4[i & 3], t[i].x, t[i].y);
+        for (int i = 0; i < kCols / 2; ++i) mx4[i & 3] = max3(mx4[i & 3], t[i].x, t[i].y);
         const float mx = max3(mx4[0], mx4[1], fmaxf(mx4[2], mx4[3]));
-        // the exponentials use a reference max that is only moved when the true max has run more than
-        // 2^8 ahead of it (so p <= 256 and the running output is rescaled rarely); l uses the same reference
+        // The exponentials use a reference max that is only moved when the true max has run more than 2^8 ahead of it (so
+        // p <= 256 and the running output is rescaled rarely); l uses the same reference.  Two threads that share a row
+        // share it: their warps agree on whether any of their rows moves (one barrier per pass), and exchange values only
+        // if so.  Past the barrier both have read their scores, so P may overwrite them.
         const bool bump = mx > m + thr;
-        const float m_use = bump ? mx : m;
-        const float alpha = bump ? ex2((m - m_use) * mul) : 1.f;
+        float m_use = m;
+        bool moved = bump;
+        if constexpr (kHalves == 1) {
+          m_use = bump ? mx : m;
+        } else if ((moved = named_barrier_or(pair_bar, 64, bump))) {
+          m_use = bump ? mx : m;
+          if (half == 0) *xrow = m_use;
+          named_barrier_sync(pair_bar, 64);
+          if (half == 1) { m_use = fmaxf(m_use, *xrow); *xrow = m_use; }
+          named_barrier_sync(pair_bar, 64);
+          if (half == 0) m_use = *xrow;
+        }
+        FPROBE(5);
+        const float alpha = m_use > m ? ex2((m - m_use) * mul) : 1.f;
         const float neg = m_use == -INFINITY ? 0.f : -m_use * mul;
         const float2 neg2 = make_float2(neg, neg);
         float2 sum2[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
-        uint32_t pk[kSub / 2];
+        uint32_t pk[kCols / 2];
 #pragma unroll
-        for (int i = 0; i < kSub / 2; ++i) {
+        for (int i = 0; i < kCols / 2; ++i) {
           const float2 x = __ffma2_rn(t[i], mul2, neg2);
-          // every kPolyPeriod-th pair takes its exponentials on the FMA pipe (see ex2_poly2)
-          const float2 p = (kAlias && kPolyPeriod > 0 && i % (kPolyPeriod > 0 ? kPolyPeriod : 1) == 0) ? ex2_poly2(x)
-                                                                                             : make_float2(ex2(x.x), ex2(x.y));
+          // every kPoly-th pair takes its exponentials on the FMA pipe (see ex2_poly2)
+          const float2 p = (kPoly > 0 && i % (kPoly > 0 ? kPoly : 1) == 0) ? ex2_poly2(x) : make_float2(ex2(x.x), ex2(x.y));
           sum2[i & 1] = __fadd2_rn(sum2[i & 1], p);
           pk[i] = pack2<kBf16>(p.x, p.y);
         }
         l = l * alpha + ((sum2[0].x + sum2[0].y) + (sum2[1].x + sum2[1].y));
-        const bool rescale = !first && __any_sync(0xffffffffu, bump);
+        const bool rescale = !first && (kHalves == 1 || moved) && __any_sync(0xffffffffu, m_use > m);
         if constexpr (!kAlias) {
           // O_g and P_g are still in use by the previous tile's output MMA until it has completed
           // (the first tile of an item follows the previous item's epilogue, which waited for that)
-          if (j > 0) {
-            ok = wait_or_abort(bar(PV_DONE + g), (gt - 1) & 1, abort_flag, a.status, 112);
-            if (!ok) break;
-            tc_fence_after_sync();
-          }
+          if (j > 0) ok = ok && wait_or_abort(bar(PV_DONE + g), (gt - 1) & 1, abort_flag, a.status, 112);
+          tc_fence_after_sync();
         } else if (rescale) {
           // O_g is being accumulated into by the previous half's output MMA until that has completed (its P buffer
           // is the other one, and this buffer's earlier reader ran before these scores).  Output MMA number
           // 2 gt + hf - 1 of this query tile: at most one phase of the barrier is outstanding, so parity names it.
-          ok = wait_or_abort(bar(PV_DONE + g), (2 * gt + hf - 1) & 1, abort_flag, a.status, 112);
-          if (!ok) break;
+          ok = ok && wait_or_abort(bar(PV_DONE + g), (2 * gt + hf - 1) & 1, abort_flag, a.status, 112);
           tc_fence_after_sync();
         }
         FPROBE(6);
-        // rescale the running output when some row of this warp moved its reference max
+        // rescale the running output (this thread's columns) when some row of this warp moved its reference max
         if (rescale) {
 #pragma unroll
-          for (int c = 0; c < D / 32; ++c) {
+          for (int c = 0; c < kOutCols / 32; ++c) {
             uint32_t o[32];
             tmem_ld32(tO + c * 32, o);
             tmem_wait_ld();
@@ -813,34 +851,47 @@ sdpa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
             tmem_st32(tO + c * 32, o);
           }
         }
-        m = m_use;
         FPROBE(7);
         // P as 16-bit pairs: half as many columns as keys (over its own S buffer when aliased)
-        const uint32_t tPh = kAlias ? tSh : tP;
+        if constexpr (kCols == 32) {
+          tmem_st16(tP + (kAlias ? hf * kSub : 0), pk);
+        } else {
 #pragma unroll
-        for (int c = 0; c < kSub / 64; ++c) tmem_st32(tPh + c * 32, *reinterpret_cast<const uint32_t(*)[32]>(&pk[c * 32]));
+          for (int c = 0; c < kCols / 64; ++c)
+            tmem_st32(tP + (kAlias ? hf * kSub : 0) + c * 32, *reinterpret_cast<const uint32_t(*)[32]>(&pk[c * 32]));
+        }
         tmem_wait_st();
         tc_fence_before_sync();
         __syncwarp();
         if (lane == 0) mbar_arrive(bar(P_READY + sbar));
         FPROBE(8);
+        m = m_use;
         }
       }
 
       FPROBE(9);
       // ---------------- epilogue: out = O / l, lse = m * mul + log2 l ----------------
-      if (ok && my_nt > 0) ok = wait_or_abort(bar(O_DONE + g), oc & 1, abort_flag, a.status, 110);
+      if (my_nt > 0) {
+        if constexpr (kHalves == 2) {   // l over both halves of the keys
+          if (half == 0) *xrow = l;
+          named_barrier_sync(pair_bar, 64);
+          if (half == 1) { l += *xrow; *xrow = l; }
+          named_barrier_sync(pair_bar, 64);
+          if (half == 0) l = *xrow;
+        }
+        ok = ok && wait_or_abort(bar(O_DONE + g), oc & 1, abort_flag, a.status, 110);
+      }
       if (ok && my_nt > 0) {
         tc_fence_after_sync();
         const float inv = 1.f / l;  // l == 0 (no kept key): 0 * inf = NaN, as the reference's softmax gives
-        const int64_t out_off = 2 * (b * a.os[0] + h * a.os[1] + int64_t(row) * a.os[2]);
+        const int64_t out_off = 2 * (b * a.os[0] + h * a.os[1] + int64_t(row) * a.os[2] + half * kOutCols);
         uint8_t* orow = reinterpret_cast<uint8_t*>(a.out) + out_off;
 #pragma unroll
-        for (int c = 0; c < D / 32; ++c) {
+        for (int c = 0; c < kOutCols / 32; ++c) {
           uint32_t o[32];
           tmem_ld32(tO + c * 32, o);
           tmem_wait_ld();
-          if (c == D / 32 - 1) {
+          if (c == kOutCols / 32 - 1) {
             // O_g is in registers: the next item's first output MMA may overwrite it
             tc_fence_before_sync();
             __syncwarp();
@@ -855,7 +906,14 @@ sdpa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
               x.y = pack2<kBf16>(__uint_as_float(o[i + 2]) * inv, __uint_as_float(o[i + 3]) * inv);
               x.z = pack2<kBf16>(__uint_as_float(o[i + 4]) * inv, __uint_as_float(o[i + 5]) * inv);
               x.w = pack2<kBf16>(__uint_as_float(o[i + 6]) * inv, __uint_as_float(o[i + 7]) * inv);
-              *reinterpret_cast<uint4*>(orow + (c * 32 + i) * 2) = x;
+            }
+            // (every lane of a store is in a row of its own: half as many stores where whole sectors fit)
+            if (a.out_v8) {
+              st_global_v8(orow + c * 64, w[0], w[1]);
+              st_global_v8(orow + c * 64 + 32, w[2], w[3]);
+            } else {
+#pragma unroll
+              for (int i = 0; i < 4; ++i) *reinterpret_cast<uint4*>(orow + c * 64 + i * 16) = w[i];
             }
             // fused all-gather: the same 64 bytes go to every peer's copy, two whole 32-byte sectors per thread
             for (int pi = 0; pi < a.n_out_peers; ++pi) {
@@ -865,11 +923,11 @@ sdpa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
             }
           }
         }
-        if (row < a.S) a.lse[(int64_t(b) * a.H + h) * a.S + row] = m * mul + log2f(l);
+        if (half == 0 && row < a.S) a.lse[(int64_t(b) * a.H + h) * a.S + row] = m * mul + log2f(l);
       }
       tc += my_nt;
       oc += my_nt > 0 ? 1 : 0;
-      seq_base += 2 * (it.nt[0] + it.nt[1]);
+      seq_base += 2 * (it.nt0 + it.nt1);
       FPROBE(10);
       FPROBE_TILES(my_nt);
     }
@@ -886,10 +944,10 @@ sdpa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   }
 }
 
-template <int D, bool kBf16, bool kTileBias>
+template <int D, bool kBf16, bool kTileBias, int kAdd>
 int launch_one(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tb,
                FwdArgs a, cudaStream_t st) {
-  auto kernel = sdpa_fwd_tc_kernel<D, kBf16, kTileBias>;
+  auto kernel = sdpa_fwd_tc_kernel<D, kBf16, kTileBias, kAdd>;
   using L = FwdSmem<D, kTileBias>;
   constexpr int kLimit = 232448;  // 227 KB per CTA
   const int smem = L::kTotal + 1024 <= kLimit ? L::kTotal + 1024 : kLimit;
@@ -902,9 +960,9 @@ int launch_one(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& 
   if (dev < 0 || !ready[dev]) {
     cudaFuncAttributes attr;
     cudaError_t e = cudaFuncGetAttributes(&attr, kernel);
-    if (e != cudaSuccess || attr.numRegs != kLaunchRegs) {
-      // the register hand-over inside the kernel is balanced for exactly kLaunchRegs per thread at launch
-      set_error("sdpa_fwd_tc_kernel was built with %d registers per thread, expected %d", attr.numRegs, kLaunchRegs);
+    if (e != cudaSuccess || attr.numRegs != Split<D>::kLaunchRegs) {
+      // the register hand-over inside the kernel is balanced for exactly that many per thread at launch
+      set_error("sdpa_fwd_tc_kernel was built with %d registers per thread, expected %d", attr.numRegs, Split<D>::kLaunchRegs);
       return NB200_ERR_LAUNCH;
     }
     e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
@@ -917,7 +975,7 @@ int launch_one(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& 
   const int n_items = a.n_qblocks * a.bh_count;
   const int sms = sm_count();
   dim3 grid(n_items < sms ? n_items : sms);
-  kernel<<<grid, kThreads, smem, st>>>(tq, tk, tv, tb, a);
+  kernel<<<grid, Split<D>::kThreads, smem, st>>>(tq, tk, tv, tb, a);
   count_launch();
   return check_launch("sdpa_fwd_tc_kernel");
 }
@@ -928,12 +986,15 @@ int launch_one(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& 
 int launch_fwd(int D, bool bf16, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
                const CUtensorMap& tb, const FwdArgs& a, cudaStream_t st) {
   const bool tiles = a.bias_mode == kBiasTile;
-  if (D == 64) {
-    if (tiles) return bf16 ? launch_one<64, true, true>(tq, tk, tv, tb, a, st) : launch_one<64, false, true>(tq, tk, tv, tb, a, st);
-    return bf16 ? launch_one<64, true, false>(tq, tk, tv, tb, a, st) : launch_one<64, false, false>(tq, tk, tv, tb, a, st);
-  }
-  if (tiles) return bf16 ? launch_one<128, true, true>(tq, tk, tv, tb, a, st) : launch_one<128, false, true>(tq, tk, tv, tb, a, st);
-  return bf16 ? launch_one<128, true, false>(tq, tk, tv, tb, a, st) : launch_one<128, false, false>(tq, tk, tv, tb, a, st);
+  const int add = (a.bias_mode == kBiasNone || a.bias_mma || a.key_mma) && a.scale >= 0.f ? kAddNone : (tiles ? kAddTile : kAddAny);
+  auto go = [&](auto of) { return bf16 ? of(std::true_type()) : of(std::false_type()); };
+  if (D == 64 && tiles && add == kAddNone) return go([&](auto t) { return launch_one<64, t.value, true, kAddNone>(tq, tk, tv, tb, a, st); });
+  if (D == 64 && tiles) return go([&](auto t) { return launch_one<64, t.value, true, kAddTile>(tq, tk, tv, tb, a, st); });
+  if (D == 64 && add == kAddNone) return go([&](auto t) { return launch_one<64, t.value, false, kAddNone>(tq, tk, tv, tb, a, st); });
+  if (D == 64) return go([&](auto t) { return launch_one<64, t.value, false, kAddAny>(tq, tk, tv, tb, a, st); });
+  if (tiles) return go([&](auto t) { return launch_one<128, t.value, true, kAddTile>(tq, tk, tv, tb, a, st); });
+  if (add == kAddNone) return go([&](auto t) { return launch_one<128, t.value, false, kAddNone>(tq, tk, tv, tb, a, st); });
+  return go([&](auto t) { return launch_one<128, t.value, false, kAddAny>(tq, tk, tv, tb, a, st); });
 }
 
 }  // namespace tc

@@ -39,6 +39,7 @@ struct FwdArgs {
   int n_out_peers;
   void* out_peers[NB200_MAX_OUT_PEERS];
   int* status;
+  int out_v8;                   // rows of out are 32-byte aligned
   int smem_bytes;               // dynamic shared memory the launch requested (filled in by launch_fwd)
 };
 

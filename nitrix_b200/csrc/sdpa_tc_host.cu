@@ -584,6 +584,7 @@ int tc_forward(const Problem& original, int dtype, int bias_dtype, void* ws, siz
     a.key_mma = 1;
   a.out = pr.out;
   for (int i = 0; i < 3; ++i) a.os[i] = pr.os[i];
+  a.out_v8 = reinterpret_cast<uintptr_t>(pr.out) % 32 == 0 && pr.os[0] % 16 == 0 && pr.os[1] % 16 == 0 && pr.os[2] % 16 == 0;
   a.lse = pr.lse;
   a.n_out_peers = pr.n_out_peers;
   for (int i = 0; i < pr.n_out_peers; ++i) {
@@ -604,7 +605,7 @@ int tc_forward(const Problem& original, int dtype, int bias_dtype, void* ws, siz
   // more than the K / V locality of the head-major order
   if (a.head_major && pr.causal && int64_t(a.n_qblocks) * pr.bh_count <= 16 * int64_t(tc::sm_count())) a.head_major = 2;
   // key padding: items by kept length, longest first (the kernel ranks the batch elements itself)
-  if (a.head_major && !pr.causal && a.mask.kv_len && a.mask.len_h_stride == 0 && a.mask.len_b_stride != 0 && pr.B > 1 && pr.B <= 384)
+  if (a.head_major && !pr.causal && a.mask.kv_len && a.mask.len_h_stride == 0 && a.mask.len_b_stride != 0 && pr.B > 1 && pr.B <= 288)
     a.head_major = 3;
   return tc::launch_fwd(pr.D, dtype == NB200_BF16, tq, tk, tv, tb, a, stream);
 }

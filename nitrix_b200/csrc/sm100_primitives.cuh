@@ -113,6 +113,19 @@ __device__ __forceinline__ void named_barrier_sync(uint32_t id, uint32_t threads
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
 
+// Named barrier over `threads` threads with an OR of `value`: true for all of them when it is true for any.
+__device__ __forceinline__ bool named_barrier_or(uint32_t id, uint32_t threads, bool value) {
+  uint32_t out;
+  asm volatile(
+      "{\n\t.reg .pred P, Q;\n\tsetp.ne.u32 Q, %3, 0;\n\t"
+      "barrier.cta.red.or.pred P, %1, %2, Q;\n\t"
+      "selp.u32 %0, 1, 0, P;\n\t}"
+      : "=r"(out)
+      : "r"(id), "r"(threads), "r"(uint32_t(value))
+      : "memory");
+  return out != 0;
+}
+
 // ---- TMA (tiled loads into this CTA's shared memory; no multicast) ----------
 __device__ __forceinline__ void tma_prefetch_desc(const void* tmap) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(tmap)) : "memory");
