@@ -247,8 +247,11 @@ __global__ void __launch_bounds__(256) copy16_rows_kernel(const uint16_t* __rest
   }
 }
 
-// (BH, S) fp32 rows -> (BH, Sp) rows, zero beyond S
-__global__ void pad_rows_kernel(const float* __restrict__ src, float* __restrict__ dst, int S, int Sp, int64_t n) {
+// two (BH, S) fp32 arrays -> (BH, Sp) rows, zero beyond S (one launch for lse and delta)
+__global__ void pad_rows_kernel(const float* __restrict__ src0, float* __restrict__ dst0, const float* __restrict__ src1,
+                                float* __restrict__ dst1, int S, int Sp, int64_t n) {
+  const float* src = blockIdx.y ? src1 : src0;
+  float* dst = blockIdx.y ? dst1 : dst0;
   for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) {
     const int64_t bh = i / Sp;
     const int r = int(i - bh * Sp);
@@ -347,9 +350,8 @@ int stage_in(const Problem& pr, const Problem& v, const Staging& sg, int pass, c
   if (sg.rows && pass == NB200_PASS_BWD) {
     const int64_t n = int64_t(pr.B) * pr.H * sg.Sp;
     const int blocks = int(((n + 255) / 256) < 148 * 16 ? ((n + 255) / 256) : 148 * 16);
-    pad_rows_kernel<<<blocks, 256, 0, stream>>>(pr.lse, v.lse, pr.S, sg.Sp, n);
-    pad_rows_kernel<<<blocks, 256, 0, stream>>>(pr.delta, v.delta, pr.S, sg.Sp, n);
-    count_launch(2);
+    pad_rows_kernel<<<dim3(blocks, 2), 256, 0, stream>>>(pr.lse, v.lse, pr.delta, v.delta, pr.S, sg.Sp, n);
+    count_launch();
     if (int rc = check_launch("pad_rows_kernel")) return rc;
   }
   return NB200_OK;
