@@ -22,10 +22,10 @@
 // Merged variant (key-major, D = 64, no bias gradient): ds goes to shared memory instead of TMEM and also feeds
 // dQ = ds K per pair of steps (a 128 x 64 tile at TMEM column 320), which the element-wise warps add to an fp32
 // accumulator in global memory; the query-major kernel is then not needed.
-// Twelve warps: 0 issues the accumulating MMAs, 1 the TMA copies of the step loop (ring refills and bias tiles, one
+// Twelve warps (query-major: twenty): 0 issues the accumulating MMAs, 1 the TMA copies of the step loop (ring refills and bias tiles, one
 // thread serving both), 2 issues the products, 3 owns TMEM and builds the per-query (key-major) or per-key
 // (query-major) addends as MMA operands, 4-7 / 8-11 are two element-wise groups that take alternate steps (one
-// owner row per thread).  The owner tiles and the first ring stages are issued by thread 0 during start-up.  All
+// owner row per thread; query-major: 32 columns of one per thread, 12-15 / 16-19 take the others).  The owner tiles and the first ring stages are issued by thread 0 during start-up.  All
 // waits are bounded.  At head dim 128 these kernels only serve what the one-kernel backward of
 // sdpa_tc_bwd_d128.cu declines (a bias gradient that needs fp32 sums).
 #include <math.h>
@@ -40,31 +40,44 @@ using namespace sm100;
 
 namespace {
 
-constexpr int kThreads = 384;
 constexpr int kStep = 64;                     // streamed rows per step
 constexpr int kYBoxBytes = kStep * 128;       // one 64-row x 128-byte TMA box
-// register split after start-up (setmaxnreg): 128 * kProducerRegs + 256 * kWorkerRegs <= 65536
-constexpr int kProducerRegs = 88;
-constexpr int kWorkerRegs = 208;
-// setmaxnreg.inc blocks (without bound) until the CTA's OWN pool -- the registers it was launched with, here
-// kLaunchRegs per thread -- holds enough released registers, so the hand-over must balance at compile time.
-constexpr int kLaunchRegs = 168;  // what __launch_bounds__(384, 1) gives: 65536 / 384 rounded down to a multiple of 8
-static_assert((kLaunchRegs - kProducerRegs) * 128 >= (kWorkerRegs - kLaunchRegs) * 256,
-              "worker warps would wait forever for registers the producer warps never release");
+// Element-wise warps: two groups that take alternate steps, of four warps (a thread owns an owner row of the step) or eight
+// (two threads share one, 32 of its columns each).  Eight where the element-wise work is the bound, query-major with its
+// dbias tiles or sums: B4 H32 L4096 D64 2580 -> 2395 us, windows of 217 35.4 -> 32.7, D128 137 -> 129; key-major they gained
+// nothing (1540 -> 1605) and merged they lost (204 -> 214; with the longer ring 196 against 200).
+template <bool kKeyMajor, bool kMerged>
+struct Split {
+  static constexpr int kHalves = kKeyMajor ? 1 : 2;
+  static constexpr int kThreads = 128 + 256 * kHalves;
+  // register split after start-up (setmaxnreg).  setmaxnreg.inc blocks (without bound) until the CTA's OWN pool -- the
+  // registers it was launched with, kLaunchRegs per thread -- holds enough released registers, so the hand-over must
+  // balance at compile time.
+  static constexpr int kLaunchRegs = kHalves == 1 ? 168 : 96;   // 65536 / kThreads rounded down to a multiple of 8
+  static constexpr int kProducerRegs = kHalves == 1 ? 88 : 64;
+  static constexpr int kWorkerRegs = kHalves == 1 ? 208 : 104;
+  static_assert((kLaunchRegs - kProducerRegs) * 128 >= (kWorkerRegs - kLaunchRegs) * 256 * kHalves,
+                "worker warps would wait forever for registers the producer warps never release");
+};
 
-
-template <int D, bool kMerged>
+// kTiles: bias tiles are fetched (only told apart in the merged kernel, whose ring takes their place otherwise)
+template <int D, bool kMerged, bool kTiles>
 struct BwdSmem {
   static constexpr int kXBytes = kTile * D * 2;                 // one owner operand
   static constexpr int kYBytes = kStep * D * 2;                 // one streamed operand
-  static constexpr int kYStages = D == 64 ? 4 : 3;
+  // The merged kernel without bias tiles has six ring stages and four addend slots in their place: its issuing warps waited
+  // 655 of 1600 cycles a step for Q and dO, which a stage holds from its fetch to the accumulating MMAs (fp16 B32 H8 L1024
+  // 275 -> 264 us, with key padding 205 -> 197, bf16 causal B8 H16 L2048 292 -> 277).  Five stages beside bias tiles were
+  // no better than four (302 and 303 us, with a mask 1871 and 1950).
+  static constexpr int kYStages = kMerged && !kTiles ? 6 : (D == 64 ? 4 : 3);
   static constexpr int kYStageBytes = 2 * kYBytes + 1024;       // Y1, Y2, then lse[64] + delta[64] (key-major)
-  static constexpr int kBiasSlots = 2;                          // 16 KB each
+  static constexpr int kBiasSlots = kMerged && !kTiles ? 0 : 2;   // 16 KB each
   static constexpr int kX = 0;
   static constexpr int kY = kX + 2 * kXBytes;
   static constexpr int kBias = kY + kYStages * kYStageBytes;
-  // hi * I and lo * I (64 x 64 each), the second operand of the MMAs that add a bias tile to the transposed scores
-  static constexpr int kIdentBytes = 2 * kStep * 128;
+  // hi * I and lo * I, the second operand of the MMAs that add a bias tile to the transposed scores, 16 queries at a time
+  // (16 x 16 each); the other kernels use the space as well
+  static constexpr int kIdentBytes = kMerged ? (kTiles ? 1024 : 0) : 2 * kStep * 128;
   static constexpr int kIdent = kBias + kBiasSlots * kBoxBytes;
   // Key-major: -lse / (scale log2e) and -delta of a step's 64 queries are added to the two products by one more
   // K = 16 MMA step each, products += W * C^T with W (128 x 16) the same row of weights for every key and
@@ -74,28 +87,36 @@ struct BwdSmem {
   static constexpr int kAugTileBytes = (kStep / 8) * 256;
   static constexpr int kAugSlotBytes = 2 * kAugTileBytes;      // lse tile, delta tile
   static constexpr int kWeights = kIdent + kIdentBytes;
-  static constexpr int kAug = kWeights + kWeightBytes;          // two slots
+  static constexpr int kAugSlots = kMerged && !kTiles ? 4 : 2;
+  static constexpr int kAug = kWeights + kWeightBytes;
   // Merged kernel: ds tiles (128 keys x 64 queries, 16-bit, 128-byte-swizzled rows) of the last four steps.  The
   // tensor core reads a tile K-major for dK and a pair of tiles MN-major for dQ.  Must stay 1024-byte aligned.
   static constexpr int kDsSlots = 4;
-  static constexpr int kDs = (kAug + 2 * kAugSlotBytes + 1023) / 1024 * 1024;
+  static constexpr int kDs = (kAug + kAugSlots * kAugSlotBytes + 1023) / 1024 * 1024;
   static constexpr int kBars = kDs + (kMerged ? kDsSlots * kBoxBytes : 0);
   // x_full, y_full[n], y_empty[n], prod_full[2], e_ready[2], acc_done, bias_full[2], bias_empty[2], p_free[2], e_free[2],
-  // aug_full[2], aug_free[2], dq_full, dq_free
-  static constexpr int kNumBars = 1 + 2 * kYStages + 2 + 2 + 1 + 4 + 4 + 4 + 2;
+  // aug_full[n], aug_free[n], dq_full, dq_free
+  static constexpr int kNumBars = 1 + 2 * kYStages + 2 + 2 + 1 + 4 + 4 + 2 * kAugSlots + 2;
   static constexpr int kMisc = kBars + 8 * kNumBars;
   static constexpr int kTotal = kMisc + 16;
 };
 
-template <int D, bool kBf16, bool kKeyMajor, bool kMerged>
-__global__ void __launch_bounds__(kThreads, 1)
+template <int D, bool kBf16, bool kKeyMajor, bool kMerged, bool kTiles>
+__global__ void __launch_bounds__(Split<kKeyMajor, kMerged>::kThreads, 1)
 sdpa_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constant__ CUtensorMap tm_x2,
                    const __grid_constant__ CUtensorMap tm_y1, const __grid_constant__ CUtensorMap tm_y2,
                    const __grid_constant__ CUtensorMap tm_bias, const BwdArgs a) {
   static_assert(!kMerged || (kKeyMajor && D == 64), "the merged kernel is the key-major kernel at head dim 64");
-  using L = BwdSmem<D, kMerged>;
+  using L = BwdSmem<D, kMerged, kTiles>;
+  constexpr int kThreads = Split<kKeyMajor, kMerged>::kThreads, kHalves = Split<kKeyMajor, kMerged>::kHalves;
+  constexpr int kCols = kStep / kHalves;   // columns of a step that one element-wise thread takes
+  constexpr int kAugSlots = L::kAugSlots;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  if (smem + L::kTotal > smem_raw + dynamic_smem_bytes()) {  // never expected; refuse rather than overrun
+    if (threadIdx.x == 0) atomicExch(a.status, 299);
+    return;
+  }
   const uint32_t sbase = smem_u32(smem);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::kBars);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + L::kMisc);
@@ -104,7 +125,7 @@ sdpa_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_const
   constexpr int NY = L::kYStages;
   constexpr int X_FULL = 0, Y_FULL = 1, Y_EMPTY = Y_FULL + NY, PROD_FULL = Y_EMPTY + NY, E_READY = PROD_FULL + 2,
                 ACC_DONE = E_READY + 2, B_FULL = ACC_DONE + 1, B_EMPTY = B_FULL + 2, P_FREE = B_EMPTY + 2,
-                E_FREE = P_FREE + 2, AUG_FULL = E_FREE + 2, AUG_FREE = AUG_FULL + 2, DQ_FULL = AUG_FREE + 2, DQ_FREE = DQ_FULL + 1;
+                E_FREE = P_FREE + 2, AUG_FULL = E_FREE + 2, AUG_FREE = AUG_FULL + kAugSlots, DQ_FULL = AUG_FREE + kAugSlots, DQ_FREE = DQ_FULL + 1;
   // D = 64 has TMEM room for E tiles of their own.  Then a stage's products can be recomputed as soon as the
   // element-wise group has read them out (P_FREE).  At D = 128 the E tiles lie over the products, which can be
   // recomputed only once the accumulating MMAs of two steps earlier have read them (E_FREE).
@@ -139,10 +160,10 @@ sdpa_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_const
   if (threadIdx.x < L::kNumBars) {
     const int i = threadIdx.x;
     uint32_t count = 1;
-    if (i >= E_READY && i < E_READY + 2) count = 4;   // one lane per warp of the group
-    if (i >= P_FREE && i < P_FREE + 2) count = 4;
-    if (i >= B_EMPTY && i < B_EMPTY + 2) count = a.bias_mma ? 1 : 4;   // released by the MMA issuer or by the group's warps
-    if (i == DQ_FREE) count = 8;                       // every element-wise warp has read its part of the dq tile
+    if (i >= E_READY && i < E_READY + 2) count = 4 * kHalves;   // one lane per warp of the group
+    if (i >= P_FREE && i < P_FREE + 2) count = 4 * kHalves;
+    if (i >= B_EMPTY && i < B_EMPTY + 2) count = a.bias_mma ? 1 : 4 * kHalves;   // released by the MMA issuer or by the group's warps
+    if (i == DQ_FREE) count = 8 * kHalves;                       // every element-wise warp has read its part of the dq tile
     mbar_init(bar(i), count);
     if (i == 0) *abort_flag = 0;
     mbar_init_fence();
@@ -174,7 +195,7 @@ sdpa_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_const
         bulk_load(ybase + 2 * L::kYBytes, a.lse + ro, row_bytes, bar(Y_FULL + n));
         bulk_load(ybase + 2 * L::kYBytes + 256, a.delta + ro, row_bytes, bar(Y_FULL + n));
       }
-      if (a.bias_mode == kBiasTile && n < 2) {
+      if (kTiles && a.bias_mode == kBiasTile && n < 2) {
         mbar_expect_tx(bar(B_FULL + n), kBoxBytes);
         const uint32_t dst = sbase + L::kBias + n * kBoxBytes;
         if (kKeyMajor) {
@@ -196,22 +217,20 @@ sdpa_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_const
       for (int idx = threadIdx.x; idx < L::kWeightBytes / 16; idx += kThreads)
         wt[idx] = (idx & 8) ? make_uint4(0, 0, 0, 0) : make_uint4(w01, w2, 0, 0);
       uint4* aug = reinterpret_cast<uint4*>(smem + L::kAug);
-      for (int idx = threadIdx.x; idx < 2 * L::kAugSlotBytes / 16; idx += kThreads) aug[idx] = make_uint4(0, 0, 0, 0);
+      for (int idx = threadIdx.x; idx < kAugSlots * L::kAugSlotBytes / 16; idx += kThreads) aug[idx] = make_uint4(0, 0, 0, 0);
       fence_proxy_async_smem();
     }
-    if (kKeyMajor && a.bias_mma) {
-      // Two 64 x 64 tiles, hi * I and lo * I with hi + lo = 1 / scale to 16 + 16 bits, as K-major 128-byte-swizzled
-      // operands (rows of 64 elements = 128 bytes).  Tile 0 at kIdent, tile 1 at kIdent + 8 KB.
-      uint4* ident = reinterpret_cast<uint4*>(smem + L::kIdent);
-      for (int idx = threadIdx.x; idx < 2 * kStep * 8; idx += kThreads) {   // one 16-byte chunk each
-        const int tile = idx / (kStep * 8), rem = idx - tile * kStep * 8;
-        const int row = rem >> 3, chunk = (rem & 7) ^ (row & 7);             // logical chunk stored at this slot
-        const int col0 = chunk * 8;                                          // first logical column of the chunk
+    if (kKeyMajor && kTiles && a.bias_mma) {
+      // two 16 x 16 tiles, hi * I and lo * I with hi + lo = 1 / scale to 16 + 16 bits: K-major without swizzle, 8-row groups
+      // of 256 bytes = [8 rows x 16 bytes (K 0-7)][8 rows x 16 bytes (K 8-15)]; one 16-byte chunk per thread
+      if (threadIdx.x < 64) {
+        const int tile = threadIdx.x >> 5, c = threadIdx.x & 31;       // chunk c: 8-row group, K half, row
+        const int row = (c >> 4) * 8 + (c & 7), k = row - ((c >> 3) & 1) * 8;
         const float val = tile == 0 ? a.inv_scale_hi : a.inv_scale_lo;
         const uint16_t one = kBf16 ? __bfloat16_as_ushort(__float2bfloat16_rn(val)) : __half_as_ushort(__float2half_rn(val));
         uint32_t w[4] = {0u, 0u, 0u, 0u};
-        if (row >= col0 && row < col0 + 8) w[(row - col0) >> 1] = uint32_t(one) << (((row - col0) & 1) * 16);
-        ident[idx] = make_uint4(w[0], w[1], w[2], w[3]);
+        if (k >= 0 && k < 8) w[k >> 1] = uint32_t(one) << ((k & 1) * 16);
+        reinterpret_cast<uint4*>(smem + L::kIdent + tile * 512)[c] = make_uint4(w[0], w[1], w[2], w[3]);
       }
       fence_proxy_async_smem();   // written by threads, read by the tensor core
     }
@@ -234,7 +253,7 @@ sdpa_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_const
   const uint32_t tm_acc1 = tmem + (kDeep ? 384 : 256), tm_acc2 = tm_acc1 + D;
 
   if (warp < 4) {
-  reg_dealloc<kProducerRegs>();
+  reg_dealloc<Split<kKeyMajor, kMerged>::kProducerRegs>();
   if (warp == 1) {
     // ---------------- TMA duties of the step loop: ring refills and bias tiles, ONE thread ----------------
     // (the owner tiles, the first NY stages and the first two bias slots were issued during start-up).  The thread
@@ -242,7 +261,7 @@ sdpa_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_const
     // pending, so whichever completes first is served at once.
     if (lane == 0 && n_steps > 0) {
       int yn = min(n_steps, NY);
-      int bn = a.bias_mode == kBiasTile ? min(n_steps, 2) : n_steps;
+      int bn = kTiles && a.bias_mode == kBiasTile ? min(n_steps, 2) : n_steps;
       const long long t0 = clock64();
       uint32_t idle = 0;
       while (yn < n_steps || bn < n_steps) {
@@ -330,32 +349,33 @@ sdpa_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_const
           const uint64_t yo = uint64_t(((kk / 4) * kYBoxBytes + (kk % 4) * 32) >> 4);
           mma_ss(p2, x2desc + xo, y2desc + yo, idesc_prod, kk > 0 ? 1u : 0u);
         }
-        if (a.bias_mma) {
+        if (kTiles && a.bias_mma) {
           // scores += bias * (I / scale): the bias slot is consumed straight from shared memory by the tensor core
           const int slot = n & 1;
           ok = wait_or_abort(bar(B_FULL + slot), (n >> 1) & 1, abort_flag, a.status, 211);
           if (!ok) break;
           tc_fence_after_sync();
           const uint32_t bslot = sbase + L::kBias + slot * kBoxBytes;
-          // P1[key, q] += bias^T[key, q'] (hi I + lo I)[q', q]: A = the slot (64 q' rows, two 64-key boxes) read
-          // MN-major, B = the identity tiles, K-major
-          constexpr uint32_t idesc_bias = make_idesc(kBf16, kTile, kStep, true, false);
+          // P1[key, q] += bias^T[key, q'] (hi I + lo I)[q', q], 16 queries at a time: A = 16 rows of the slot (two 64-key
+          // boxes) read MN-major, B = the identity tiles, D = 16 columns of P1
+          constexpr uint32_t idesc_bias = make_idesc(kBf16, kTile, 16, true, false);
           const uint64_t adesc = make_smem_desc(bslot, kYBoxBytes, 1024);
           const int n_tiles = a.inv_scale_lo != 0.f ? 2 : 1;
           for (int tile = 0; tile < n_tiles; ++tile) {
-            const uint64_t bdesc = make_smem_desc(sbase + L::kIdent + tile * kYBoxBytes, 16, 1024);
+            const uint64_t bdesc = make_smem_desc_noswizzle(sbase + L::kIdent + tile * 512, 128, 256);
 #pragma unroll
             for (int kk = 0; kk < kStep / 16; ++kk)
-              mma_ss(p1, adesc + uint64_t((kk * 2048) >> 4), bdesc + uint64_t((kk * 32) >> 4), idesc_bias, 1u);
+              mma_ss(p1 + kk * 16, adesc + uint64_t((kk * 2048) >> 4), bdesc, idesc_bias, 1u);
           }
         }
         if constexpr (kKeyMajor) {
           // P1 += W C1^T (C1: -lse / (scale log2e)), P2 += W C2^T (C2: -delta)
-          ok = wait_or_abort(bar(AUG_FULL + s), (n >> 1) & 1, abort_flag, a.status, 212);
+          const int as = n % kAugSlots;
+          ok = wait_or_abort(bar(AUG_FULL + as), (n / kAugSlots) & 1, abort_flag, a.status, 212);
           if (!ok) break;
           tc_fence_after_sync();
           const uint64_t wdesc = make_smem_desc_noswizzle(sbase + L::kWeights, 128, 256);
-          const uint32_t aslot = sbase + L::kAug + s * L::kAugSlotBytes;
+          const uint32_t aslot = sbase + L::kAug + as * L::kAugSlotBytes;
           mma_ss(p1, wdesc, make_smem_desc_noswizzle(aslot, 128, 256), idesc_prod, 1u);
           mma_ss(p2, wdesc, make_smem_desc_noswizzle(aslot + L::kAugTileBytes, 128, 256), idesc_prod, 1u);
         }
@@ -370,8 +390,8 @@ sdpa_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_const
           }
         }
         mma_commit(bar(PROD_FULL + s));
-        if (kKeyMajor || a.key_aug) mma_commit(bar(AUG_FREE + s));
-        if (a.bias_mma) mma_commit(bar(B_EMPTY + (n & 1)));   // the slot may be refilled once these MMAs are done
+        if (kKeyMajor || a.key_aug) mma_commit(bar(AUG_FREE + n % kAugSlots));
+        if (kTiles && a.bias_mma) mma_commit(bar(B_EMPTY + (n & 1)));   // the slot may be refilled once these MMAs are done
       }
     }
   } else if (warp == 0) {
@@ -421,8 +441,10 @@ sdpa_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_const
 #pragma unroll
           for (int kk = 0; kk < kStep / 16; ++kk) {
             const uint32_t acc = (m > 0 || kk > 0) ? 1u : 0u;
-            if (kKeyMajor) mma_ts(tm_acc1, e1 + kk * 8, y2mn + uint64_t((kk * 2048) >> 4), idesc_acc, acc);
-            mma_ts(tm_acc2, e2 + kk * 8, y1mn + uint64_t((kk * 2048) >> 4), idesc_acc, acc);
+            // (D = 128 with two threads per row: each half's E tile lies over its own half of the products)
+            const uint32_t ek = kDeep || kHalves == 1 ? kk * 8 : (kk >> 1) * kCols + (kk & 1) * 8;
+            if (kKeyMajor) mma_ts(tm_acc1, e1 + ek, y2mn + uint64_t((kk * 2048) >> 4), idesc_acc, acc);
+            mma_ts(tm_acc2, e2 + ek, y1mn + uint64_t((kk * 2048) >> 4), idesc_acc, acc);
           }
           mma_commit(bar(Y_EMPTY + st));
         }
@@ -490,9 +512,9 @@ sdpa_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_const
     const float inv_mul = 1.f / (a.scale * kLog2e);
     bool ok = true;
     for (int n = 0; n < n_steps && ok; ++n) {
-      const int st = n % NY, s = n & 1;
+      const int st = n % NY, s = n % kAugSlots;
       ok = wait_or_abort(bar(Y_FULL + st), (n / NY) & 1, abort_flag, a.status, 213);
-      if (ok && n >= 2) ok = wait_or_abort(bar(AUG_FREE + s), ((n - 2) >> 1) & 1, abort_flag, a.status, 214);
+      if (ok && n >= kAugSlots) ok = wait_or_abort(bar(AUG_FREE + s), (n / kAugSlots - 1) & 1, abort_flag, a.status, 214);
       if (!ok) break;
       const float* ld = reinterpret_cast<const float*>(smem + L::kY + st * L::kYStageBytes + 2 * L::kYBytes);
       uint8_t* slot = smem + L::kAug + s * L::kAugSlotBytes;
@@ -533,9 +555,9 @@ sdpa_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_const
     }
   }
   } else {
-    reg_alloc<kWorkerRegs>();
-    // ---------------- element-wise groups (one owner row per thread) ----------------
-    const int grp = (warp - 4) >> 2;
+    reg_alloc<Split<kKeyMajor, kMerged>::kWorkerRegs>();
+    // ---------------- element-wise groups (an owner row, or 32 columns of one, per thread) ----------------
+    const int grp = ((warp - 4) >> 2) & 1, half = kHalves == 1 ? 0 : (warp - 4) >> 3;
     const int wq = warp & 3;
     const int r = wq * 32 + lane;
     const int orow = o0 + r;                       // query row (query-major) or key (key-major)
@@ -591,8 +613,10 @@ sdpa_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_const
     auto drain_pair = [&](int j) -> bool {
       if (!wait_or_abort(bar(DQ_FULL), j & 1, abort_flag, a.status, 216)) return false;
       tc_fence_after_sync();
-      uint32_t v[32];
-      tmem_ld32(tm_dq + lane_addr + grp * 32, v);
+      constexpr int kDq = 32 / kHalves;   // columns of it per thread
+      uint32_t v[kDq];
+      if constexpr (kHalves == 1) tmem_ld32(tm_dq + lane_addr + grp * 32, v);
+      else tmem_ld16(tm_dq + lane_addr + grp * 32 + half * kDq, v);
       tmem_wait_ld();
       tc_fence_before_sync();
       __syncwarp();
@@ -600,16 +624,16 @@ sdpa_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_const
       // The accumulator is laid out so that one warp-wide reduction covers 512 contiguous bytes: per 128-query tile
       // [column half g][warp w][4-column chunk c][lane][4] holds dq[128 tile + 32 w + lane][32 g + 4 c + 0..3].
       const int64_t tile = int64_t(blockIdx.y) * (a.S / kTile) + ((s_begin + 2 * j) >> 1);
-      float* dst = a.dq_acc + tile * (kTile * D) + ((grp * 4 + wq) * 8) * 128 + lane * 4;
+      float* dst = a.dq_acc + tile * (kTile * D) + ((grp * 4 + wq) * 8 + half * (kDq / 4)) * 128 + lane * 4;
 #pragma unroll
-      for (int c = 0; c < 8; ++c) red_add_v4(dst + c * 128, v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
+      for (int c = 0; c < kDq / 4; ++c) red_add_v4(dst + c * 128, v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
       return true;
     };
 
     for (int n = grp; n < n_steps && ok; n += 2) {
       const int s = n & 1;
       const int st = n % NY;
-      const int r0 = (s_begin + n) * kStep;          // first streamed row of the step
+      const int r0 = (s_begin + n) * kStep + half * kCols;   // first streamed row of this thread's columns
       if constexpr (kMerged) {
         // group 0 takes pair j before step 2j + 4, group 1 after step 2j + 3: both between the pair's MMAs
         // (issued after the products of step 2j + 3) and the next pair's (after the products of step 2j + 5)
@@ -618,29 +642,34 @@ sdpa_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_const
           if (!ok) break;
         }
       }
-      // keep bits over the step's 64 streamed rows
-      uint32_t keep[2] = {0xffffffffu, 0xffffffffu};
+      // keep bits over these streamed rows
+      uint32_t keep[kCols / 32];
+#pragma unroll
+      for (int i = 0; i < kCols / 32; ++i) keep[i] = 0xffffffffu;
       if (mbits) {
-        const uint2 w = __ldg(reinterpret_cast<const uint2*>(mbits + (r0 >> 5)));
-        keep[0] = w.x; keep[1] = w.y;
+        if constexpr (kCols == 32) {
+          keep[0] = __ldg(mbits + (r0 >> 5));
+        } else {
+          const uint2 w = __ldg(reinterpret_cast<const uint2*>(mbits + (r0 >> 5)));
+          keep[0] = w.x; keep[kCols / 32 - 1] = w.y;
+        }
       }
       if (kKeyMajor) {
         // queries r0 + c: need c < S - r0, and (causal) r0 + c >= key
         const int hi = a.S - r0;
         const int lo = a.causal ? orow - r0 : 0;
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {
+        for (int i = 0; i < kCols / 32; ++i) {
           const int nh = hi - 32 * i, nl = lo - 32 * i;
           const uint32_t mh = nh >= 32 ? 0xffffffffu : (nh <= 0 ? 0u : ((1u << nh) - 1u));
           const uint32_t ml = nl <= 0 ? 0xffffffffu : (nl >= 32 ? 0u : ~((1u << nl) - 1u));
-          keep[i] &= mh & ml;
+          keep[i] &= key_dropped ? 0u : mh & ml;
         }
-        if (key_dropped) keep[0] = keep[1] = 0u;
       } else {
         int n_keep = a.T - r0;
         if (a.causal) n_keep = min(n_keep, orow - r0 + 1);
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {
+        for (int i = 0; i < kCols / 32; ++i) {
           const int nk = n_keep - 32 * i;
           keep[i] &= nk >= 32 ? 0xffffffffu : (nk <= 0 ? 0u : ((1u << nk) - 1u));
         }
@@ -649,15 +678,15 @@ sdpa_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_const
       ok = wait_or_abort(bar(PROD_FULL + s), (n >> 1) & 1, abort_flag, a.status, 206);
       if (!ok) break;
       tc_fence_after_sync();
-      const uint32_t tP1 = tmem + s * 128 + lane_addr, tP2 = tP1 + 64;
-      // both products of the step: four TMEM loads in flight, one wait; handled as fp32 pairs
-      float2 t[kStep / 2], dp[kStep / 2];
+      const uint32_t tP1 = tmem + s * 128 + half * kCols + lane_addr, tP2 = tP1 + 64;
+      // this thread's part of both products: all TMEM loads in flight, one wait; handled as fp32 pairs
+      float2 t[kCols / 2], dp[kCols / 2];
       {
-        uint32_t raw[2 * kStep];
+        uint32_t raw[2 * kCols];
 #pragma unroll
-        for (int c = 0; c < 2; ++c) {
+        for (int c = 0; c < kCols / 32; ++c) {
           tmem_ld32(tP1 + c * 32, *reinterpret_cast<uint32_t(*)[32]>(&raw[c * 32]));
-          tmem_ld32(tP2 + c * 32, *reinterpret_cast<uint32_t(*)[32]>(&raw[kStep + c * 32]));
+          tmem_ld32(tP2 + c * 32, *reinterpret_cast<uint32_t(*)[32]>(&raw[kCols + c * 32]));
         }
         tmem_wait_ld();
         if constexpr (kDeep) {
@@ -667,23 +696,23 @@ sdpa_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_const
           if (lane == 0) mbar_arrive(bar(P_FREE + s));
         }
 #pragma unroll
-        for (int i = 0; i < kStep / 2; ++i) {
+        for (int i = 0; i < kCols / 2; ++i) {
           t[i] = make_float2(__uint_as_float(raw[2 * i]), __uint_as_float(raw[2 * i + 1]));
-          dp[i] = make_float2(__uint_as_float(raw[kStep + 2 * i]), __uint_as_float(raw[kStep + 2 * i + 1]));
+          dp[i] = make_float2(__uint_as_float(raw[kCols + 2 * i]), __uint_as_float(raw[kCols + 2 * i + 1]));
         }
       }
       // logits t = s * scale + bias
-      if (a.bias_mode == kBiasTile && !a.bias_mma) {
+      if (kTiles && a.bias_mode == kBiasTile && !a.bias_mma) {
         const int slot = n & 1;
         ok = wait_or_abort(bar(B_FULL + slot), (n >> 1) & 1, abort_flag, a.status, 207);
         if (!ok) break;
         const uint8_t* sl = smem + L::kBias + slot * kBoxBytes;
         if (kKeyMajor) {
           // element (query c, key r): box r / 64, row c, 16-byte chunk ((r % 64) / 8) ^ (c % 8)
-          const uint8_t* colbase = sl + (r >> 6) * kYBoxBytes + (r & 7) * 2;
+          const uint8_t* colbase = sl + (r >> 6) * kYBoxBytes + half * (kCols * 128) + (r & 7) * 2;
           const int chunk = (r & 63) >> 3;
 #pragma unroll
-          for (int c = 0; c < kStep / 2; ++c) {
+          for (int c = 0; c < kCols / 2; ++c) {
             const uint16_t r0w = *reinterpret_cast<const uint16_t*>(colbase + (2 * c) * 128 + ((chunk ^ ((2 * c) & 7)) << 4));
             const uint16_t r1w =
                 *reinterpret_cast<const uint16_t*>(colbase + (2 * c + 1) * 128 + ((chunk ^ ((2 * c + 1) & 7)) << 4));
@@ -693,8 +722,8 @@ sdpa_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_const
         } else {
           const uint8_t* srow = sl + r * 128;
 #pragma unroll
-          for (int c = 0; c < 8; ++c) {
-            const uint4 w = *reinterpret_cast<const uint4*>(srow + ((c ^ (r & 7)) << 4));
+          for (int c = 0; c < kCols / 8; ++c) {
+            const uint4 w = *reinterpret_cast<const uint4*>(srow + (((half * (kCols / 8) + c) ^ (r & 7)) << 4));
             const uint32_t ww[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
             for (int e = 0; e < 4; ++e) t[c * 4 + e] = __ffma2_rn(t[c * 4 + e], scale2, unpack2<kBf16>(ww[e]));
@@ -705,7 +734,7 @@ sdpa_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_const
       } else if (a.bias_mode == kBiasKey && !kKeyMajor && !key_aug) {
         const uint4* bk = reinterpret_cast<const uint4*>(bias_key + 2 * r0);
 #pragma unroll
-        for (int c = 0; c < 8; ++c) {
+        for (int c = 0; c < kCols / 8; ++c) {
           const uint4 w = r0 + 8 * c < a.T ? __ldg(bk + c) : make_uint4(0, 0, 0, 0);   // T is a multiple of 8
           const uint32_t ww[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
@@ -714,13 +743,13 @@ sdpa_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_const
       } else if (!fold_scale) {
         const float2 own2 = make_float2(bias_own, bias_own);
 #pragma unroll
-        for (int c = 0; c < kStep / 2; ++c) t[c] = __ffma2_rn(t[c], scale2, own2);
+        for (int c = 0; c < kCols / 2; ++c) t[c] = __ffma2_rn(t[c], scale2, own2);
       }
       // p = exp2(t log2e - lse), ds = p (dp - delta); key-major products arrive with -lse and -delta already added
-      uint32_t e1[kStep / 2], e2[kStep / 2];
-      const bool need_mask = __any_sync(0xffffffffu, (keep[0] & keep[1]) != 0xffffffffu);
+      uint32_t e1[kCols / 2], e2[kCols / 2];
+      const bool need_mask = __any_sync(0xffffffffu, (keep[0] & keep[kCols / 32 - 1]) != 0xffffffffu);
 #pragma unroll
-      for (int c4 = 0; c4 < kStep / 4; ++c4) {
+      for (int c4 = 0; c4 < kCols / 4; ++c4) {
         const float2 nls = make_float2(-lse_row, -lse_row), ndl = make_float2(-delta_row, -delta_row);  // query-major
         float2 ds4[2];
 #pragma unroll
@@ -761,7 +790,7 @@ sdpa_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_const
         if (a.dbias_acc) {
           float2 sum2 = make_float2(0.f, 0.f);
 #pragma unroll
-          for (int c = 0; c < kStep / 2; ++c) sum2 = __fadd2_rn(sum2, unpack2<kBf16>(e2[c]));
+          for (int c = 0; c < kCols / 2; ++c) sum2 = __fadd2_rn(sum2, unpack2<kBf16>(e2[c]));
           *key_ds_sum += sum2.x + sum2.y;
         }
       }
@@ -773,18 +802,23 @@ sdpa_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_const
           tc_fence_after_sync();
         }
       }
-      const uint32_t tE1 = tm_e + s * kEStage + lane_addr, tE2 = tE1 + kE2Off;
-      if (kKeyMajor) tmem_st32(tE1, e1);
+      const uint32_t tE1 = tm_e + s * kEStage + half * (kDeep ? kCols / 2 : kCols) + lane_addr, tE2 = tE1 + kE2Off;
+      if constexpr (kKeyMajor) {
+        if constexpr (kHalves == 1) tmem_st32(tE1, e1);
+        else tmem_st16(tE1, e1);
+      }
       if constexpr (kMerged) {
         // ds row of this key: 64 queries = 128 bytes, chunks swizzled as TMA would have written them.  The slot was
         // last read by MMAs issued before this step's products, and those have completed (PROD_FULL came after).
         uint8_t* dsrow = smem + L::kDs + (n % L::kDsSlots) * kBoxBytes + r * 128;
 #pragma unroll
-        for (int c = 0; c < 8; ++c)
-          *reinterpret_cast<uint4*>(dsrow + ((c ^ (r & 7)) << 4)) = make_uint4(e2[c * 4], e2[c * 4 + 1], e2[c * 4 + 2], e2[c * 4 + 3]);
+        for (int c = 0; c < kCols / 8; ++c)
+          *reinterpret_cast<uint4*>(dsrow + (((half * (kCols / 8) + c) ^ (r & 7)) << 4)) = make_uint4(e2[c * 4], e2[c * 4 + 1], e2[c * 4 + 2], e2[c * 4 + 3]);
         fence_proxy_async_smem();
-      } else {
+      } else if constexpr (kHalves == 1) {
         tmem_st32(tE2, e2);
+      } else {
+        tmem_st16(tE2, e2);
       }
       tmem_wait_st();
       tc_fence_before_sync();
@@ -795,27 +829,29 @@ sdpa_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_const
       }
       if constexpr (!kKeyMajor) {
         if (a.dbias) {
-          // dbias[row, r0 .. r0+63] = ds in bias dtype (the 16-bit pairs already packed in e2).  A thread holds one
-          // row, so direct stores would touch 32 lines per instruction; the warp turns its 32 x 64 tile over in
-          // shared memory (two halves of 32 keys; the space of the identity tiles is free in this kernel) and
+          // dbias[row, r0 .. r0+31] = ds in bias dtype (the 16-bit pairs already packed in e2).  A thread holds one
+          // row, so direct stores would touch 32 lines per instruction; the warp turns its 32 x 32 tile over in
+          // shared memory (16 rows x 32 keys at a time; the space of the identity tiles is free in this kernel) and
           // stores 8 rows x 64 contiguous bytes per instruction.
-          uint8_t* stage = smem + L::kIdent + (warp - 4) * 2048;
+          static_assert(kHalves == 2, "32 keys per thread");
+          uint8_t* stage = smem + L::kIdent + (warp - 4) * 1024;
           uint8_t* dbase = reinterpret_cast<uint8_t*>(a.dbias) + 2 * (b * a.dbs[0] + h * a.dbs[1] + r0);
 #pragma unroll
-          for (int half = 0; half < 2; ++half) {
+          for (int part = 0; part < 2; ++part) {
+            if ((lane >> 4) == part) {
 #pragma unroll
-            for (int c = 0; c < 4; ++c)
-              *reinterpret_cast<uint4*>(stage + lane * 64 + ((c ^ ((lane >> 1) & 3)) << 4)) =
-                  make_uint4(e2[half * 16 + c * 4], e2[half * 16 + c * 4 + 1], e2[half * 16 + c * 4 + 2],
-                             e2[half * 16 + c * 4 + 3]);
+              for (int c = 0; c < 4; ++c)
+                *reinterpret_cast<uint4*>(stage + (lane & 15) * 64 + ((c ^ ((lane >> 1) & 3)) << 4)) =
+                    make_uint4(e2[c * 4], e2[c * 4 + 1], e2[c * 4 + 2], e2[c * 4 + 3]);
+            }
             __syncwarp();
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
+            for (int i = 0; i < 2; ++i) {
               const int rl = 8 * i + (lane >> 2), ch = lane & 3;
               const uint4 v = *reinterpret_cast<const uint4*>(stage + rl * 64 + ((ch ^ ((rl >> 1) & 3)) << 4));
-              const int row = o0 + wq * 32 + rl;
-              if (row < a.S && r0 + half * 32 + ch * 8 < a.T)
-                *reinterpret_cast<uint4*>(dbase + 2 * (int64_t(row) * a.dbs[2] + half * 32 + ch * 8)) = v;
+              const int row = o0 + wq * 32 + part * 16 + rl;
+              if (row < a.S && r0 + ch * 8 < a.T)
+                *reinterpret_cast<uint4*>(dbase + 2 * (int64_t(row) * a.dbs[2] + ch * 8)) = v;
             }
             __syncwarp();
           }
@@ -826,7 +862,7 @@ sdpa_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_const
     // ---------------- epilogue ----------------
     if (!kKeyMajor && a.dbias && orow < a.S) {
       // key steps past the diagonal (causal) or past the last kept key are never visited: their dbias is exactly zero
-      if (grp == 0) {
+      if (grp == 0 && half == 0) {
         uint8_t* dst = reinterpret_cast<uint8_t*>(a.dbias) + 2 * (b * a.dbs[0] + h * a.dbs[1] + int64_t(orow) * a.dbs[2]);
         for (int k0 = s_end * kStep; k0 < a.T; k0 += 8)
           *reinterpret_cast<uint4*>(dst + 2 * k0) = make_uint4(0, 0, 0, 0);
@@ -844,32 +880,32 @@ sdpa_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_const
     if (ok) {
       tc_fence_after_sync();
       // key-major: group 0 writes dv (ACC1), group 1 writes dk (ACC2 * scale).
-      // query-major: both groups write dq (ACC2 * scale), half of the columns each.
+      // query-major: all four quarters of the warps write dq (ACC2 * scale), a part of the columns each.
       const uint32_t tacc = ((kKeyMajor && grp == 0) ? tm_acc1 : tm_acc2) + lane_addr;
       const float mul = (kKeyMajor && grp == 0) ? 1.f : a.scale;
       void* outp = (kKeyMajor && grp == 0) ? a.out1 : a.out2;
       const int64_t* os = (kKeyMajor && grp == 0) ? a.o1s : a.o2s;
       uint8_t* orow_ptr = reinterpret_cast<uint8_t*>(outp) + 2 * (b * os[0] + h * os[1] + int64_t(orow) * os[2]);
-      const int c_begin = kKeyMajor ? 0 : grp * (D / 64);
-      const int c_end = kKeyMajor ? D / 32 : (grp + 1) * (D / 64);
-      for (int c = c_begin; c < c_end; ++c) {
-        uint32_t o[32];
+      constexpr int kOut = (kKeyMajor ? D : D / 2) / kHalves;   // columns per thread
+      const int col0 = kKeyMajor ? half * kOut : (grp * kHalves + half) * kOut;
+      for (int c = col0; c < col0 + kOut; c += 16) {
+        uint32_t o[16];
         if (n_steps > 0) {
-          tmem_ld32(tacc + c * 32, o);
+          tmem_ld16(tacc + c, o);
           tmem_wait_ld();
         } else {
 #pragma unroll
-          for (int i = 0; i < 32; ++i) o[i] = 0u;
+          for (int i = 0; i < 16; ++i) o[i] = 0u;
         }
         if (orow < n_owner) {
 #pragma unroll
-          for (int i = 0; i < 32; i += 8) {
+          for (int i = 0; i < 16; i += 8) {
             uint4 w;
             w.x = pack2<kBf16>(__uint_as_float(o[i]) * mul, __uint_as_float(o[i + 1]) * mul);
             w.y = pack2<kBf16>(__uint_as_float(o[i + 2]) * mul, __uint_as_float(o[i + 3]) * mul);
             w.z = pack2<kBf16>(__uint_as_float(o[i + 4]) * mul, __uint_as_float(o[i + 5]) * mul);
             w.w = pack2<kBf16>(__uint_as_float(o[i + 6]) * mul, __uint_as_float(o[i + 7]) * mul);
-            *reinterpret_cast<uint4*>(orow_ptr + (c * 32 + i) * 2) = w;
+            *reinterpret_cast<uint4*>(orow_ptr + (c + i) * 2) = w;
           }
         }
       }
@@ -885,10 +921,13 @@ sdpa_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_const
   }
 }
 
-template <int D, bool kBf16, bool kKeyMajor, bool kMerged = false>
+template <int D, bool kBf16, bool kKeyMajor, bool kMerged = false, bool kTiles = true>
 int launch_one(const CUtensorMap* maps, const BwdArgs& a, int n_tiles, int bh_count, cudaStream_t st) {
-  auto kernel = sdpa_bwd_tc_kernel<D, kBf16, kKeyMajor, kMerged>;
-  const int smem = BwdSmem<D, kMerged>::kTotal + 1024;
+  using S = Split<kKeyMajor, kMerged>;
+  auto kernel = sdpa_bwd_tc_kernel<D, kBf16, kKeyMajor, kMerged, kTiles>;
+  constexpr int kLimit = 232448;  // 227 KB per CTA
+  constexpr int kTotal = BwdSmem<D, kMerged, kTiles>::kTotal, smem = kTotal + 1024 <= kLimit ? kTotal + 1024 : kLimit;
+  static_assert(kTotal <= kLimit, "backward shared memory exceeds the per-CTA limit");
   // checked and configured once per device and kernel instance (setting it again would be harmless)
   static bool ready[64] = {};
   int dev = 0;
@@ -896,9 +935,9 @@ int launch_one(const CUtensorMap* maps, const BwdArgs& a, int n_tiles, int bh_co
   if (dev < 0 || !ready[dev]) {
     cudaFuncAttributes attr;
     cudaError_t e = cudaFuncGetAttributes(&attr, kernel);
-    if (e != cudaSuccess || attr.numRegs != kLaunchRegs) {
-      // the register hand-over inside the kernel is balanced for exactly kLaunchRegs per thread at launch
-      set_error("sdpa_bwd_tc_kernel was built with %d registers per thread, expected %d", attr.numRegs, kLaunchRegs);
+    if (e != cudaSuccess || attr.numRegs != S::kLaunchRegs) {
+      // the register hand-over inside the kernel is balanced for exactly that many per thread at launch
+      set_error("sdpa_bwd_tc_kernel was built with %d registers per thread, expected %d", attr.numRegs, S::kLaunchRegs);
       return NB200_ERR_LAUNCH;
     }
     e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
@@ -909,7 +948,7 @@ int launch_one(const CUtensorMap* maps, const BwdArgs& a, int n_tiles, int bh_co
     if (dev >= 0) ready[dev] = true;
   }
   dim3 grid(n_tiles, bh_count);
-  kernel<<<grid, kThreads, smem, st>>>(maps[0], maps[1], maps[2], maps[3], maps[4], a);
+  kernel<<<grid, S::kThreads, smem, st>>>(maps[0], maps[1], maps[2], maps[3], maps[4], a);
   count_launch();
   return check_launch(kMerged ? "sdpa_bwd_tc_kernel<merged>"
                               : (kKeyMajor ? "sdpa_bwd_tc_kernel<key-major>" : "sdpa_bwd_tc_kernel<query-major>"));
@@ -1092,8 +1131,11 @@ int launch_bwd(const Problem& pr, const TcBwdPrepared& prep, int dtype, int bias
     ak.out2 = pr.dk;
     for (int i = 0; i < 3; ++i) { ak.o1s[i] = pr.dvs[i]; ak.o2s[i] = pr.dks[i]; }
     const CUtensorMap maps[5] = {k128, v128, q64, g64, bias_k};
-    const int rc = bf16 ? launch_one<64, true, true, true>(maps, ak, (pr.T + kTile - 1) / kTile, pr.bh_count, stream)
-                        : launch_one<64, false, true, true>(maps, ak, (pr.T + kTile - 1) / kTile, pr.bh_count, stream);
+    const int n_tiles = (pr.T + kTile - 1) / kTile;
+    const int rc = a.bias_mode == kBiasTile ? (bf16 ? launch_one<64, true, true, true, true>(maps, ak, n_tiles, pr.bh_count, stream)
+                                                    : launch_one<64, false, true, true, true>(maps, ak, n_tiles, pr.bh_count, stream))
+                                            : (bf16 ? launch_one<64, true, true, true, false>(maps, ak, n_tiles, pr.bh_count, stream)
+                                                    : launch_one<64, false, true, true, false>(maps, ak, n_tiles, pr.bh_count, stream));
     if (rc) return rc;
     const int64_t n_chunks = int64_t(pr.bh_count) * pr.S * 8;
     const int blocks = int((n_chunks + 255) / 256);
