@@ -22,7 +22,7 @@
 // Two warps per scheduler cannot keep the special-function unit busy (a pair of exponentials with its arithmetic takes 17.8
 // cycles of it with two warps, 16.7 with four, 16 being its rate, and nothing covers the rest of a pass); four do, where
 // their registers suffice: D = 64 forward, fp16 B1 H16 L8192 512 -> 427 us, causal with a shared bias B8 H16 L2048 192 ->
-// 157, key padding B32 H8 L1024 114 -> 104.  At D = 128 the same split spills (1559 -> 2149 us on B4 H32 L4096 with bias and
+// 162, key padding B32 H8 L1024 114 -> 104.  At D = 128 the same split spills (1559 -> 2149 us on B4 H32 L4096 with bias and
 // mask); there the passes without tests for what a problem does not have took 1068 -> 951 (B1 H16 L16384 causal, per-key
 // bias) and 1617 -> 1551.
 // TMEM (512 columns).  D = 128: [0,128) S0, [128,256) S1, then O0, O1.  There is no
@@ -65,16 +65,13 @@ struct Split {
   static_assert((kLaunchRegs - kProducerRegs) * 128 >= (kSoftmaxRegs - kLaunchRegs) * 256 * kHalves,
                 "softmax warps would wait forever for registers the producer warps never release");
 };
-#ifndef NB200_POLY64
-#define NB200_POLY64 0
-#endif
 #ifndef NB200_POLY_PERIOD
 #define NB200_POLY_PERIOD 4
 #endif
-// One pair in this many computes 2^x without the special-function unit, which all softmax warps share; at D = 64 only bf16
-// with bias tiles, where the tensor core's bias add leaves issue slots (163 -> 156 us causal, 1227 -> 1151 B4 H32 L4096 with
-// bias and mask; without tiles 427 -> 447).
-constexpr int kPolyPeriod = NB200_POLY_PERIOD, kPolyPeriod64 = 16;
+// D = 128: one pair in this many computes 2^x without the special-function unit, which both query tiles' warps share (every
+// third or second: 994 and 1005 us for 984, B1 H16 L16384 causal with a per-key bias).  None at D = 64 (every 8th or 16th pair
+// 474 and 448 us for 427, B1 H16 L8192).
+constexpr int kPolyPeriod = NB200_POLY_PERIOD;
 #ifdef NB200_PROBE
 // Development aid (not compiled into the library): cycles one softmax warp spends in each phase of its tiles.
 __device__ unsigned long long g_fprobe[16];
@@ -220,7 +217,7 @@ sdpa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   //   are computed while the softmax warps work on the current one.
   // D = 64 leaves room for separate P tiles, so the next score MMA can run under the current softmax.
   constexpr bool kAlias = D == 128;
-  constexpr int kPoly = kAlias ? kPolyPeriod : NB200_POLY64;
+  constexpr int kPoly = kAlias ? kPolyPeriod : 0;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n_items = a.n_qblocks * a.bh_count;
