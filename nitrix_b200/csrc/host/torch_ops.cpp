@@ -92,6 +92,9 @@ struct Attention {
   double scale;
   bool causal;
   int kernel;
+  // The mask's strides when it was packed, which are the layout of its bits.  A saved-tensor hook may hand the backward the
+  // mask in another layout: an expanded axis, which has no bits of its own, comes back from t.cpu() as a dense one.
+  std::vector<int64_t> packed_strides;
 
   nb200_sdpa_params params() const {
     nb200_sdpa_params p{};
@@ -109,7 +112,8 @@ struct Attention {
     }
     if (mask.defined()) {
       p.mask = static_cast<const uint8_t*>(packed.defined() ? packed.data_ptr() : mask.data_ptr());
-      copy_strides(p.mask_stride, mask, full);
+      if (packed.defined()) std::copy(packed_strides.begin(), packed_strides.end(), p.mask_stride);
+      else copy_strides(p.mask_stride, mask, full);
       p.mask_is_bitpacked = packed.defined() ? 2 : 0;
     }
     p.scale = float(scale);
@@ -159,17 +163,34 @@ struct Attention {
     return ws;
   }
 
-  void pack_mask() {
+  // The problem as the packing entry points take it, and the bytes its bits take.
+  nb200_sdpa_params pack_params(size_t* bytes) const {
     nb200_sdpa_params p = params();
     p.out = q.data_ptr();
     p.lse = static_cast<float*>(q.data_ptr());
     copy_strides(p.out_stride, q);
     p.bias = nullptr;
+    p.mask_is_bitpacked = 0;
+    check(lib.nb200_mask_pack_bytes(&p, 1, bytes), "nb200_mask_pack_bytes");
+    return p;
+  }
+
+  void pack_mask() {
     size_t need = 0;
-    check(lib.nb200_mask_pack_bytes(&p, 1, &need), "nb200_mask_pack_bytes");
+    const nb200_sdpa_params p = pack_params(&need);
     Tensor bits = scratch(need ? need : 1, q);
     check(lib.nb200_mask_pack(&p, 1, bits.data_ptr(), size_t(bits.numel()), stream_of(q)), "nb200_mask_pack");
     packed = bits;
+    packed_strides.assign(p.mask_stride, p.mask_stride + 4);
+  }
+
+  // Bits of another layout than the one described would be read out of their buffer.
+  void check_packed() const {
+    if (!packed.defined()) return;
+    size_t need = 0;
+    pack_params(&need);
+    TORCH_CHECK(size_t(packed.numel()) == (need ? need : 1), "scaled_dot_product_attention: the packed mask holds ", packed.numel(),
+                " bytes, its layout takes ", need);
   }
 
   std::pair<Tensor, Tensor> forward() const {
@@ -199,6 +220,7 @@ struct Attention {
       p.dbias = dbias.data_ptr();
       copy_strides(p.dbias_stride, dbias);
     }
+    check_packed();
     const Tensor ws = workspace(p, NB200_PASS_BWD);
     check(lib.nb200_sdpa_bwd(&p, stream_of(q)), "nb200_sdpa_bwd");
     return {dq, dk, dv, dbias};
@@ -210,7 +232,7 @@ struct Attention {
 struct AttentionRule : torch::autograd::Function<AttentionRule> {
   static tensor_list forward(AutogradContext* ctx, const Tensor& q, const Tensor& k, const Tensor& v, const MaybeTensor& bias,
                              const MaybeTensor& mask, double scale, bool causal, int64_t kernel, bool tensor_core) {
-    Attention a{q, k, v, bias.value_or(Tensor()), mask.value_or(Tensor()), Tensor(), scale, causal, int(kernel)};
+    Attention a{q, k, v, bias.value_or(Tensor()), mask.value_or(Tensor()), Tensor(), scale, causal, int(kernel), {}};
     const bool want_dbias = bias && bias->requires_grad();
     // (a stride of 0 is a broadcast axis to the library, which has one gradient for it)
     if (want_dbias && has_expanded_axis(a.bias)) a.bias = a.bias.contiguous();
@@ -219,7 +241,10 @@ struct AttentionRule : torch::autograd::Function<AttentionRule> {
     if (tensor_core && mask && a.plan(NB200_PASS_BWD, want_dbias) == NB200_KERNEL_TCGEN05) a.pack_mask();
     auto [out, lse] = a.forward();
     ctx->save_for_backward({q, k, v, a.bias, a.mask, out, lse});
-    if (a.packed.defined()) ctx->saved_data["packed"] = a.packed;
+    if (a.packed.defined()) {
+      ctx->saved_data["packed"] = a.packed;
+      ctx->saved_data["packed_strides"] = a.packed_strides;
+    }
     ctx->saved_data["scale"] = scale;
     ctx->saved_data["flags"] = (kernel << 2) | (int64_t(want_dbias) << 1) | int64_t(causal);
     ctx->mark_non_differentiable({lse});
@@ -232,8 +257,11 @@ struct AttentionRule : torch::autograd::Function<AttentionRule> {
     const int64_t flags = ctx->saved_data["flags"].toInt();
     const auto packed = ctx->saved_data.find("packed");
     const c10::cuda::CUDAGuard guard(s[0].device());
-    const Attention a{s[0], s[1], s[2], s[3], s[4], packed == ctx->saved_data.end() ? Tensor() : packed->second.toTensor(),
-                      ctx->saved_data["scale"].toDouble(), (flags & 1) != 0, int(flags >> 2)};
+    Attention a{s[0], s[1], s[2], s[3], s[4], Tensor(), ctx->saved_data["scale"].toDouble(), (flags & 1) != 0, int(flags >> 2), {}};
+    if (packed != ctx->saved_data.end()) {
+      a.packed = packed->second.toTensor();
+      a.packed_strides = ctx->saved_data["packed_strides"].toIntVector();
+    }
     tensor_list g = a.backward(s[5], s[6], grads[0], (flags & 2) != 0);
     g.resize(9);
     return g;
@@ -266,7 +294,7 @@ AttentionResult attention(const Tensor& q, const Tensor& k, const Tensor& v, con
                           double scale, bool causal, int64_t kernel, bool any_family) {
   if (!operands_fit(q, k, v, bias, mask)) return {std::nullopt, std::nullopt, false};
   const c10::cuda::CUDAGuard guard(q.device());
-  const Attention a{q, k, v, bias.value_or(Tensor()), mask.value_or(Tensor()), Tensor(), scale, causal, int(kernel)};
+  const Attention a{q, k, v, bias.value_or(Tensor()), mask.value_or(Tensor()), Tensor(), scale, causal, int(kernel), {}};
   int family = NB200_KERNEL_SIMT;
   if (kernel == NB200_KERNEL_AUTO) {
     family = a.plan(NB200_PASS_FWD, false);

@@ -79,3 +79,25 @@ def test_what_has_no_rule_is_refused(op):
     z.add_(1)
     with pytest.raises(RuntimeError, match="inplace"):
         y.float().sum().backward()
+
+
+@pytest.mark.parametrize("expand", [True, False])
+@pytest.mark.parametrize("D,S,T", [(64, 128, 200), (128, 100, 130)])
+def test_packed_masks_keep_the_layout_they_were_packed_from(D, S, T, expand):
+    # a hook that copies hands the backward an expanded mask with dense strides, while its bits were packed per key alone
+    from nitrix_b200.nn import scaled_dot_product_attention
+
+    g = torch.Generator(device="cuda").manual_seed(D)
+    q, k, v = (torch.randn(3, 4, n, D, generator=g, device="cuda").bfloat16().requires_grad_(True) for n in (S, T, T))
+    dout = torch.randn(3, 4, S, D, generator=g, device="cuda").bfloat16()
+    mask = torch.rand(3, 1, 1 if expand else S, T, generator=g, device="cuda") > 0.3
+    mask[..., 0] = True
+    mask = mask.expand(3, 4, S, T) if expand else mask
+    want = torch.autograd.grad(scaled_dot_product_attention(q, k, v, mask=mask), (q, k, v), dout)
+    restored = []
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: t.cpu(), lambda t: (restored.append(t.cuda()), restored[-1])[1]):
+        out = scaled_dot_product_attention(q, k, v, mask=mask)
+    got = torch.autograd.grad(out, (q, k, v), dout)
+    assert any(t.shape == mask.shape and t.is_contiguous() for t in restored if t.dtype in (torch.bool, torch.uint8))
+    for a, b in zip(got, want):   # (fp32 sums of dq added in any order, then rounded to bf16)
+        assert float((a.float() - b.float()).norm()) <= 1e-2 * float(b.float().norm())
