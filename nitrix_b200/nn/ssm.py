@@ -91,7 +91,7 @@ def _workspace(need: int, least: int, like: torch.Tensor) -> torch.Tensor:
 @functools.lru_cache(maxsize=1)
 def _ops():
     ops = _cabi.torch_ops()
-    ops.set_scan_allocator(_workspace)
+    ops.set_scan_allocator(lambda need, least, like: _workspace(need, least, like))   # (whatever this module's is by then)
     return ops
 
 

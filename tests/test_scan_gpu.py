@@ -92,20 +92,19 @@ def test_ragged_channels_and_states_and_several_chunks_per_cta(batch, length, d,
 def test_backward_in_ranges_of_a_smaller_workspace(monkeypatch, batch, length, d, n, pairs, dtype):
     # room for the adjoint states of `pairs` (batch element, channel) pairs: two elements at a time and a last one, one
     # element, groups of 64 channels with a last one cut short, the least
-    from nitrix_b200 import _cabi
     from nitrix_b200.nn import ssm
 
-    def small(p, device):
-        full, least = (ssm._bytes(getattr(_cabi.lib(), f"nb200_selective_scan_workspace{q}_bytes"), p) for q in ("", "_least"))
+    sizes = []
+
+    def small(need, least, like):
         states = 4 * ((length + 7) // 8) * n
-        size = full - (batch * d - pairs) * states
-        assert least == full - (batch * d - min(d, 64)) * states and least <= size
-        ws = torch.empty(size, dtype=torch.uint8, device=device)
-        p.workspace, p.workspace_bytes = ws.data_ptr(), size
-        return ws
+        sizes.append(need - (batch * d - pairs) * states)
+        assert least == need - (batch * d - min(d, 64)) * states and least <= sizes[-1]
+        return torch.empty(sizes[-1], dtype=torch.uint8, device=like.device)
 
     monkeypatch.setattr(ssm, "_workspace", small)
     _run((batch,), length, d, n, dtype)
+    assert len(sizes) == 1
 
 
 def test_a_device_without_room_for_all_adjoint_states_runs_in_ranges(monkeypatch):
