@@ -239,6 +239,18 @@ template <int kN, bool kUsed>
 struct Segment {
   float h[kScanCh][kN];
   float span[kScanCh];   // sum of delta
+  // The state behind a segment: end + state * 2^(d rate).  The ends of the range are those of a walk step by step: a state
+  // that is zero stays it whatever the decay (no 0 * inf), the factor is applied as two halves where it would leave the range
+  // that the product need not leave, and past that (a rate of -inf: no memory) there is no rounding to put back.
+  static __device__ __forceinline__ float through(float state, float d, float rate, float end) {
+    const float x = __fmul_rn(d, rate);
+    const bool wide = fabsf(x) > 126.f;
+    const float e = ex2_ss(wide ? 0.5f * x : x);
+    // (the exponent of a whole segment is large: its rounding goes back in as a factor 1 + ln 2 * rest)
+    const float f = fabsf(x) < 256.f ? fmaf(e * fmaf(d, rate, -x), 0.6931471805599453f, e) : e;
+    const float to = fmaf(wide ? state * e : state, f, end);
+    return state == 0.f ? end : to;
+  }
   // Publishes this segment's end; returns in `state` what enters it, from segments first, first + step .. own - step.
   template <int kPairs>
   __device__ __forceinline__ void join(int first, int own, int step, int ch, int part, float my_span, const float2 (&rate)[kPairs],
@@ -257,11 +269,8 @@ struct Segment {
       const float d = *cluster.map_shared_rank(&span[ch], s);
 #pragma unroll
       for (int k = 0; k < kPairs; ++k) {
-        // (the exponent of a whole segment is large: its rounding goes back in as a factor 1 + ln 2 * rest)
-        const float2 x = __fmul2_rn(both(d), rate[k]);
-        const float2 rest = __ffma2_rn(both(d), rate[k], make_float2(-x.x, -x.y));
-        const float2 a = ex2_ss2(x), decay = __ffma2_rn(__fmul2_rn(a, rest), both(0.6931471805599453f), a);
-        state[k] = __ffma2_rn(decay, state[k], make_float2(rh[2 * k], rh[2 * k + 1]));
+        state[k].x = through(state[k].x, d, rate[k].x, rh[2 * k]);
+        state[k].y = through(state[k].y, d, rate[k].y, rh[2 * k + 1]);
       }
     }
   }

@@ -145,3 +145,60 @@ def test_many_sequences_of_few_channels(batch, length, d, n):
 def test_walks_split_in_time(lead, length, d, n, dtype):
     """Few channels: segments of the sequence walked side by side, joined by their decays."""
     _run(lead, length, d, n, dtype, seed=length)
+
+
+# Nine steps whose decays multiply to 2^exponent lie in one segment of the split walks; the other steps' are 2^-0.003.
+_ENDS = {"growth over an empty state": (0.0, 200.0), "growth of a small state": (1e-30, 135.0),
+         "decay of a large state": (1e30, -140.0), "growth out of the range": (0.0, 600.0)}
+
+
+@pytest.mark.parametrize("length,n", [(256, 8), (112, 33)])   # eight segments, four with a short one
+@pytest.mark.parametrize("form", _ENDS)
+def test_segments_join_at_the_ends_of_the_range(form, length, n):
+    """What enters a segment passes its whole decay as it would step by step: forward, and mirrored through dx.  Tolerance:
+    an exponent of 97 (140 ln 2) times its rate and its span, rounded to 2^-24 three or four times (2e-5), some 45
+    exponentials of 2^-22 and as many products of 2^-24 behind it (1.3e-5): 4e-5 of the largest."""
+    from nitrix_b200.nn import selective_scan
+
+    start, exponent = _ENDS[form]
+    g = torch.Generator(device="cuda").manual_seed(length)
+    lead, d, seg = 2, 20, 32
+    A = torch.full((d, n), 1.0 if exponent > 0 else -1.0, device="cuda")
+    delta = torch.full((lead, length, d), 2.0 ** -9, device="cuda")
+    delta[:, seg + 4:seg + 13] = abs(exponent) / 9 * float(np.log(2.0))
+    x = torch.zeros(lead, length, d, device="cuda")
+    x[:, :4] = start
+    C = torch.rand(lead, length, n, generator=g, device="cuda") + 0.5
+    C[:, :length - 16] = 0.0    # (what is read is what has passed the segment)
+    B = torch.rand(lead, length, n, generator=g, device="cuda") + 0.5
+    if start == 0.0:
+        x[:, length - 16:] = 1.0
+    want = S.selective_scan_torch(*(t.double() for t in (x, delta, A, B, C)))
+    y = selective_scan(x, delta, A, B, C)
+    assert float((y.double() - want).abs().max()) <= 4e-5 * float(want.abs().max()), form
+    # the adjoint walk is the same recurrence last step first, one step later: dy for x, C for B
+    rx, rd, rB, rC = (t.flip(1).contiguous() for t in (x, delta, B, C))
+    dx, dx64 = [], []
+    for z, to, fn in ((torch.zeros_like(x), dx, selective_scan), (torch.zeros_like(x).double(), dx64, S.selective_scan_torch)):
+        z.requires_grad_(True)
+        to.append(torch.autograd.grad(fn(z, *(t.to(z.dtype) for t in (rd, A, rC, rB))), z, rx.to(z.dtype))[0])
+    assert float(dx64[0].abs().max()) > 0
+    assert float((dx[0].double() - dx64[0]).abs().max()) <= 4e-5 * float(dx64[0].abs().max()), form
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
+@pytest.mark.parametrize("length,n", [(256, 8), (112, 33)])
+def test_segments_of_states_without_memory(length, n, dtype):
+    """A rate of -inf (an fp16 -exp(A_log) overflows to it): the state is what its own step put in, in every segment."""
+    from nitrix_b200.nn import selective_scan
+
+    x, delta, A, B, C, _, dy = _operands((2,), length, 20, n, dtype, False, 5)
+    A[::3, 1::2] = -float("inf")
+    leaves = [t.detach().clone().requires_grad_(True) for t in (x, B, C)]
+    y = selective_scan(leaves[0], delta, A, *leaves[1:])
+    grads = torch.autograd.grad(y, leaves, dy)
+    ref = [t.detach().double().requires_grad_(True) for t in (x, B, C)]
+    want = S.selective_scan_torch(ref[0], delta.double(), A.double(), *ref[1:])
+    tol = 2e-5 if dtype == torch.float32 else 2e-3   # as above
+    for a, r in zip((y.detach(), *grads), (want.detach(), *torch.autograd.grad(want, ref, dy.double()))):
+        assert float((a.double() - r).abs().max()) <= tol * float(r.abs().max())
