@@ -31,8 +31,7 @@ using MaybeTensor = std::optional<Tensor>;
   X(nb200_last_error) X(nb200_sdpa_plan) X(nb200_sdpa_workspace_bytes) X(nb200_sdpa_workspace_least_bytes)                 \
   X(nb200_sdpa_fwd) X(nb200_sdpa_bwd) X(nb200_mask_pack_bytes) X(nb200_mask_pack) X(nb200_qk_rms_norm)                     \
   X(nb200_qk_rms_norm_grad) X(nb200_layer_norm_fwd) X(nb200_layer_norm_bwd) X(nb200_layer_norm_workspace_bytes)            \
-  X(nb200_selective_scan_fwd) X(nb200_selective_scan_bwd) X(nb200_selective_scan_workspace_bytes)                          \
-  X(nb200_selective_scan_workspace_least_bytes) X(nb200_selective_scan_checkpoint_bytes)
+  X(nb200_selective_scan_fwd) X(nb200_selective_scan_bwd) X(nb200_selective_scan_checkpoint_bytes)
 
 struct Library {
 #define X(name) decltype(&::name) name = nullptr;
@@ -465,9 +464,9 @@ Tensor sum_to_operand(const Tensor& g3, at::IntArrayRef lead, at::IntArrayRef sh
 
 // The backward's scratch comes from nitrix_b200.nn.ssm, which decides what a device without room for all of it gets.
 PyObject* scan_allocator = nullptr;
-Tensor scan_workspace(size_t need, size_t least, const Tensor& like) {
+Tensor scan_workspace(nb200_selective_scan_params& p, const Tensor& like) {   // (fills in p's workspace)
   py::gil_scoped_acquire gil;
-  return py::reinterpret_borrow<py::object>(scan_allocator)(need, least, like).cast<Tensor>();
+  return py::reinterpret_borrow<py::object>(scan_allocator)(reinterpret_cast<uintptr_t>(&p), like).cast<Tensor>();
 }
 
 // Saves the operands and the forward's checkpoints.
@@ -513,12 +512,7 @@ struct ScanRule : torch::autograd::Function<ScanRule> {
     p.dy = dy3.data_ptr();
     p.dx = dx.data_ptr(); p.ddelta = ddelta.data_ptr(); p.dA = dA.data_ptr(); p.dB = dB.data_ptr(); p.dC = dC.data_ptr();
     p.dD = dD.defined() ? dD.data_ptr() : nullptr;
-    size_t need = 0, least = 0;
-    check(lib.nb200_selective_scan_workspace_bytes(&p, &need), "nb200_selective_scan_workspace_bytes");
-    check(lib.nb200_selective_scan_workspace_least_bytes(&p, &least), "nb200_selective_scan_workspace_least_bytes");
-    const Tensor ws = scan_workspace(need, least, x3);
-    p.workspace = ws.data_ptr();
-    p.workspace_bytes = size_t(ws.numel());
+    const Tensor ws = scan_workspace(p, x3);
     check(lib.nb200_selective_scan_bwd(&p, stream_of(x3)), "nb200_selective_scan_bwd");
     const auto xs = ctx->saved_data["x"].toIntVector(), types = ctx->saved_data["types"].toIntVector();
     const at::IntArrayRef lead(xs.data(), xs.size() - 2);

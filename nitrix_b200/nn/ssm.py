@@ -79,19 +79,23 @@ def selective_scan_forward(x3, delta3, A, B3, C3, D, want_checkpoints: bool):
     return y, ck
 
 
-def _workspace(need: int, least: int, like: torch.Tensor) -> torch.Tensor:
+def _workspace(p, device) -> torch.Tensor:
     """The backward's scratch; where the device has no room for the adjoint states of the whole batch at once (as large as
     the checkpoints), the least with which it runs, a range after the other."""
     try:
-        return torch.empty(max(need, 16), dtype=torch.uint8, device=like.device)
+        ws = torch.empty(max(_bytes(_cabi.lib().nb200_selective_scan_workspace_bytes, p), 16), dtype=torch.uint8, device=device)
     except torch.OutOfMemoryError:
-        return torch.empty(max(least, 16), dtype=torch.uint8, device=like.device)
+        ws = torch.empty(max(_bytes(_cabi.lib().nb200_selective_scan_workspace_least_bytes, p), 16), dtype=torch.uint8,
+                         device=device)
+    p.workspace, p.workspace_bytes = ws.data_ptr(), ws.numel()
+    return ws
 
 
 @functools.lru_cache(maxsize=1)
 def _ops():
     ops = _cabi.torch_ops()
-    ops.set_scan_allocator(lambda need, least, like: _workspace(need, least, like))   # (whatever this module's is by then)
+    # (the module's _workspace at the time of the call, not the one there was at the first)
+    ops.set_scan_allocator(lambda address, like: _workspace(_cabi.SelectiveScanParams.from_address(address), like.device))
     return ops
 
 
@@ -106,9 +110,7 @@ def selective_scan_backward(x3, delta3, A, B3, C3, D, ck, dy3):
     p.checkpoints = None if ck is None else ck.data_ptr()
     p.dx, p.ddelta, p.dA, p.dB, p.dC = (t.data_ptr() for t in (dx, ddelta, dA, dB, dC))
     p.dD = None if dD is None else dD.data_ptr()
-    ws = _workspace(_bytes(_cabi.lib().nb200_selective_scan_workspace_bytes, p),
-                    _bytes(_cabi.lib().nb200_selective_scan_workspace_least_bytes, p), x3)
-    p.workspace, p.workspace_bytes = ws.data_ptr(), ws.numel()
+    ws = _workspace(p, x3.device)
     _check(_cabi.enqueue(_cabi.lib().nb200_selective_scan_bwd, p, x3.device), "nb200_selective_scan_bwd")
     del ws  # same-stream reuse is ordered by the caching allocator
     return dx, ddelta, dA, dB, dC, dD

@@ -92,19 +92,20 @@ def test_ragged_channels_and_states_and_several_chunks_per_cta(batch, length, d,
 def test_backward_in_ranges_of_a_smaller_workspace(monkeypatch, batch, length, d, n, pairs, dtype):
     # room for the adjoint states of `pairs` (batch element, channel) pairs: two elements at a time and a last one, one
     # element, groups of 64 channels with a last one cut short, the least
+    from nitrix_b200 import _cabi
     from nitrix_b200.nn import ssm
 
-    sizes = []
-
-    def small(need, least, like):
+    def small(p, device):
+        full, least = (ssm._bytes(getattr(_cabi.lib(), f"nb200_selective_scan_workspace{q}_bytes"), p) for q in ("", "_least"))
         states = 4 * ((length + 7) // 8) * n
-        sizes.append(need - (batch * d - pairs) * states)
-        assert least == need - (batch * d - min(d, 64)) * states and least <= sizes[-1]
-        return torch.empty(sizes[-1], dtype=torch.uint8, device=like.device)
+        size = full - (batch * d - pairs) * states
+        assert least == full - (batch * d - min(d, 64)) * states and least <= size
+        ws = torch.empty(size, dtype=torch.uint8, device=device)
+        p.workspace, p.workspace_bytes = ws.data_ptr(), size
+        return ws
 
     monkeypatch.setattr(ssm, "_workspace", small)
     _run((batch,), length, d, n, dtype)
-    assert len(sizes) == 1
 
 
 def test_a_device_without_room_for_all_adjoint_states_runs_in_ranges(monkeypatch):
@@ -202,3 +203,13 @@ def test_segments_of_states_without_memory(length, n, dtype):
     tol = 2e-5 if dtype == torch.float32 else 2e-3   # as above
     for a, r in zip((y.detach(), *grads), (want.detach(), *torch.autograd.grad(want, ref, dy.double()))):
         assert float((a.double() - r).abs().max()) <= tol * float(r.abs().max())
+
+
+def test_the_backward_asks_this_module_for_its_scratch_each_time(monkeypatch):
+    from nitrix_b200.nn import ssm
+
+    own, calls = ssm._workspace, []
+    _run((2,), 40, 24, 8, torch.float32)
+    monkeypatch.setattr(ssm, "_workspace", lambda p, device: (calls.append(device), own(p, device))[1])
+    _run((2,), 40, 24, 8, torch.float32)
+    assert len(calls) == 1
