@@ -199,36 +199,42 @@ inline int round_up(int x, int m) { return (x + m - 1) / m * m; }
 namespace {
 
 // dst[i0][i1][i2][i3] = src[...] for 16-bit elements, both sides described by element strides.
-// Bound: HBM, each element read and written once.  A warp takes one row at a time and a contiguous run of rows, so an
-// index is divided once per warp and not three times per element in 64 bits; a lane writes aligned words of two elements
-// whatever the row's alignment (odd lengths put every other row at an odd element), read as one word where the source is
-// aligned like the destination and as two elements otherwise, four words in flight.  One element per thread was bound by
-// its divisions: (3, 16, 5158, 5158) 6640 us per copy, now 1070 (2.55 GB each way: 4.8 TB/s); (2, 32, 1223, 6617) 2700 ->
-// 580; (1, 8, 217, 217) 4.7 -> 3.0.
+// Bound: HBM, each element read and written once.  A warp takes one row, or one piece of a row, at a time and a contiguous run
+// of them, so an index is divided once per warp and not three times per element in 64 bits; a lane writes aligned words of two
+// elements whatever the row's alignment (odd lengths put every other row at an odd element), read as one word where the
+// source is aligned like the destination and as two elements otherwise, four words in flight.  One element per thread was
+// bound by its divisions: (3, 16, 5158, 5158) 6640 us per copy, now 1070 (2.55 GB each way: 4.8 TB/s); (2, 32, 1223, 6617)
+// 2700 -> 580.  Whole rows leave most of the GPU idle where they are few: (1, 8, 4, 65537) 129 us, in pieces 10.
 template <bool kSrcUnit, bool kDstUnit>
 __global__ void __launch_bounds__(256) copy16_rows_kernel(const uint16_t* __restrict__ src, int64_t s0, int64_t s1, int64_t s2,
                                                           int64_t s3, uint16_t* __restrict__ dst, int64_t d0, int64_t d1,
-                                                          int64_t d2, int64_t d3, int64_t e1, int64_t e2, int e3,
-                                                          int64_t rows, int64_t rows_per_warp) {
+                                                          int64_t d2, int64_t d3, int64_t e1, int64_t e2, int e3, int piece,
+                                                          int pieces, int64_t units, int64_t units_per_warp) {
   const int lane = threadIdx.x & 31;
-  const int64_t first = (int64_t(blockIdx.x) * 8 + (threadIdx.x >> 5)) * rows_per_warp;
-  if (first >= rows) return;
-  const int64_t last = min(rows, first + rows_per_warp);
-  int64_t i2 = first % e2, i1 = (first / e2) % e1, i0 = first / e2 / e1;
-  for (int64_t row = first; row < last; ++row) {
-    const uint16_t* sp = src + i0 * s0 + i1 * s1 + i2 * s2;
-    uint16_t* dp = dst + i0 * d0 + i1 * d1 + i2 * d2;
-    if (++i2 == e2) {
-      i2 = 0;
-      if (++i1 == e1) { i1 = 0; ++i0; }
+  const int64_t first = (int64_t(blockIdx.x) * 8 + (threadIdx.x >> 5)) * units_per_warp;
+  if (first >= units) return;
+  const int64_t last = min(units, first + units_per_warp), row = first / pieces;
+  int col = int(first - row * pieces) * piece;
+  int64_t i2 = row % e2, i1 = (row / e2) % e1, i0 = row / e2 / e1;
+  for (int64_t u = first; u < last; ++u) {
+    const uint16_t* sp = src + i0 * s0 + i1 * s1 + i2 * s2 + col * (kSrcUnit ? 1 : s3);
+    uint16_t* dp = dst + i0 * d0 + i1 * d1 + i2 * d2 + col * (kDstUnit ? 1 : d3);
+    const int n = min(piece, e3 - col);   // >= 1
+    col += piece;
+    if (col >= e3) {
+      col = 0;
+      if (++i2 == e2) {
+        i2 = 0;
+        if (++i1 == e1) { i1 = 0; ++i0; }
+      }
     }
     if constexpr (!kDstUnit) {
-      for (int w = lane; w < e3; w += 32) dp[w * d3] = sp[w * s3];
+      for (int w = lane; w < n; w += 32) dp[w * d3] = sp[w * s3];
       continue;
     }
     const int head = int((reinterpret_cast<uintptr_t>(dp) >> 1) & 1);   // elements in front of the first whole word
-    const int words = (e3 - head) >> 1;                                 // (e3 >= 1)
-    const bool tail = ((e3 - head) & 1) != 0;
+    const int words = (n - head) >> 1;
+    const bool tail = ((n - head) & 1) != 0;
     const uint16_t* se = sp + head * (kSrcUnit ? 1 : s3);
     uint32_t* dw = reinterpret_cast<uint32_t*>(dp + head);
     if (kSrcUnit && (reinterpret_cast<uintptr_t>(se) & 3) == 0) {
@@ -243,7 +249,18 @@ __global__ void __launch_bounds__(256) copy16_rows_kernel(const uint16_t* __rest
       }
     }
     if (lane == 0 && head) dp[0] = sp[0];
-    if (lane == 1 && tail) dp[e3 - 1] = sp[kSrcUnit ? e3 - 1 : (e3 - 1) * s3];
+    if (lane == 1 && tail) dp[n - 1] = sp[kSrcUnit ? n - 1 : (n - 1) * s3];
+  }
+}
+
+// The same, an element per thread and turn, for rows that are short or few in all; `I` holds the number of elements.
+template <typename I>
+__global__ void __launch_bounds__(256) copy16_elements_kernel(const uint16_t* __restrict__ src, int64_t s0, int64_t s1, int64_t s2,
+                                                              int64_t s3, uint16_t* __restrict__ dst, int64_t d0, int64_t d1,
+                                                              int64_t d2, int64_t d3, I e1, I e2, I e3, I n) {
+  for (I i = I(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += I(gridDim.x) * blockDim.x) {
+    const I r = i / e3, i3 = i - r * e3, r2 = r / e2, i2 = r - r2 * e2, i0 = r2 / e1, i1 = r2 - i0 * e1;
+    dst[i0 * d0 + i1 * d1 + i2 * d2 + i3 * d3] = __ldg(src + i0 * s0 + i1 * s1 + i2 * s2 + i3 * s3);
   }
 }
 
@@ -264,19 +281,35 @@ inline bool aligned16(const void* p) { return reinterpret_cast<uintptr_t>(p) % 1
 
 int launch_copy16(const void* src, const int64_t ss[4], void* dst, const int64_t ds[4], const int64_t e[4], cudaStream_t st,
                   const char* what) {
-  const int64_t rows = e[0] * e[1] * e[2];
-  if (rows <= 0 || e[3] <= 0) return NB200_OK;
-  // eight CTAs of eight warps per SM
-  const int64_t warps = int64_t(sm_count()) * 64;
-  const int64_t per_warp = (rows + warps - 1) / warps;
-  const int blocks = int((rows + 8 * per_warp - 1) / (8 * per_warp));
+  const int64_t rows = e[0] * e[1] * e[2], n = rows * e[3];
+  if (n <= 0) return NB200_OK;
   const uint16_t* s16 = static_cast<const uint16_t*>(src);
   uint16_t* d16 = static_cast<uint16_t*>(dst);
-  const bool src_unit = e[3] == 1 || ss[3] == 1, dst_unit = e[3] == 1 || ds[3] == 1;
-  auto kernel = !dst_unit ? copy16_rows_kernel<false, false>
-                          : (src_unit ? copy16_rows_kernel<true, true> : copy16_rows_kernel<false, true>);
-  kernel<<<blocks, 256, 0, st>>>(s16, ss[0], ss[1], ss[2], ss[3], d16, ds[0], ds[1], ds[2], ds[3], e[1], e[2], int(e[3]), rows,
-                                 per_warp);
+  // By elements below 64 of them a row, where most lanes of a warp per row have nothing to do ((8, 16, 4096, 1) 8 us against
+  // 61, 12 keys 27 against 78, 47 keys 82 against 102, 63 level), and up to one element per thread of a full GPU (17680: 6
+  // us against 8); from there on by rows ((1, 8, 48, 8191) 12 us against 16, (2, 8, 1000, 1001) 27 against 55).
+  if (e[3] < 64 || n <= (int64_t(1) << 19)) {
+    const int64_t want = (n + 255) / 256, most = int64_t(sm_count()) * 16;
+    const int blocks = int(want < most ? want : most);
+    if (n < (int64_t(1) << 31))
+      copy16_elements_kernel<uint32_t><<<blocks, 256, 0, st>>>(s16, ss[0], ss[1], ss[2], ss[3], d16, ds[0], ds[1], ds[2], ds[3],
+                                                               uint32_t(e[1]), uint32_t(e[2]), uint32_t(e[3]), uint32_t(n));
+    else
+      copy16_elements_kernel<int64_t><<<blocks, 256, 0, st>>>(s16, ss[0], ss[1], ss[2], ss[3], d16, ds[0], ds[1], ds[2], ds[3],
+                                                              e[1], e[2], e[3], n);
+    count_launch();
+    return check_launch(what);
+  }
+  // eight CTAs of eight warps per SM; fewer rows than that are cut into pieces of an even length, from 256 elements on
+  const int64_t warps = int64_t(sm_count()) * 64;
+  const int64_t by_rows = (warps + rows - 1) / rows, by_length = (e[3] + 255) / 256, cut = by_rows < by_length ? by_rows : by_length;
+  const int piece = int((e[3] + 2 * cut - 1) / (2 * cut) * 2), pieces = int((e[3] + piece - 1) / piece);
+  const int64_t units = rows * pieces, per_warp = (units + warps - 1) / warps;
+  const int blocks = int((units + 8 * per_warp - 1) / (8 * per_warp));
+  auto kernel = ds[3] != 1 ? copy16_rows_kernel<false, false>
+                           : (ss[3] == 1 ? copy16_rows_kernel<true, true> : copy16_rows_kernel<false, true>);
+  kernel<<<blocks, 256, 0, st>>>(s16, ss[0], ss[1], ss[2], ss[3], d16, ds[0], ds[1], ds[2], ds[3], e[1], e[2], int(e[3]), piece,
+                                 pieces, units, per_warp);
   count_launch();
   return check_launch(what);
 }

@@ -46,6 +46,13 @@ def test_padded_copies_of_a_bias_keep_every_element(S, T, layout):
     assert float((grads[0][3].double() - ref).abs().max()) <= 2e-2 * max(1.0, float(ref.abs().max()))
 
 
+@pytest.mark.parametrize("layout", ["dense", "odd_start", "key_strided"])
+@pytest.mark.parametrize("S,T", [(4, 30011), (1, 90003), (1500, 65), (1500, 63), (400, 257)])
+def test_padded_copies_of_few_long_and_of_many_short_rows(S, T, layout):
+    # rows cut into pieces (the last one shorter), whole rows, and rows taken element by element
+    test_padded_copies_of_a_bias_keep_every_element(S, T, layout)
+
+
 def _words(bits):
     """(..., n) booleans -> (..., ceil(n / 32) rounded up to 4) 32-bit words, bit i of word w = element 32 w + i."""
     n = bits.shape[-1]
