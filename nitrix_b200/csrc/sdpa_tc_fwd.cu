@@ -50,7 +50,6 @@ using namespace sm100;
 
 namespace {
 
-constexpr int kMaxOrder = 288;   // batch elements that a CTA ranks by kept length (item order 3)
 // Softmax warps per query tile: four (a thread owns a row) or eight (two threads share a row, each half of a pass's keys).
 template <int D>
 struct Split {
@@ -946,6 +945,8 @@ int launch_one(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& 
                FwdArgs a, cudaStream_t st) {
   auto kernel = sdpa_fwd_tc_kernel<D, kBf16, kTileBias, kAdd>;
   using L = FwdSmem<D, kTileBias>;
+  static_assert(kMaxOrder <= Split<D>::kThreads, "a thread per ranked batch element");
+  // (with bias tiles at head dim 64 the room left for rounding the base up is 840 bytes; the driver's base needs none)
   constexpr int kLimit = 232448;  // 227 KB per CTA
   const int smem = L::kTotal + 1024 <= kLimit ? L::kTotal + 1024 : kLimit;
   static_assert(L::kTotal <= kLimit, "forward shared memory exceeds the per-CTA limit");

@@ -6,6 +6,8 @@
 namespace nb200 {
 namespace tc {
 
+constexpr int kMaxOrder = 384;   // batch elements that a CTA ranks by kept length (item order 3), one thread each
+
 struct FwdArgs {
   int B, H, S, T;
   int bh_begin, bh_count;       // flattened (batch, head) range this launch covers

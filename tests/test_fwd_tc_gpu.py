@@ -57,3 +57,23 @@ def test_forward_against_fp64(D, dtype, S, T, kind):
         tol = (2.0 if dtype == torch.bfloat16 else 0.25) * 2.0 ** -7
         assert float((got.double() - want).abs().max()) <= tol * max(1.0, float(want.abs().max()))
         assert float((lse.double() - want_lse).abs().max()) <= 1e-3 * max(1.0, float(want_lse.abs().max()))
+
+
+@pytest.mark.parametrize("D,tile", [(64, True), (64, False), (128, True), (128, False)])
+@pytest.mark.parametrize("B", [289, 384, 385])
+def test_many_key_padded_batch_elements_whatever_their_order(B, D, tile):
+    # items are dealt by kept length up to the largest batch that a CTA ranks; an element's rows depend on nothing else
+    from nitrix_b200.nn.attention import sdpa_forward
+
+    g = torch.Generator(device="cuda").manual_seed(B)
+    S, T = 40, 264
+    q = torch.randn(B, 1, S, D, generator=g, device="cuda").bfloat16()
+    k, v = (torch.randn(B, 1, T, D, generator=g, device="cuda").bfloat16() for _ in range(2))
+    bias = torch.randn(1, 1, S, T, generator=g, device="cuda").bfloat16() if tile else None
+    lengths = torch.randint(1, T + 1, (B, 1), generator=g, device="cuda")
+    mask = (torch.arange(T, device="cuda") < lengths).reshape(B, 1, 1, T)
+    out, lse = sdpa_forward(q, k, v, bias, mask, scale=0.125)
+    for i in range(0, B, 100):
+        part = slice(i, i + 100)
+        out_i, lse_i = sdpa_forward(q[part], k[part], v[part], bias, mask[part], scale=0.125)
+        assert torch.equal(out[part], out_i) and torch.equal(lse[part], lse_i)
