@@ -233,8 +233,9 @@ __device__ __forceinline__ float2 both(float v) { return make_float2(v, v); }
 // cluster of up to eight CTAs takes the sequence in segments: each walks its own from an empty state, keeping its end and
 // the sum of its deltas (whose exponential is the segment's whole decay), reads those of the segments before it over
 // distributed shared memory, and walks again from the state they give.  About 1.6 times the work, four or eight times the
-// SMs (walk_splits has the figures).  Error against 64 bits, f32, mean over 14 problems, half of them with slow decays, one walk /
-// segments: y 3.1e-7 / 2.3e-7, dA 1.8e-6 / 1.2e-6.
+// SMs (walk_splits has the figures).  Error against 64 bits, f32, norms, mean over (1, 2048, 128, 16), (2, 1024, 96, 8), (1, 1500,
+// 64, 32), (2, 600, 40, 64) and (4, 512, 64, 16), each with rates of 0.2 to 1.7 and a hundredth of that, one walk / segments:
+// y 1.2e-6 / 7.4e-7, dA 2.4e-6 / 1.4e-6.
 template <int kN, bool kUsed>
 struct Segment {
   float h[kScanCh][kN];
@@ -813,18 +814,33 @@ int segment_steps(int length, int splits) {
   return (stages + splits - 1) / splits * kStage;
 }
 // Segments of the walks, 1: not split.  Two give nothing (1.6 times the work: (1, 2048, 2048, 16) 352 -> 341 us, (4, 2048,
-// 1024, 16) 446 -> 465), so four or eight, as many as leave up to eight CTAs per SM -- four from 32 states on, whose CTAs
-// hold more registers and shared memory: (4, 600, 300, 64) 248, as four segments 227, as eight 302 -- and 24 steps each.
-// All kernels of forward and backward, us before / now: bf16 (5, 1847, 136, 8) 280 / 124, (2, 1274, 277, 32) 276 / 142, f32
-// (1, 2048, 128, 16) 264 / 85, (1, 2048, 2048, 16) 352 / 219, (4, 2048, 1024, 16) 446 / 406, (3, 166, 297, 8) 37 / 32.
-int walk_splits(int64_t ctas, int64_t length, int states) {
+// 1024, 16) 446 -> 465), so four or eight.  `load` is the CTAs that they put on an SM.  Up to one wave of clusters a step
+// costs its latencies whatever the load, and the segments gain; past it they only add work (f32 forward, N = 16, 296 CTAs of
+// one walk, 256 / 2048 steps: 21 / 139 us, in four 28 / 166, in eight 34 / 143; N = 64, 148 CTAs: 40 / 285, in four 68 / 389,
+// in eight 173 / 424).  More states hold more registers and shared memory and take longer to join, so the room shrinks and
+// the least length, which grows with the load, rises with them.  The lines lie where one walk and segments were level over 2
+// to 592 CTAs of one walk and 97 to 2048 steps, N = 8 / 16 / 32 / 64: on 74 CTAs of 2048 steps one walk takes 105 / 132 /
+// 167 / 285 us, four 64 / 72 / 105 / 210, eight 40 / 50 / 81 / 243; on 148 of 256 steps 17 / 20 / 25 / 40, 15 / 17 / 26 / 68
+// and 17 / 22 / 61 / 173.  As many as left eight CTAs per SM (four from 32 states on) and 24 steps each, as the rule was before,
+// made one in ten of these slower than one walk (N = 64, 74 CTAs, 192 steps: 31 -> 84 us).
+int walk_splits(int64_t ctas, int64_t length, int states, bool half, bool adjoint) {
   int sms = 0, dev = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (sms <= 0) sms = 148;
-  const int64_t room = (states > 16 ? 4 : 8) * int64_t(sms);
-  for (int splits = 8; splits >= 4; splits /= 2)
-    if (splits * ctas <= room && length >= 24 * splits) return splits;
+  const float load4 = 4.f * float(ctas) / float(sms), load8 = 2.f * load4, steps = float(length);
+  struct Rule { float room8, least8, slope8, room4, slope4; };   // most load; least steps, in all and per load
+  const int n = pick_n(states);
+  Rule r;
+  if (n == 8) r = {7.f, 192.f, 32.f, 7.6f, half && !adjoint ? 16.f : 25.f};
+  else if (n == 16) r = adjoint ? Rule{7.f, 192.f, 96.f, 6.f, 50.f} : Rule{7.f, 192.f, 64.f, 7.6f, 25.f};
+  else if (n == 32) r = {5.f, 384.f, 192.f, 5.5f, adjoint ? 100.f : 75.f};
+  else if (half && !adjoint) r = {2.f, 768.f, 0.f, 5.5f, 45.f};   // (its one walk is slow: 74 CTAs, 2048 steps 521 us, f32 285)
+  else r = {2.f, 768.f, 0.f, 3.f, 150.f};
+  if (load8 <= r.room8 && steps >= fmaxf(r.least8, r.slope8 * load8)) return 8;
+  if (load4 <= r.room4 && steps >= fmaxf(96.f, r.slope4 * load4)) return 4;
+  // 16-bit storage of few states: a little past one wave too (296 CTAs, 2048 steps: N = 8 128 -> 115 us, N = 16 140 -> 136)
+  if (half && !adjoint && n <= 16 && load8 <= 20.f && steps >= 128.f * float(n)) return 8;
   return 1;
 }
 
@@ -866,7 +882,8 @@ template <typename T>
 int fwd_t(const nb200_selective_scan_params* p, cudaStream_t st) {
   SsArgs a = args_of<T>(p);
   if (p->length <= kStage - 4) return fwd_launch<T, true, false>(p, a, 1, st);
-  const int splits = walk_splits(int64_t(p->channels + kScanCh - 1) / kScanCh * p->batch, p->length, p->states);
+  const int64_t ctas = int64_t(p->channels + kScanCh - 1) / kScanCh * p->batch;
+  const int splits = walk_splits(ctas, p->length, p->states, sizeof(T) == 2, false);
   if (splits == 1) return fwd_launch<T, false, false>(p, a, 1, st);
   a.seg = segment_steps(p->length, splits);
   return fwd_launch<T, false, true>(p, a, splits, st);
@@ -950,7 +967,7 @@ template <typename T, bool kRange>
 int bwd_range(const nb200_selective_scan_params* p, const SsArgs& a, Range r, cudaStream_t st) {
   if (a.chunks > 1) {
     const dim3 grid((r.channels + kScanCh - 1) / kScanCh, r.batch);
-    const int splits = kRange ? 1 : walk_splits(int64_t(grid.x) * grid.y, p->length, p->states);
+    const int splits = kRange ? 1 : walk_splits(int64_t(grid.x) * grid.y, p->length, p->states, sizeof(T) == 2, true);
     SsArgs w = a;
     w.seg = segment_steps(p->length, splits);
     if (int rc = splits == 1 ? adjoint_launch<T, kRange, false>(p, w, grid, 1, st) : adjoint_launch<T, false, true>(p, w, grid, splits, st)) return rc;
