@@ -22,12 +22,12 @@
 // Merged variant (key-major, D = 64, no bias gradient): ds goes to shared memory instead of TMEM and also feeds
 // dQ = ds K per pair of steps (a 128 x 64 tile at TMEM column 320), which the element-wise warps add to an fp32
 // accumulator in global memory; the query-major kernel is then not needed.
-// Twelve warps (query-major: twenty): 0 issues the accumulating MMAs, 1 the TMA copies of the step loop (ring refills and bias tiles, one
-// thread serving both), 2 issues the products, 3 owns TMEM and builds the per-query (key-major) or per-key
-// (query-major) addends as MMA operands, 4-7 / 8-11 are two element-wise groups that take alternate steps (one
-// owner row per thread; query-major: 32 columns of one per thread, 12-15 / 16-19 take the others).  The owner tiles and the first ring stages are issued by thread 0 during start-up.  All
-// waits are bounded.  At head dim 128 these kernels only serve what the one-kernel backward of
-// sdpa_tc_bwd_d128.cu declines (a bias gradient that needs fp32 sums).
+// Twelve warps (query-major: twenty): 0 issues the accumulating MMAs, 1 the TMA copies of the step loop (ring refills and
+// bias tiles, one thread serving both), 2 issues the products, 3 owns TMEM and builds the per-query (key-major) or per-key
+// (query-major) addends as MMA operands, 4-7 / 8-11 are two element-wise groups that take alternate steps (one owner row
+// per thread; query-major: 32 columns of one per thread, 12-15 / 16-19 take the others).  The owner tiles and the first ring
+// stages are issued by thread 0 during start-up.  All waits are bounded.  At head dim 128 these kernels only serve what the
+// one-kernel backward of sdpa_tc_bwd_d128.cu declines (a bias gradient that needs fp32 sums).
 #include <math.h>
 #include <stdlib.h>
 
@@ -46,7 +46,7 @@ constexpr int kYBoxBytes = kStep * 128;       // one 64-row x 128-byte TMA box
 // (two threads share one, 32 of its columns each).  Eight where the element-wise work is the bound, query-major with its
 // dbias tiles or sums: B4 H32 L4096 D64 2580 -> 2395 us, windows of 217 35.4 -> 32.7, D128 137 -> 129; key-major they gained
 // nothing (1540 -> 1605) and merged they lost (204 -> 214; with the longer ring 196 against 200).
-template <bool kKeyMajor, bool kMerged>
+template <bool kKeyMajor>
 struct Split {
   static constexpr int kHalves = kKeyMajor ? 1 : 2;
   static constexpr int kThreads = 128 + 256 * kHalves;
@@ -102,13 +102,13 @@ struct BwdSmem {
 };
 
 template <int D, bool kBf16, bool kKeyMajor, bool kMerged, bool kTiles>
-__global__ void __launch_bounds__(Split<kKeyMajor, kMerged>::kThreads, 1)
+__global__ void __launch_bounds__(Split<kKeyMajor>::kThreads, 1)
 sdpa_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_constant__ CUtensorMap tm_x2,
                    const __grid_constant__ CUtensorMap tm_y1, const __grid_constant__ CUtensorMap tm_y2,
                    const __grid_constant__ CUtensorMap tm_bias, const BwdArgs a) {
   static_assert(!kMerged || (kKeyMajor && D == 64), "the merged kernel is the key-major kernel at head dim 64");
   using L = BwdSmem<D, kMerged, kTiles>;
-  constexpr int kThreads = Split<kKeyMajor, kMerged>::kThreads, kHalves = Split<kKeyMajor, kMerged>::kHalves;
+  constexpr int kThreads = Split<kKeyMajor>::kThreads, kHalves = Split<kKeyMajor>::kHalves;
   constexpr int kCols = kStep / kHalves;   // columns of a step that one element-wise thread takes
   constexpr int kAugSlots = L::kAugSlots;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -253,7 +253,7 @@ sdpa_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_const
   const uint32_t tm_acc1 = tmem + (kDeep ? 384 : 256), tm_acc2 = tm_acc1 + D;
 
   if (warp < 4) {
-  reg_dealloc<Split<kKeyMajor, kMerged>::kProducerRegs>();
+  reg_dealloc<Split<kKeyMajor>::kProducerRegs>();
   if (warp == 1) {
     // ---------------- TMA duties of the step loop: ring refills and bias tiles, ONE thread ----------------
     // (the owner tiles, the first NY stages and the first two bias slots were issued during start-up).  The thread
@@ -555,7 +555,7 @@ sdpa_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_const
     }
   }
   } else {
-    reg_alloc<Split<kKeyMajor, kMerged>::kWorkerRegs>();
+    reg_alloc<Split<kKeyMajor>::kWorkerRegs>();
     // ---------------- element-wise groups (an owner row, or 32 columns of one, per thread) ----------------
     const int grp = ((warp - 4) >> 2) & 1, half = kHalves == 1 ? 0 : (warp - 4) >> 3;
     const int wq = warp & 3;
@@ -613,10 +613,8 @@ sdpa_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_const
     auto drain_pair = [&](int j) -> bool {
       if (!wait_or_abort(bar(DQ_FULL), j & 1, abort_flag, a.status, 216)) return false;
       tc_fence_after_sync();
-      constexpr int kDq = 32 / kHalves;   // columns of it per thread
-      uint32_t v[kDq];
-      if constexpr (kHalves == 1) tmem_ld32(tm_dq + lane_addr + grp * 32, v);
-      else tmem_ld16(tm_dq + lane_addr + grp * 32 + half * kDq, v);
+      uint32_t v[32];
+      tmem_ld32(tm_dq + lane_addr + grp * 32, v);
       tmem_wait_ld();
       tc_fence_before_sync();
       __syncwarp();
@@ -624,19 +622,19 @@ sdpa_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_const
       // The accumulator is laid out so that one warp-wide reduction covers 512 contiguous bytes: per 128-query tile
       // [column half g][warp w][4-column chunk c][lane][4] holds dq[128 tile + 32 w + lane][32 g + 4 c + 0..3].
       const int64_t tile = int64_t(blockIdx.y) * (a.S / kTile) + ((s_begin + 2 * j) >> 1);
-      float* dst = a.dq_acc + tile * (kTile * D) + ((grp * 4 + wq) * 8 + half * (kDq / 4)) * 128 + lane * 4;
+      float* dst = a.dq_acc + tile * (kTile * D) + (grp * 4 + wq) * 8 * 128 + lane * 4;
 #pragma unroll
-      for (int c = 0; c < kDq / 4; ++c) red_add_v4(dst + c * 128, v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
+      for (int c = 0; c < 8; ++c) red_add_v4(dst + c * 128, v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
       return true;
     };
 
     for (int n = grp; n < n_steps && ok; n += 2) {
       const int s = n & 1;
-      const int st = n % NY;
       const int r0 = (s_begin + n) * kStep + half * kCols;   // first streamed row of this thread's columns
       if constexpr (kMerged) {
-        // group 0 takes pair j before step 2j + 4, group 1 after step 2j + 3: both between the pair's MMAs
-        // (issued after the products of step 2j + 3) and the next pair's (after the products of step 2j + 5)
+        // group 0 takes pair j before step 2j + 4, group 1 after step 2j + 3.  The pair's MMAs follow those that accumulate
+        // step 2j + 1, the next pair's those of step 2j + 3 and both groups' DQ_FREE of this one, whatever the products
+        // (another warp's, up to the ring's depth ahead) have reached.
         if (grp == 0 && n >= 4) {
           ok = drain_pair(next_pair++);
           if (!ok) break;
@@ -709,7 +707,7 @@ sdpa_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_const
         const uint8_t* sl = smem + L::kBias + slot * kBoxBytes;
         if (kKeyMajor) {
           // element (query c, key r): box r / 64, row c, 16-byte chunk ((r % 64) / 8) ^ (c % 8)
-          const uint8_t* colbase = sl + (r >> 6) * kYBoxBytes + half * (kCols * 128) + (r & 7) * 2;
+          const uint8_t* colbase = sl + (r >> 6) * kYBoxBytes + (r & 7) * 2;
           const int chunk = (r & 63) >> 3;
 #pragma unroll
           for (int c = 0; c < kCols / 2; ++c) {
@@ -804,16 +802,18 @@ sdpa_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_const
       }
       const uint32_t tE1 = tm_e + s * kEStage + half * (kDeep ? kCols / 2 : kCols) + lane_addr, tE2 = tE1 + kE2Off;
       if constexpr (kKeyMajor) {
-        if constexpr (kHalves == 1) tmem_st32(tE1, e1);
-        else tmem_st16(tE1, e1);
+        tmem_st32(tE1, e1);
       }
       if constexpr (kMerged) {
-        // ds row of this key: 64 queries = 128 bytes, chunks swizzled as TMA would have written them.  The slot was
-        // last read by MMAs issued before this step's products, and those have completed (PROD_FULL came after).
+        // ds row of this key: 64 queries = 128 bytes, chunks swizzled as TMA would have written them.  The slot's last
+        // readers are the MMAs of step n - 4 and of the pair it belongs to, issued at step n - 3 at the latest.  The wait above
+        // tells that they are done: the commit of step n - 2 covers all that its thread issued before it.  (The ring is
+        // deeper than the slots, so this step's products say nothing about them.)
+        static_assert(kDeep && L::kDsSlots == 4, "the wait for step n - 2 covers the slot of step n - 4");
         uint8_t* dsrow = smem + L::kDs + (n % L::kDsSlots) * kBoxBytes + r * 128;
 #pragma unroll
         for (int c = 0; c < kCols / 8; ++c)
-          *reinterpret_cast<uint4*>(dsrow + (((half * (kCols / 8) + c) ^ (r & 7)) << 4)) = make_uint4(e2[c * 4], e2[c * 4 + 1], e2[c * 4 + 2], e2[c * 4 + 3]);
+          *reinterpret_cast<uint4*>(dsrow + ((c ^ (r & 7)) << 4)) = make_uint4(e2[c * 4], e2[c * 4 + 1], e2[c * 4 + 2], e2[c * 4 + 3]);
         fence_proxy_async_smem();
       } else if constexpr (kHalves == 1) {
         tmem_st32(tE2, e2);
@@ -887,7 +887,7 @@ sdpa_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_const
       const int64_t* os = (kKeyMajor && grp == 0) ? a.o1s : a.o2s;
       uint8_t* orow_ptr = reinterpret_cast<uint8_t*>(outp) + 2 * (b * os[0] + h * os[1] + int64_t(orow) * os[2]);
       constexpr int kOut = (kKeyMajor ? D : D / 2) / kHalves;   // columns per thread
-      const int col0 = kKeyMajor ? half * kOut : (grp * kHalves + half) * kOut;
+      const int col0 = kKeyMajor ? 0 : (grp * kHalves + half) * kOut;
       for (int c = col0; c < col0 + kOut; c += 16) {
         uint32_t o[16];
         if (n_steps > 0) {
@@ -923,7 +923,7 @@ sdpa_bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_x1, const __grid_const
 
 template <int D, bool kBf16, bool kKeyMajor, bool kMerged = false, bool kTiles = true>
 int launch_one(const CUtensorMap* maps, const BwdArgs& a, int n_tiles, int bh_count, cudaStream_t st) {
-  using S = Split<kKeyMajor, kMerged>;
+  using S = Split<kKeyMajor>;
   auto kernel = sdpa_bwd_tc_kernel<D, kBf16, kKeyMajor, kMerged, kTiles>;
   constexpr int kLimit = 232448;  // 227 KB per CTA
   constexpr int kTotal = BwdSmem<D, kMerged, kTiles>::kTotal, smem = kTotal + 1024 <= kLimit ? kTotal + 1024 : kLimit;
