@@ -41,20 +41,6 @@ constexpr int kLaunchRegs = 168;              // what __launch_bounds__(384, 1) 
 static_assert((kLaunchRegs - kProducerRegs) * 128 >= (kWorkerRegs - kLaunchRegs) * 256,
               "worker warps would wait forever for registers the producer warps never release");
 
-#ifdef NB200_PROBE
-// Development aid (not compiled into the library): cycles one element-wise warp spends in each phase of its steps.
-__device__ long long g_probe[32];
-#define PROBE_DECL long long pt_ = clock64(); const bool probe_ = blockIdx.x == 3 && blockIdx.y == 1 && warp == 4 && lane == 0
-#define IPROBE_DECL long long ipt_ = clock64(); const bool iprobe_ = blockIdx.x == 3 && blockIdx.y == 1
-#define IPROBE(i) do { const long long now_ = clock64(); if (iprobe_) g_probe[i] += now_ - ipt_; ipt_ = now_; } while (0)
-#define PROBE(i) do { const long long now_ = clock64(); if (probe_) g_probe[i] += now_ - pt_; pt_ = now_; } while (0)
-#else
-#define PROBE_DECL
-#define PROBE(i)
-#define IPROBE_DECL
-#define IPROBE(i)
-#endif
-
 template <bool kTileBias>
 struct Smem {
   static constexpr int kXBytes = kTile * kD * 2;                // K or V tile
@@ -292,19 +278,14 @@ sdpa_bwd_tc_d128_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
       const uint64_t kdesc = make_smem_desc(sbase + L::kX, 16, 1024);
       const uint64_t vdesc = make_smem_desc(sbase + L::kX + L::kXBytes, 16, 1024);
       const uint64_t wdesc = make_smem_desc_noswizzle(sbase + L::kWeights, 128, 256);
-      IPROBE_DECL;
       for (int n = 0; n < n_steps && ok; ++n) {
         const int st = n % NY, s = n & 1;
-        IPROBE(16);
         ok = wait_or_abort(bar(Y_FULL + st), (n / NY) & 1, abort_flag, a.status, 304);
-        IPROBE(17);
         // One stage per product, each with its own pair of barriers (PROD_FULL / P_FREE + 0, 1: scores; + 2, 3: dP):
         // a product may be overwritten once the warps of step n - 1 hold it in registers, and the warps take the
         // scores of step n -- and start on their exponentials -- while the tensor core still computes its dP.
         if (ok && n >= 1) ok = wait_or_abort(bar(P_FREE + ((n - 1) & 1)), ((n - 1) >> 1) & 1, abort_flag, a.status, 309);
-        IPROBE(18);
         if (ok) ok = wait_or_abort(bar(AUG_FULL + s), (n >> 1) & 1, abort_flag, a.status, 312);
-        IPROBE(19);
         if (!ok) break;
         tc_fence_after_sync();
         const uint32_t ybase = sbase + L::kY + st * L::kYStageBytes;
@@ -321,9 +302,7 @@ sdpa_bwd_tc_d128_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
         if constexpr (kTileBias) {
           // P1[key, q] += bias^T[key, q'] (hi I + lo I)[q', q], 16 queries at a time: A = 16 rows of the slot read
           // MN-major (two 64-key boxes), B = the 16 x 16 scaled identity, D = 16 columns of P1
-          IPROBE(16);
           ok = wait_or_abort(bar(B_FULL + s), (n >> 1) & 1, abort_flag, a.status, 311);
-          IPROBE(20);
           if (!ok) break;
           tc_fence_after_sync();
           const uint64_t adesc = make_smem_desc(sbase + L::kBias + s * kBoxBytes, kYBoxBytes, 1024);
@@ -337,9 +316,7 @@ sdpa_bwd_tc_d128_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
           mma_commit(bar(B_EMPTY + s));
         }
         mma_commit(bar(PROD_FULL + s));
-        IPROBE(16);
         if (n >= 1) ok = wait_or_abort(bar(P_FREE + 2 + ((n - 1) & 1)), ((n - 1) >> 1) & 1, abort_flag, a.status, 319);
-        IPROBE(23);
         if (!ok) break;
         tc_fence_after_sync();
 #pragma unroll
@@ -495,11 +472,8 @@ sdpa_bwd_tc_d128_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
     // dq accumulator of this (batch, head): [query / 4][d][query % 4] floats, so that one warp-wide reduction of
     // four queries covers 512 contiguous bytes (lanes = 32 consecutive d)
 
-    PROBE_DECL;
     auto drain = [&](int j) -> bool {
-      PROBE(0);
       if (!wait_or_abort(bar(DQ_FULL + (j & 1)), (j >> 1) & 1, abort_flag, a.status, 316)) return false;
-      PROBE(10);
       tc_fence_after_sync();
       uint32_t v[kStep];
       tmem_ld32(tm_dq + lane_addr, *reinterpret_cast<uint32_t(*)[32]>(&v[0]));
@@ -508,11 +482,9 @@ sdpa_bwd_tc_d128_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) mbar_arrive(bar(DQ_FREE + (j & 1)));
-      PROBE(11);
       float* dst = a.dq_acc + int64_t(blockIdx.y) * a.acc_rows * kD + r * 4 + int64_t(step_row(j) / 4) * (kD * 4);
 #pragma unroll
       for (int c = 0; c < kStep / 4; ++c) red_add_v4(dst + c * (kD * 4), v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
-      PROBE(12);
       return true;
     };
 
@@ -538,10 +510,8 @@ sdpa_bwd_tc_d128_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
         if (key_dropped) keep[0] = keep[1] = 0u;
       }
 
-      PROBE(1);
       ok = wait_or_abort(bar(PROD_FULL + s), (n >> 1) & 1, abort_flag, a.status, 306);
       if (!ok) break;
-      PROBE(2);
       tc_fence_after_sync();
       // the scores first: p = exp2(t log2e) (they arrive with -lse already added) while dP is still being computed
       float2 t[kStep / 2];
@@ -554,7 +524,6 @@ sdpa_bwd_tc_d128_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
         tc_fence_before_sync();
         __syncwarp();
         if (lane == 0) mbar_arrive(bar(P_FREE + s));
-        PROBE(3);
 #pragma unroll
         for (int i = 0; i < kStep / 2; ++i) t[i] = make_float2(__uint_as_float(raw[2 * i]), __uint_as_float(raw[2 * i + 1]));
       }
@@ -575,19 +544,16 @@ sdpa_bwd_tc_d128_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
         t[c] = make_float2(ex2(x.x), ex2(x.y));
         e1[c] = pack2<kBf16>(t[c].x, t[c].y);
       }
-      PROBE(4);
       // p of this stage is still being read by dV of step n - 2
       if (n >= 2) {
         ok = wait_or_abort(bar(E_FREE + s), ((n - 2) >> 1) & 1, abort_flag, a.status, 310);
         if (!ok) break;
         tc_fence_after_sync();
       }
-      PROBE(5);
       tmem_st32(tm_e + s * 32 + lane_addr, e1);
       // ds = p dP (dP arrives with -delta already added)
       ok = wait_or_abort(bar(PROD_FULL + 2 + s), (n >> 1) & 1, abort_flag, a.status, 318);
       if (!ok) break;
-      PROBE(9);
       // p is in TMEM by now (its store was issued before the wait): dV += p^T dO may start while ds is formed
       tmem_wait_st();
       tc_fence_before_sync();
@@ -608,14 +574,12 @@ sdpa_bwd_tc_d128_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
           e2[c] = pack2<kBf16>(ds.x, ds.y);
         }
       }
-      PROBE(13);
       // the ds^T buffer was last read by the MMAs (and the dbias store) of step n - NDS
       if (n >= NDS) {
         const int m = n - NDS;
         ok = wait_or_abort(bar(DS_FREE + (m & 1)), (m >> 1) & 1, abort_flag, a.status, 317);
         if (!ok) break;
       }
-      PROBE(6);
       {
         const uint32_t tile = sbase + L::kDs + (n % NDS) * kBoxBytes + ds_thread;
         if constexpr (kDbias) {
@@ -634,12 +598,10 @@ sdpa_bwd_tc_d128_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
         }
         fence_proxy_async_smem();
       }
-      PROBE(7);
       tmem_wait_st();
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) mbar_arrive(bar(E_READY + s));
-      PROBE(8);
       // dQ^T of the previous step (the other group's) is complete by now: add it to the accumulator
       if (n >= 1) ok = drain(n - 1);
     }
@@ -803,12 +765,3 @@ int launch_dq_finish_d128(const Problem& pr, const float* acc, int acc_rows, boo
 
 }  // namespace tc
 }  // namespace nb200
-
-#ifdef NB200_PROBE
-extern "C" NB200_API int nb200_debug_probe(long long* out32, int reset) {
-  long long zero[32] = {};
-  if (out32) cudaMemcpyFromSymbol(out32, nb200::tc::g_probe, sizeof(zero));
-  if (reset) cudaMemcpyToSymbol(nb200::tc::g_probe, zero, sizeof(zero));
-  return 0;
-}
-#endif

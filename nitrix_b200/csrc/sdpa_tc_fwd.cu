@@ -64,26 +64,10 @@ struct Split {
   static_assert((kLaunchRegs - kProducerRegs) * 128 >= (kSoftmaxRegs - kLaunchRegs) * 256 * kHalves,
                 "softmax warps would wait forever for registers the producer warps never release");
 };
-#ifndef NB200_POLY_PERIOD
-#define NB200_POLY_PERIOD 4
-#endif
 // D = 128: one pair in this many computes 2^x without the special-function unit, which both query tiles' warps share (every
 // third or second: 994 and 1005 us for 984, B1 H16 L16384 causal with a per-key bias).  None at D = 64 (every 8th or 16th pair
 // 474 and 448 us for 427, B1 H16 L8192).
-constexpr int kPolyPeriod = NB200_POLY_PERIOD;
-#ifdef NB200_PROBE
-// Development aid (not compiled into the library): cycles one softmax warp spends in each phase of its tiles.
-__device__ unsigned long long g_fprobe[16];
-#define FPROBE_DECL long long fpt_ = clock64(); const bool fprobe_ = blockIdx.x == 5 && warp == 4 && lane == 0; unsigned fp_[12] = {}
-#define FPROBE(i) do { const long long now_ = clock64(); fp_[i] += unsigned(now_ - fpt_); fpt_ = now_; } while (0)
-#define FPROBE_FLUSH do { if (fprobe_) for (int i_ = 0; i_ < 12; ++i_) g_fprobe[i_] += fp_[i_]; } while (0)
-#define FPROBE_TILES(n) do { fp_[11] += unsigned(n); } while (0)
-#else
-#define FPROBE_DECL
-#define FPROBE(i)
-#define FPROBE_FLUSH
-#define FPROBE_TILES(n)
-#endif
+constexpr int kPolyPeriod = 4;
 
 template <int D, bool kTileBias>
 struct FwdSmem {
@@ -216,6 +200,7 @@ sdpa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   //   are computed while the softmax warps work on the current one.
   // D = 64 leaves room for separate P tiles, so the next score MMA can run under the current softmax.
   constexpr bool kAlias = D == 128;
+  static_assert(kAlias == (kHalves == 1), "two threads per row where P has columns of its own");
   constexpr int kPoly = kAlias ? kPolyPeriod : 0;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -229,7 +214,7 @@ sdpa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       if (i >= V_EMPTY && i < V_EMPTY + kStages) count = 2;
       if (i >= O_FREE && i < O_FREE + 2) count = 4 * kHalves;                         // one lane per softmax warp of the tile
       if (i >= S_FREE && i < S_FREE + 2) count = 4 * kHalves;
-      if (i >= B_EMPTY && i < B_EMPTY + L::kBiasSlots) count = a.bias_mma ? 1 : (kAlias ? 4 * kHalves : 4);   // MMA issuer or the warps that read it
+      if (i >= B_EMPTY && i < B_EMPTY + L::kBiasSlots) count = a.bias_mma ? 1 : 4;   // MMA issuer or the warps that read it
       if (i >= AUG_FREE && i < AUG_FREE + L::kAugSlots) count = 2;        // one arrival per MMA issuer
       mbar_init(bar(i), count);
     }
@@ -621,6 +606,7 @@ sdpa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     constexpr int kSub = kAlias ? kTile / 2 : kTile;   // keys per pass
     constexpr int kSubs = kTile / kSub;
     constexpr int kCols = kSub / kHalves;              // keys per pass and thread
+    static_assert(kCols == 64, "two mask words, two TMEM loads and one bias slot per pass and thread");
     constexpr int kOutCols = D / kHalves;              // output columns per thread
     const uint32_t tS = tm_S(g) + half * kCols + lane_addr, tO = tm_O(g) + half * kOutCols + lane_addr;
     const uint32_t tP = tm_P(g) + half * (kCols / 2) + lane_addr;
@@ -635,7 +621,6 @@ sdpa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     const float2 scale2 = make_float2(a.scale, a.scale), mul2 = make_float2(mul, mul);
     uint32_t bias_phase = 0;  // bit s = parity of this tile's next wait on its "full" barrier of slot s
     int tc = 0, oc = 0, seq_base = 0;
-    FPROBE_DECL;
 
     // A warp that gives up (`ok` false) waits no more and stores nothing, but walks on through its passes -- nothing in a
     // pass can leave its TMEM or shared memory -- because its partner waits for it at the pair's barrier, which has no time
@@ -658,15 +643,8 @@ sdpa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
 
       uint32_t mnext[kCols / 32];   // keep-bits of this row for the coming pass
       auto load_mask_words = [](const uint32_t* src, uint32_t (&dst)[kCols / 32]) {
-        if constexpr (kCols == 32) {
-          dst[0] = __ldg(src);
-        } else if constexpr (kCols == 128) {
-          const uint4 w = __ldg(reinterpret_cast<const uint4*>(src));
-          dst[0] = w.x; dst[1] = w.y; dst[2] = w.z; dst[3] = w.w;
-        } else {
-          const uint2 w = __ldg(reinterpret_cast<const uint2*>(src));
-          dst[0] = w.x; dst[1] = w.y;
-        }
+        const uint2 w = __ldg(reinterpret_cast<const uint2*>(src));
+        dst[0] = w.x; dst[1] = w.y;
       };
 #pragma unroll
       for (int i = 0; i < kCols / 32; ++i) mnext[i] = 0xffffffffu;
@@ -708,9 +686,7 @@ sdpa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         }
         need_mask = __any_sync(0xffffffffu, need_mask);
 
-        FPROBE(0);
         ok = ok && wait_or_abort(bar(S_FULL + sbar), gt & 1, abort_flag, a.status, 108);
-        FPROBE(1);
         tc_fence_after_sync();
 
         // this thread's scores of the pass: all TMEM loads in flight, one wait; handled as fp32 pairs
@@ -731,29 +707,24 @@ sdpa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
             t[i] = make_float2(__uint_as_float(raw[2 * i]), __uint_as_float(raw[2 * i + 1]));
         }
         // logits: t = s * scale + bias (natural units); with nothing to add the scale is folded into the exponent
-        FPROBE(2);
         if constexpr (kAdd == kAddTile) {
           // slots filled before this (tile, query tile): every live query tile of the earlier key tiles, and
-          // query tile 0 of this one when this is query tile 1.  One slot per 64 keys: of two warps that share rows both
-          // read the pass's slot at D = 128; at D = 64 each has its own and only follows the other's phase.
+          // query tile 0 of this one when this is query tile 1.  One slot per 64 keys; of two threads that share a row each
+          // reads its own and only follows the other's phase.
           const int seq0 = seq_base + 2 * (min(j, it.nt0) + min(j, it.nt1) + ((g == 1 && j < it.nt0) ? 1 : 0));
 #pragma unroll
           for (int hh = 0; hh < kSub / 64; ++hh) {
             const int slot = (seq0 + (kAlias ? hf : hh)) % L::kBiasSlots;
-            if (kAlias || kHalves == 1 || hh == half) {
+            if (kAlias || hh == half) {
               ok = ok && wait_or_abort(bar(B_FULL + g * L::kBiasSlots + slot), (bias_phase >> slot) & 1u, abort_flag, a.status,
                                        109);
               const uint8_t* srow = smem + L::kBias + slot * kBoxBytes + r * 128;
-              const int c0 = kAlias ? half * (kCols / 8) : 0;   // first 16-byte chunk
-              constexpr int kChunks = kCols < 64 ? kCols / 8 : 8;
-              const int t0 = kCols > 64 ? hh * 32 : 0;          // (a compile-time constant: hh is unrolled)
 #pragma unroll
-              for (int c = 0; c < kChunks; ++c) {
-                const uint4 w = *reinterpret_cast<const uint4*>(srow + (((c0 + c) ^ (r & 7)) << 4));
+              for (int c = 0; c < 8; ++c) {
+                const uint4 w = *reinterpret_cast<const uint4*>(srow + ((c ^ (r & 7)) << 4));
                 const uint32_t ww[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
-                for (int e = 0; e < 4; ++e)
-                  t[t0 + c * 4 + e] = __ffma2_rn(t[t0 + c * 4 + e], scale2, unpack2<kBf16>(ww[e]));
+                for (int e = 0; e < 4; ++e) t[c * 4 + e] = __ffma2_rn(t[c * 4 + e], scale2, unpack2<kBf16>(ww[e]));
               }
               __syncwarp();
               if (lane == 0) mbar_arrive(bar(B_EMPTY + slot));
@@ -775,7 +746,6 @@ sdpa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
             for (int i = 0; i < kCols / 2; ++i) t[i] = __fmul2_rn(t[i], scale2);
           }
         }
-        FPROBE(3);
         if (need_mask) {
 #pragma unroll
           for (int i = 0; i < kCols / 2; ++i) {
@@ -783,7 +753,6 @@ sdpa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
             if (!((keep[i >> 4] >> ((2 * i + 1) & 31)) & 1u)) t[i].y = -INFINITY;
           }
         }
-        FPROBE(4);
         // max of these keys: four independent chains of three-input max
         float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
@@ -792,7 +761,7 @@ sdpa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         // The exponentials use a reference max that is only moved when the true max has run more than 2^8 ahead of it (so
         // p <= 256 and the running output is rescaled rarely); l uses the same reference.  Two threads that share a row
         // share it: their warps agree on whether any of their rows moves (one barrier per pass), and exchange values only
-        // if so.  Past the barrier both have read their scores, so P may overwrite them.
+        // if so.
         const bool bump = mx > m + thr;
         float m_use = m;
         bool moved = bump;
@@ -806,7 +775,6 @@ sdpa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
           named_barrier_sync(pair_bar, 64);
           if (half == 0) m_use = *xrow;
         }
-        FPROBE(5);
         const float alpha = m_use > m ? ex2((m - m_use) * mul) : 1.f;
         const float neg = m_use == -INFINITY ? 0.f : -m_use * mul;
         const float2 neg2 = make_float2(neg, neg);
@@ -834,7 +802,6 @@ sdpa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
           ok = ok && wait_or_abort(bar(PV_DONE + g), (2 * gt + hf - 1) & 1, abort_flag, a.status, 112);
           tc_fence_after_sync();
         }
-        FPROBE(6);
         // rescale the running output (this thread's columns) when some row of this warp moved its reference max
         if (rescale) {
 #pragma unroll
@@ -847,25 +814,16 @@ sdpa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
             tmem_st32(tO + c * 32, o);
           }
         }
-        FPROBE(7);
         // P as 16-bit pairs: half as many columns as keys (over its own S buffer when aliased)
-        if constexpr (kCols == 32) {
-          tmem_st16(tP + (kAlias ? hf * kSub : 0), pk);
-        } else {
-#pragma unroll
-          for (int c = 0; c < kCols / 64; ++c)
-            tmem_st32(tP + (kAlias ? hf * kSub : 0) + c * 32, *reinterpret_cast<const uint32_t(*)[32]>(&pk[c * 32]));
-        }
+        tmem_st32(tP + (kAlias ? hf * kSub : 0), pk);
         tmem_wait_st();
         tc_fence_before_sync();
         __syncwarp();
         if (lane == 0) mbar_arrive(bar(P_READY + sbar));
-        FPROBE(8);
         m = m_use;
         }
       }
 
-      FPROBE(9);
       // ---------------- epilogue: out = O / l, lse = m * mul + log2 l ----------------
       if (my_nt > 0) {
         if constexpr (kHalves == 2) {   // l over both halves of the keys
@@ -924,10 +882,7 @@ sdpa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       tc += my_nt;
       oc += my_nt > 0 ? 1 : 0;
       seq_base += 2 * (it.nt0 + it.nt1);
-      FPROBE(10);
-      FPROBE_TILES(my_nt);
     }
-    FPROBE_FLUSH;
   }
 
   // ---------------- teardown ----------------
@@ -997,12 +952,3 @@ int launch_fwd(int D, bool bf16, const CUtensorMap& tq, const CUtensorMap& tk, c
 
 }  // namespace tc
 }  // namespace nb200
-
-#ifdef NB200_PROBE
-extern "C" NB200_API int nb200_debug_fprobe(unsigned long long* out16, int reset) {
-  unsigned long long zero[16] = {};
-  if (out16) cudaMemcpyFromSymbol(out16, nb200::tc::g_fprobe, sizeof(zero));
-  if (reset) cudaMemcpyToSymbol(nb200::tc::g_fprobe, zero, sizeof(zero));
-  return 0;
-}
-#endif
