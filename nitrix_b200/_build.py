@@ -78,10 +78,21 @@ def host_module_path() -> pathlib.Path:
     return LIBDIR / (HOST_MODULE + ".so")
 
 
-def _host_digest() -> str:
+def host_runtime() -> str:
+    """What the host module is built against; kept beside it, so that it can be compared before the module is loaded."""
     import torch
 
-    h = hashlib.sha256(" ".join([*HOST_FLAGS, torch.__version__, sysconfig.get_python_version()]).encode())
+    return f"torch {torch.__version__}, Python {sysconfig.get_python_version()}"
+
+
+def host_module_runtime() -> str:
+    """:func:`host_runtime` at the time the host module was built."""
+    stamp = LIBDIR / "build_host.runtime"
+    return stamp.read_text().strip() if stamp.exists() else "an unknown torch"
+
+
+def _host_digest() -> str:
+    h = hashlib.sha256(" ".join([*HOST_FLAGS, host_runtime()]).encode())
     for f in [HOST_SOURCE, *sorted(INCLUDE.glob("*.h"))]:
         h.update(f.read_bytes())
     return h.hexdigest()
@@ -111,6 +122,7 @@ def _compile_host() -> None:
     if res.returncode != 0:
         raise RuntimeError("host compiler failed:\n" + " ".join(cmd) + "\n" + res.stdout + res.stderr)
     os.replace(tmp, host_module_path())
+    (LIBDIR / "build_host.runtime").write_text(host_runtime() + "\n")
     (LIBDIR / "build_host.sha256").write_text(_host_digest() + "\n")
 
 
@@ -158,8 +170,6 @@ def build(force: bool = False, verbose: bool = False) -> pathlib.Path:
             stamp.write_text(want + "\n")
             if verbose:
                 print(f"==== {src.name}\n{log}")
-        if host is not None:
-            host.result()
     tmp = LIBDIR / (LIBNAME + ".tmp")
     cmd = [nvcc, *LINK_FLAGS, "-o", str(tmp), *map(str, objs)]
     res = subprocess.run(cmd, capture_output=True, text=True)
@@ -167,6 +177,8 @@ def build(force: bool = False, verbose: bool = False) -> pathlib.Path:
         raise RuntimeError("nvcc link failed:\n" + " ".join(cmd) + "\n" + res.stdout + res.stderr)
     os.replace(tmp, lib_path())
     (LIBDIR / "build.sha256").write_text(_digest() + "\n")
+    if host is not None:
+        host.result()   # (after the library, which does without the module)
     return lib_path()
 
 

@@ -174,16 +174,15 @@ def torch_ops():
     import importlib.machinery
     import importlib.util
 
-    import torch
-
     path = _build.host_module_path()
     if not path.exists():
         raise NativeLibraryError(f"{path} is missing: build it with `python -m nitrix_b200._build`.")
+    # before it is loaded: a module built against another torch fails on a symbol, or worse
+    if _build.host_module_runtime() != _build.host_runtime():
+        raise NativeLibraryError(f"{path} was built for {_build.host_module_runtime()}, this is {_build.host_runtime()}: build it anew")
     loader = importlib.machinery.ExtensionFileLoader(_build.HOST_MODULE, str(path))
     module = importlib.util.module_from_spec(importlib.util.spec_from_loader(_build.HOST_MODULE, loader))
     loader.exec_module(module)
-    if module.torch_version != torch.__version__.split("+")[0]:
-        raise NativeLibraryError(f"{path} was built for torch {module.torch_version}, this is {torch.__version__}: build it anew")
     L = lib()
     module.bind({name: C.cast(getattr(L, name), C.c_void_p).value for name in module.entry_points()})
     return module

@@ -14,7 +14,6 @@
 #include <torch/csrc/autograd/grad_mode.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/utils/pybind.h>
-#include <torch/version.h>
 
 #include "nitrix_b200_attention.h"
 #include "nitrix_b200_norm.h"
@@ -539,7 +538,6 @@ Tensor selective_scan(const Tensor& x, const Tensor& delta, const Tensor& A, con
 }  // namespace
 
 PYBIND11_MODULE(_torch_ops, m) {
-  m.attr("torch_version") = TORCH_VERSION;
   m.def("entry_points", &entry_points);
   m.def("bind", &bind);
   // (torch's wrapper: its exception types, and no interpreter lock while the library is called)

@@ -501,3 +501,36 @@ def test_jax_scan_ffi_layer_is_complete_and_consistent():
         assert name in header, name
     ck, ws = J.scratch_bytes(8, 1024, 2048, 16, "bfloat16")
     assert ck == 8 * 128 * 2048 * 16 * 4 and ws >= 2 * 8 * 1024 * 16 * 4
+
+
+def test_a_host_module_of_another_torch_is_refused_before_it_is_loaded(monkeypatch, tmp_path):
+    from nitrix_b200 import _build, _cabi
+
+    monkeypatch.setattr(_build, "LIBDIR", tmp_path)
+    load = _cabi.torch_ops.__wrapped__
+    with pytest.raises(_cabi.NativeLibraryError, match="is missing"):
+        load()
+    _build.host_module_path().write_bytes(b"no module at all")
+    for stamp, named in ((None, "an unknown torch"), ("torch 1.2.3, Python 3.12", "torch 1.2.3")):
+        if stamp:
+            (tmp_path / "build_host.runtime").write_text(stamp + "\n")
+        with pytest.raises(_cabi.NativeLibraryError, match=named):
+            load()
+    # a pre-release is compared whole with what it was built against
+    monkeypatch.setattr(torch, "__version__", "9.0.0.dev20300101+cu999")
+    (tmp_path / "build_host.runtime").write_text(_build.host_runtime() + "\n")
+    with pytest.raises(ImportError):
+        load()
+
+
+def test_the_library_is_linked_where_the_host_module_does_not_compile(monkeypatch, tmp_path):
+    from nitrix_b200 import _build
+
+    (tmp_path / "one.cu").write_text('extern "C" __attribute__((visibility("default"))) int one() { return 1; }\n')
+    (tmp_path / "host.cpp").write_text("#error not today\n")
+    for name, at in (("CSRC", tmp_path), ("LIBDIR", tmp_path / "lib"), ("OBJDIR", tmp_path / "lib" / "obj"),
+                     ("HOST_SOURCE", tmp_path / "host.cpp")):
+        monkeypatch.setattr(_build, name, at)
+    with pytest.raises(RuntimeError, match="host compiler failed"):
+        _build.build()
+    assert C.CDLL(str(_build.lib_path())).one() == 1
