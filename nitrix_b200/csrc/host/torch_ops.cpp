@@ -72,6 +72,12 @@ bool has_expanded_axis(const Tensor& t) {
   return false;
 }
 
+// There are no forward-mode rules.  (torch's own refusal for C++ functions is a RuntimeError, after the kernels have run.)
+void refuse_tangents(const char* what, std::initializer_list<MaybeTensor> operands) {
+  for (const MaybeTensor& t : operands)
+    TORCH_CHECK_NOT_IMPLEMENTED(!t || !t->defined() || !t->_fw_grad(0).defined(), what, ": forward-mode differentiation is not implemented");
+}
+
 Tensor dense_like(const Tensor& t) { return at::empty(t.sizes(), t.options()); }
 
 void copy_strides(int64_t (&dst)[4], const Tensor& t) {
@@ -300,6 +306,7 @@ AttentionResult attention(const Tensor& q, const Tensor& k, const Tensor& v, con
   }
   if (c10::GradMode::is_enabled() &&
       (q.requires_grad() || k.requires_grad() || v.requires_grad() || (bias && bias->requires_grad()))) {
+    refuse_tangents("scaled_dot_product_attention", {q, k, v, bias});
     tensor_list r = AttentionRule::apply(q, k, v, bias, mask, scale, causal, kernel, family == NB200_KERNEL_TCGEN05);
     return {r[0], r[1], true};
   }
@@ -357,6 +364,7 @@ bool qk_norm_fits(const Tensor& q, const Tensor& k) {
 
 std::tuple<Tensor, Tensor> qk_norm(const Tensor& q, const Tensor& k) {
   const c10::cuda::CUDAGuard guard(q.device());
+  refuse_tangents("qk_rms_norm", {q, k});
   const tensor_list r = QkNormRule::apply(q, k);
   return {r[0], r[1]};
 }
@@ -431,6 +439,7 @@ struct LayerNormRule : torch::autograd::Function<LayerNormRule> {
 
 Tensor layer_norm(const Tensor& x, const MaybeTensor& weight, const MaybeTensor& bias, double eps, double out_scale) {
   const c10::cuda::CUDAGuard guard(x.device());
+  refuse_tangents("layer_norm", {x, weight, bias});
   return LayerNormRule::apply(x, weight, bias, eps, out_scale);
 }
 
@@ -527,6 +536,7 @@ struct ScanRule : torch::autograd::Function<ScanRule> {
 
 Tensor selective_scan(const Tensor& x, const Tensor& delta, const Tensor& A, const Tensor& B, const Tensor& C, const MaybeTensor& D) {
   const c10::cuda::CUDAGuard guard(x.device());
+  refuse_tangents("selective_scan", {x, delta, A, B, C, D});
   bool differentiate = false;
   if (c10::GradMode::is_enabled()) {
     for (const Tensor* t : {&x, &delta, &A, &B, &C}) differentiate = differentiate || t->requires_grad();

@@ -101,3 +101,12 @@ def test_packed_masks_keep_the_layout_they_were_packed_from(D, S, T, expand):
     assert any(t.shape == mask.shape and t.is_contiguous() for t in restored if t.dtype in (torch.bool, torch.uint8))
     for a, b in zip(got, want):   # (fp32 sums of dq added in any order, then rounded to bf16)
         assert float((a.float() - b.float()).norm()) <= 1e-2 * float(b.float().norm())
+
+
+@pytest.mark.parametrize("op", _OPS)
+def test_forward_mode_is_not_implemented(op):
+    # (the class that a Python autograd function without a jvp raises, whichever operand has the tangent)
+    leaves, fn = _OPS[op]()
+    for i in range(len(leaves)):
+        with pytest.raises(NotImplementedError), torch.autograd.forward_ad.dual_level():
+            fn(*(torch.autograd.forward_ad.make_dual(t, torch.ones_like(t)) if j == i else t for j, t in enumerate(leaves)))
