@@ -73,9 +73,11 @@ bool has_expanded_axis(const Tensor& t) {
 }
 
 // There are no forward-mode rules.  (torch's own refusal for C++ functions is a RuntimeError, after the kernels have run.)
-void refuse_tangents(const char* what, std::initializer_list<MaybeTensor> operands) {
-  for (const MaybeTensor& t : operands)
-    TORCH_CHECK_NOT_IMPLEMENTED(!t || !t->defined() || !t->_fw_grad(0).defined(), what, ": forward-mode differentiation is not implemented");
+bool has_tangent(const Tensor& t) { return t._fw_grad(0).defined(); }
+bool has_tangent(const MaybeTensor& t) { return t && has_tangent(*t); }
+template <typename... T>
+void refuse_tangents(const char* what, const T&... operands) {
+  TORCH_CHECK_NOT_IMPLEMENTED(!(has_tangent(operands) || ...), what, ": forward-mode differentiation is not implemented");
 }
 
 Tensor dense_like(const Tensor& t) { return at::empty(t.sizes(), t.options()); }
@@ -306,7 +308,7 @@ AttentionResult attention(const Tensor& q, const Tensor& k, const Tensor& v, con
   }
   if (c10::GradMode::is_enabled() &&
       (q.requires_grad() || k.requires_grad() || v.requires_grad() || (bias && bias->requires_grad()))) {
-    refuse_tangents("scaled_dot_product_attention", {q, k, v, bias});
+    refuse_tangents("scaled_dot_product_attention", q, k, v, bias);
     tensor_list r = AttentionRule::apply(q, k, v, bias, mask, scale, causal, kernel, family == NB200_KERNEL_TCGEN05);
     return {r[0], r[1], true};
   }
@@ -364,7 +366,7 @@ bool qk_norm_fits(const Tensor& q, const Tensor& k) {
 
 std::tuple<Tensor, Tensor> qk_norm(const Tensor& q, const Tensor& k) {
   const c10::cuda::CUDAGuard guard(q.device());
-  refuse_tangents("qk_rms_norm", {q, k});
+  refuse_tangents("qk_rms_norm", q, k);
   const tensor_list r = QkNormRule::apply(q, k);
   return {r[0], r[1]};
 }
@@ -439,7 +441,7 @@ struct LayerNormRule : torch::autograd::Function<LayerNormRule> {
 
 Tensor layer_norm(const Tensor& x, const MaybeTensor& weight, const MaybeTensor& bias, double eps, double out_scale) {
   const c10::cuda::CUDAGuard guard(x.device());
-  refuse_tangents("layer_norm", {x, weight, bias});
+  refuse_tangents("layer_norm", x, weight, bias);
   return LayerNormRule::apply(x, weight, bias, eps, out_scale);
 }
 
@@ -474,7 +476,7 @@ Tensor sum_to_operand(const Tensor& g3, at::IntArrayRef lead, at::IntArrayRef sh
 PyObject* scan_allocator = nullptr;
 Tensor scan_workspace(nb200_selective_scan_params& p, const Tensor& like) {   // (fills in p's workspace)
   py::gil_scoped_acquire gil;
-  return py::reinterpret_borrow<py::object>(scan_allocator)(reinterpret_cast<uintptr_t>(&p), like).cast<Tensor>();
+  return py::reinterpret_borrow<py::object>(scan_allocator)(reinterpret_cast<uintptr_t>(&p), int(like.device().index())).cast<Tensor>();
 }
 
 // Saves the operands and the forward's checkpoints.
@@ -536,7 +538,7 @@ struct ScanRule : torch::autograd::Function<ScanRule> {
 
 Tensor selective_scan(const Tensor& x, const Tensor& delta, const Tensor& A, const Tensor& B, const Tensor& C, const MaybeTensor& D) {
   const c10::cuda::CUDAGuard guard(x.device());
-  refuse_tangents("selective_scan", {x, delta, A, B, C, D});
+  refuse_tangents("selective_scan", x, delta, A, B, C, D);
   bool differentiate = false;
   if (c10::GradMode::is_enabled()) {
     for (const Tensor* t : {&x, &delta, &A, &B, &C}) differentiate = differentiate || t->requires_grad();

@@ -94,8 +94,9 @@ def _workspace(p, device) -> torch.Tensor:
 @functools.lru_cache(maxsize=1)
 def _ops():
     ops = _cabi.torch_ops()
+    params_at = _cabi.SelectiveScanParams.from_address
     # (the module's _workspace at the time of the call, not the one there was at the first)
-    ops.set_scan_allocator(lambda address, like: _workspace(_cabi.SelectiveScanParams.from_address(address), like.device))
+    ops.set_scan_allocator(lambda address, device_index: _workspace(params_at(address), device_index))
     return ops
 
 
