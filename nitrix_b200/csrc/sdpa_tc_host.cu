@@ -122,11 +122,15 @@ __device__ __forceinline__ uint32_t join_bits(uint32_t bits, int lane) {
 // before.  Bound: HBM, the mask once.  32 x 32 tiles of single bytes, or 256 x 256 tiles with a ballot per bit for lengths
 // that are multiples of 256, and a memset took (12, 1, 1216, 1216) with the transposed words 58 us, now 7.4; (4, 1, 7424,
 // 7424) 108 -> 68, without them 46 -> 47; (3, 1, 1217, 1331) without 15 -> 7; (2, 2, 256, 256) with 7.6 -> 3.1.
-template <int kKeys>
+// kNarrow: up to 32 keys, one word, 64 x 32 tiles: a lane takes one row's eight keys, where four lanes of a warp would take
+// those of eight rows one by one ((1, 8, 3974, 12) with the transposed words 11.2 -> 4.5 us, (4, 16, 1024, 31) 16.8 ->
+// 6.5).
+template <int kKeys, bool kNarrow>
 __global__ void __launch_bounds__(256) mask_pack_kernel(const uint8_t* mask, int64_t sb, int64_t sh, int64_t ss, int64_t st,
                                                         int Hm, int S, int T, uint32_t* rows_out, int words_per_row,
                                                         uint32_t* cols_out, int words_per_col) {
-  constexpr int kLaneKeys = kKeys == 16 ? 16 : 8, kRowLanes = 256 / kLaneKeys, kLoads = 8 * kRowLanes / 32;
+  static_assert(!kNarrow || kKeys != 16, "a load per lane");
+  constexpr int kLaneKeys = kKeys == 16 ? 16 : 8, kRowLanes = (kNarrow ? 32 : 256) / kLaneKeys, kLoads = 8 * kRowLanes / 32;
   __shared__ uint32_t sw[64][9];   // [row][key word], padded against bank conflicts
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int bm = blockIdx.z / Hm, hm = blockIdx.z - bm * Hm;
@@ -135,22 +139,32 @@ __global__ void __launch_bounds__(256) mask_pack_kernel(const uint8_t* mask, int
   const int rl0 = warp * 8 + lane / kRowLanes;   // first row of this lane; the next ones 32 / kRowLanes further
   const uint8_t* base = mask + bm * sb + hm * sh + key * st;
   uint32_t bits[kLoads];
+  if (row0 + warp * 8 < S) {
 #pragma unroll
-  for (int i = 0; i < kLoads; ++i) {
-    const int row = row0 + rl0 + i * (32 / kRowLanes);
-    bits[i] = keep_bits<kKeys>(base + int64_t(row) * ss, mask, st, row < S ? T - key : 0);
+    for (int i = 0; i < kLoads; ++i) {
+      const int row = row0 + rl0 + i * (32 / kRowLanes);
+      bits[i] = keep_bits<kKeys>(base + int64_t(row) * ss, mask, st, row < S ? T - key : 0);
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < kLoads; ++i) bits[i] = 0u;
   }
 #pragma unroll
   for (int i = 0; i < kLoads; ++i) {
     const int rl = rl0 + i * (32 / kRowLanes);
     const uint32_t w = join_bits<kKeys>(bits[i], lane);
-    if ((kl & 31) == 0) {
+    if constexpr (kNarrow) {
+      // (a row is four words, three of them padding: its four lanes write one each)
+      if ((lane & 3) == 0) sw[rl][0] = w;
+      if (row0 + rl < S) rows_out[(int64_t(blockIdx.z) * S + row0 + rl) * words_per_row + (lane & 3)] = (lane & 3) ? 0u : w;
+    } else if ((kl & 31) == 0) {
       sw[rl][kl >> 5] = w;
       if (row0 + rl < S && (key >> 5) < words_per_row) rows_out[(int64_t(blockIdx.z) * S + row0 + rl) * words_per_row + (key >> 5)] = w;
     }
   }
   if (!cols_out) return;
   __syncthreads();
+  if (kNarrow && warp > 0) return;
   uint32_t x[2] = {sw[lane][warp], sw[32 + lane][warp]};   // lane = row
 #pragma unroll
   for (int m = 16; m; m >>= 1) {
@@ -479,7 +493,8 @@ int launch_mask_pack(const Problem& pr, const MaskPackPlan& plan, void* ws, Mask
     kernel<<<Bm * Hm, 32 * (warps < 32 ? warps : 32), 0, stream>>>(mask, pr.ms[0], pr.ms[1], pr.ms[3], Hm, pr.T, rows,
                                                                    plan.words_per_row, kv_len);
   } else {
-    auto kernel = whole(16) ? mask_pack_kernel<16> : (whole(8) ? mask_pack_kernel<8> : mask_pack_kernel<1>);
+    auto kernel = pr.T <= 32 ? (whole(8) ? mask_pack_kernel<8, true> : mask_pack_kernel<1, true>)
+                  : whole(16) ? mask_pack_kernel<16, false> : (whole(8) ? mask_pack_kernel<8, false> : mask_pack_kernel<1, false>);
     // (with the transposed copy: all of its words, a multiple of 4 per key)
     const dim3 grid((pr.T + 255) / 256, cols ? plan.words_per_col / 2 : (pr.S + 63) / 64, Bm * Hm);
     kernel<<<grid, 256, 0, stream>>>(mask, pr.ms[0], pr.ms[1], pr.ms[2], pr.ms[3], Hm, pr.S, pr.T, rows, plan.words_per_row,

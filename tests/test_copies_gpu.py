@@ -90,6 +90,12 @@ def test_packed_mask_bits(S, T, layout):
     assert torch.equal(blob[at:at + cols.numel() * 4].view(torch.int32).reshape(cols.shape), cols)
 
 
+@pytest.mark.parametrize("layout", ["dense", "rows_of_8", "odd_start", "key_strided"])
+@pytest.mark.parametrize("S,T", [(64, 32), (65, 24), (9, 8), (130, 7), (200, 33), (9, 100)])
+def test_packed_mask_bits_of_narrow_masks_and_of_warps_without_rows(S, T, layout):
+    test_packed_mask_bits(S, T, layout)
+
+
 @pytest.mark.parametrize("T", [1, 31, 256, 257, 1000, 8200])
 def test_packed_key_mask_bits_and_kept_lengths(T):
     from nitrix_b200.nn.attention import pack_mask
