@@ -14,7 +14,7 @@
 // shared over the batch, batch-fastest so concurrent CTAs hit the same bias
 // tiles in L2.  Twelve warps at D = 128, twenty at D = 64:
 //   warp 0      TMA producer for Q (per item) and the K / V rings
-//   warp 1      TMA producer for the bias ring (128 x 64 slots)
+//   warp 1      TMA producer for the bias ring (128 x 64 slots); without one, per-key addends and, at D = 64, mask words
 //   warp 2      issues tcgen05.mma for query tile 0 (one elected lane)
 //   warp 3      issues tcgen05.mma for query tile 1; owns the TMEM allocation
 //   warps 4-7   softmax of query tile 0, warps 8-11 that of query tile 1: one row per thread at D = 128, at D = 64 the
@@ -69,7 +69,7 @@ struct Split {
 // 474 and 448 us for 427, B1 H16 L8192).
 constexpr int kPolyPeriod = 4;
 
-template <int D, bool kTileBias>
+template <int D, bool kTileBias, bool kStagedMask>
 struct FwdSmem {
   static constexpr int kTileBytes = kTile * D * 2;        // one Q / K / V tile
   // K and V ring depth.  A TMA tile takes 1-2 us from L2 / HBM while a key tile is consumed in well under
@@ -91,11 +91,16 @@ struct FwdSmem {
   // no swizzle, 4 KB) and a ring of three 128-key x 16 tiles (4 KB each).
   static constexpr int kAugSlots = 3;
   static constexpr int kAugTileBytes = (kTile / 8) * 256;
-  static constexpr int kNumBars = 4 + 4 * kStages + 16 + 3 * kBiasSlots + 2 * kAugSlots;
+  static constexpr int kMaskSlots = kStagedMask ? 3 : 0;   // kStagedMask: per query tile (mask_full[2][slots] mask_empty[2][slots])
+  static constexpr int kNumBars = 4 + 4 * kStages + 16 + 3 * kBiasSlots + 2 * kAugSlots + 4 * kMaskSlots;
   static constexpr int kMisc = kBars + 8 * kNumBars;      // tmem base (4 B) + abort flag (4 B)
   static constexpr int kOrder = kMisc + 16;               // batch indices by kept length (item order 3), 16-bit each
   static constexpr int kExchange = kOrder + 2 * kMaxOrder;   // one fp32 per query row of both tiles
-  static constexpr int kTotal = kExchange + 2 * kTile * 4;
+  // the keep words of a pass, 16 bytes per query row
+  static constexpr int kMaskSlotBytes = kTile * 16;
+  static constexpr int kMaskWords = (kExchange + 2 * kTile * 4 + 15) / 16 * 16;
+  static_assert(kMaskWords % 16 == 0 && kMaskSlotBytes % 16 == 0, "copied in words of 16 bytes");
+  static constexpr int kTotal = kMaskWords + 2 * kMaskSlots * kMaskSlotBytes;
 };
 
 // One work item: two query tiles of one (batch, head).
@@ -170,12 +175,18 @@ __device__ __forceinline__ Item decode_item(const FwdArgs& a, int item, const ui
 // loop neither tests for the others at every pass nor holds registers for them.
 enum SoftmaxAdd : int { kAddNone = 0, kAddTile = 1, kAddAny = 2 };
 
-template <int D, bool kBf16, bool kTileBias, int kAdd>
+// kMasked: the softmax warps apply a mask (every one of the instances that are not compiled apart for it is).  Two threads per row
+// have no registers for words fetched a pass ahead (spilled, such a load is waited for on the spot), and 16 warps that fetch
+// 8 bytes of 32 rows each keep the load units busy.  So the warp that has no bias tiles to fetch copies them, 16 bytes per row
+// and pass, to a ring in shared memory: (4, 8, 2048, 2048, 64) with a mask of 80 % of the keys 100 us with words in registers,
+// 90 now, one that keeps all 92, 78, no mask 74, 72.5.
+template <int D, bool kBf16, bool kTileBias, int kAdd, bool kMasked>
 __global__ void __launch_bounds__(Split<D>::kThreads, 1)
 sdpa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                    const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_bias,
                    const FwdArgs a) {
-  using L = FwdSmem<D, kTileBias>;
+  constexpr bool kStagedMask = kMasked && Split<D>::kHalves == 2 && !kTileBias;
+  using L = FwdSmem<D, kTileBias, kStagedMask>;
   constexpr int kStages = L::kStages;
   constexpr int kThreads = Split<D>::kThreads, kHalves = Split<D>::kHalves;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -194,7 +205,8 @@ sdpa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   constexpr int Q_FULL = 0, Q_EMPTY = 2, K_FULL = 4, K_EMPTY = K_FULL + kStages, V_FULL = K_EMPTY + kStages,
                 V_EMPTY = V_FULL + kStages, S_FULL = V_EMPTY + kStages, P_READY = S_FULL + 4, O_DONE = P_READY + 4,
                 O_FREE = O_DONE + 2, S_FREE = O_FREE + 2, PV_DONE = S_FREE + 2, B_FULL = PV_DONE + 2,
-                B_EMPTY = B_FULL + 2 * L::kBiasSlots, AUG_FULL = B_EMPTY + L::kBiasSlots, AUG_FREE = AUG_FULL + L::kAugSlots;
+                B_EMPTY = B_FULL + 2 * L::kBiasSlots, AUG_FULL = B_EMPTY + L::kBiasSlots, AUG_FREE = AUG_FULL + L::kAugSlots,
+                M_FULL = AUG_FREE + L::kAugSlots, M_EMPTY = M_FULL + 2 * L::kMaskSlots;
   // D = 128 fills TMEM (2 x 128 S + 2 x 128 O), so P must overwrite S: a key tile is taken as two halves of 64
   //   keys, each with its own 64-column S buffer and P written over that buffer, and the scores of the next half
   //   are computed while the softmax warps work on the current one.
@@ -216,6 +228,8 @@ sdpa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       if (i >= S_FREE && i < S_FREE + 2) count = 4 * kHalves;
       if (i >= B_EMPTY && i < B_EMPTY + L::kBiasSlots) count = a.bias_mma ? 1 : 4;   // MMA issuer or the warps that read it
       if (i >= AUG_FREE && i < AUG_FREE + L::kAugSlots) count = 2;        // one arrival per MMA issuer
+      if (i >= M_FULL && i < M_EMPTY) count = 32;                         // every lane of the warp that copies
+      if (i >= M_EMPTY && i < M_EMPTY + 2 * L::kMaskSlots) count = 4 * kHalves;
       mbar_init(bar(i), count);
     }
     *abort_flag = 0;
@@ -323,13 +337,56 @@ sdpa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       }
     }
   } else if (warp == 1) {
-    // ---------------- bias producer ----------------
+    // ---------------- bias and mask producer ----------------
     if constexpr (!kTileBias) {
-      if (a.key_mma) {
+      if (kStagedMask || a.key_mma) {
         // per-key addends of each streamed key tile as an MMA operand: lane -> keys lane, lane + 32, ...
         const float inv_scale = 1.f / a.scale;
         int kv = 0;
+        int mc[2] = {0, 0};   // tiles that query tile g has had before this item
         bool ok = true;
+        // The keep words of key tile j for both query tiles: lane -> rows lane, lane + 32, ...  An item's first tiles go through
+        // registers, all loads in flight, which is the sooner there (4 key tiles of (30, 2, 433, 433, 64) 18.9 us, with copies
+        // alone 22.7); the others by copies that arrive by themselves and leave L1 to the softmax warps' spilled registers
+        // (16 key tiles of (4, 8, 2048, 2048, 64) 78.2 us, with loads alone 81.7).
+        auto copy_mask_words = [&](const Item& it, int j) {
+          if constexpr (kStagedMask) {
+            const uint32_t* rows = a.mask.rows + it.b * a.mask.b_stride + it.h * a.mask.h_stride + j * 4;
+            auto row = [&](int g, int i) { return rows + int64_t(min(it.q0 + g * kTile + lane + 32 * i, a.S - 1)) * a.mask.row_stride; };
+            auto slot = [&](int g) { return g * L::kMaskSlots + (mc[g] + j) % L::kMaskSlots; };
+            auto address = [&](int g, int i) { return sbase + L::kMaskWords + slot(g) * L::kMaskSlotBytes + (lane + 32 * i) * 16; };
+#pragma unroll
+            for (int g = 0; g < 2; ++g) {
+              const int n = mc[g] + j;
+              if (j < it.nt(g) && n >= L::kMaskSlots && ok)   // (a warp that gives up leaves its loops together)
+                ok = __all_sync(0xffffffffu, wait_or_abort(bar(M_EMPTY + slot(g)), (n / L::kMaskSlots - 1) & 1, abort_flag, a.status, 119));
+            }
+            if (!ok) return;
+            if (j < L::kMaskSlots) {
+              uint4 w[2][4];
+#pragma unroll
+              for (int g = 0; g < 2; ++g)
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                  if (j < it.nt(g)) w[g][i] = ldg_no_allocate(reinterpret_cast<const uint4*>(row(g, i)));
+#pragma unroll
+              for (int g = 0; g < 2; ++g) {
+                if (j >= it.nt(g)) continue;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) st_shared_v4(address(g, i), w[g][i]);
+                mbar_arrive(bar(M_FULL + slot(g)));
+              }
+            } else {
+#pragma unroll
+              for (int g = 0; g < 2; ++g) {
+                if (j >= it.nt(g)) continue;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) cp_async16(address(g, i), row(g, i));
+                cp_async_arrive(bar(M_FULL + slot(g)));
+              }
+            }
+          }
+        };
         for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
           const Item it = decode_item(a, item, order);
           const uint16_t* bk = a.bias_mode == kBiasKey
@@ -337,9 +394,12 @@ sdpa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                                    : nullptr;
           const uint32_t* mk = a.mask.kv_len ? a.mask.rows + it.b * a.mask.b_stride + it.h * a.mask.h_stride : nullptr;
           for (int j = 0; j < it.nt_max && ok; ++j, ++kv) {
+            copy_mask_words(it, j);
+            if (!ok) break;
+            if (!a.key_mma) continue;
             const int slot = kv % L::kAugSlots;
             if (kv >= L::kAugSlots)
-              ok = wait_or_abort(bar(AUG_FREE + slot), ((kv / L::kAugSlots) - 1) & 1, abort_flag, a.status, 117);
+              ok = __all_sync(0xffffffffu, wait_or_abort(bar(AUG_FREE + slot), ((kv / L::kAugSlots) - 1) & 1, abort_flag, a.status, 117));
             if (!ok) break;
             uint8_t* ctile = smem + L::kBias + L::kAugTileBytes * (1 + slot);
 #pragma unroll
@@ -378,7 +438,10 @@ sdpa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
             __syncwarp();
             if (lane == 0) mbar_arrive(bar(AUG_FULL + slot));
           }
+          mc[0] += it.nt0;
+          mc[1] += it.nt1;
         }
+        if (kStagedMask) cp_async_wait_all();   // (in flight still only where the softmax warps gave up)
       }
     }
     if (a.bias_mode == kBiasTile && elect_one()) {
@@ -633,7 +696,7 @@ sdpa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       float m = -INFINITY, l = 0.f;  // m: reference max in logit units (see the lazy rescale below); l: this thread's keys
 
       const uint32_t* mrow = nullptr;
-      if (a.mask.rows && !(key_mma && a.mask.kv_len)) {   // a key-only mask was added to the scores as -inf
+      if (kMasked && !kStagedMask && a.mask.rows && !(key_mma && a.mask.kv_len)) {   // a key-only mask was added to the scores as -inf
         mrow = a.mask.rows + b * a.mask.b_stride + h * a.mask.h_stride + int64_t(min(row, a.S - 1)) * a.mask.row_stride +
                half * (kCols / 32);
       }
@@ -648,7 +711,7 @@ sdpa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       };
 #pragma unroll
       for (int i = 0; i < kCols / 32; ++i) mnext[i] = 0xffffffffu;
-      if (mrow && my_nt > 0) load_mask_words(mrow, mnext);
+      if (!kStagedMask && mrow && my_nt > 0) load_mask_words(mrow, mnext);
       for (int j = 0; j < my_nt; ++j) {
         const int gt = tc + j;   // this tile's running index for this query tile
 #pragma unroll 1
@@ -662,7 +725,15 @@ sdpa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
 #pragma unroll
         for (int i = 0; i < kCols / 32; ++i) keep[i] = 0xffffffffu;
         bool need_mask = false;
-        if (mrow) {
+        if constexpr (kStagedMask) {
+          const int slot = g * L::kMaskSlots + gt % L::kMaskSlots;
+          ok = ok && wait_or_abort(bar(M_FULL + slot), (gt / L::kMaskSlots) & 1, abort_flag, a.status, 120);
+          const uint2 w = *reinterpret_cast<const uint2*>(smem + L::kMaskWords + slot * L::kMaskSlotBytes + r * 16 + half * 8);
+          keep[0] = w.x; keep[1] = w.y;
+          __syncwarp();
+          if (lane == 0) mbar_arrive(bar(M_EMPTY + slot));
+          need_mask = (keep[0] & keep[1]) != 0xffffffffu;
+        } else if (mrow) {
           // this pass's words were fetched a pass ago; the next pass's fetch runs under this pass's arithmetic
           uint32_t all = 0xffffffffu;
 #pragma unroll
@@ -895,11 +966,11 @@ sdpa_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   }
 }
 
-template <int D, bool kBf16, bool kTileBias, int kAdd>
+template <int D, bool kBf16, bool kTileBias, int kAdd, bool kMasked = true>
 int launch_one(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tb,
                FwdArgs a, cudaStream_t st) {
-  auto kernel = sdpa_fwd_tc_kernel<D, kBf16, kTileBias, kAdd>;
-  using L = FwdSmem<D, kTileBias>;
+  auto kernel = sdpa_fwd_tc_kernel<D, kBf16, kTileBias, kAdd, kMasked>;
+  using L = FwdSmem<D, kTileBias, kMasked && Split<D>::kHalves == 2 && !kTileBias>;
   static_assert(kMaxOrder <= Split<D>::kThreads, "a thread per ranked batch element");
   // (with bias tiles at head dim 64 the room left for rounding the base up is 840 bytes; the driver's base needs none)
   constexpr int kLimit = 232448;  // 227 KB per CTA
@@ -943,8 +1014,13 @@ int launch_fwd(int D, bool bf16, const CUtensorMap& tq, const CUtensorMap& tk, c
   auto go = [&](auto of) { return bf16 ? of(std::true_type()) : of(std::false_type()); };
   if (D == 64 && tiles && add == kAddNone) return go([&](auto t) { return launch_one<64, t.value, true, kAddNone>(tq, tk, tv, tb, a, st); });
   if (D == 64 && tiles) return go([&](auto t) { return launch_one<64, t.value, true, kAddTile>(tq, tk, tv, tb, a, st); });
-  if (D == 64 && add == kAddNone) return go([&](auto t) { return launch_one<64, t.value, false, kAddNone>(tq, tk, tv, tb, a, st); });
-  if (D == 64) return go([&](auto t) { return launch_one<64, t.value, false, kAddAny>(tq, tk, tv, tb, a, st); });
+  const bool masked = a.mask.rows && !(a.key_mma && a.mask.kv_len);   // by the softmax warps
+  if (D == 64 && add == kAddNone)
+    return masked ? go([&](auto t) { return launch_one<64, t.value, false, kAddNone, true>(tq, tk, tv, tb, a, st); })
+                  : go([&](auto t) { return launch_one<64, t.value, false, kAddNone, false>(tq, tk, tv, tb, a, st); });
+  if (D == 64)
+    return masked ? go([&](auto t) { return launch_one<64, t.value, false, kAddAny, true>(tq, tk, tv, tb, a, st); })
+                  : go([&](auto t) { return launch_one<64, t.value, false, kAddAny, false>(tq, tk, tv, tb, a, st); });
   if (tiles) return go([&](auto t) { return launch_one<128, t.value, true, kAddTile>(tq, tk, tv, tb, a, st); });
   if (add == kAddNone) return go([&](auto t) { return launch_one<128, t.value, false, kAddNone>(tq, tk, tv, tb, a, st); });
   return go([&](auto t) { return launch_one<128, t.value, false, kAddAny>(tq, tk, tv, tb, a, st); });

@@ -77,3 +77,27 @@ def test_many_key_padded_batch_elements_whatever_their_order(B, D, tile):
         part = slice(i, i + 100)
         out_i, lse_i = sdpa_forward(q[part], k[part], v[part], bias, mask[part], scale=0.125)
         assert torch.equal(out[part], out_i) and torch.equal(lse[part], lse_i)
+
+
+@pytest.mark.parametrize("kind", ["mask", "mask_shared", "mask_causal", "mask_key_bias", "mask_neg", "key_mask_neg", "key_bias_neg_mask"])
+@pytest.mark.parametrize("S,T", [(300, 700), (130, 385), (257, 90)])
+def test_staged_mask_words_over_several_items_per_cta(kind, S, T):
+    """Head dim 64 without bias tiles: the ring of mask words wraps within an item and from one to the next, query tiles of
+    different (causal) and of no (past the last row) key tiles among them.  Tolerance as above."""
+    from nitrix_b200.nn.attention import sdpa_forward
+
+    g = torch.Generator(device="cuda").manual_seed(S * 1000 + T)
+    B, H, D = 23, 8, 64
+    q = torch.randn(B, H, S, D, generator=g, device="cuda").half()
+    k, v = (torch.randn(B, H, T, D, generator=g, device="cuda").half() for _ in range(2))
+    scale = -0.125 if "neg" in kind else 0.125
+    rows = 1 if kind == "key_mask_neg" else S
+    mask = torch.rand(1 if kind == "mask_shared" else B, 1, rows, T, generator=g, device="cuda") < 0.7
+    mask[..., 0] = True
+    bias = torch.randn(1, H, 1, (T + 7) // 8 * 8, generator=g, device="cuda").half()[..., :T] if "bias" in kind else None
+    out, lse = sdpa_forward(q, k, v, bias, mask, scale=scale, causal=kind == "mask_causal")
+    for i in range(0, B, 4):
+        p = slice(i, i + 4)
+        want, want_lse = _reference(q[p], k[p], v[p], bias, mask if kind == "mask_shared" else mask[p], kind == "mask_causal", scale)
+        assert float((out[p].double() - want).abs().max()) <= 0.25 * 2.0 ** -7 * max(1.0, float(want.abs().max()))
+        assert float((lse[p].double() - want_lse).abs().max()) <= 1e-3 * max(1.0, float(want_lse.abs().max()))
