@@ -30,7 +30,8 @@ using MaybeTensor = std::optional<Tensor>;
   X(nb200_last_error) X(nb200_sdpa_plan) X(nb200_sdpa_workspace_bytes) X(nb200_sdpa_workspace_least_bytes)                 \
   X(nb200_sdpa_fwd) X(nb200_sdpa_bwd) X(nb200_mask_pack_bytes) X(nb200_mask_pack) X(nb200_qk_rms_norm)                     \
   X(nb200_qk_rms_norm_grad) X(nb200_layer_norm_fwd) X(nb200_layer_norm_bwd) X(nb200_layer_norm_workspace_bytes)            \
-  X(nb200_selective_scan_fwd) X(nb200_selective_scan_bwd) X(nb200_selective_scan_checkpoint_bytes)
+  X(nb200_selective_scan_fwd) X(nb200_selective_scan_bwd) X(nb200_selective_scan_checkpoint_bytes)                         \
+  X(nb200_selective_scan_workspace_bytes)
 
 struct Library {
 #define X(name) decltype(&::name) name = nullptr;
@@ -474,7 +475,9 @@ Tensor sum_to_operand(const Tensor& g3, at::IntArrayRef lead, at::IntArrayRef sh
 
 // The backward's scratch comes from nitrix_b200.nn.ssm, which decides what a device without room for all of it gets.
 PyObject* scan_allocator = nullptr;
-Tensor scan_workspace(nb200_selective_scan_params& p, const Tensor& like) {   // (fills in p's workspace)
+// It gets the block with the bytes that are wanted and fills in the workspace.
+Tensor scan_workspace(nb200_selective_scan_params& p, const Tensor& like) {
+  check(lib.nb200_selective_scan_workspace_bytes(&p, &p.workspace_bytes), "nb200_selective_scan_workspace_bytes");
   py::gil_scoped_acquire gil;
   return py::reinterpret_borrow<py::object>(scan_allocator)(reinterpret_cast<uintptr_t>(&p), int(like.device().index())).cast<Tensor>();
 }

@@ -833,7 +833,7 @@ int walk_splits(int64_t ctas, int64_t length, int states, bool half, bool adjoin
   const int n = pick_n(states);
   Rule r;
   if (n == 8) r = {7.f, 192.f, 32.f, 7.6f, half && !adjoint ? 16.f : 25.f};
-  else if (n == 16) r = adjoint ? Rule{7.f, 192.f, 96.f, 6.f, 50.f} : Rule{7.f, 192.f, 64.f, 7.6f, 25.f};
+  else if (n == 16) r = adjoint ? Rule{7.f, 192.f, 96.f, 6.f, 50.f} : Rule{7.7f, 192.f, load8 > 7.f ? 120.f : 64.f, 7.6f, 25.f};   // (the wave's end: (4, 927, 550, 16))
   else if (n == 32) r = {5.f, 384.f, 192.f, 5.5f, adjoint ? 100.f : 75.f};
   else if (half && !adjoint) r = {2.f, 768.f, 0.f, 5.5f, 45.f};   // (its one walk is slow: 74 CTAs, 2048 steps 521 us, f32 285)
   else r = {2.f, 768.f, 0.f, 3.f, 150.f};

@@ -80,10 +80,12 @@ def selective_scan_forward(x3, delta3, A, B3, C3, D, want_checkpoints: bool):
 
 
 def _workspace(p, device) -> torch.Tensor:
-    """The backward's scratch; where the device has no room for the adjoint states of the whole batch at once (as large as
-    the checkpoints), the least with which it runs, a range after the other."""
+    """The backward's scratch (``p.workspace_bytes`` where the caller has asked already); where the device has no room for
+    the adjoint states of the whole batch at once (as large as the checkpoints), the least with which it runs, a range after
+    the other."""
+    need = p.workspace_bytes or _bytes(_cabi.lib().nb200_selective_scan_workspace_bytes, p)
     try:
-        ws = torch.empty(max(_bytes(_cabi.lib().nb200_selective_scan_workspace_bytes, p), 16), dtype=torch.uint8, device=device)
+        ws = torch.empty(max(need, 16), dtype=torch.uint8, device=device)
     except torch.OutOfMemoryError:
         ws = torch.empty(max(_bytes(_cabi.lib().nb200_selective_scan_workspace_least_bytes, p), 16), dtype=torch.uint8,
                          device=device)
