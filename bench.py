@@ -80,10 +80,10 @@ KERNEL_FLOP_SHARE = {
 NCU_TRAFFIC_BYTES = {
     # profiles/c3_b1_attention_kernels_ncu_full.md: captured at batch 1 (the recipe's size rule), x 4 for the bench's
     # batch 4 -- every (batch, head) pair has its own bias / dbias, so traffic grows in proportion
-    "c3": {"sdpa_bwd_tc_kernel<one-pass d128>": 4 * (1.355364e9 + 1.181375e9), "sdpa_fwd_tc_kernel": 4 * (1.191293e9 + 0.039252e9)},
+    "c3": {"sdpa_bwd_tc_kernel<one-pass d128>": 4 * (1.347099e9 + 1.179926e9), "sdpa_fwd_tc_kernel": 4 * (1.189577e9 + 0.034012e9)},
     # profiles/c2_attention_kernels_ncu_full.md, profiles/c4_attention_kernels_ncu_full.md: captured at full size
-    "c2": {"sdpa_bwd_tc_kernel<merged>": 671.002368e6 + 123.455744e6, "sdpa_fwd_tc_kernel": 250.225664e6 + 25.214464e6},
-    "c4": {"sdpa_bwd_tc_kernel<merged>": 176.488704e6 + 84.309760e6, "sdpa_fwd_tc_kernel": 74.746368e6 + 6.363136e6},
+    "c2": {"sdpa_bwd_tc_kernel<merged>": 668.139776e6 + 121.411584e6, "sdpa_fwd_tc_kernel": 249.546240e6 + 25.904128e6},
+    "c4": {"sdpa_bwd_tc_kernel<merged>": 176.477184e6 + 84.955648e6, "sdpa_fwd_tc_kernel": 73.766656e6 + 8.738304e6},
 }
 
 METRIC = "fwd+bwd attention TFLOP/s"
